@@ -1,4 +1,5 @@
-// USFFT gather and scatter for scans that revisit their directions.
+// USFFT for scans that revisit their directions: the formulation of both operators,
+// and the adjoint scatter (the forward gather is gather_dir.cu).
 //
 // A scan over several half-turns sees every direction (theta modulo pi) more
 // than once: rays theta, theta + pi, theta + 2 pi, ... sample the same points
@@ -36,7 +37,7 @@
 // cores: 16 complex products per ray sample, against 1296 for the taps of the
 // per-ray formulation).
 //
-// Both kernels take 16 time samples [jbase, jbase + 16) per launch.
+// The scatter takes 16 time samples [jbase, jbase + 16) per launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,27 +50,7 @@ namespace rectv {
 namespace {
 
 constexpr int kT = 16;
-constexpr int kFW = kT + 2 * kR;   // footprint side (24)
-constexpr int kCells = kFW * kFW;  // 576
 constexpr int kChunks = 8;         // 16-byte chunks of a cell: time samples (2i, 2i+1), complex
-
-// ---- forward ----
-constexpr int kFThr = 256;
-constexpr int kFCap = 128;  // positions per forward item
-
-constexpr int kWt = 5 * kTaps;  // weights per position (odd row pitch: the four positions of a warp on distinct banks)
-
-struct FwdSmem {
-    float4 fp[kCells * kChunks];  // footprint of 16 time samples, cell-major; chunk i of cell c at
-                                  // slot (i + 2 (c & 3)) & 7
-    // per position: [0,9) (-1)^b w_b of the x taps, [9,18) their derivatives
-    // along x, [18,27) (-1)^a w_a of the y taps times the stencil origin's
-    // fftshift sign, [27,36) those times cos, [36,45) minus sin times their
-    // derivatives along y (cos, sin of the direction): S_perp's row weights
-    float wt[kFCap][kWt];
-    int org[kFCap];               // footprint cell of the stencil origin
-    int pid[kFCap];               // d*n + q, -1: none
-};
 
 // ---- adjoint ----
 constexpr int kAThr = 256;             // two threads per cell of a tile (8 time samples each), one slice per block
@@ -105,237 +86,6 @@ __device__ __forceinline__ float2 cmulc(float2 a, float2 b) {
 }
 
 }  // namespace
-
-// ---------------------------------------------------------------------------
-// Forward: one block (256 threads) per (work item, slices); an item is at
-// most 128 positions whose stencils start in one 16x16 tile of the
-// oversampled grid.  Per slice the tile's 24x24-cell footprint of 16 time
-// samples is copied (coalesced loads, cell-major stores) from the halo-padded
-// spectra (tiles right of the Nyquist column read the mirrored cells and
-// conjugate), then eight lanes per position (two time samples each) sum the
-// 81 taps, and mix the position's rays: each lane forms its two time
-// samples' share of all eight rays of a round, the eight lanes add their
-// shares by recursive halving (14 shuffles) and lane i keeps ray i.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kFThr, 2)
-    k_gather_dir(float2 *__restrict__ rows, const float2 *__restrict__ spec, const uint32_t *__restrict__ pos,
-                 const int4 *__restrict__ items, const float2 *__restrict__ dsincos,
-                 const int *__restrict__ ray_start, const uint32_t *__restrict__ rays,
-                 const float *__restrict__ tau, const float2 *__restrict__ kmat, const float2 *__restrict__ shiftf,
-                 UsGeo g, int zb, int jbase, int accumulate, int *__restrict__ err) {
-    extern __shared__ __align__(16) unsigned char dir_fwd_smem[];
-    FwdSmem &sm = *reinterpret_cast<FwdSmem *>(dir_fwd_smem);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int4 it = items[blockIdx.x];
-    const int z0 = blockIdx.y * g.zper, z1 = min(zb, z0 + g.zper);
-    const int tyi = it.x / g.NT, txi = it.x - tyi * g.NT;
-    const int cnt = min(it.z, kFCap);
-    const bool mirrored = txi * kT > g.n + 2;
-    const int KY0 = tyi * kT - kR, KX0 = txi * kT - kR;  // footprint cell (0, 0) in the periodic spectrum
-
-    // ---- the item's positions (the same for every slice) ----
-    // derivative of a tap weight exp(-pi^2/mu d^2) along the position, per
-    // grid cell: c1 d w, c1 = 2 (pi^2/mu) / (2n)
-    const float c1 = 2.f * g.wexp / g.tn;
-    for (int e = tid; e < kFCap; e += kFThr) {
-        int id = -1, org = 0;
-        float *wt = sm.wt[e];
-        if (e < cnt) {
-            const uint32_t u = __ldg(pos + it.y + e);
-            const int d = u / (uint32_t)g.n, q = u - d * g.n;
-            const float2 sc = __ldg(dsincos + d);
-            float x0, y0;
-            int fx, fy;
-            sample_pos(q, sc, g, x0, y0, fx, fy);
-            const int lx0 = g.n + fx - txi * kT, ly0 = g.n + fy - tyi * kT;
-            if (lx0 < 0 || lx0 >= kT || ly0 < 0 || ly0 >= kT) {  // host/device bin disagreement
-                atomicAdd(err, 1);
-            } else {
-                id = (int)u;
-                org = ly0 * kFW + lx0;
-                const float sgn = ((lx0 + ly0) & 1) ? -1.f : 1.f;
-#pragma unroll
-                for (int b = 0; b < kTaps; ++b) {
-                    const float dx = (float)(fx - kR + b) * g.inv2n - x0, dy = (float)(fy - kR + b) * g.inv2n - y0;
-                    const float a = tap_weight(fx, b, x0, g), c = tap_weight(fy, b, y0, g) * sgn;
-                    const float sb = (b & 1) ? -1.f : 1.f;
-                    wt[b] = sb * a;
-                    wt[kTaps + b] = sb * c1 * dx * a;
-                    wt[2 * kTaps + b] = sb * c;
-                    wt[3 * kTaps + b] = sb * c * sc.y;
-                    wt[4 * kTaps + b] = -sb * c1 * dy * c * sc.x;
-                }
-            }
-        }
-        if (id < 0)
-            for (int b = 0; b < kWt; ++b) wt[b] = 0.f;
-        sm.pid[e] = id;
-        sm.org[e] = org;
-    }
-
-    const int ngroups = (cnt + 3) / 4;  // four positions per warp
-    const int pi = lane >> 3, ci = lane & 7;
-    const int fc = lane & 3, fj = lane >> 2;  // footprint copies: cell of four, time sample of eight
-    const int j0 = jbase + 2 * ci;      // this lane's time samples j0, j0 + 1
-    for (int z = z0; z < z1; ++z) {
-        // ---- footprint of slice z: lane = (cell cl of four, time sample jj of
-        // eight), warp w copies rows w, w + 8, w + 16: a half-warp writes four
-        // cells x four time samples on distinct banks, a warp reads eight
-        // 32-byte runs ----
-        // (all 36 loads of a thread in flight, then the stores)
-        const float2 *simg = spec + ((long long)z * g.m + jbase) * g.img_fwd;
-        float2 fv[2][kFW / 8][kFW / 4];
-#pragma unroll
-        for (int jh = 0; jh < 2; ++jh) {
-            const int j = 8 * jh + fj;
-            const float2 *sj = simg + (long long)j * g.img_fwd;
-#pragma unroll
-            for (int rr = 0; rr < kFW / 8; ++rr) {
-                const int KY = KY0 + wid + 8 * rr;
-                const float2 *srow = sj + (long long)((mirrored ? g.P - KY : KY) + kHalo) * g.qp;
-#pragma unroll
-                for (int cq = 0; cq < kFW / 4; ++cq) {
-                    const int KX = KX0 + 4 * cq + fc;
-                    fv[jh][rr][cq] = (jbase + j < g.m) ? __ldg(srow + (mirrored ? g.P - KX : KX) + kHalo)
-                                                       : make_float2(0.f, 0.f);
-                }
-            }
-        }
-#pragma unroll
-        for (int jh = 0; jh < 2; ++jh) {
-            const int j = 8 * jh + fj;
-#pragma unroll
-            for (int rr = 0; rr < kFW / 8; ++rr) {
-                const int row = wid + 8 * rr;
-                float2 *drow = reinterpret_cast<float2 *>(sm.fp) + (row * kFW + fc) * 16 + ((j + 4 * fc) & 15);
-#pragma unroll
-                for (int cq = 0; cq < kFW / 4; ++cq) drow[64 * cq] = fv[jh][rr][cq];
-            }
-        }
-        __syncthreads();
-
-        for (int gi = wid; gi < ngroups; gi += kFThr / 32) {
-            const int e = 4 * gi + pi;
-            const int id = sm.pid[e];
-            const int org = sm.org[e];
-            const int lx0 = org % kFW;
-            // four base pointers (one per rotation of the column's chunks): every
-            // tap is then a load at a constant offset from one of them
-            const float4 *fq[4];
-#pragma unroll
-            for (int bq = 0; bq < 4; ++bq) fq[bq] = sm.fp + org * kChunks + ((ci + 2 * ((lx0 + bq) & 3)) & 7);
-            const float *wt = sm.wt[e];
-            float wx[kTaps], wxd[kTaps];
-#pragma unroll
-            for (int b = 0; b < kTaps; ++b) {
-                wx[b] = wt[b];
-                wxd[b] = wt[kTaps + b];
-            }
-            // ---- S_j and S_perp_j of this lane's two time samples: 81 taps ----
-            float2 s0 = make_float2(0.f, 0.f), s1 = make_float2(0.f, 0.f);
-            float2 p0 = make_float2(0.f, 0.f), p1 = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int a = 0; a < kTaps; ++a) {
-                float2 r0 = make_float2(0.f, 0.f), r1 = make_float2(0.f, 0.f);
-                float2 d0 = make_float2(0.f, 0.f), d1 = make_float2(0.f, 0.f);
-#pragma unroll
-                for (int b = 0; b < kTaps; ++b) {
-                    const float4 f = fq[b & 3][(a * kFW + b) * kChunks];
-                    r0 = ffma2(make_float2(wx[b], wx[b]), make_float2(f.x, f.y), r0);
-                    r1 = ffma2(make_float2(wx[b], wx[b]), make_float2(f.z, f.w), r1);
-                    d0 = ffma2(make_float2(wxd[b], wxd[b]), make_float2(f.x, f.y), d0);
-                    d1 = ffma2(make_float2(wxd[b], wxd[b]), make_float2(f.z, f.w), d1);
-                }
-                const float w = wt[2 * kTaps + a], wc = wt[3 * kTaps + a], ws = wt[4 * kTaps + a];
-                s0 = ffma2(make_float2(w, w), r0, s0);
-                s1 = ffma2(make_float2(w, w), r1, s1);
-                p0 = ffma2(make_float2(wc, wc), d0, ffma2(make_float2(ws, ws), r0, p0));
-                p1 = ffma2(make_float2(wc, wc), d1, ffma2(make_float2(ws, ws), r1, p1));
-            }
-            if (mirrored) {  // the footprint held the conjugate-mirrored cells
-                s0.y = -s0.y;
-                s1.y = -s1.y;
-                p0.y = -p0.y;
-                p1.y = -p1.y;
-            }
-            // ---- rays of the position, eight per round ----
-            int q = 0, rs = 0, nr = 0;
-            if (id >= 0) {
-                const int d = id / g.n;
-                q = id - d * g.n;
-                rs = __ldg(ray_start + d);
-                nr = __ldg(ray_start + d + 1) - rs;
-            }
-            const float qp = __fdiv_rn((float)(q - g.n / 2), (float)g.n);
-            const int rounds = __reduce_max_sync(0xffffffffu, (nr + 7) >> 3);
-            for (int rd = 0; rd < rounds; ++rd) {
-                // lane ci fetches ray 8 rd + ci of its position; the eight lanes share them by shuffles
-                uint32_t rv = 0;
-                float tv = 0.f;
-                if (8 * rd + ci < nr) {
-                    rv = __ldg(rays + rs + 8 * rd + ci);
-                    tv = __ldg(tau + rs + 8 * rd + ci);
-                }
-                float v[16];
-#pragma unroll
-                for (int rr = 0; rr < 8; ++rr) {
-                    const uint32_t rvr = __shfl_sync(0xffffffffu, rv, (lane & ~7) | rr);
-                    const float tvr = __shfl_sync(0xffffffffu, tv, (lane & ~7) | rr);
-                    float2 k0 = make_float2(0.f, 0.f), k1 = make_float2(0.f, 0.f);
-                    float dl = 0.f;
-                    if (8 * rd + rr < nr) {
-                        const long long th = rvr & 0x7fffffffu;
-                        dl = qp * tvr;  // this ray's offset across the direction
-                        if (j0 < g.m) k0 = __ldg(kmat + th * g.m + j0);
-                        if (j0 + 1 < g.m) k1 = __ldg(kmat + th * g.m + j0 + 1);
-                    }
-                    const float2 t0 = make_float2(fmaf(dl, p0.x, s0.x), fmaf(dl, p0.y, s0.y));
-                    const float2 t1 = make_float2(fmaf(dl, p1.x, s1.x), fmaf(dl, p1.y, s1.y));
-                    v[2 * rr] = k0.x * t0.x - k0.y * t0.y + k1.x * t1.x - k1.y * t1.y;
-                    v[2 * rr + 1] = k0.x * t0.y + k0.y * t0.x + k1.x * t1.y + k1.y * t1.x;
-                }
-                // sum over the eight lanes of the position by recursive halving;
-                // lane ci ends with ray 8 rd + ci
-                float w8[8], w4[4], w2[2];
-                const bool b4 = ci & 4, b2 = ci & 2, b1 = ci & 1;
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const float send = b4 ? v[t] : v[8 + t];
-                    const float keep = b4 ? v[8 + t] : v[t];
-                    w8[t] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float send = b2 ? w8[t] : w8[4 + t];
-                    const float keep = b2 ? w8[4 + t] : w8[t];
-                    w4[t] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-                }
-#pragma unroll
-                for (int t = 0; t < 2; ++t) {
-                    const float send = b1 ? w4[t] : w4[2 + t];
-                    const float keep = b1 ? w4[2 + t] : w4[t];
-                    w2[t] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-                }
-                const int ri = 8 * rd + ci;
-                if (ri < nr) {
-                    const long long th = rv & 0x7fffffffu;
-                    const int k = (rv >> 31) ? g.n - q : q;
-                    const float2 sh = __ldg(shiftf + k);
-                    const float cf = (k & 1) ? g.cw : -g.cw;  // (-1)^(k+1) (pi/mu)/n
-                    float2 o = cmul(make_float2(w2[0], w2[1]), make_float2(sh.x * cf, sh.y * cf));
-                    float2 *dst = rows + ((long long)z * g.ntheta + th) * g.n + k;
-                    if (accumulate) {
-                        const float2 p = *dst;
-                        o.x += p.x;
-                        o.y += p.y;
-                    }
-                    *dst = o;
-                }
-            }
-        }
-        __syncthreads();  // the footprint buffer is refilled for the next slice
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Adjoint, step 1: E_j and E_perp_j of every position and slice (time
@@ -785,26 +535,13 @@ void launch_adj_tabinfo_dir(const GeoDev &gd, cudaStream_t s) {
 }
 
 void dir_prepare() {
-    CUDA_CHECK(cudaFuncSetAttribute(k_gather_dir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem)));
+    gather_dir_prepare();
     CUDA_CHECK(cudaFuncSetAttribute(k_scatter_dir, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(AdjSmem)));
 }
 
-int dir_fwd_capacity() { return kFCap; }
 int dir_adj_table_capacity() { return kATab; }
 int dir_adj_table_dirs() { return kAMaxSeg; }
 size_t dir_mix_bytes(int zb, int ndir, int n) { return (size_t)zb * ndir * n * 16 * sizeof(float4); }
-
-void launch_gather_dir(float2 *rows, const float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
-                       int accumulate, cudaStream_t s) {
-    if (gd.n_dfwd_items == 0) return;
-    if (g.T != kT) throw Error(1, "tile size must be 16");
-    if (g.zper < 1) throw Error(1, "slices per block must be positive");
-    const dim3 gs(gd.n_dfwd_items, (zb + g.zper - 1) / g.zper);
-    k_gather_dir<<<gs, kFThr, sizeof(FwdSmem), s>>>(rows, spec, gd.dfwd_pos, gd.dfwd_items, gd.sincos, gd.dray_start,
-                                                     gd.drays, gd.dtau, gd.kmat, gd.shiftfwd, g, zb, jbase, accumulate,
-                                                     gd.err);
-    LAUNCH_CHECK("k_gather_dir");
-}
 
 void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
                         cudaStream_t s) {

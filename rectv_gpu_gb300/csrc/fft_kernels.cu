@@ -222,6 +222,8 @@ __device__ __forceinline__ void fft_core(float2 *v, float2 *sh, int c, int t, co
 }
 
 constexpr int kRowThreads = 512;  // threads per block of the row kernels
+// values per tile of the vector layout's column passes (32- to 128-byte runs; 512 threads but for P = 256)
+constexpr int vec_col_c(int N) { return N >= 2048 ? 4 : (N == 1024 ? 8 : 16); }
 constexpr int kColC = 4;          // columns per block of the column kernels (32-byte row runs, two blocks per SM)
 
 // ---------------------------------------------------------------------------
@@ -277,6 +279,72 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     }
 }
 
+// ---------------------------------------------------------------------------
+// Forward rows into the vector layout (UsGeo): one row y of the images of one
+// plane.  The two images of a value pair (2p, 2p+1) are the real and imaginary
+// part of one complex FFT, so that the split half spectra leave as 16-byte
+// stores and the C pairs of a block as C x 16 contiguous bytes per cell
+// (64-128 bytes).  Thread = (pair c, point t) with c fastest: C transforms
+// interleaved in shared memory as in the column kernels, R rows per block.
+// ---------------------------------------------------------------------------
+template <int N>
+struct VecRows {
+    static constexpr int N1 = N / 16;
+    static constexpr int C = N1 * 8 <= kRowThreads ? 8 : 4;  // pairs per block
+    static constexpr int R = kRowThreads / (N1 * C);         // rows per block
+    using L = FftLayout<N, true, C>;
+    static constexpr size_t SMEM = sizeof(float2) * (size_t)L::S * C * R;
+};
+
+template <int N>
+__global__ void __launch_bounds__(kRowThreads, 2)
+    k_fft_rows_fwd_vec(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp,
+                       const float2 *__restrict__ tw, UsGeo g, int zb, float inv4n2) {
+    using V = VecRows<N>;
+    using L = typename V::L;
+    constexpr int N1 = V::N1, C = V::C, R = V::R;
+    extern __shared__ float2 fft_sh[];
+    const int n = N / 2;
+    const int c = threadIdx.x % C, t = (threadIdx.x / C) % N1, rr = threadIdx.x / (C * N1);
+    const int y = (blockIdx.x / (8 / C)) * R + rr, pl = blockIdx.y;
+    const int v0 = 2 * ((blockIdx.x % (8 / C)) * C + c);  // the pair's values v0, v0 + 1 of the plane
+    float2 *sh = fft_sh + rr * (L::S * C);
+    const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
+    const int zc = vec_slice(g, pl, v0 + 1), tc_ = vec_time(g, pl, v0 + 1);
+    const bool oka = za < zb && ta < g.m, okb = zc < zb && tc_ < g.m;
+    float2 v[16];
+    {
+        const float *ua = u + (((long long)(oka ? za : 0) * g.m + (oka ? ta : 0)) * n + y) * n;
+        const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tc_ : 0)) * n + y) * n;
+        const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * inv4n2;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            v[r] = make_float2(0.f, 0.f);
+            if (r >= 4 && r < 12) {  // X = t + N1 r in [n/2, 3n/2)
+                const int x = t + N1 * (r - 4), X = x + n / 2;
+                const float w = ((X & 1) ? -__ldg(dp + x) : __ldg(dp + x)) * sy;
+                if (oka) v[r].x = __ldg(ua + x) * w;
+                if (okb) v[r].y = __ldg(ub + x) * w;
+            }
+        }
+    }
+    fft_core<N, -1, L>(v, sh, c, t, tw);
+    // Z in natural order, then A(k) = (Z(k) + conj Z(-k))/2, B(k) = (Z(k) - conj Z(-k))/(2i)
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 16 / L::R3; ++q)
+#pragma unroll
+        for (int j1 = 0; j1 < L::R3; ++j1) sh[(t + N1 * q + 256 * j1) * C + c] = v[q * L::R3 + j1];
+    __syncthreads();
+    if (!oka && !okb) return;
+    float4 *row = reinterpret_cast<float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0);
+    for (int k = t; k <= n; k += N1) {
+        const float2 zk = sh[k * C + c], zm = sh[((N - k) & (N - 1)) * C + c];
+        row[(long long)k * 8] = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y),
+                                            0.5f * (zm.x - zk.x));
+    }
+}
+
 // TMA tile copies of the column kernels: boxes of 4 columns (8 floats) x BR
 // rows of one image, landing in shared memory as [row][column].
 __device__ __forceinline__ void tma_load3(void *dst, const CUtensorMap *map, int x, int y, int z, void *bar) {
@@ -316,27 +384,40 @@ __device__ __forceinline__ void mbar_expect(void *bar, uint32_t bytes) {
 // Inverse: inverse P-point FFT of columns kx .. kx+3 of the Hermitian half
 // planes [img][P][hpitch]; only rows [n/2, 3n/2) are written back (columns
 // past the row pitch read as zeros and are not stored).
+//
+// VEC: the vector layout.  A tile is C values of one column's cells (C x 8
+// contiguous bytes), tiles of a cell's values fastest, so that the blocks in
+// flight share the cells' 128-byte lines.
 // ---------------------------------------------------------------------------
-template <int N, int C, int DIR>
+template <int N, int C, int DIR, bool VEC>
 struct ColPass {
     static constexpr int n = N / 2;
     static constexpr int BR = n < 256 ? n : 256;                // rows per TMA box
     static constexpr int IN_ROWS = DIR < 0 ? n : N;              // rows loaded per tile
     static constexpr int OUT_ROWS = DIR < 0 ? N : n;             // rows stored per tile
-    static constexpr int IN_Y0 = DIR < 0 ? kHalo + n / 2 : 0;    // first loaded row (map coordinates)
-    static constexpr int OUT_Y0 = DIR < 0 ? kHalo : n / 2;       // first stored row
-    static constexpr int XOFF = DIR < 0 ? kHalo : 0;             // column offset of the map window
+    static constexpr int Y0 = VEC ? kVH : (DIR < 0 ? kHalo : 0);  // row 0 in map coordinates
+    static constexpr int IN_Y0 = DIR < 0 ? Y0 + n / 2 : Y0;       // first loaded row
+    static constexpr int OUT_Y0 = DIR < 0 ? Y0 : Y0 + n / 2;      // first stored row
+    // first float of tile group gr of an image; VEC: nlv groups of values per cell
+    __device__ static __forceinline__ int x0(int gr, int nlv) {
+        if constexpr (VEC) {
+            const int k = gr / nlv;
+            return 32 * (kVH + k) + 2 * C * (gr - k * nlv);
+        } else {
+            return 2 * ((DIR < 0 ? kHalo : 0) + gr * C);  // column offset of the planar map window
+        }
+    }
     using L = FftLayout<N, true, C>;
     static constexpr size_t EX = (size_t)L::S * C > (size_t)OUT_ROWS * C ? (size_t)L::S * C : (size_t)OUT_ROWS * C;
     static constexpr size_t LAND = (size_t)IN_ROWS * C;          // float2 per landing buffer
     static constexpr size_t SMEM = sizeof(float2) * (EX + 2 * LAND);
 };
 
-template <int N, int C, int DIR>
+template <int N, int C, int DIR, bool VEC>
 __global__ void __launch_bounds__(C *(N / 16), 1)
-    k_fft_cols(const __grid_constant__ CUtensorMap tmap, const float2 *__restrict__ tw, int ngroups, int ntiles,
-               int *__restrict__ err) {
-    using CP = ColPass<N, C, DIR>;
+    k_fft_cols(const __grid_constant__ CUtensorMap tmap, const float2 *__restrict__ tw, int ngroups, int nlv,
+               int ntiles, int *__restrict__ err) {
+    using CP = ColPass<N, C, DIR, VEC>;
     using L = typename CP::L;
     constexpr int N1 = N / 16, n = N / 2, BR = CP::BR;
     extern __shared__ __align__(1024) float2 fft_sh[];
@@ -350,7 +431,7 @@ __global__ void __launch_bounds__(C *(N / 16), 1)
     }
     __syncthreads();
     auto fetch = [&](int tile, int buf) {  // one thread
-        const int x = 2 * (CP::XOFF + (tile % ngroups) * C), img = tile / ngroups;
+        const int x = CP::x0(tile % ngroups, nlv), img = tile / ngroups;
         mbar_expect(&bar[buf], (uint32_t)(CP::LAND * sizeof(float2)));
         for (int i = 0; i < CP::IN_ROWS / BR; ++i)
             tma_load3(fft_sh + CP::EX + buf * CP::LAND + i * BR * C, &tmap, x, CP::IN_Y0 + i * BR, img, &bar[buf]);
@@ -391,7 +472,7 @@ __global__ void __launch_bounds__(C *(N / 16), 1)
         tc::fence_proxy_async();
         __syncthreads();
         if (threadIdx.x == 0) {
-            const int x = 2 * (CP::XOFF + (tile % ngroups) * C), img = tile / ngroups;
+            const int x = CP::x0(tile % ngroups, nlv), img = tile / ngroups;
             for (int i = 0; i < CP::OUT_ROWS / BR; ++i) tma_store3(&tmap, x, CP::OUT_Y0 + i * BR, img, ex + i * BR * C);
             asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
         }
@@ -476,7 +557,8 @@ size_t rows_smem() {
 // costs one inverse and one forward n-point FFT; the residual never goes to
 // memory.  Rows are the flattened (slice, angle) index; N = n.
 // ---------------------------------------------------------------------------
-template <int N>
+// HALF: the rows hold H(k) itself, k = 0 .. n/2 (direction path).
+template <int N, bool HALF>
 __global__ void __launch_bounds__(kRowThreads, 2)
     k_resid_rows(const float2 *__restrict__ rows, const float *__restrict__ gdata, float2 *__restrict__ out,
                  const float2 *__restrict__ tw, long long nrows, float scale) {
@@ -486,12 +568,26 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     const int t = threadIdx.x % N1, c = threadIdx.x / N1;
     const long long ra = 2 * ((long long)blockIdx.x * RP + c), rb = ra + 1;
     const bool oka = ra < nrows, okb = rb < nrows;
-    const float2 *ga = rows + (oka ? ra : 0) * N, *gb = rows + (okb ? rb : 0) * N;
+    constexpr int RN = HALF ? N / 2 + 1 : N;  // values per row
+    const float2 *ga = rows + (oka ? ra : 0) * RN, *gb = rows + (okb ? rb : 0) * RN;
     float2 v[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) {  // Ha + i Hb at k = t + N1 r
         const int k = t + N1 * r, km = (N - k) & (N - 1);
         float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
+        if constexpr (HALF) {
+            const bool hi = k > N / 2;
+            if (oka) a = __ldg(ga + (hi ? km : k));
+            if (okb) b = __ldg(gb + (hi ? km : k));
+            if (hi) {
+                a.y = -a.y;
+                b.y = -b.y;
+            } else if (k == N / 2) {  // the transform's output is real: its Nyquist bin is too
+                a.y = b.y = 0.f;
+            }
+            v[r] = make_float2(a.x - b.y, a.y + b.x);
+            continue;
+        }
         if (oka) {
             const float2 p = ga[k], q = ga[km];
             a = make_float2(0.5f * (p.x + q.x), 0.5f * (p.y - q.y));
@@ -536,26 +632,30 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     }
 }
 
-template <int N>
+template <int N, bool HALF>
 void resid_n(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, long long nrows, float scale,
              cudaStream_t s) {
     constexpr int N1 = N / 16, RP = kRowThreads / N1;
     const long long npairs = (nrows + 1) / 2;
     const long long nblk = (npairs + RP - 1) / RP;
     if (nblk > 2147483647LL) throw Error(1, "residual rows: too many rows");
-    k_resid_rows<N><<<(unsigned)nblk, kRowThreads, rows_smem<N>(), s>>>(rows, gdata, out, tw, nrows, scale);
+    k_resid_rows<N, HALF><<<(unsigned)nblk, kRowThreads, rows_smem<N>(), s>>>(rows, gdata, out, tw, nrows, scale);
     LAUNCH_CHECK("k_resid_rows");
 }
 
 template <int N>
 void set_attrs_n() {
-    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
+    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
+    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd_vec<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, vec_col_c(N), -1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ColPass<N, vec_col_c(N), -1, true>::SMEM));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, -1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, kColC, -1>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, kColC, 1>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ColPass<N, kColC, -1, false>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ColPass<N, kColC, 1, false>::SMEM));
 }
 
 int sm_count() {
@@ -568,15 +668,42 @@ int sm_count() {
     return nsm;
 }
 
-template <int N, int DIR>
-void launch_cols(const CUtensorMap &map, const float2 *tw, int nimg, int *err, cudaStream_t s) {
-    const int ngroups = (N / 2 + 1 + kColC - 1) / kColC;
+template <int N, int C, int DIR, bool VEC>
+void launch_cols(const CUtensorMap &map, const float2 *tw, int nimg, int ngroups, int nlv, int *err, cudaStream_t s) {
     const long long ntiles = (long long)ngroups * nimg;
-    if (ntiles > 2147483647LL) throw Error(1, "pad FFT: too many column tiles");
-    const int grid = (int)std::min<long long>(ntiles, sm_count());
-    k_fft_cols<N, kColC, DIR><<<grid, kColC * (N / 16), ColPass<N, kColC, DIR>::SMEM, s>>>(map, tw, ngroups,
-                                                                                         (int)ntiles, err);
+    if (ntiles > 2147483647LL - 65536) throw Error(1, "pad FFT: too many column tiles");
+    constexpr int thr = C * (N / 16);
+    constexpr size_t smem = ColPass<N, C, DIR, VEC>::SMEM;
+    // persistent: as many blocks per SM as shared memory and 1024 threads allow
+    const int per_sm = std::max(1, std::min((int)((size_t)227 * 1024 / (smem + 1024)), 1024 / thr));
+    const int grid = (int)std::min<long long>(ntiles, (long long)per_sm * sm_count());
+    k_fft_cols<N, C, DIR, VEC><<<grid, thr, smem, s>>>(map, tw, ngroups, nlv, (int)ntiles, err);
     LAUNCH_CHECK(DIR < 0 ? "k_fft_cols (forward)" : "k_fft_cols (inverse)");
+}
+
+template <int N, int DIR>
+void launch_cols_planar(const CUtensorMap &map, const float2 *tw, int nimg, int *err, cudaStream_t s) {
+    launch_cols<N, kColC, DIR, false>(map, tw, nimg, (N / 2 + 1 + kColC - 1) / kColC, 1, err, s);
+}
+
+template <int N, int DIR>
+void launch_cols_vec(const CUtensorMap &map, const float2 *tw, int zb, int *err, const UsGeo &g, cudaStream_t s) {
+    constexpr int C = vec_col_c(N);
+    // value groups of a cell that hold data (fewer than all with 9 .. 15 time samples)
+    const int nlv = g.tg == 16 && g.jg == 1 ? (g.m + C - 1) / C : 16 / C;
+    launch_cols<N, C, DIR, true>(map, tw, vec_planes(g, zb), (N / 2 + 1) * nlv, nlv, err, s);
+}
+
+template <int N>
+void fwd_vec_n(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const CUtensorMap &map,
+               int *err, const UsGeo &g, cudaStream_t s) {
+    using V = VecRows<N>;
+    const int n = N / 2;
+    const float inv4n2 = (float)(1.0 / (4.0 * n * (double)n));
+    const dim3 gr(n / V::R * (8 / V::C), vec_planes(g, zb));
+    k_fft_rows_fwd_vec<N><<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g, zb, inv4n2);
+    LAUNCH_CHECK("k_fft_rows_fwd_vec");
+    launch_cols_vec<N, -1>(map, tw, zb, err, g, s);
 }
 
 template <int N>
@@ -588,7 +715,7 @@ void fwd_n(const float *u, float2 *spec, int nimg, const float *deapod, const fl
     dim3 gr((n / 2 + RP - 1) / RP, nimg);
     k_fft_rows_fwd<N><<<gr, kRowThreads, rows_smem<N>(), s>>>(u, spec, deapod, tw, g, inv4n2);
     LAUNCH_CHECK("k_fft_rows_fwd");
-    launch_cols<N, -1>(map, tw, nimg, err, s);
+    launch_cols_planar<N, -1>(map, tw, nimg, err, s);
 }
 
 template <int N>
@@ -596,7 +723,7 @@ void inv_n(float2 *spec, float *u, int nimg, float cscale, const float *deapod, 
            const CUtensorMap &map, int *err, int hpitch, cudaStream_t s) {
     constexpr int N1 = N / 16, RP = kRowThreads / N1;
     const int n = N / 2;
-    launch_cols<N, 1>(map, tw, nimg, err, s);
+    launch_cols_planar<N, 1>(map, tw, nimg, err, s);
     dim3 gr((n / 2 + RP - 1) / RP, nimg);
     k_fft_rows_inv<N><<<gr, kRowThreads, rows_smem<N>(), s>>>(spec, u, deapod, tw, cscale, hpitch);
     LAUNCH_CHECK("k_fft_rows_inv");
@@ -613,13 +740,13 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
     return encode;
 }
 
-// float view [nimg][rows][row_floats] (pitches in bytes), boxes of 8 floats x
+// float view [nimg][rows][row_floats] (pitches in bytes), boxes of 2 c floats x
 // min(n, 256) rows x 1 image
 void encode_cols_map(CUtensorMap *map, void *base, long long row_floats, long long rows, long long nimg,
-                     long long row_pitch, long long img_pitch, int n, const char *what) {
+                     long long row_pitch, long long img_pitch, int n, const char *what, int c = kColC) {
     const cuuint64_t dims[3] = {(cuuint64_t)row_floats, (cuuint64_t)rows, (cuuint64_t)nimg};
     const cuuint64_t strides[2] = {(cuuint64_t)row_pitch, (cuuint64_t)img_pitch};
-    const cuuint32_t box[3] = {2 * kColC, (cuuint32_t)(n < 256 ? n : 256), 1};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * c), (cuuint32_t)(n < 256 ? n : 256), 1};
     const cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = tmap_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es,
                                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -664,6 +791,23 @@ void make_pad_fft_maps(CUtensorMap *fwd, CUtensorMap *inv, float2 *spec, int nim
                     "the inverse column FFT");
 }
 
+void make_vec_fft_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g) {
+    encode_cols_map(map, spec, 32LL * g.vp, g.vrows, npl, 128LL * g.vp, 8LL * g.vplane, g.n,
+                    "the vector layout's column FFT", vec_col_c(g.P));
+}
+
+void launch_pad_fft_fwd_vec(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
+                            const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
+    if (vec_planes(g, zb) > 65535) throw Error(1, "pad FFT: too many planes per batch");
+    switch (g.P) {
+        case 256: fwd_vec_n<256>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 512: fwd_vec_n<512>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 1024: fwd_vec_n<1024>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 2048: fwd_vec_n<2048>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        default: throw Error(1, "pad FFT: unsupported grid size");
+    }
+}
+
 void launch_pad_fft_fwd(const float *u, float2 *spec, int nimg, const float *deapod, const float2 *tw,
                         const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
     if (nimg > 65535) throw Error(1, "pad FFT: too many images per batch");
@@ -679,14 +823,14 @@ void launch_pad_fft_fwd(const float *u, float2 *spec, int nimg, const float *dea
 bool resid_rows_supported(int n) { return n >= 256 && n <= 1024 && (n & (n - 1)) == 0; }
 
 // tw_n: the twiddle table of the n-point transforms, pad_fft_twiddles(n)
-void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb,
+void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb, bool half,
                        const UsGeo &g, cudaStream_t s) {
     const long long nrows = (long long)zb * g.ntheta;
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
     switch (g.n) {
-        case 256: resid_n<256>(rows, gdata, out, tw_n, nrows, scale, s); break;
-        case 512: resid_n<512>(rows, gdata, out, tw_n, nrows, scale, s); break;
-        case 1024: resid_n<1024>(rows, gdata, out, tw_n, nrows, scale, s); break;
+        case 256: (half ? resid_n<256, true> : resid_n<256, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
+        case 512: (half ? resid_n<512, true> : resid_n<512, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
+        case 1024: (half ? resid_n<1024, true> : resid_n<1024, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
         default: throw Error(1, "residual rows: unsupported detector width");
     }
 }

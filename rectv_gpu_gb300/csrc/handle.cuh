@@ -80,6 +80,7 @@ struct Layout {
     bool pad_fft = false;     // hand-written padded-grid 2D FFTs
     bool fused_rows = false;  // fused residual rows (k_resid_rows)
     bool iter_plans = false;  // the outer iteration runs cuFFT plans
+    int tg = 1, zs = 1, jg = 1;  // vector layout of the direction path (UsGeo)
     long long slab = 0, gp = 0, img_spec = 0;
     size_t spec_elems = 0;
     double bytes = 0;         // estimate of all device memory, geometry included
@@ -126,7 +127,17 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     }
     L.zb = nzp * d;
     L.nbatch = L.nchunks / d;
-    L.spec_elems = std::max<size_t>((size_t)L.zb * m * (size_t)L.img_spec,
+    if (m > 16) {
+        L.tg = 16;
+        L.jg = (m + 15) / 16;
+    } else {
+        while (L.tg < m) L.tg *= 2;
+        L.zs = 16 / L.tg;
+    }
+    const long long vec_pl = L.jg > 1 ? (long long)L.zb * L.jg : (L.zb + L.zs - 1) / L.zs;
+    const long long vec_plane = (P + 2 * kVH) * (n + 1 + 2 * kVH) * 16;
+    L.spec_elems = std::max<size_t>(std::max<size_t>((size_t)L.zb * m * (size_t)L.img_spec,
+                                                     L.tc_scatter ? (size_t)(vec_pl * vec_plane) : 0),
                                     (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
@@ -185,9 +196,15 @@ struct Handle {
     GeoDev gd;
     std::vector<void *> geo_owned;
 
-    // cuFFT
-    cufftHandle p_r2c2d = 0, p_c2c2d = 0, p_rows_c2c = 0, p_rows_r2c = 0, p_c2r2d = 0;
+    // cuFFT plans, made as a geometry's path needs them (ensure_plans)
+    enum { kR2C2D, kC2C2D, kC2R2D, kRowsC2C, kRowsR2C, kRowsC2R, kVecR2C, kNPlans };
+    cufftHandle plan[kNPlans] = {};
+    bool plan_made[kNPlans] = {};
+    size_t fft_work_bytes = 0;
+    int vec_slices = 1;          // slices per cuFFT call of the direction path without the hand-written FFTs
+    float2 *planar = nullptr;    // its planar images [vec_slices m][P][n + 2] (geometry)
     CUtensorMap spec_tmap;  // TMA boxes of the forward spectra (tensor-core gather)
+    CUtensorMap vec_tmap, vec_fft_map;  // vector layout: gather footprints, column FFT tiles
     // key of the geometry on the device (set_geometry)
     bool geo_valid = false, geo_has_phi = false, geo_tc_scatter = false;
     float geo_center = 0.f, geo_tc_spr = 0.f;
@@ -196,7 +213,6 @@ struct Handle {
     // key of the captured graphs besides the geometry (setup)
     int graph_titer = -1;
     float graph_lambda0 = 0.f, graph_lambda1 = 0.f;
-    bool plans_made = false;
     int img_per_fft = 0;
     void *fft_work = nullptr;
     // hand-written padded-grid FFTs (P a power of two in [256, 2048]) instead
@@ -277,6 +293,12 @@ struct Handle {
         ug.sc_grid = 0;
 
         lay = make_layout(n, ntheta, m, nz, nzp, batch_bytes);
+        ug.tg = lay.tg;
+        ug.zs = lay.zs;
+        ug.jg = lay.jg;
+        ug.vp = n + 1 + 2 * kVH;
+        ug.vrows = P + 2 * kVH;
+        ug.vplane = (long long)ug.vrows * ug.vp * 16;
         slab = lay.slab;
         gp = lay.gp;
         zb = lay.zb;
@@ -294,6 +316,19 @@ struct Handle {
         // the float4 gradient scratch of check_adjoints
         spec = alloc<float2>(lay.spec_elems);
         make_spec_tensor_map(&spec_tmap, spec, zb * m, ug);
+        make_vec_gather_map(&vec_tmap, spec, vec_planes(ug, zb), ug);
+        {  // cuFFT calls of the direction path: as many slices as keep its images near the L2
+            const double img = (double)m * P * (n + 2) * 8.0;
+            vec_slices = (int)std::max(1.0, std::min((double)zb, 64e6 / img));
+            vec_slices = std::max(lay.zs, vec_slices / lay.zs * lay.zs);
+            img_per_fft = zb * m;
+            const double cap = 8.0 * (1ull << 30), one = (double)P * P * 8.0;
+            while (img_per_fft > 1 && img_per_fft * one > cap) {
+                int nx = img_per_fft - 1;
+                while (nx > 1 && (zb * m) % nx) --nx;
+                img_per_fft = nx;
+            }
+        }
         rows = alloc<float2>((size_t)zb * ntheta * (size_t)std::max(n, n / 2 + 1));
 
         tv.n = n;
@@ -323,6 +358,7 @@ struct Handle {
                 CUDA_CHECK(cudaStreamSynchronize(stream));
                 ug.hpitch = P / 2 + 2;  // 16-byte half-plane rows for the TMA tiles
                 make_pad_fft_maps(&fft_fwd_map, &fft_inv_map, spec, zb * m, ug);
+                make_vec_fft_map(&vec_fft_map, spec, vec_planes(ug, zb), ug);
                 fused_rows = lay.fused_rows;
                 if (fused_rows) {
                     const std::vector<float2> wn = pad_fft_twiddles(n);
@@ -339,9 +375,18 @@ struct Handle {
 
     // cuFFT plans are made on first need (never during stream capture): the
     // outer iteration needs them only off the hand-written path
-    // (lay.iter_plans), the operator API, check_adjoints and FBP always.
+    // (lay.iter_plans), the operator API, check_adjoints and FBP always.  The
+    // geometry must be set: its path decides which plans run.
     void ensure_plans() {
-        if (!plans_made) make_fft_plans();
+        bool need[kNPlans] = {};
+        need[kRowsR2C] = true;
+        need[gd.dirs ? kRowsC2R : kRowsC2C] = true;
+        if (!pad_fft) need[gd.dirs ? kVecR2C : kR2C2D] = true;
+        if (!gd.tc_scatter)
+            need[kC2C2D] = true;
+        else if (!pad_fft)
+            need[kC2R2D] = true;
+        make_fft_plans(need);
     }
 
     template <class T>
@@ -361,69 +406,57 @@ struct Handle {
         tv.sd = (float)(1.0 / (4.0 * std::cbrt(2.0) * ((double)l1 / 2.0)));
     }
 
-    void make_fft_plans() {
-        const int P = 2 * n;
-        const double img_bytes = (double)P * P * 8.0;
-        const int nimg = zb * m;
-        int per = nimg;
-        const double cap = 8.0 * (1ull << 30);
-        while (per > 1 && per * img_bytes > cap) {
-            int nx = per - 1;
-            while (nx > 1 && nimg % nx) --nx;
-            per = nx;
-        }
-        img_per_fft = per;
-        size_t ws = 0, w1 = 0;
-        CUFFT_CHECK(cufftCreate(&p_r2c2d));
-        CUFFT_CHECK(cufftCreate(&p_c2c2d));
-        CUFFT_CHECK(cufftCreate(&p_c2r2d));
-        CUFFT_CHECK(cufftCreate(&p_rows_c2c));
-        CUFFT_CHECK(cufftCreate(&p_rows_r2c));
-        plans_made = true;
-        for (cufftHandle h : {p_r2c2d, p_c2c2d, p_rows_c2c, p_rows_r2c, p_c2r2d})
-            CUFFT_CHECK(cufftSetAutoAllocation(h, 0));
-        {  // 2D R2C in place inside the padded forward images: real rows of
-           // 2 qp floats -> P/2+1 complex of a qp-complex row
-            int nn[2] = {P, P};
-            int inem[2] = {P, 2 * ug.qp};
-            int onem[2] = {P, ug.qp};
-            CUFFT_CHECK(cufftMakePlanMany(p_r2c2d, 2, nn, inem, 1, (int)(2 * ug.img_fwd), onem, 1, (int)ug.img_fwd,
-                                          CUFFT_R2C, per, &w1));
+    void make_fft_plans(const bool (&need)[kNPlans]) {
+        const int P = 2 * n, per = img_per_fft, nrows = zb * ntheta, hn = n / 2 + 1;
+        size_t ws = fft_work_bytes;
+        bool any = false;
+        for (int i = 0; i < kNPlans; ++i) {
+            if (!need[i] || plan_made[i]) continue;
+            any = true;
+            CUFFT_CHECK(cufftCreate(&plan[i]));
+            plan_made[i] = true;
+            CUFFT_CHECK(cufftSetAutoAllocation(plan[i], 0));
+            size_t w1 = 0;
+            // 2D (rows of iem / oem elements, images of idist / odist) or rows of n
+            auto make = [&](int rank, int len, int iem, int idist, int oem, int odist, cufftType type, int batch) {
+                int nn[2] = {len, len}, in[2] = {len, iem}, on[2] = {len, oem};
+                if (rank == 1) {
+                    in[0] = iem;
+                    on[0] = oem;
+                }
+                CUFFT_CHECK(cufftMakePlanMany(plan[i], rank, nn, in, 1, idist, on, 1, odist, type, batch, &w1));
+            };
+            switch (i) {
+                case kR2C2D:  // in place inside the padded forward images
+                    make(2, P, 2 * ug.qp, (int)(2 * ug.img_fwd), ug.qp, (int)ug.img_fwd, CUFFT_R2C, per);
+                    break;
+                case kC2R2D:  // in place: Hermitian half planes of P/2+1 complex -> real rows of P+2 floats
+                    make(2, P, P / 2 + 1, P * (P / 2 + 1), P + 2, P * (P + 2), CUFFT_C2R, per);
+                    break;
+                case kC2C2D: make(2, P, P, P * P, P, P * P, CUFFT_C2C, per); break;  // full planes
+                case kVecR2C:  // in place, rows of n + 2 complex
+                    make(2, P, 2 * (n + 2), 2 * (n + 2) * P, n + 2, (n + 2) * P, CUFFT_R2C, vec_slices * m);
+                    break;
+                case kRowsC2C: make(1, n, n, n, n, n, CUFFT_C2C, nrows); break;
+                case kRowsR2C: make(1, n, 2 * hn, 2 * hn, hn, hn, CUFFT_R2C, nrows); break;  // in place (adjoint)
+                case kRowsC2R: make(1, n, hn, hn, 2 * hn, 2 * hn, CUFFT_C2R, nrows); break;  // in place (forward)
+            }
+            CUFFT_CHECK(cufftSetStream(plan[i], stream));
             ws = std::max(ws, w1);
         }
-        {  // 2D C2R in place: Hermitian half planes of P/2+1 complex -> real rows of P+2 floats
-            int nn[2] = {P, P};
-            int inem[2] = {P, P / 2 + 1};
-            int onem[2] = {P, P + 2};
-            CUFFT_CHECK(cufftMakePlanMany(p_c2r2d, 2, nn, inem, 1, P * (P / 2 + 1), onem, 1, P * (P + 2), CUFFT_C2R,
-                                          per, &w1));
-            ws = std::max(ws, w1);
+        if (!any) return;
+        if (ws > fft_work_bytes) {
+            if (fft_work) {
+                drop_graphs();  // they hold the work area's address
+                cudaFreeAsync(fft_work, stream);
+                owned.erase(std::find(owned.begin(), owned.end(), fft_work));
+                dev_bytes -= fft_work_bytes;
+            }
+            fft_work = alloc<char>(ws);
+            fft_work_bytes = ws;
         }
-        {  // 2D C2C full plane
-            int nn[2] = {P, P};
-            CUFFT_CHECK(cufftMakePlanMany(p_c2c2d, 2, nn, nullptr, 1, P * P, nullptr, 1, P * P, CUFFT_C2C, per,
-                                          &w1));
-            ws = std::max(ws, w1);
-        }
-        const int nrows = zb * ntheta;
-        {  // rows C2C (forward operator's inverse transform)
-            int nn[1] = {n};
-            CUFFT_CHECK(cufftMakePlanMany(p_rows_c2c, 1, nn, nullptr, 1, n, nullptr, 1, n, CUFFT_C2C, nrows, &w1));
-            ws = std::max(ws, w1);
-        }
-        {  // rows R2C in place (adjoint): 2(n/2+1) floats -> n/2+1 complex
-            int nn[1] = {n};
-            int inem[1] = {2 * (n / 2 + 1)};
-            int onem[1] = {n / 2 + 1};
-            CUFFT_CHECK(cufftMakePlanMany(p_rows_r2c, 1, nn, inem, 1, 2 * (n / 2 + 1), onem, 1, n / 2 + 1,
-                                          CUFFT_R2C, nrows, &w1));
-            ws = std::max(ws, w1);
-        }
-        if (ws > 0) fft_work = alloc<char>(ws);
-        for (cufftHandle h : {p_r2c2d, p_c2c2d, p_rows_c2c, p_rows_r2c, p_c2r2d}) {
-            CUFFT_CHECK(cufftSetWorkArea(h, fft_work));
-            CUFFT_CHECK(cufftSetStream(h, stream));
-        }
+        for (int i = 0; i < kNPlans; ++i)
+            if (plan_made[i]) CUFFT_CHECK(cufftSetWorkArea(plan[i], fft_work));
     }
 
     void drop_graphs() {
@@ -439,6 +472,7 @@ struct Handle {
         for (void *p : geo_owned) cudaFreeAsync(p, stream);
         geo_owned.clear();
         geo_bytes = 0;
+        planar = nullptr;
         int *err = gd.err;
         gd = GeoDev();
         gd.err = err;
@@ -449,9 +483,8 @@ struct Handle {
     // the handle's earlier work (the engine binds only idle handles).
     void bind_stream(cudaStream_t s) {
         stream = s ? s : own_stream;
-        if (plans_made)
-            for (cufftHandle h : {p_r2c2d, p_c2c2d, p_rows_c2c, p_rows_r2c, p_c2r2d})
-                CUFFT_CHECK(cufftSetStream(h, stream));
+        for (int i = 0; i < kNPlans; ++i)
+            if (plan_made[i]) CUFFT_CHECK(cufftSetStream(plan[i], stream));
     }
 
     void release() {
@@ -460,14 +493,11 @@ struct Handle {
         stream = own_stream;
         drop_graphs();
         free_geo();
-        if (plans_made) {
-            cufftDestroy(p_r2c2d);
-            cufftDestroy(p_c2c2d);
-            cufftDestroy(p_c2r2d);
-            cufftDestroy(p_rows_c2c);
-            cufftDestroy(p_rows_r2c);
-            plans_made = false;
-        }
+        for (int i = 0; i < kNPlans; ++i)
+            if (plan_made[i]) {
+                cufftDestroy(plan[i]);
+                plan_made[i] = false;
+            }
         for (void *p : owned) cudaFreeAsync(p, stream);
         owned.clear();
         if (stats_host) cudaFreeHost(stats_host);
@@ -650,6 +680,24 @@ struct Handle {
                 kmat[(size_t)th * m + j] = make_float2((float)acc.real(), (float)acc.imag());
             }
         gd.kmat = (float2 *)up(kmat.data(), kmat.size() * sizeof(float2));
+        std::vector<float2> dk;  // K' in direction order, rows padded to whole groups of time samples
+        if (dirs) {
+            const int ks = ug.jg > 1 ? 16 * ug.jg : ug.tg;
+            dk.assign((size_t)ntheta * ks, make_float2(0.f, 0.f));
+            for (int r = 0; r < ntheta; ++r) {
+                const size_t th = dplan.rays[r] & 0x7fffffffu;
+                std::copy(kmat.begin() + th * m, kmat.begin() + (th + 1) * m, dk.begin() + (size_t)r * ks);
+            }
+            gd.dkmat = (float2 *)up(dk.data(), dk.size() * sizeof(float2));
+            if (!pad_fft) {
+                const size_t bytes = (size_t)vec_slices * m * ug.P * (n + 2) * sizeof(float2);
+                void *p = nullptr;
+                CUDA_CHECK(cudaMallocAsync(&p, bytes, stream));
+                geo_owned.push_back(p);
+                geo_bytes += bytes;
+                planar = (float2 *)p;
+            }
+        }
         // set_center (radonusfft.cu:70-75, takeshift kernels_radonusfft.cuh:191-198)
         std::vector<float2> sf(n), sa(n);
         for (int k = 0; k < n; ++k) {
@@ -694,21 +742,49 @@ struct Handle {
     // out = tau R_apr u  (residual: out = R_apr u - gb)
     void forward(const float *u, const float *gb, float *out, float tau, int residual) {
         forward_rows(u);
-        CUFFT_CHECK(cufftExecC2C(p_rows_c2c, reinterpret_cast<cufftComplex *>(rows),
+        if (gd.dirs) {  // Hermitian half rows
+            CUFFT_CHECK(cufftExecC2R(plan[kRowsC2R], reinterpret_cast<cufftComplex *>(rows),
+                                     reinterpret_cast<cufftReal *>(rows)));
+            launch_finish_fwd_real(reinterpret_cast<const float *>(rows), gb, out, zb, tau, residual, ug, stream);
+            return;
+        }
+        CUFFT_CHECK(cufftExecC2C(plan[kRowsC2C], reinterpret_cast<cufftComplex *>(rows),
                                  reinterpret_cast<cufftComplex *>(rows), CUFFT_INVERSE));
         launch_finish_fwd(rows, gb, out, zb, tau, residual, ug, stream);
     }
 
-    // the gathered row spectra of R_apr u (before the inverse row FFT) in rows
+    // the gathered row spectra of R_apr u (before the inverse row FFT) in rows:
+    // whole rows, or their Hermitian halves on the direction path
     void forward_rows(const float *u) {
         const int nimg = zb * m;
+        if (gd.dirs) {
+            if (pad_fft) {
+                launch_pad_fft_fwd_vec(u, spec, zb, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+            } else {
+                UsGeo gp2 = ug;  // planar images of rows of n + 2 complex
+                gp2.qp = n + 2;
+                gp2.qoff = 0;
+                gp2.img_fwd = (long long)ug.P * (n + 2);
+                for (int z = 0; z < zb; z += vec_slices) {
+                    const int nzg = std::min(vec_slices, zb - z);
+                    launch_deapod_pad(u + (long long)z * slab, reinterpret_cast<float *>(planar), nzg * m, gd.deapod,
+                                      gp2, stream);
+                    CUFFT_CHECK(cufftExecR2C(plan[kVecR2C], reinterpret_cast<cufftReal *>(planar),
+                                             reinterpret_cast<cufftComplex *>(planar)));
+                    launch_planar_to_vec(planar, spec, z, nzg, ug, stream);
+                }
+            }
+            launch_vec_halo(spec, vec_planes(ug, zb), ug, stream);
+            launch_gather_fwd(spec, rows, zb, gd, ug, &vec_tmap, stream);
+            return;
+        }
         if (pad_fft) {
             launch_pad_fft_fwd(u, spec, nimg, gd.deapod, fft_tw, fft_fwd_map, gd.err, ug, stream);
         } else {
             launch_deapod_pad(u, reinterpret_cast<float *>(spec), nimg, gd.deapod, ug, stream);
             for (int i = 0; i < nimg; i += img_per_fft) {
                 cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * ug.img_fwd + ug.qoff);
-                CUFFT_CHECK(cufftExecR2C(p_r2c2d, reinterpret_cast<cufftReal *>(p), p));
+                CUFFT_CHECK(cufftExecR2C(plan[kR2C2D], reinterpret_cast<cufftReal *>(p), p));
             }
         }
         launch_spec_halo(spec, nimg, ug, stream);
@@ -718,7 +794,7 @@ struct Handle {
     // u += tau R_apr^T h
     void adjoint(const float *h, float *u, float tau, const float *row_filter = nullptr) {
         launch_adj_prep(h, reinterpret_cast<float *>(rows), zb, ug, stream);
-        CUFFT_CHECK(cufftExecR2C(p_rows_r2c, reinterpret_cast<cufftReal *>(rows),
+        CUFFT_CHECK(cufftExecR2C(plan[kRowsR2C], reinterpret_cast<cufftReal *>(rows),
                                  reinterpret_cast<cufftComplex *>(rows)));
         if (row_filter) launch_filter_rows(rows, row_filter, (long long)zb * ntheta, n, stream);
         adjoint_rows(rows, u, tau);
@@ -740,7 +816,7 @@ struct Handle {
             }
             for (int i = 0; i < nimg; i += img_per_fft) {
                 cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * img_half);
-                CUFFT_CHECK(cufftExecC2R(p_c2r2d, p, reinterpret_cast<cufftReal *>(p)));
+                CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], p, reinterpret_cast<cufftReal *>(p)));
             }
             launch_crop_accum_real(reinterpret_cast<const float *>(spec), u, zb, tau, gd.deapod, ug, stream);
             return;
@@ -751,7 +827,7 @@ struct Handle {
         launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
         for (int i = 0; i < nimg; i += img_per_fft) {
             cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * ug.img_adj);
-            CUFFT_CHECK(cufftExecC2C(p_c2c2d, p, p, CUFFT_INVERSE));
+            CUFFT_CHECK(cufftExecC2C(plan[kC2C2D], p, p, CUFFT_INVERSE));
         }
         launch_crop_accum(spec, u, zb, tau, gd.deapod, ug, stream);
     }
@@ -768,7 +844,7 @@ struct Handle {
                 const int c0 = bb * dpb;
                 if (fused_rows) {  // residual rows straight into the adjoint's row spectra
                     forward_rows(U[src] + z0 * slab);
-                    launch_resid_rows(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, zb, ug, stream);
+                    launch_resid_rows(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, zb, gd.dirs, ug, stream);
                 } else {
                     forward(U[src] + z0 * slab, gdata + z0 * ntheta * n, h1, 1.0f, 1);
                 }
@@ -1039,8 +1115,8 @@ struct Handle {
         check_live();
         session = false;
         drop_graphs();
-        ensure_plans();
         set_geometry(theta_h, nullptr, center);
+        ensure_plans();
         std::vector<float> w(n / 2 + 1);
         for (int k = 0; k <= n / 2; ++k) {
             const float rho = (float)(k - n / 2) / (float)n;
@@ -1080,11 +1156,13 @@ struct Handle {
         // samples, per group of 16 time samples the tensor-core gather (8+ time
         // samples) and the direct one (items with few samples per ray), then the
         // fused residual rows or the forward epilogue
+        // (direction path: deapodise/pad and the layout change per cuFFT call, no zeroing)
+        const int vcalls = (zb + vec_slices - 1) / vec_slices;
         const int gather_k =
-            1 + ng * (gd.dirs ? (gd.n_dfwd_items > 0 ? 1 : 0)
-                              : ((m >= 8 && gd.n_fwd_tc_items > 0) ? 1 : 0) + (gd.n_fwd_items > 0 ? 1 : 0));
-        const int fwd_k = (pad_fft ? 2 : 1) + 1 + gather_k + 1;
-        const int fwd_f = (pad_fft ? 0 : f2) + (fused_rows ? 0 : 1);
+            gd.dirs ? (gd.n_dfwd_items > 0 ? ng : 0)
+                    : 1 + ng * (((m >= 8 && gd.n_fwd_tc_items > 0) ? 1 : 0) + (gd.n_fwd_items > 0 ? 1 : 0));
+        const int fwd_k = (pad_fft ? 2 : (gd.dirs ? 2 * vcalls : 1)) + 1 + gather_k + 1;
+        const int fwd_f = (pad_fft ? 0 : (gd.dirs ? vcalls : f2)) + (fused_rows ? 0 : 1);
         // adjoint: [row preparation], the zeroing of split tiles (direct scatter),
         // one scatter per group, then [columns + rows | crop]
         const int adj_k = (fused_rows ? 0 : 1) + ((!gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
@@ -1146,7 +1224,7 @@ struct Handle {
             throw Error(RECTV_ERR_ARG, "rectv_launch_kernel: no padded-grid FFT at this size");
         for (int r = 0; r < reps; ++r) {
             switch (which) {
-                case 0: launch_gather_fwd(spec, rows, zb, gd, ug, &spec_tmap, stream); break;
+                case 0: launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &vec_tmap : &spec_tmap, stream); break;
                 case 1: launch_scatter_adj(fused_rows ? rows_adj : rows, spec, zb, gd, ug, stream); break;
                 case 2:  // the inner steps after the first (w = mu - rho psi as stored by the last iteration)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 2 : 0, rho_d, 0,
@@ -1156,7 +1234,10 @@ struct Handle {
                     launch_shrink(U[cur], U[cur], psi, mu, rho_d, lambda0, 0, nchunks, tv, partials, stream);
                     break;
                 case 4:  // padded-grid forward FFT of the batch (rows + columns)
-                    launch_pad_fft_fwd(U[cur], spec, zb * m, gd.deapod, fft_tw, fft_fwd_map, gd.err, ug, stream);
+                    if (gd.dirs)
+                        launch_pad_fft_fwd_vec(U[cur], spec, zb, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+                    else
+                        launch_pad_fft_fwd(U[cur], spec, zb * m, gd.deapod, fft_tw, fft_fwd_map, gd.err, ug, stream);
                     break;
                 case 6:  // the first inner step (psi, mu in; stores w = mu - rho psi, unchanged values)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 1 : 0, rho_d, 0,
@@ -1178,8 +1259,8 @@ struct Handle {
             throw Error(RECTV_ERR_ARG, "rectv: check_adjoints needs nz == nzp (one chunk), as in rectv.cu:258");
         session = false;
         drop_graphs();
-        ensure_plans();
         set_geometry(theta_h, phi_h, center);
+        ensure_plans();
         set_lambda1(lambda1_);
         CUDA_CHECK(cudaMemcpyAsync(gdata, g_h, sizeof(float) * (size_t)nz * ntheta * n, cudaMemcpyHostToDevice,
                                    stream));

@@ -212,6 +212,7 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, i
 bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, double tol_cells, double min_group,
                     DirPlan &dp) {
     dp = DirPlan();
+    if (n % 2) return false;  // sample k of a ray mirrors sample n - k for an even detector width only
     const double pi = 3.14159265358979323846;
     const double tol = tol_cells / (double)n;
     std::vector<double> alpha(ntheta);
@@ -284,7 +285,7 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
             if (y0 >= 0.5f) y0 = 0.5f - 1e-5f;
             const int KX = n + (int)std::floor(tn * x0), KY = n + (int)std::floor(tn * y0);
             ftile[ip] = (KY / T) * NT + (KX / T);
-            fcnt[ftile[ip]]++;
+            if (q <= n / 2) fcnt[ftile[ip]]++;  // the pair (q, n - q) is gathered at q
             const int xa = wrapi(KX - kR, P) / T, xb = wrapi(KX + kR, P) / T;
             const int ya = wrapi(KY - kR, P) / T, yb = wrapi(KY + kR, P) / T;
             const int nx = (xa == xb) ? 1 : 2, ny = (ya == yb) ? 1 : 2;
@@ -309,7 +310,7 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
         for (int d = 0; d < dp.ndir; ++d)
             for (int q = 1; q < n; ++q, ++ip) {
                 const uint32_t id = (uint32_t)d * (uint32_t)n + (uint32_t)q;
-                dp.fwd_pos[fp[ftile[ip]]++] = id;
+                if (q <= n / 2) dp.fwd_pos[fp[ftile[ip]]++] = (uint32_t)d * (uint32_t)(n / 2) + (uint32_t)(q - 1);
                 const int4 a = atiles[ip];
                 const int tl[4] = {a.x, a.y, a.z, a.w};
                 for (int i = 0; i < 4; ++i)

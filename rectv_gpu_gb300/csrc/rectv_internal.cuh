@@ -67,7 +67,31 @@ struct UsGeo {
     // scatter (0: one per SM)
     int zper;
     int sc_grid;
+    // Vector layout of the direction path (dir_kernels.cu): the spectra of 16
+    // (slice, time sample) pairs are stored together, cell by cell:
+    // [plane][row][column][16] complex over the window rows [-kVH, P + kVH) x
+    // columns [-kVH, n + kVH] of the half plane.  One plane holds tg time
+    // samples (1, 2, 4, 8 or 16, at least m) of zs = 16 / tg slices; with
+    // m > 16 a slice takes jg = ceil(m / 16) planes of 16 samples.
+    int tg, zs, jg;
+    int vp;             // row pitch in cells: n + 1 + 2 kVH
+    int vrows;          // P + 2 kVH
+    long long vplane;   // complex elements per plane
 };
+
+// halo cells of the vector layout (a stencil and its mirror image reach from
+// 4 cells before to 5 cells after the origin)
+constexpr int kVH = 8;
+__host__ __device__ inline int vec_planes(const UsGeo &g, int zb) {  // planes of zb slices
+    return g.jg > 1 ? zb * g.jg : (zb + g.zs - 1) / g.zs;
+}
+// slice and time sample of entry v of plane pl
+__host__ __device__ inline int vec_slice(const UsGeo &g, int pl, int v) {
+    return g.jg > 1 ? pl / g.jg : pl * g.zs + v / g.tg;
+}
+__host__ __device__ inline int vec_time(const UsGeo &g, int pl, int v) {
+    return g.jg > 1 ? (pl % g.jg) * 16 + v : v & (g.tg - 1);
+}
 
 // Weights of one polar sample restricted to one 16x16 tile of the adjoint
 // plan (zero outside the sample's 9x9 stencil), with its ray and the mask of
@@ -119,9 +143,10 @@ struct GeoDev {
     int *dray_start = nullptr;    // [ndir + 1]
     uint32_t *drays = nullptr;    // theta | opposite << 31
     float *dtau = nullptr;        // per ray: offset across the direction (DirPlan::tau)
+    float2 *dkmat = nullptr;      // K' in the order of drays, [ray][max(tg, 16 jg)], zero past m
     float4 *demix = nullptr;      // adjoint E, E_perp per (slice, position): dir_mix_bytes(demix_slices, ndir, n)
     int demix_slices = 0;
-    uint32_t *dfwd_pos = nullptr; // positions d*n + q sorted by origin tile
+    uint32_t *dfwd_pos = nullptr; // position pairs d*(n/2) + q - 1 sorted by origin tile
     int4 *dfwd_items = nullptr;   // (tile, start, count, 0)
     int n_dfwd_items = 0;
 };
@@ -152,7 +177,7 @@ struct DirPlan {
     std::vector<uint32_t> rays;     // theta index | opposite << 31 (sample k of an opposite ray is position n - k)
     std::vector<float> tau;         // per ray (order of rays): its samples' offset across the direction, in
                                     // grid cells per unit of (q - n/2)/n
-    std::vector<uint32_t> fwd_pos;  // positions d*n + q (1 <= q < n) sorted by the tile of the stencil origin
+    std::vector<uint32_t> fwd_pos;  // position pairs d*(n/2) + q - 1 (1 <= q <= n/2) sorted by the tile of the stencil origin
     std::vector<int4> fwd_items;    // (tile, start, count, 0): at most fwd_cap positions of one tile
     std::vector<uint32_t> adj_pos;  // one entry per tile a position's stencil touches
     std::vector<int4> adj_items;    // (tile, start, count, 0), one per tile, busiest first
@@ -189,6 +214,9 @@ void launch_gather_fwd(const float2 *spec, float2 *rows, int zb, const GeoDev &g
                        const CUtensorMap *tmap, cudaStream_t s);
 void launch_finish_fwd(const float2 *rows, const float *gdata, float *out, int zb, float tau,
                        int residual, const UsGeo &g, cudaStream_t s);
+// the same from the real output of the rows' C2R inverse (rows of 2 (n/2+1) floats)
+void launch_finish_fwd_real(const float *rows, const float *gdata, float *out, int zb, float tau, int residual,
+                            const UsGeo &g, cudaStream_t s);
 void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaStream_t s);
 void launch_zero_split(float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
 void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
@@ -223,8 +251,16 @@ void launch_adj_tabinfo(const GeoDev &gd, cudaStream_t s);
 // positions' interpolated spectra (time samples [jbase, jbase + 16),
 // accumulated into rows when accumulate != 0), and the adjoint scatter into
 // the zeroed Hermitian half planes (as launch_scatter_tc)
-void launch_gather_dir(float2 *rows, const float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
-                       int accumulate, cudaStream_t s);
+void launch_gather_dir(float2 *hrows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &vmap,
+                       cudaStream_t s);
+// TMA descriptor of the gather's footprints in the vector layout (npl planes)
+void make_vec_gather_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
+// fills the halo of the forward spectra in the vector layout
+void launch_vec_halo(float2 *spec, int npl, const UsGeo &g, cudaStream_t s);
+// cuFFT's spectra of slices z0 .. z0 + nz - 1 (planar, rows of n + 2 complex,
+// image (z - z0) m + t) into the vector layout
+void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, const UsGeo &g, cudaStream_t s);
+void gather_dir_prepare();
 void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
                         cudaStream_t s);
 // geometry records of the direction path's adjoint entries (as
@@ -250,13 +286,18 @@ std::vector<float2> pad_fft_twiddles(int P);
 void make_pad_fft_maps(CUtensorMap *fwd, CUtensorMap *inv, float2 *spec, int nimg, const UsGeo &g);
 void launch_pad_fft_fwd(const float *u, float2 *spec, int nimg, const float *deapod, const float2 *tw,
                         const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
+// the forward pass into the vector layout (halo not filled)
+void make_vec_fft_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
+void launch_pad_fft_fwd_vec(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
+                            const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 // fused residual rows of the inner step (fft_kernels.cu), n a power of two in
 // [256, 1024]: gathered rows [z][theta][n] and data g -> the adjoint's row
 // spectra [z][theta][n/2+1] (inverse row FFT, residual, fftshift, R2C)
 bool resid_rows_supported(int n);
-void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb,
+// half: the rows hold the Hermitian half k = 0 .. n/2 (direction path)
+void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb, bool half,
                        const UsGeo &g, cudaStream_t s);
 size_t gather_tc_smem();
 int gather_tc_table_capacity();

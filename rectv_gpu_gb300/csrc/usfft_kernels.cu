@@ -356,14 +356,14 @@ __global__ void k_zero_k0(float2 *rows, long long nrows, int n) {
 
 void launch_gather_fwd(const float2 *spec, float2 *rows, int zb, const GeoDev &gd, const UsGeo &g,
                        const CUtensorMap *tmap, cudaStream_t s) {
+    if (g.T != 16) throw Error(1, "tile size must be 16");
+    if (gd.dirs) {  // rays grouped by direction: one interpolation per position pair (gather_dir.cu), half rows
+        launch_gather_dir(rows, zb, gd, g, *tmap, s);
+        return;
+    }
     const long long nrows = (long long)zb * g.ntheta;
     k_zero_k0<<<(unsigned)((nrows + 255) / 256), 256, 0, s>>>(rows, nrows, g.n);
     LAUNCH_CHECK("k_zero_k0");
-    if (g.T != 16) throw Error(1, "tile size must be 16");
-    if (gd.dirs) {  // rays grouped by direction: one interpolation per position (dir_kernels.cu)
-        for (int jb = 0; jb < g.m; jb += 16) launch_gather_dir(rows, spec, zb, gd, g, jb, jb > 0, s);
-        return;
-    }
     const int mp = mp_for(g.m);
     for (int jb = 0; jb < g.m; jb += 16) {
         const int acc = jb > 0;
@@ -407,6 +407,27 @@ void launch_finish_fwd(const float2 *rows, const float *gdata, float *out, int z
     k_finish_fwd<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(rows, gdata, out, total, g.n, scale, tau,
                                                                  residual);
     LAUNCH_CHECK("k_finish_fwd");
+}
+
+// The same after the C2R inverse of Hermitian half rows: real rows of 2 (n/2+1) floats.
+__global__ void k_finish_fwd_real(const float *__restrict__ rows, const float *__restrict__ gdata,
+                                  float *__restrict__ out, long long total, int n, float scale, float tau,
+                                  int residual) {
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (i >= total) return;
+    const long long r = i / n;
+    const int sidx = (int)(i - r * n);
+    const float v = rows[r * (2 * (n / 2 + 1)) + sidx] * ((sidx & 1) ? scale : -scale);
+    out[i] = residual ? v - gdata[i] : tau * v;
+}
+
+void launch_finish_fwd_real(const float *rows, const float *gdata, float *out, int zb, float tau, int residual,
+                            const UsGeo &g, cudaStream_t s) {
+    const long long total = (long long)zb * g.ntheta * g.n;
+    const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
+    k_finish_fwd_real<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(rows, gdata, out, total, g.n, scale, tau,
+                                                                      residual);
+    LAUNCH_CHECK("k_finish_fwd_real");
 }
 
 // ---------------------------------------------------------------------------

@@ -152,7 +152,7 @@ int rectv_get_launch_counts(rectv_handle *h, int *kernels, int *fft_execs, int *
  * reference interpolates every ray, kernels_radonusfft.cuh:81-144).  *ndir =
  * number of ray directions (theta modulo pi) when the rays of a direction
  * share their sample positions (scans over several half-turns: the
- * interpolation runs once per position, dir_kernels.cu), 0 when every ray is
+ * interpolation runs once per position, gather_dir.cu), 0 when every ray is
  * interpolated (tensor-core or FP32 kernels); *nrays = ntheta.  Selected at
  * geometry set-up: directions are used when the rays average at least 2.5
  * per direction (RECTV_DIRS=0 never, RECTV_DIRS=1 whenever possible) and

@@ -115,12 +115,10 @@ Tune autotune(Handle &h, bool force) {
         best.gather_ms = tbest;
         h.ug.zper = best.zper;
     }
-    if (h.gd.tc_scatter) {
+    if (h.gd.tc_scatter && !h.gd.dirs) {  // the direction scatter's grid follows from the problem
         const int nsm = sm_count(h.device);
         double tbest = 1e30;
-        // persistent blocks: nsm * frac / 4 (tensor-core scatter, one block per
-        // SM at most), nsm * frac / 2 (direction scatter, two per SM at most)
-        const int per = h.gd.dirs ? 2 : 4;
+        const int per = 4;  // persistent blocks: nsm * frac / 4, one block per SM at most
         for (int frac : {4, 3, 2}) {
             h.ug.sc_grid = nsm * frac / per;
             const double t = time_kernel(h, 1, reps);

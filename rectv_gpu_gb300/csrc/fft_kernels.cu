@@ -294,6 +294,19 @@ struct VecRows {
     static constexpr int R = kRowThreads / (N1 * C);         // rows per block
     using L = FftLayout<N, true, C>;
     static constexpr size_t SMEM = sizeof(float2) * (size_t)L::S * C * R;
+    // real rows of the block's 2C images in shared memory, image c of the
+    // pairs' first values, C + c of their second ones: 16-byte rows whose
+    // pitch spreads the lanes (c, t) over the banks
+    static constexpr int n = N / 2;
+    static constexpr int RP = n + (C == 8 ? 4 : 8);
+    static_assert(2 * C * RP <= 2 * L::S * C, "real rows fit the exchange buffer");
+    static constexpr int PER = 2 * C * (n / 4) / (C * N1);  // float4 of the rows per thread (4)
+    // the 16-byte piece i of this row's thread tr: image j, column x (a multiple of 4)
+    __device__ static __forceinline__ void piece(int i, int tr, int &j, int &x) {
+        const int e = i * (C * N1) + tr;
+        j = e / (n / 4);
+        x = 4 * (e - j * (n / 4));
+    }
 };
 
 template <int N>
@@ -310,12 +323,12 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     const int v0 = 2 * ((blockIdx.x % (8 / C)) * C + c);  // the pair's values v0, v0 + 1 of the plane
     float2 *sh = fft_sh + rr * (L::S * C);
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
-    const int zc = vec_slice(g, pl, v0 + 1), tc_ = vec_time(g, pl, v0 + 1);
-    const bool oka = za < zb && ta < g.m, okb = zc < zb && tc_ < g.m;
+    const int zc = vec_slice(g, pl, v0 + 1), tb = vec_time(g, pl, v0 + 1);
+    const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m;
     float2 v[16];
     {
         const float *ua = u + (((long long)(oka ? za : 0) * g.m + (oka ? ta : 0)) * n + y) * n;
-        const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tc_ : 0)) * n + y) * n;
+        const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y) * n;
         const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * inv4n2;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
@@ -540,6 +553,88 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         }
 }
 
+// ---------------------------------------------------------------------------
+// Adjoint rows from the vector layout: the two images of a value pair are the
+// real and imaginary part of one inverse FFT (as k_fft_rows_fwd_vec); the
+// centre outputs pass through shared memory once more so that the rows of u
+// are read and written as whole lines.
+// ---------------------------------------------------------------------------
+template <int N>
+__global__ void __launch_bounds__(kRowThreads, 2)
+    k_fft_rows_inv_vec(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp,
+                       const float2 *__restrict__ tw, UsGeo g, int zb, float cscale) {
+    using V = VecRows<N>;
+    using L = typename V::L;
+    constexpr int N1 = V::N1, C = V::C, R = V::R, n = N / 2;
+    extern __shared__ float2 fft_sh[];
+    const int c = threadIdx.x % C, t = (threadIdx.x / C) % N1, rr = threadIdx.x / (C * N1);
+    const int y = (blockIdx.x / (8 / C)) * R + rr, pl = blockIdx.y;
+    const int vb = 2 * (blockIdx.x % (8 / C)) * C;  // the block's first value
+    float2 *sh = fft_sh + rr * (L::S * C);
+    const float4 *row =
+        reinterpret_cast<const float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + vb) + c;
+    // A + i B at k = t + N1 r: the stored half k <= n is read once; its mirror
+    // image at N - k belongs to thread N1 - t and goes there through shared memory
+    float2 v[16];
+    {
+        float4 f[9];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) f[r] = row[(long long)(t + N1 * r) * 8];
+        f[8] = t == 0 ? row[(long long)n * 8] : make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t == 0) f[0].y = f[0].w = f[8].y = f[8].w = 0.f;  // columns 0 and n of a real image's spectrum
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            v[r] = make_float2(f[r].x - f[r].w, f[r].y + f[r].z);
+            const int k = t + N1 * r;
+            if (k > 0) sh[(N - k - n) * C + c] = make_float2(f[r].x + f[r].w, f[r].z - f[r].y);
+        }
+        if (t == 0) sh[c] = make_float2(f[8].x - f[8].w, f[8].y + f[8].z);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 8; r < 16; ++r) v[r] = sh[(t + N1 * r - n) * C + c];
+    __syncthreads();
+    fft_core<N, 1, L>(v, sh, c, t, tw);
+    __syncthreads();
+    float *rows = reinterpret_cast<float *>(sh);
+#pragma unroll
+    for (int q = 0; q < 16 / L::R3; ++q)
+#pragma unroll
+        for (int j1 = 0; j1 < L::R3; ++j1) {
+            const int x = t + N1 * q + 256 * j1 - n / 2;
+            if (x >= 0 && x < n) {
+                rows[c * V::RP + x] = v[q * L::R3 + j1].x;
+                rows[(C + c) * V::RP + x] = v[q * L::R3 + j1].y;
+            }
+        }
+    const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * cscale;
+    float4 *up[V::PER], f[V::PER];
+    const int tr = threadIdx.x % (C * N1);
+#pragma unroll
+    for (int i = 0; i < V::PER; ++i) {  // the rows of u are on their way during the barrier
+        int j, x;
+        V::piece(i, tr, j, x);
+        const int vj = vb + 2 * (j % C) + j / C, z = vec_slice(g, pl, vj), tt = vec_time(g, pl, vj);
+        up[i] = z < zb && tt < g.m ? reinterpret_cast<float4 *>(u + (((long long)z * g.m + tt) * n + y) * n + x) : nullptr;
+        if (up[i]) f[i] = *up[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < V::PER; ++i) {
+        if (!up[i]) continue;
+        int j, x;
+        V::piece(i, tr, j, x);
+        const float4 o = *reinterpret_cast<const float4 *>(rows + j * V::RP + x);
+        const float4 d = __ldg(reinterpret_cast<const float4 *>(dp + x));
+        const float s0 = ((x + n / 2) & 1) ? -sy : sy;  // (-1)^X of column x; the next ones alternate
+        f[i].x += o.x * d.x * s0;
+        f[i].y -= o.y * d.y * s0;
+        f[i].z += o.z * d.z * s0;
+        f[i].w -= o.w * d.w * s0;
+        *up[i] = f[i];
+    }
+}
+
 template <int N>
 size_t rows_smem() {
     return sizeof(float2) * (size_t)FftLayout<N, false, kRowThreads / (N / 16)>::S * (kRowThreads / (N / 16));
@@ -648,6 +743,9 @@ void set_attrs_n() {
     CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
     CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd_vec<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv_vec<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, vec_col_c(N), 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)ColPass<N, vec_col_c(N), 1, true>::SMEM));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, vec_col_c(N), -1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)ColPass<N, vec_col_c(N), -1, true>::SMEM));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
@@ -704,6 +802,16 @@ void fwd_vec_n(const float *u, float2 *spec, int zb, const float *deapod, const 
     k_fft_rows_fwd_vec<N><<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g, zb, inv4n2);
     LAUNCH_CHECK("k_fft_rows_fwd_vec");
     launch_cols_vec<N, -1>(map, tw, zb, err, g, s);
+}
+
+template <int N>
+void inv_vec_n(float2 *spec, float *u, int zb, float cscale, const float *deapod, const float2 *tw,
+               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
+    using V = VecRows<N>;
+    launch_cols_vec<N, 1>(map, tw, zb, err, g, s);
+    const dim3 gr(N / 2 / V::R * (8 / V::C), vec_planes(g, zb));
+    k_fft_rows_inv_vec<N><<<gr, kRowThreads, V::SMEM, s>>>(spec, u, deapod, tw, g, zb, cscale);
+    LAUNCH_CHECK("k_fft_rows_inv_vec");
 }
 
 template <int N>
@@ -847,6 +955,20 @@ void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const f
         case 512: inv_n<512>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
         case 1024: inv_n<1024>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
         case 2048: inv_n<2048>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
+        default: throw Error(1, "pad FFT: unsupported grid size");
+    }
+}
+
+void launch_pad_fft_inv_accum_vec(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
+                                  const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
+    if (vec_planes(g, zb) > 65535) throw Error(1, "pad FFT: too many planes per batch");
+    const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
+    const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
+    switch (g.P) {
+        case 256: inv_vec_n<256>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 512: inv_vec_n<512>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 1024: inv_vec_n<1024>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 2048: inv_vec_n<2048>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
         default: throw Error(1, "pad FFT: unsupported grid size");
     }
 }

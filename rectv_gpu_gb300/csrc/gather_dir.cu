@@ -1,6 +1,6 @@
 // Forward USFFT gather for scans that revisit their directions (direction
 // path; the geometry and the first-order offset correction are described in
-// dir_kernels.cu).
+// scatter_dir.cu).
 //
 // Only the real part of the inverse row FFT is used (addreal,
 // kernels_operators.cuh:75-84), so a ray needs the Hermitian half of its row

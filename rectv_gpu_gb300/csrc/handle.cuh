@@ -197,7 +197,7 @@ struct Handle {
     std::vector<void *> geo_owned;
 
     // cuFFT plans, made as a geometry's path needs them (ensure_plans)
-    enum { kR2C2D, kC2C2D, kC2R2D, kRowsC2C, kRowsR2C, kRowsC2R, kVecR2C, kNPlans };
+    enum { kR2C2D, kC2C2D, kC2R2D, kRowsC2C, kRowsR2C, kRowsC2R, kVecR2C, kVecC2R, kNPlans };
     cufftHandle plan[kNPlans] = {};
     bool plan_made[kNPlans] = {};
     size_t fft_work_bytes = 0;
@@ -270,7 +270,8 @@ struct Handle {
         usfft_prepare();
         gather_tc_prepare();
         scatter_tc_prepare();
-        dir_prepare();
+        gather_dir_prepare();
+        scatter_dir_prepare();
         pad_fft_prepare();
         const int P = 2 * n;
         ug.n = n;
@@ -382,10 +383,10 @@ struct Handle {
         need[kRowsR2C] = true;
         need[gd.dirs ? kRowsC2R : kRowsC2C] = true;
         if (!pad_fft) need[gd.dirs ? kVecR2C : kR2C2D] = true;
-        if (!gd.tc_scatter)
+        if (!gd.dirs && !gd.tc_scatter)
             need[kC2C2D] = true;
         else if (!pad_fft)
-            need[kC2R2D] = true;
+            need[gd.dirs ? kVecC2R : kC2R2D] = true;
         make_fft_plans(need);
     }
 
@@ -436,6 +437,9 @@ struct Handle {
                 case kC2C2D: make(2, P, P, P * P, P, P * P, CUFFT_C2C, per); break;  // full planes
                 case kVecR2C:  // in place, rows of n + 2 complex
                     make(2, P, 2 * (n + 2), 2 * (n + 2) * P, n + 2, (n + 2) * P, CUFFT_R2C, vec_slices * m);
+                    break;
+                case kVecC2R:
+                    make(2, P, n + 2, (n + 2) * P, 2 * (n + 2), 2 * (n + 2) * P, CUFFT_C2R, vec_slices * m);
                     break;
                 case kRowsC2C: make(1, n, n, n, n, n, CUFFT_C2C, nrows); break;
                 case kRowsR2C: make(1, n, 2 * hn, 2 * hn, hn, hn, CUFFT_R2C, nrows); break;  // in place (adjoint)
@@ -535,7 +539,7 @@ struct Handle {
         // adjoint: tensor-core time-sample mixing (k_scatter_tc) as fixed by
         // the layout at creation
         const bool tc_scatter = lay.tc_scatter;
-        // direction path (dir_kernels.cu): rays that revisit a direction over
+        // direction path (scatter_dir.cu): rays that revisit a direction over
         // several half-turns share its sample positions, so the USFFT
         // interpolates once per position.  Used when the rays average at least
         // 2.5 per direction (RECTV_DIRS=1: whenever it can run, RECTV_DIRS=0:
@@ -563,7 +567,7 @@ struct Handle {
         if (dirs) {  // per-direction sincos and adjoint entries; no per-ray items
             hp.sincos = dplan.sincos;
             hp.adj_pts = std::move(dplan.adj_pos);
-            hp.adj_items = std::move(dplan.adj_items);
+            hp.adj_items = dir_adj_work(dplan.adj_items, vec_planes(ug, zb) / ug.jg);
         } else {
             hp = build_plan(theta_h, n, ntheta, ug.T, table_capacity(), 1 << 30, tc_min_spr);
         }
@@ -598,8 +602,8 @@ struct Handle {
             gd.dfwd_pos = (uint32_t *)up(dplan.fwd_pos.data(), dplan.fwd_pos.size() * 4);
             gd.dfwd_items = (int4 *)up(dplan.fwd_items.data(), dplan.fwd_items.size() * sizeof(int4));
             gd.n_dfwd_items = (int)dplan.fwd_items.size();
-            {  // the adjoint's E, E_perp per (slice, position) of one batch
-                const size_t bytes = dir_mix_bytes(zb, dplan.ndir, n);
+            {  // the adjoint's mixed rays per (plane, position pair) of one batch
+                const size_t bytes = dir_mix_bytes(ug, zb, dplan.ndir);
                 void *p = nullptr;
                 CUDA_CHECK(cudaMallocAsync(&p, bytes, stream));
                 geo_owned.push_back(p);
@@ -610,19 +614,18 @@ struct Handle {
         }
         std::vector<int> tab_base(1, 0);  // uploaded asynchronously: kept until the stream sync below
         std::vector<int4> tabs;
-        if (tc_scatter) {
+        if (tc_scatter && !dirs) {
             void *p = nullptr;
             CUDA_CHECK(cudaMallocAsync(&p, std::max<size_t>(hp.adj_pts.size() * sizeof(AdjRec), 16), stream));
             geo_owned.push_back(p);
             geo_bytes += std::max<size_t>(hp.adj_pts.size() * sizeof(AdjRec), 16);
             gd.adj_recs = (AdjRec *)p;
             // tables of the busy items and the size of their ray segmentation
-            const int cap = dirs ? dir_adj_table_capacity() : scatter_tc_table_capacity();
+            const int cap = scatter_tc_table_capacity();
             long long words = 0;
             // a table holds whole rays (runs of equal theta), at most one MMA
-            // batch of them (scatter_tc_batch_rays()) and at most cap entries;
-            // on the direction path whole directions, at most dir_adj_table_dirs()
-            const int max_rays = dirs ? dir_adj_table_dirs() : scatter_tc_batch_rays();
+            // batch of them (scatter_tc_batch_rays()) and at most cap entries
+            const int max_rays = scatter_tc_batch_rays();
             for (int i = 0; i < gd.n_adj_busy; ++i) {
                 const int4 it = hp.adj_items[i];
                 const uint32_t *pts = hp.adj_pts.data() + it.y;
@@ -637,7 +640,7 @@ struct Handle {
                         c1 = r;
                         ++nseg;
                     }
-                    const int w = dirs ? dir_adj_info_words(nseg) : scatter_tc_info_words(nseg);
+                    const int w = scatter_tc_info_words(nseg);
                     tabs.push_back(make_int4(it.y + c0, c1 - c0, (int)words, w));
                     words += w;
                     if (words > 2147483647LL) throw Error(RECTV_ERR_ARG, "rectv: adjoint plan too large");
@@ -716,14 +719,9 @@ struct Handle {
             dp[x] = (float)std::exp((double)mu_us * d * d);
         }
         gd.deapod = (float *)up(dp.data(), n * sizeof(float));
-        if (gd.tc_scatter) {
-            if (gd.dirs) {
-                launch_adj_records_dir(gd.adj_recs, gd, ug, stream);
-                launch_adj_tabinfo_dir(gd, stream);
-            } else {
-                launch_adj_records(gd.adj_recs, gd, ug, stream);
-                launch_adj_tabinfo(gd, stream);
-            }
+        if (gd.tc_scatter && !gd.dirs) {
+            launch_adj_records(gd.adj_recs, gd, ug, stream);
+            launch_adj_tabinfo(gd, stream);
         }
         CUDA_CHECK(cudaStreamSynchronize(stream));  // host vectors go out of scope
         geo_theta.assign(theta_h, theta_h + ntheta);
@@ -803,12 +801,27 @@ struct Handle {
     // u += tau R_apr^T of the row spectra rowsc [zb][ntheta][n/2+1]
     void adjoint_rows(const float2 *rowsc, float *u, float tau) {
         const int nimg = zb * m;
+        if (gd.dirs) {  // Hermitian half planes in the vector layout
+            launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
+            if (pad_fft) {
+                launch_pad_fft_inv_accum_vec(spec, u, zb, tau, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+                return;
+            }
+            for (int z = 0; z < zb; z += vec_slices) {
+                const int nzg = std::min(vec_slices, zb - z);
+                launch_vec_to_planar(spec, planar, z, nzg, ug, stream);
+                CUFFT_CHECK(cufftExecC2R(plan[kVecC2R], reinterpret_cast<cufftComplex *>(planar),
+                                         reinterpret_cast<cufftReal *>(planar)));
+                launch_crop_accum_real(reinterpret_cast<const float *>(planar), u + (long long)z * slab, nzg, tau,
+                                       gd.deapod, 2 * (n + 2), ug, stream);
+            }
+            return;
+        }
         if (gd.tc_scatter) {
             // Re IFFT2 of the scattered grids as a C2R of their Hermitian part,
             // which the tensor-core scatter adds into zeroed half planes
             const long long img_half = (long long)ug.P * ug.hpitch;
-            // (the direction path clears them inside k_adj_mix)
-            if (!gd.dirs) CUDA_CHECK(cudaMemsetAsync(spec, 0, sizeof(float2) * (size_t)nimg * img_half, stream));
+            CUDA_CHECK(cudaMemsetAsync(spec, 0, sizeof(float2) * (size_t)nimg * img_half, stream));
             launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
             if (pad_fft) {
                 launch_pad_fft_inv_accum(spec, u, zb, tau, gd.deapod, fft_tw, fft_inv_map, gd.err, ug, stream);
@@ -818,7 +831,7 @@ struct Handle {
                 cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * img_half);
                 CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], p, reinterpret_cast<cufftReal *>(p)));
             }
-            launch_crop_accum_real(reinterpret_cast<const float *>(spec), u, zb, tau, gd.deapod, ug, stream);
+            launch_crop_accum_real(reinterpret_cast<const float *>(spec), u, zb, tau, gd.deapod, ug.P + 2, ug, stream);
             return;
         }
         if (lay.img_spec < (long long)ug.P * ug.P)
@@ -1165,10 +1178,10 @@ struct Handle {
         const int fwd_f = (pad_fft ? 0 : (gd.dirs ? vcalls : f2)) + (fused_rows ? 0 : 1);
         // adjoint: [row preparation], the zeroing of split tiles (direct scatter),
         // one scatter per group, then [columns + rows | crop]
+        // (direction path: mixing and scatter per group, the fold of the border)
         const int adj_k = (fused_rows ? 0 : 1) + ((!gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
-                          ng * (gd.dirs ? 2 : 1) +
-                          (own2d ? 2 : 1);
-        const int adj_f = (fused_rows ? 0 : 1) + (own2d ? 0 : f2);
+                          (gd.dirs ? 2 * ng + 1 : ng) + (own2d ? 2 : (gd.dirs ? 2 * vcalls : 1));
+        const int adj_f = (fused_rows ? 0 : 1) + (own2d ? 0 : (gd.dirs ? vcalls : f2));
         // per outer iteration: titer inner steps per batch (forward, graddiv,
         // adjoint), one shrink per batch, the two-stage rho reduction
         *kern = titer * nbatch * (fwd_k + 1 + adj_k) + nbatch + 2;
@@ -1244,8 +1257,12 @@ struct Handle {
                                    nchunks, tv, stream);
                     break;
                 case 5:  // padded-grid inverse FFT (columns + rows), added into the scratch iterate
-                    launch_pad_fft_inv_accum(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, fft_inv_map, gd.err,
-                                             ug, stream);
+                    if (gd.dirs)
+                        launch_pad_fft_inv_accum_vec(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, vec_fft_map,
+                                                     gd.err, ug, stream);
+                    else
+                        launch_pad_fft_inv_accum(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, fft_inv_map,
+                                                 gd.err, ug, stream);
                     break;
                 default: throw Error(RECTV_ERR_ARG, "rectv_launch_kernel: unknown kernel id");
             }

@@ -212,7 +212,9 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, i
 bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, double tol_cells, double min_group,
                     DirPlan &dp) {
     dp = DirPlan();
-    if (n % 2) return false;  // sample k of a ray mirrors sample n - k for an even detector width only
+    // sample k of a ray mirrors sample n - k for an even detector width only (and the border cells that
+    // fold into each other must be distinct)
+    if (n % 2 || n < 32) return false;
     const double pi = 3.14159265358979323846;
     const double tol = tol_cells / (double)n;
     std::vector<double> alpha(ntheta);
@@ -263,68 +265,81 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
     dp.ndir = (int)dp.sincos.size();
     if ((double)ntheta < min_group * dp.ndir || dp.ndir >= 65536) return false;
 
-    // positions (d, q), 1 <= q < n: the same float sequence as the kernels
-    // (sample_pos), binned by the tile of the stencil origin (forward) and by
-    // every tile the stencil touches (adjoint), direction-major inside a tile
-    const int P = 2 * n;
-    const int NT = (P + T - 1) / T;
-    const int ntiles = NT * NT;
+    // position pairs (d, q), 1 <= q <= n/2 (sample n - q is the mirror image):
+    // the same float sequence as the kernels (sample_pos), binned by the tile
+    // of the stencil origin (forward) and by every tile of the vector layout's
+    // window that the pair's joint 10x10 cells touch (adjoint; the window
+    // starts kVH cells before cell 0, so they never leave it), direction-major
+    // inside a tile
+    const int P = 2 * n, nh = n / 2;
+    const int NT = (P + T - 1) / T, WX = (n + 1 + 2 * kVH + T - 1) / T, WY = (P + 2 * kVH + T - 1) / T;
+    const int ntiles = NT * NT, nwin = WX * WY;
     const float tn = (float)(2 * n);
     std::vector<float> qk(n);
     for (int k = 1; k < n; ++k) qk[k] = (float)(k - n / 2) / (float)n;
-    const long long npos = (long long)dp.ndir * (n - 1);
+    const long long npos = (long long)dp.ndir * nh;
     std::vector<int> ftile(npos);
     std::vector<int4> atiles(npos);
-    std::vector<long long> fcnt(ntiles + 1, 0), acnt(ntiles + 1, 0);
+    std::vector<long long> fcnt(ntiles + 1, 0), acnt(nwin + 1, 0);
     long long ip = 0;
     for (int d = 0; d < dp.ndir; ++d) {
         const float s = dp.sincos[d].x, c = dp.sincos[d].y;
-        for (int q = 1; q < n; ++q, ++ip) {
+        for (int q = 1; q <= nh; ++q, ++ip) {
             float x0 = qk[q] * s, y0 = qk[q] * c;
             if (x0 >= 0.5f) x0 = 0.5f - 1e-5f;
             if (y0 >= 0.5f) y0 = 0.5f - 1e-5f;
             const int KX = n + (int)std::floor(tn * x0), KY = n + (int)std::floor(tn * y0);
             ftile[ip] = (KY / T) * NT + (KX / T);
-            if (q <= n / 2) fcnt[ftile[ip]]++;  // the pair (q, n - q) is gathered at q
-            const int xa = wrapi(KX - kR, P) / T, xb = wrapi(KX + kR, P) / T;
-            const int ya = wrapi(KY - kR, P) / T, yb = wrapi(KY + kR, P) / T;
+            fcnt[ftile[ip]]++;
+            const int xa = (KX - kR + kVH) / T, xb = (KX + kR + 1 + kVH) / T;
+            const int ya = (KY - kR + kVH) / T, yb = (KY + kR + 1 + kVH) / T;
             const int nx = (xa == xb) ? 1 : 2, ny = (ya == yb) ? 1 : 2;
             const int xs[2] = {xa, xb}, ys[2] = {ya, yb};
             int tl[4] = {-1, -1, -1, -1}, nt = 0;
             for (int a = 0; a < ny; ++a)
-                for (int b = 0; b < nx; ++b) tl[nt++] = ys[a] * NT + xs[b];
+                for (int b = 0; b < nx; ++b) tl[nt++] = ys[a] * WX + xs[b];
             atiles[ip] = make_int4(tl[0], tl[1], tl[2], tl[3]);
             for (int i = 0; i < nt; ++i) acnt[tl[i]]++;
         }
     }
-    std::vector<long long> foff(ntiles + 1, 0), aoff(ntiles + 1, 0);
-    for (int t = 0; t < ntiles; ++t) {
-        foff[t + 1] = foff[t] + fcnt[t];
-        aoff[t + 1] = aoff[t] + acnt[t];
-    }
+    std::vector<long long> foff(ntiles + 1, 0), aoff(nwin + 1, 0);
+    for (int t = 0; t < ntiles; ++t) foff[t + 1] = foff[t] + fcnt[t];
+    for (int t = 0; t < nwin; ++t) aoff[t + 1] = aoff[t] + acnt[t];
     dp.fwd_pos.resize(foff[ntiles]);
-    dp.adj_pos.resize(aoff[ntiles]);
+    dp.adj_pos.resize(aoff[nwin]);
     {
         std::vector<long long> fp(foff.begin(), foff.end() - 1), ap(aoff.begin(), aoff.end() - 1);
-        ip = 0;
-        for (int d = 0; d < dp.ndir; ++d)
-            for (int q = 1; q < n; ++q, ++ip) {
-                const uint32_t id = (uint32_t)d * (uint32_t)n + (uint32_t)q;
-                if (q <= n / 2) dp.fwd_pos[fp[ftile[ip]]++] = (uint32_t)d * (uint32_t)(n / 2) + (uint32_t)(q - 1);
-                const int4 a = atiles[ip];
-                const int tl[4] = {a.x, a.y, a.z, a.w};
-                for (int i = 0; i < 4; ++i)
-                    if (tl[i] >= 0) dp.adj_pos[ap[tl[i]]++] = id;
-            }
+        for (ip = 0; ip < npos; ++ip) {  // id = d nh + q - 1
+            dp.fwd_pos[fp[ftile[ip]]++] = (uint32_t)ip;
+            const int4 a = atiles[ip];
+            const int tl[4] = {a.x, a.y, a.z, a.w};
+            for (int i = 0; i < 4; ++i)
+                if (tl[i] >= 0) dp.adj_pos[ap[tl[i]]++] = (uint32_t)ip;
+        }
     }
     for (int t = 0; t < ntiles; ++t)
         for (long long i = foff[t]; i < foff[t + 1]; i += fwd_cap)
             dp.fwd_items.push_back(make_int4(t, (int)i, (int)std::min<long long>(fwd_cap, foff[t + 1] - i), 0));
-    for (int t = 0; t < ntiles; ++t) dp.adj_items.push_back(make_int4(t, (int)aoff[t], (int)acnt[t], 0));
-    // heaviest tiles first (the empty ones last)
-    std::stable_sort(dp.adj_items.begin(), dp.adj_items.end(),
-                     [](const int4 &a, const int4 &b) { return a.z > b.z; });
+    for (int t = 0; t < nwin; ++t) dp.adj_items.push_back(make_int4(t, (int)aoff[t], (int)acnt[t], 0));
     return true;
+}
+
+// A tile's planes are split so that a block has about an eighth of a wave's
+// share of the work (the tiles at the centre of the spectrum hold thousands of
+// pairs, the others tens), but no block has fewer than 256 pairs x planes.
+std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz) {
+    constexpr long long kBlocks = 304;  // resident blocks: two per SM
+    long long total = 0;
+    for (const int4 &t : tiles) total += (long long)t.z * npz;
+    const long long budget = std::max<long long>(256, total / (8 * kBlocks));
+    std::vector<int4> work;
+    for (const int4 &t : tiles) {
+        const int per = (int)std::max<long long>(1, std::min<long long>(npz, budget / std::max(1, t.z)));
+        for (int p = 0; p < npz; p += per) work.push_back(make_int4(t.x, t.y, t.z, p | std::min(npz, p + per) << 16));
+    }
+    auto cost = [](const int4 &a) { return (long long)a.z * ((a.w >> 16) - (a.w & 0xffff)); };
+    std::stable_sort(work.begin(), work.end(), [&](const int4 &a, const int4 &b) { return cost(a) > cost(b); });
+    return work;
 }
 
 }  // namespace rectv

@@ -67,7 +67,7 @@ struct UsGeo {
     // scatter (0: one per SM)
     int zper;
     int sc_grid;
-    // Vector layout of the direction path (dir_kernels.cu): the spectra of 16
+    // Vector layout of the direction path (scatter_dir.cu): the spectra of 16
     // (slice, time sample) pairs are stored together, cell by cell:
     // [plane][row][column][16] complex over the window rows [-kVH, P + kVH) x
     // columns [-kVH, n + kVH] of the half plane.  One plane holds tg time
@@ -135,16 +135,16 @@ struct GeoDev {
     int *adj_tab_base = nullptr;
     uint32_t *adj_info = nullptr;
     int n_adj_tabs = 0;
-    // direction path (dir_kernels.cu, DirPlan): sincos then holds one
-    // (sin, cos) per direction, adj_pts / adj_items / adj_recs / adj_tabs the
-    // direction positions' adjoint entries (ray index := direction index)
+    // direction path (gather_dir.cu, scatter_dir.cu, DirPlan): sincos then holds
+    // one (sin, cos) per direction, adj_pts / adj_items the position pairs
+    // touching each 16x16 tile of the window
     bool dirs = false;
     int ndir = 0;
     int *dray_start = nullptr;    // [ndir + 1]
     uint32_t *drays = nullptr;    // theta | opposite << 31
     float *dtau = nullptr;        // per ray: offset across the direction (DirPlan::tau)
     float2 *dkmat = nullptr;      // K' in the order of drays, [ray][max(tg, 16 jg)], zero past m
-    float4 *demix = nullptr;      // adjoint E, E_perp per (slice, position): dir_mix_bytes(demix_slices, ndir, n)
+    float4 *demix = nullptr;      // the adjoint's mixed rays per (plane, position pair): dir_mix_bytes
     int demix_slices = 0;
     uint32_t *dfwd_pos = nullptr; // position pairs d*(n/2) + q - 1 sorted by origin tile
     int4 *dfwd_items = nullptr;   // (tile, start, count, 0)
@@ -169,7 +169,7 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, i
 
 // Rays grouped by direction (theta modulo pi), for scans that revisit their
 // angles over several half-turns: the rays of one direction sample the same
-// positions, so the USFFT interpolates once per position (dir_kernels.cu).
+// positions, so the USFFT interpolates once per position (scatter_dir.cu).
 struct DirPlan {
     int ndir = 0;
     std::vector<float2> sincos;     // [ndir] (sin, cos) of each direction's representative ray
@@ -179,8 +179,8 @@ struct DirPlan {
                                     // grid cells per unit of (q - n/2)/n
     std::vector<uint32_t> fwd_pos;  // position pairs d*(n/2) + q - 1 (1 <= q <= n/2) sorted by the tile of the stencil origin
     std::vector<int4> fwd_items;    // (tile, start, count, 0): at most fwd_cap positions of one tile
-    std::vector<uint32_t> adj_pos;  // one entry per tile a position's stencil touches
-    std::vector<int4> adj_items;    // (tile, start, count, 0), one per tile, busiest first
+    std::vector<uint32_t> adj_pos;  // pairs, one entry per tile of the vector layout's window their cells touch
+    std::vector<int4> adj_items;    // (tile, start, count, 0), one per tile
 };
 // Defaults of the direction path: rays are grouped when their samples agree
 // within kDirTolCells grid cells, and the path is taken when the rays average
@@ -198,12 +198,6 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
 // 2w+1 of the tile (lo | hi << 16), then the first row of every ray and the
 // table size as 16-bit values; padded to 16 bytes.
 __host__ __device__ constexpr int adj_info_words(int nseg) { return (4 + 8 * nseg + (nseg + 2) / 2 + 3) & ~3; }
-// The direction path's form: [4 + 16 s + b] the rows [lo, hi) of direction s
-// whose stencils touch 4x4-cell block b of the tile (rows 4 (b >> 2) .. + 3,
-// columns 4 (b & 3) .. + 3).
-__host__ __device__ constexpr int dir_adj_info_words(int nseg) {
-    return (4 + 16 * nseg + (nseg + 2) / 2 + 3) & ~3;
-}
 
 // ---- USFFT kernel launchers (usfft_kernels.cu) ----
 void launch_deapod_pad(const float *u, float *spec, int nimg, const float *deapod, const UsGeo &g,
@@ -224,8 +218,9 @@ void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev 
 void launch_crop_accum(const float2 *spec, float *u, int zb, float tau, const float *deapod,
                        const UsGeo &g, cudaStream_t s);
 // the same from the real output of the C2R inverse (rows of 2 (P/2+1) floats)
-void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, const UsGeo &g,
-                            cudaStream_t s);
+// (rowf: floats per row, 2 (P/2+1), or 2 (n+2) on the direction path)
+void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, int rowf,
+                            const UsGeo &g, cudaStream_t s);
 // tensor-core gather (gather_tc.cu): items of fwd_tc_items, time samples
 // [jbase, jbase + 16)
 void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &tmap, int jbase,
@@ -247,34 +242,27 @@ int scatter_tc_batch_rays();  // rays per tensor-core batch
 int scatter_tc_info_words(int nseg);
 // fill adj_info from the records (after launch_adj_records)
 void launch_adj_tabinfo(const GeoDev &gd, cudaStream_t s);
-// direction path (dir_kernels.cu): forward rows of all rays from the
-// positions' interpolated spectra (time samples [jbase, jbase + 16),
-// accumulated into rows when accumulate != 0), and the adjoint scatter into
-// the zeroed Hermitian half planes (as launch_scatter_tc)
+// direction path (gather_dir.cu, scatter_dir.cu): the Hermitian half rows
+// [z][theta][n/2+1] of all rays from the spectra in the vector layout, and the
+// adjoint: half rows into the Hermitian half planes in the vector layout
 void launch_gather_dir(float2 *hrows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &vmap,
                        cudaStream_t s);
+void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
 // TMA descriptor of the gather's footprints in the vector layout (npl planes)
 void make_vec_gather_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
 // fills the halo of the forward spectra in the vector layout
 void launch_vec_halo(float2 *spec, int npl, const UsGeo &g, cudaStream_t s);
 // cuFFT's spectra of slices z0 .. z0 + nz - 1 (planar, rows of n + 2 complex,
-// image (z - z0) m + t) into the vector layout
+// image (z - z0) m + t) into the vector layout, and back
 void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, const UsGeo &g, cudaStream_t s);
-void gather_dir_prepare();
-void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
-                        cudaStream_t s);
-// geometry records of the direction path's adjoint entries (as
-// launch_adj_records, with sf = (A, Bx), k = float bits of By: the first-order
-// weight of entry p at tile cell (cx, cy) is w (A + B . (cx, cy)),
-// B = c1/(2n) (cos, -sin) of the direction, c1 = 2 pi^2/mu / (2n))
-void launch_adj_records_dir(AdjRec *recs, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
-// their segmentation (dir_adj_info_words per table)
-void launch_adj_tabinfo_dir(const GeoDev &gd, cudaStream_t s);
-void dir_prepare();           // kernel attributes; once, outside stream capture
-int dir_fwd_capacity();       // positions per forward item
-int dir_adj_table_capacity(); // entries per adjoint table
-int dir_adj_table_dirs();     // directions per adjoint table
-size_t dir_mix_bytes(int zb, int ndir, int n);  // the adjoint's per-position mixing buffer
+void launch_vec_to_planar(const float2 *spec, float2 *planar, int z0, int nz, const UsGeo &g, cudaStream_t s);
+void gather_dir_prepare();    // kernel attributes; once, outside stream capture
+void scatter_dir_prepare();
+int dir_fwd_capacity();       // position pairs per forward item
+// work items of the adjoint over npz planes: (tile, start, count, first plane |
+// end plane << 16) of a plan's (tile, start, count), the most work first
+std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz);
+size_t dir_mix_bytes(const UsGeo &g, int zb, int ndir);  // the adjoint's per-position mixing buffer
 // hand-written 2D FFTs of the zero-padded grids (fft_kernels.cu), P = 2n a
 // power of two in [256, 2048]: forward = deapodise/pad/modulate + R2C into
 // the halo-padded spectra (halo not filled); inverse = C2R of the Hermitian
@@ -292,6 +280,9 @@ void launch_pad_fft_fwd_vec(const float *u, float2 *spec, int zb, const float *d
                             const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
+// the same from half planes in the vector layout (make_vec_fft_map)
+void launch_pad_fft_inv_accum_vec(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
+                                  const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 // fused residual rows of the inner step (fft_kernels.cu), n a power of two in
 // [256, 1024]: gathered rows [z][theta][n] and data g -> the adjoint's row
 // spectra [z][theta][n/2+1] (inverse row FFT, residual, fftshift, R2C)

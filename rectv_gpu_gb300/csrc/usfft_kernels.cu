@@ -667,8 +667,8 @@ static void scatter_adj_t(const float2 *rowsc, float2 *spec, int zb, const GeoDe
 void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
                         const UsGeo &g, cudaStream_t s) {
     if (g.T != 16) throw Error(1, "tile size must be 16");
-    if (gd.dirs) {  // rays grouped by direction, into the Hermitian half planes (dir_kernels.cu)
-        for (int jb = 0; jb < g.m; jb += 16) launch_scatter_dir(rowsc, spec, zb, gd, g, jb, s);
+    if (gd.dirs) {  // rays grouped by direction, into the vector layout's half planes (scatter_dir.cu)
+        launch_scatter_dir(rowsc, spec, zb, gd, g, s);
         return;
     }
     const int mp = mp_for(g.m);
@@ -716,26 +716,26 @@ void launch_crop_accum(const float2 *spec, float *u, int zb, float tau, const fl
 }
 
 // Same epilogue after the C2R inverse of the Hermitian half planes: real
-// images with rows of 2 (P/2+1) floats.
+// images with rows of rowf floats.
 __global__ void k_crop_accum_real(const float *__restrict__ out, float *__restrict__ u,
-                                  const float *__restrict__ dp, int n, int P, long long img_real, float c) {
+                                  const float *__restrict__ dp, int n, int rowf, long long img_real, float c) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
     const long long img = blockIdx.z;
     if (x >= n) return;
     const int X = x + n / 2, Y = y + n / 2;
-    float v = out[img * img_real + (long long)Y * (P + 2) + X];
+    float v = out[img * img_real + (long long)Y * rowf + X];
     v = ((X + Y) & 1) ? -v : v;
     u[(img * n + y) * n + x] += c * v * dp[x] * dp[y];
 }
 
-void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, const UsGeo &g,
-                            cudaStream_t s) {
+void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, int rowf,
+                            const UsGeo &g, cudaStream_t s) {
     dim3 gs((g.n + 255) / 256, g.n, zb * g.m);
     const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
     const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
-    const long long img_real = 2LL * g.P * (g.P / 2 + 1);
-    k_crop_accum_real<<<gs, 256, 0, s>>>(out, u, deapod, g.n, g.P, img_real, c);
+    const long long img_real = (long long)g.P * rowf;
+    k_crop_accum_real<<<gs, 256, 0, s>>>(out, u, deapod, g.n, rowf, img_real, c);
     LAUNCH_CHECK("k_crop_accum_real");
 }
 

@@ -326,18 +326,25 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
 
 // A tile's planes are split so that a block has about an eighth of a wave's
 // share of the work (the tiles at the centre of the spectrum hold thousands of
-// pairs, the others tens), but no block has fewer than 256 pairs x planes.
+// pairs, the others tens), but no block has fewer than 256 pairs x planes.  A
+// tile with more than half a resident block's whole share of the work (small
+// problems: few tiles, most of them dense) goes to four blocks per plane, one
+// per four rows (item.x = 5 tile + 1 + row group; 5 tile for whole tiles).
 std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz) {
-    constexpr long long kBlocks = 304;  // resident blocks: two per SM
+    constexpr long long kBlocks = 456;  // resident blocks: three per SM
     long long total = 0;
     for (const int4 &t : tiles) total += (long long)t.z * npz;
-    const long long budget = std::max<long long>(256, total / (8 * kBlocks));
+    const long long budget = std::max<long long>(256, total / (8 * kBlocks)), share = total / kBlocks;
     std::vector<int4> work;
     for (const int4 &t : tiles) {
-        const int per = (int)std::max<long long>(1, std::min<long long>(npz, budget / std::max(1, t.z)));
-        for (int p = 0; p < npz; p += per) work.push_back(make_int4(t.x, t.y, t.z, p | std::min(npz, p + per) << 16));
+        const bool split = t.z >= 32 && 2LL * t.z > share;
+        const int per =
+            split ? 1 : (int)std::max<long long>(1, std::min<long long>(npz, budget / std::max(1, t.z)));
+        for (int p = 0; p < npz; p += per)
+            for (int r = 0; r < (split ? 4 : 1); ++r)
+                work.push_back(make_int4(5 * t.x + (split ? 1 + r : 0), t.y, t.z, p | std::min(npz, p + per) << 16));
     }
-    auto cost = [](const int4 &a) { return (long long)a.z * ((a.w >> 16) - (a.w & 0xffff)); };
+    auto cost = [](const int4 &a) { return (long long)a.z * ((a.w >> 16) - (a.w & 0xffff)) * (a.x % 5 ? 1 : 4); };
     std::stable_sort(work.begin(), work.end(), [&](const int4 &a, const int4 &b) { return cost(a) > cost(b); });
     return work;
 }

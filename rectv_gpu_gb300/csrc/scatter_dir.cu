@@ -72,21 +72,26 @@ constexpr int kVec = 24;      // float4 per position pair: M0, M0perp, M2 of 16 
 // ---- mixing ----
 constexpr int kMThr = 256;    // 32 position pairs x 8 lanes
 constexpr int kMFly = 8;      // rays in flight per thread
+constexpr int kMRays = 64;    // rays of a direction in shared memory
 
 // ---- scatter ----
 constexpr int kSWarps = 8;               // consumer warps; one more warp issues the copies
 constexpr int kSThr = 32 * (kSWarps + 1);
 constexpr int kSChunk = 32;              // entries per stage
-constexpr int kSStages = 4;
-constexpr int kSCap = 192;               // entries whose weights are held
+constexpr int kSStages = 3;
+constexpr int kSCap = 128;               // entries whose weights are held
+
+struct SEntry {
+    float wx[kT], wxd[kT];  // wx1 and its first-order weight over the tile's columns
+    float2 wy[kT];          // (y weight of the joint 10 taps, first-order weight) over the rows
+    float4 hd;              // first column and row of the joint window (int bits), wx2 - wx1 at its columns 0, 9
+};
 
 struct ScatSmem {
     float4 m[kSStages][kSChunk][kVec];   // the entries' M0, M0perp, M2 (bulk copies)
-    float wx[kSCap][kT], wxd[kSCap][kT]; // wx1 and its first-order weight over the tile's columns
-    float2 wy[kSCap][kT];                // (y weight of the joint 10 taps, first-order weight) over the rows
-    float4 hd[kSCap];                    // first column and row of the joint window (int bits), wx2 - wx1 at its columns 0, 9
+    SEntry ent[kSCap];
     uint32_t id[kSCap];
-    uint32_t mask[kSCap / kSChunk][kSWarps];  // entries of a chunk whose window touches a warp's cells
+    uint32_t mask[kSCap / kSChunk][8];   // entries of a chunk whose window touches a pair of rows
     unsigned long long full[kSStages], empty[kSStages];
 };
 
@@ -98,99 +103,138 @@ __device__ __forceinline__ float2 mul2(float w, float2 a) { return make_float2(w
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Adjoint, step 1: M0, M0perp, M2 of every position pair and plane.  Eight
-// lanes per pair, two of the plane's 16 values each: a pair's 384 bytes leave
-// as three full 128-byte lines.  The row values of eight rays are in flight
-// per thread.  Out: emix[((pl ndir + d) n/2 + q - 1)][3][8] float4.
-// Writes 1.13 GB at n = 1024, 360 directions, 16 slices: 0.92 ms a launch
-// (1.46 ms for the kernel that mixed every position and cleared the half
-// planes): bound by the latency of the ray -> row load chain.
+// Adjoint, step 1: M0, M0perp, M2 of every position pair and plane.  One block
+// per (32 pairs of a direction, planes); eight lanes per pair, two of the
+// plane's 16 values each, so that a pair's 384 bytes leave as three full
+// 128-byte lines.  The direction's rays (index, offset, K' rows) sit in shared
+// memory for all planes of the block; a thread has the row values of eight
+// rays in flight.
+// Writes 1.13 GB at n = 1024, 360 directions, 16 slices: 0.45 ms a launch
+// (0.92 ms with one plane per block, where every block waits through the chain
+// of loads from the ray index to the row).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kMThr)
     k_adj_mix(float4 *__restrict__ emix, const float2 *__restrict__ rowsc, const int *__restrict__ ray_start,
               const uint32_t *__restrict__ rays, const float *__restrict__ tau, const float2 *__restrict__ dkmat,
-              const float2 *__restrict__ shifta, UsGeo g, int zb, int ndir, int jgrp, int kstride) {
+              const float2 *__restrict__ shifta, UsGeo g, int zb, int ndir, int npz, int per, int jgrp, int kstride) {
+    __shared__ float4 ks[kMRays][8];   // K' of the plane's 16 values
+    __shared__ uint32_t rvs[kMRays];
+    __shared__ float tvs[kMRays];
     const int nh = g.n / 2, hn = nh + 1;
     const int ci = threadIdx.x & 7;
-    const int q = 1 + blockIdx.x * (kMThr / 8) + (threadIdx.x >> 3), d = blockIdx.y, pz = blockIdx.z;
-    if (q > nh) return;
-    const int z0 = g.jg > 1 ? pz : pz * g.zs + (2 * ci) / g.tg;
-    const int z1 = g.jg > 1 ? pz : pz * g.zs + (2 * ci + 1) / g.tg;
-    const bool two = z1 != z0;  // one time sample: the two values are two slices
-    const int j0 = 16 * jgrp + ((2 * ci) & (g.tg - 1));
+    const int d = blockIdx.y, q = min(nh, 1 + (int)blockIdx.x * (kMThr / 8) + (int)(threadIdx.x >> 3));
+    const bool live = 1 + (int)blockIdx.x * (kMThr / 8) + (int)(threadIdx.x >> 3) <= nh;
+    const int p0 = blockIdx.z * per, p1 = min(npz, p0 + per);
     const int rs = __ldg(ray_start + d), nr = __ldg(ray_start + d + 1) - rs;
     const float qp = __fdiv_rn((float)(q - nh), (float)g.n);
     const float2 sh = __ldg(shifta + q);
     const float cf = ((q & 1) ? g.cw : -g.cw) * (q == nh ? 0.5f : 1.f);  // the pair q = n/2 is one position
     const float2 fk = make_float2(sh.x * cf, sh.y * cf);
-    float2 a0 = dup(0.f), a1 = a0, p0 = a0, p1 = a0, i0 = a0, i1 = a0;  // sum h v, sum delta h v, sum g v (K' = h + i g)
-    for (int r0 = 0; r0 < nr; r0 += kMFly) {
-        float2 R0[kMFly], R1[kMFly];
-#pragma unroll
-        for (int i = 0; i < kMFly; ++i) {
-            R0[i] = R1[i] = dup(0.f);
-            if (r0 + i < nr) {
-                const uint32_t rv = __ldg(rays + rs + r0 + i);
-                const long long th = rv & 0x7fffffffu;
-                if (z0 < zb) R0[i] = __ldg(rowsc + ((long long)z0 * g.ntheta + th) * hn + q);
-                if (two && z1 < zb) R1[i] = __ldg(rowsc + ((long long)z1 * g.ntheta + th) * hn + q);
+    const int s0 = g.jg > 1 ? 0 : (2 * ci) / g.tg;  // slice of this lane's first value
+    const bool two = g.tg == 1;  // one time sample: the two values are two slices
+    for (int r0 = 0; r0 < nr; r0 += kMRays) {
+        const int nc = min(kMRays, nr - r0);
+        if (r0 > 0) __syncthreads();
+        for (int i = threadIdx.x; i < nc * 8; i += kMThr) {
+            const int r = i >> 3, c = i & 7;
+            const float2 *k = dkmat + (long long)(rs + r0 + r) * kstride + 16 * jgrp + ((2 * c) & (g.tg - 1));
+            if (two) {
+                const float2 k1 = __ldg(k);
+                ks[r][c] = make_float4(k1.x, k1.y, k1.x, k1.y);
+            } else {
+                ks[r][c] = __ldg(reinterpret_cast<const float4 *>(k));
+            }
+            if (c == 0) {
+                rvs[r] = __ldg(rays + rs + r0 + r);
+                tvs[r] = __ldg(tau + rs + r0 + r);
             }
         }
+        __syncthreads();
+        for (int pz = p0; pz < p1; ++pz) {
+            const int z0 = g.jg > 1 ? pz : pz * g.zs + s0;
+            const bool ok0 = live && z0 < zb, ok1 = two && live && z0 + 1 < zb;
+            const float2 *row = rowsc + (long long)z0 * g.ntheta * hn + q;
+            float4 *o = emix + (((long long)pz * ndir + d) * nh + q - 1) * kVec + ci;
+            // sums of h v, delta h v, g v (K' = h + i g); a later chunk of rays adds to the stored ones
+            float2 a0 = dup(0.f), a1 = a0, e0 = a0, e1 = a0, i0 = a0, i1 = a0;
+            if (r0 > 0 && live) {
+                const float4 A = o[0], P = o[8], M = o[16];
+                a0 = lo2(A), a1 = hi2(A), e0 = lo2(P), e1 = hi2(P);
+                i0 = make_float2(2.f * M.y - A.y, A.x - 2.f * M.x);
+                i1 = make_float2(2.f * M.w - A.w, A.z - 2.f * M.z);
+            }
+            for (int rb = 0; rb < nc; rb += kMFly) {
+                float2 R0[kMFly], R1[kMFly];
 #pragma unroll
-        for (int i = 0; i < kMFly; ++i) {
-            if (r0 + i >= nr) break;
-            const int r = rs + r0 + i;
-            const uint32_t rv = __ldg(rays + r);
-            const float dl = qp * __ldg(tau + r);  // this ray's offset across the direction
-            float4 k;
-            if (g.tg == 1) {
-                const float2 k1 = __ldg(dkmat + (long long)r * kstride + j0);
-                k = make_float4(k1.x, k1.y, k1.x, k1.y);
-            } else {
-                k = __ldg(reinterpret_cast<const float4 *>(dkmat + (long long)r * kstride + j0));
+                for (int i = 0; i < kMFly; ++i) {
+                    R0[i] = R1[i] = dup(0.f);
+                    if (rb + i < nc) {
+                        const long long off = (long long)(rvs[rb + i] & 0x7fffffffu) * hn;
+                        if (ok0) R0[i] = __ldg(row + off);
+                        if (ok1) R1[i] = __ldg(row + off + (long long)g.ntheta * hn);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < kMFly; ++i) {
+                    if (rb + i >= nc) break;
+                    const float dl = qp * tvs[rb + i];  // this ray's offset across the direction
+                    const float4 k = ks[rb + i][ci];
+                    float2 v = cmul(R0[i], fk), w = v;
+                    if (two) w = cmul(R1[i], fk);
+                    if (rvs[rb + i] >> 31) {
+                        v.y = -v.y;
+                        w.y = -w.y;
+                    }
+                    const float2 hv = mul2(k.x, v), hw = mul2(k.z, w);
+                    a0.x += hv.x;
+                    a0.y += hv.y;
+                    a1.x += hw.x;
+                    a1.y += hw.y;
+                    e0 = ffma2(dup(dl), hv, e0);
+                    e1 = ffma2(dup(dl), hw, e1);
+                    i0 = ffma2(dup(k.y), v, i0);
+                    i1 = ffma2(dup(k.w), w, i1);
+                }
             }
-            float2 v = cmul(R0[i], fk), w = two ? cmul(R1[i], fk) : v;
-            if (rv >> 31) {
-                v.y = -v.y;
-                w.y = -w.y;
+            if (live) {
+                o[0] = make_float4(a0.x, a0.y, a1.x, a1.y);
+                o[8] = make_float4(e0.x, e0.y, e1.x, e1.y);
+                o[16] = make_float4(0.5f * (a0.x - i0.y), 0.5f * (a0.y + i0.x), 0.5f * (a1.x - i1.y), 0.5f * (a1.y + i1.x));
             }
-            const float2 hv = mul2(k.x, v), hw = mul2(k.z, w);
-            a0.x += hv.x;
-            a0.y += hv.y;
-            a1.x += hw.x;
-            a1.y += hw.y;
-            p0 = ffma2(dup(dl), hv, p0);
-            p1 = ffma2(dup(dl), hw, p1);
-            i0 = ffma2(dup(k.y), v, i0);
-            i1 = ffma2(dup(k.w), w, i1);
         }
     }
-    float4 *o = emix + (((long long)pz * ndir + d) * nh + q - 1) * kVec + ci;
-    o[0] = make_float4(a0.x, a0.y, a1.x, a1.y);
-    o[8] = make_float4(p0.x, p0.y, p1.x, p1.y);
-    o[16] = make_float4(0.5f * (a0.x - i0.y), 0.5f * (a0.y + i0.x), 0.5f * (a1.x - i1.y), 0.5f * (a1.y + i1.x));
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint, step 2: one block (eight consumer warps and a copy warp, two
-// blocks per SM) per (16x16 tile of the window, planes), the most work
-// first.  The entries of a tile are the position pairs whose joint 10x10
-// window touches it; their weights over the tile's columns and rows are
-// computed once per block (per plane in the few tiles of more than 192
-// entries).  Per plane the copy warp streams the entries' M0, M0perp, M2 (one
-// 384-byte bulk copy each) through four stages of 32 entries; a warp owns 4
-// rows x 8 columns of the tile and walks the entries that touch them, its
-// lane (row, ci) two of the 16 values of the row's 8 cells:
+// Adjoint, step 2: one block (eight consumer warps and a copy warp, three
+// blocks per SM) per (16x16 tile of the window, planes), the most work first.
+// The entries of a tile are the position pairs whose joint 10x10 window
+// touches it; the weights of up to 128 of them over the tile's columns and
+// rows are computed once for all planes of the block (a tile with more takes
+// them in turn and adds to its cells).  Per plane the copy warp streams the
+// entries' M0, M0perp, M2 (384 bytes each, one bulk copy per run of
+// consecutive samples) through three stages of 32 entries; a warp owns two
+// rows of the tile and walks the entries that touch them, its lane (row, v)
+// one of the 16 values of the row's 16 cells:
 //     U = wy1 M0 + wy1' M0perp + (wy2 - wy1) M2,  V = wy1 M0perp,
-//     cell += wx1 U + wx1' V,  and wy2 M2 (wx2 - wx1) at the window's edge columns.
-// So an entry costs a lane 3 16-byte loads of M for 8 cells.  Warps wait for
-// copies only, never for each other.  All sums run in entry order; the cells
-// leave as full 128-byte lines.  Measured at n = 1024, 360 directions, 16 time
-// samples, 16 slices: 3.7 ms a launch, against 6.4 ms for a scatter of every
-// position with float2 atomics into cleared half planes.  Bound by the latency
-// of the shared loads and FMA chains (issue 54 % active, FMA pipe 42 %).
+//     cell += wx1 U + wx1' V,  and wy2 M2 (wx2 - wx1) at the window's edge columns,
+// the left and the right eight cells each only if the window reaches them.
+// Warps wait for copies only, never for each other.  All sums run in entry
+// order; the cells leave as full 128-byte lines.
+// Split items (item.x % 5 > 0): a block has four rows of the tile, its warps
+// take every fourth entry each and add up at the end in warp order: four times
+// the blocks for problems whose tiles would leave SMs idle (dir_adj_work).
+// Measured at n = 1024, 360 directions, 16 time samples, 16 slices: 3.47 ms a
+// launch (a scatter of every position with float2 atomics into cleared half
+// planes: 6.4 ms).  Bound by instruction issue (59 % active; 105 instructions
+// per entry and row pair, 22 of them the packed FMAs of the cells) and the
+// latency of the shared loads.  Other splits of a tile measured: 4 rows x 8
+// columns per warp with two values per lane and 16 consumer warps per SM
+// 3.71 ms (3.95 ms with the next entry's loads in flight), 4 rows x 16
+// columns, 128 registers, 12 consumer warps per SM 3.85 ms: fewer
+// instructions, but too few warps to hide their latency.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kSThr, 2)
+__global__ void __launch_bounds__(kSThr, 3)
     k_scatter_dir(const float4 *__restrict__ emix, float4 *__restrict__ spec, const uint32_t *__restrict__ pos,
                   const int4 *__restrict__ items, const float2 *__restrict__ dsincos, UsGeo g, int ndir, int jgrp,
                   int *__restrict__ err) {
@@ -199,7 +243,8 @@ __global__ void __launch_bounds__(kSThr, 2)
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int4 it = items[blockIdx.x];
     const int ntx = (g.vp + kT - 1) / kT;
-    const int ty = it.x / ntx, Y0 = ty * kT, X0 = (it.x - ty * ntx) * kT;  // window cell (0, 0) of the tile
+    const int tile = it.x / 5, sub = it.x - 5 * tile;  // sub > 0: row group sub - 1 alone
+    const int ty = tile / ntx, Y0 = ty * kT, X0 = (tile - ty * ntx) * kT;  // window cell (0, 0) of the tile
     const int p0 = it.w & 0xffff, p1 = it.w >> 16;
     const int nh = g.n / 2, nseg = (it.z + kSCap - 1) / kSCap;
     const long long rowp = (long long)g.vp * 8, plane = (long long)g.vrows * rowp;  // float4
@@ -221,83 +266,74 @@ __global__ void __launch_bounds__(kSThr, 2)
         tc::fence_mbar_init();
     }
     const float c1 = 2.f * g.wexp / g.tn;  // d w / d position = c1 d w per grid cell
-    // weights and warp masks of entries [s0, s0 + cnt)
+    // weights and row masks of entries [s0, s0 + cnt): thread = (entry, axis)
     auto build = [&](int s0, int cnt) {
-        for (int i = tid; i < cnt * 32; i += kSThr) {
-            const int e = i >> 5, c = i & 15, ax = (i >> 4) & 1;
-            const uint32_t id = __ldg(pos + it.y + s0 + e);
-            const int d = id / (uint32_t)nh, q = id - d * nh + 1;
-            const float2 sc = __ldg(dsincos + d);
-            float x0, y0;
-            int fx, fy;
-            sample_pos(q, sc, g, x0, y0, fx, fy);
-            const float p = ax ? y0 : x0;
-            const int f = ax ? fy : fx;
-            const int d0 = g.n + f - kR + kVH - (ax ? Y0 : X0);  // first tap of the window in the tile
-            const float v = __fmul_rn(g.tn, p);
-            const bool mir = floorf(v) != v;  // the mirrored stencil starts one cell later
-            const int b = c - d0;
-            float w = 0.f, wd = 0.f;
-            if (b >= 0 && b <= kTaps) {
-                w = tap_weight(f, b, p, g);
-                if (b == kTaps) {
-                    if (!mir) w = 0.f;
-                } else {
-                    wd = (ax ? -sc.x : sc.y) * c1 * ((float)(f - kR + b) * g.inv2n - p) * w;
+        for (int i = tid; i < 2 * kSCap; i += kSThr) {
+            const int e = i & (kSCap - 1), ax = i / kSCap;  // a warp: 32 entries of one chunk, one axis
+            int d0 = 100;
+            if (e < cnt) {
+                const uint32_t id = __ldg(pos + it.y + s0 + e);
+                const int d = id / (uint32_t)nh, q = id - d * nh + 1;
+                const float2 sc = __ldg(dsincos + d);
+                float x0, y0;
+                int fx, fy;
+                sample_pos(q, sc, g, x0, y0, fx, fy);
+                const float p = ax ? y0 : x0, cd = (ax ? -sc.x : sc.y) * c1;
+                const int f = ax ? fy : fx;
+                d0 = g.n + f - kR + kVH - (ax ? Y0 : X0);  // first tap of the window in the tile
+                const float v = __fmul_rn(g.tn, p);
+                const bool mir = floorf(v) != v;  // the mirrored stencil starts one cell later
+                SEntry &en = sm.ent[e];
+                const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 *zero = reinterpret_cast<float4 *>(ax ? reinterpret_cast<float *>(en.wy) : en.wx);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) zero[k] = z4;
+#pragma unroll
+                for (int b = 0; b <= kTaps; ++b) {
+                    float w = tap_weight(f, b, p, g);
+                    if (b == kTaps && !mir) w = 0.f;
+                    const int c = d0 + b;
+                    const float wd = cd * ((float)(f - kR + b) * g.inv2n - p) * w;
+                    if (ax == 0 && b == 0) en.hd.z = mir ? -w : 0.f;
+                    if (ax == 0 && b == kTaps) en.hd.w = w;
+                    if (c < 0 || c >= kT) continue;
+                    if (ax) {
+                        en.wy[c] = make_float2(w, b < kTaps ? wd : 0.f);
+                    } else if (b < kTaps) {
+                        en.wx[c] = w;
+                        en.wxd[c] = wd;
+                    }
                 }
-            }
-            if (ax) {
-                sm.wy[e][c] = make_float2(w, wd);
-            } else {
-                sm.wx[e][c] = b < kTaps ? w : 0.f;
-                sm.wxd[e][c] = wd;
-            }
-            if (c == 0) {
-                float *h = reinterpret_cast<float *>(&sm.hd[e]);
                 if (ax) {
-                    h[1] = __int_as_float(mir ? d0 : -1000);  // rows 0 and 9 of the window differ only when mirrored
+                    en.hd.y = __int_as_float(mir ? d0 : -1000);  // rows 0 and 9 of the window differ only when mirrored
                 } else {
-                    h[0] = __int_as_float(d0);
-                    h[2] = mir ? -tap_weight(f, 0, p, g) : 0.f;
-                    h[3] = mir ? tap_weight(f, kTaps, p, g) : 0.f;
+                    en.hd.x = __int_as_float(d0);
                     sm.id[e] = id;
                 }
             }
-        }
-        if (wid < kSWarps) {
-            const int ry0 = 4 * (wid >> 1), cx0 = 8 * (wid & 1);
-            for (int ch = 0; ch * kSChunk < cnt; ++ch) {
-                const int e = ch * kSChunk + lane;
-                bool in = false;
-                if (e < cnt) {
-                    const uint32_t id = __ldg(pos + it.y + s0 + e);
-                    const int d = id / (uint32_t)nh, q = id - d * nh + 1;
-                    float x0, y0;
-                    int fx, fy;
-                    sample_pos(q, __ldg(dsincos + d), g, x0, y0, fx, fy);
-                    const int dx = g.n + fx - kR + kVH - X0, dy = g.n + fy - kR + kVH - Y0;
-                    in = dx + kTaps >= cx0 && dx < cx0 + 8 && dy + kTaps >= ry0 && dy < ry0 + 4;
+            if (ax && e - lane < cnt) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const uint32_t mk = __ballot_sync(0xffffffffu, d0 + kTaps >= 2 * r && d0 < 2 * r + 2);
+                    if (lane == 0) sm.mask[e / kSChunk][r] = mk;
                 }
-                const uint32_t mk = __ballot_sync(0xffffffffu, in);
-                if (lane == 0) sm.mask[ch][wid] = mk;
             }
         }
     };
-    const int ci = lane & 7, ry = 4 * (wid >> 1) + (lane >> 3), cx0 = 8 * (wid & 1);
-    float2 acc[8][2];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c][0] = acc[c][1] = dup(0.f);
+    const int rg = sub ? 2 * (sub - 1) + (wid & 1) : wid & 7;  // this warp's pair of rows
+    const uint32_t part = sub ? 0x11111111u << ((wid >> 1) & 3) : 0xffffffffu;
+    const int vi = lane & 15, ry = 2 * rg + (lane >> 4);
+    float2 acc[2][8];  // [re, im][cell pair]
     bool ok = true;
     int k = 0;  // stages issued (copy warp) or consumed
-    for (int pz = p0; pz < p1; ++pz) {
-        for (int seg = 0; seg < nseg; ++seg) {
-            const int s0 = seg * kSCap, cnt = min(kSCap, it.z - s0);
-            if (nseg > 1 || pz == p0) {
-                __syncthreads();  // the previous entries are done (and the barriers initialised)
-                build(s0, cnt);
-                __syncthreads();
-            }
-            const int nch = (cnt + kSChunk - 1) / kSChunk;
+    for (int seg = 0; seg < nseg; ++seg) {
+        const int s0 = seg * kSCap, cnt = min(kSCap, it.z - s0), nch = (cnt + kSChunk - 1) / kSChunk;
+        __syncthreads();  // the previous entries are done (and the barriers initialised)
+        build(s0, cnt);
+        __syncthreads();
+        for (int pz = p0; pz < p1; ++pz) {
+            float2 *dst = reinterpret_cast<float2 *>(spec + (long long)(pz * g.jg + jgrp) * plane +
+                                                     (long long)(Y0 + ry) * rowp + (long long)X0 * 8) + vi;
             if (wid == kSWarps) {
                 for (int ch = 0; ch < nch; ++ch, ++k) {
                     const int slot = k % kSStages, ne = min(kSChunk, cnt - ch * kSChunk);
@@ -308,88 +344,133 @@ __global__ void __launch_bounds__(kSThr, 2)
                                      "r"((uint32_t)(ne * kVec * sizeof(float4)))
                                      : "memory");
                     __syncwarp();
-                    if (lane < ne) {
-                        const float4 *src = emix + ((long long)pz * ndir * nh + sm.id[ch * kSChunk + lane]) * kVec;
+                    // runs of consecutive pairs (a direction's samples inside the tile) are contiguous: one copy each
+                    const uint32_t id = lane < ne ? sm.id[ch * kSChunk + lane] : 0u;
+                    const uint32_t before = __shfl_up_sync(0xffffffffu, id, 1);
+                    const bool first = lane < ne && (lane == 0 || id != before + 1);
+                    const uint32_t rest = __ballot_sync(0xffffffffu, first) & ~((2u << lane) - 1u);
+                    if (first) {
+                        const int len = (rest ? __ffs(rest) - 1 : ne) - lane;
+                        const float4 *src = emix + ((long long)pz * ndir * nh + id) * kVec;
                         asm volatile(
                             "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
                                 tc::smem_addr(sm.m[slot][lane])),
-                            "l"(src), "r"((uint32_t)(kVec * sizeof(float4))), "r"(bar)
+                            "l"(src), "r"((uint32_t)(len * kVec * sizeof(float4))), "r"(bar)
                             : "memory");
                     }
                 }
-                continue;
-            }
-            for (int ch = 0; ch < nch; ++ch, ++k) {
-                const int slot = k % kSStages;
-                ok = tc::mbar_wait(&sm.full[slot], (uint32_t)((k / kSStages) & 1), ok) && ok;
-                for (uint32_t mk = sm.mask[ch][wid]; mk; mk &= mk - 1) {
-                    const int el = __ffs(mk) - 1, e = ch * kSChunk + el;
-                    const float4 m0 = sm.m[slot][el][ci], mp = sm.m[slot][el][8 + ci], m2 = sm.m[slot][el][16 + ci];
-                    const float2 wy = sm.wy[e][ry];
-                    const float4 h = sm.hd[e];
-                    const float4 xa = *reinterpret_cast<const float4 *>(&sm.wx[e][cx0]),
-                                 xb = *reinterpret_cast<const float4 *>(&sm.wx[e][cx0 + 4]),
-                                 da = *reinterpret_cast<const float4 *>(&sm.wxd[e][cx0]),
-                                 db = *reinterpret_cast<const float4 *>(&sm.wxd[e][cx0 + 4]);
-                    const int a = ry - __float_as_int(h.y);
-                    const float w1 = a == kTaps ? 0.f : wy.x, w2 = a == 0 ? 0.f : wy.x, we = w2 - w1;
-                    const float2 U0 = ffma2(dup(we), lo2(m2), ffma2(dup(wy.y), lo2(mp), mul2(w1, lo2(m0))));
-                    const float2 U1 = ffma2(dup(we), hi2(m2), ffma2(dup(wy.y), hi2(mp), mul2(w1, hi2(m0))));
-                    const float2 V0 = mul2(w1, lo2(mp)), V1 = mul2(w1, hi2(mp));
-                    const float wx[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
-                    const float wd[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+            } else {
 #pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        acc[c][0] = ffma2(dup(wd[c]), V0, ffma2(dup(wx[c]), U0, acc[c][0]));
-                        acc[c][1] = ffma2(dup(wd[c]), V1, ffma2(dup(wx[c]), U1, acc[c][1]));
+                for (int i = 0; i < 16; ++i) acc[i >> 3][i & 7] = dup(0.f);
+                for (int ch = 0; ch < nch; ++ch, ++k) {
+                    const int slot = k % kSStages;
+                    ok = tc::mbar_wait(&sm.full[slot], (uint32_t)((k / kSStages) & 1), ok) && ok;
+                    const float2 *mb = reinterpret_cast<const float2 *>(sm.m[slot][0]) + vi;
+                    const SEntry *eb = &sm.ent[ch * kSChunk];
+                    for (uint32_t mk = sm.mask[ch][rg] & part; mk; mk &= mk - 1) {
+                        const int el = __ffs(mk) - 1;
+                        const SEntry &en = eb[el];
+                        const float2 m0 = mb[el * 2 * kVec], mp = mb[el * 2 * kVec + 16], m2 = mb[el * 2 * kVec + 32];
+                        const float2 wy = en.wy[ry];
+                        const float4 h = en.hd;
+                        const float4 *x4 = reinterpret_cast<const float4 *>(en.wx);
+                        const int a = ry - __float_as_int(h.y);
+                        const float w1 = a == kTaps ? 0.f : wy.x, w2 = a == 0 ? 0.f : wy.x, we = w2 - w1;
+                        const float U[2] = {fmaf(we, m2.x, fmaf(wy.y, mp.x, w1 * m0.x)),
+                                            fmaf(we, m2.y, fmaf(wy.y, mp.y, w1 * m0.y))};
+                        const float V[2] = {w1 * mp.x, w1 * mp.y};
+                        const float E[2] = {w2 * m2.x, w2 * m2.y};
+                        const int dx = __float_as_int(h.x);
+                        auto half = [&](int c0) {  // cells 2 c0 .. 2 c0 + 7 (pairs c0 ..)
+                            const float4 xa = x4[c0 / 2], xb = x4[c0 / 2 + 1];
+                            const float4 da = x4[kT / 4 + c0 / 2], db = x4[kT / 4 + c0 / 2 + 1];
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                acc[i][c0] = ffma2(lo2(xa), dup(U[i]), acc[i][c0]);
+                                acc[i][c0 + 1] = ffma2(hi2(xa), dup(U[i]), acc[i][c0 + 1]);
+                                acc[i][c0 + 2] = ffma2(lo2(xb), dup(U[i]), acc[i][c0 + 2]);
+                                acc[i][c0 + 3] = ffma2(hi2(xb), dup(U[i]), acc[i][c0 + 3]);
+                            }
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                acc[i][c0] = ffma2(lo2(da), dup(V[i]), acc[i][c0]);
+                                acc[i][c0 + 1] = ffma2(hi2(da), dup(V[i]), acc[i][c0 + 1]);
+                                acc[i][c0 + 2] = ffma2(lo2(db), dup(V[i]), acc[i][c0 + 2]);
+                                acc[i][c0 + 3] = ffma2(hi2(db), dup(V[i]), acc[i][c0 + 3]);
+                            }
+                        };
+                        if (dx < 8) half(0);
+                        if (dx + kTaps >= 8) half(4);
+                        // the window's edge columns dx and dx + 9: one jump for both
+                        switch (dx) {
+#define RECTV_E0(c)                                                                         \
+    _Pragma("unroll") for (int i = 0; i < 2; ++i) {                                         \
+        if ((c) & 1) acc[i][(c) / 2].y = fmaf(h.z, E[i], acc[i][(c) / 2].y);                \
+        else acc[i][(c) / 2].x = fmaf(h.z, E[i], acc[i][(c) / 2].x);                        \
+    }
+#define RECTV_E9(c)                                                                         \
+    _Pragma("unroll") for (int i = 0; i < 2; ++i) {                                         \
+        if ((c) & 1) acc[i][(c) / 2].y = fmaf(h.w, E[i], acc[i][(c) / 2].y);                \
+        else acc[i][(c) / 2].x = fmaf(h.w, E[i], acc[i][(c) / 2].x);                        \
+    }
+#define RECTV_LEFT(c) case c - 9: RECTV_E9(c) break;
+#define RECTV_BOTH(c) case c: RECTV_E0(c) RECTV_E9(c + 9) break;
+#define RECTV_RIGHT(c) case c: RECTV_E0(c) break;
+                            RECTV_LEFT(0) RECTV_LEFT(1) RECTV_LEFT(2) RECTV_LEFT(3) RECTV_LEFT(4) RECTV_LEFT(5)
+                            RECTV_LEFT(6) RECTV_LEFT(7) RECTV_LEFT(8)
+                            RECTV_BOTH(0) RECTV_BOTH(1) RECTV_BOTH(2) RECTV_BOTH(3) RECTV_BOTH(4) RECTV_BOTH(5)
+                            RECTV_BOTH(6)
+                            RECTV_RIGHT(7) RECTV_RIGHT(8) RECTV_RIGHT(9) RECTV_RIGHT(10) RECTV_RIGHT(11)
+                            RECTV_RIGHT(12) RECTV_RIGHT(13) RECTV_RIGHT(14) RECTV_RIGHT(15)
+#undef RECTV_E0
+#undef RECTV_E9
+#undef RECTV_LEFT
+#undef RECTV_BOTH
+#undef RECTV_RIGHT
+                            default: break;
+                        }
                     }
-                    // edge columns of the window inside this warp's columns (at most one: they are 9 apart)
-                    int ce = __float_as_int(h.x) - cx0;
-                    float wv = h.z;
-                    if (ce < 0) {
-                        ce += kTaps;
-                        wv = h.w;
-                    }
-                    const float2 E0 = mul2(wv * w2, lo2(m2)), E1 = mul2(wv * w2, hi2(m2));
-                    switch (ce) {
-#define RECTV_EDGE(c)                                                        \
-    case c:                                                                  \
-        acc[c][0] = make_float2(acc[c][0].x + E0.x, acc[c][0].y + E0.y);     \
-        acc[c][1] = make_float2(acc[c][1].x + E1.x, acc[c][1].y + E1.y);     \
-        break;
-                        RECTV_EDGE(0)
-                        RECTV_EDGE(1)
-                        RECTV_EDGE(2)
-                        RECTV_EDGE(3)
-                        RECTV_EDGE(4)
-                        RECTV_EDGE(5)
-                        RECTV_EDGE(6)
-                        RECTV_EDGE(7)
-#undef RECTV_EDGE
-                        default: break;
-                    }
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_addr(&sm.empty[slot]))
+                                     : "memory");
                 }
-                __syncwarp();
-                if (lane == 0)
-                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(tc::smem_addr(&sm.empty[slot]))
-                                 : "memory");
             }
-        }
-        if (wid < kSWarps) {  // the pre-IFFT fftshift sign is applied here
-            float4 *dst = spec + (long long)(pz * g.jg + jgrp) * plane;
-            const int Y = Y0 + ry;
-            if (Y < g.vrows) {
+            if (sub) {  // add the four warps' sums, in warp order, through the (idle) stages
+                __syncthreads();
+                float2 *red = reinterpret_cast<float2 *>(sm.m);
+                static_assert(sizeof(sm.m) >= 6 * 16 * 32 * sizeof(float2), "six warps' sums");
+                if (wid > 1 && wid < kSWarps) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int X = X0 + cx0 + c;
-                    const float sg = ((X + Y) & 1) ? -1.f : 1.f;
-                    if (X < g.vp)
-                        dst[Y * rowp + (long long)X * 8 + ci] =
-                            make_float4(sg * acc[c][0].x, sg * acc[c][0].y, sg * acc[c][1].x, sg * acc[c][1].y);
+                    for (int i = 0; i < 16; ++i) red[((wid - 2) * 16 + i) * 32 + lane] = acc[i >> 3][i & 7];
+                }
+                __syncthreads();
+                if (wid < 2) {
+                    for (int w = wid; w < 6; w += 2)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 o = red[(w * 16 + i) * 32 + lane];
+                            acc[i >> 3][i & 7].x += o.x;
+                            acc[i >> 3][i & 7].y += o.y;
+                        }
+                }
+                tc::fence_proxy_async();  // before the next copies into the stages
+                __syncthreads();
+            }
+            if (wid < (sub ? 2 : kSWarps) && Y0 + ry < g.vrows) {  // the pre-IFFT fftshift sign is applied here
+                const float sy = ((X0 + Y0 + ry) & 1) ? -1.f : 1.f;
+#pragma unroll
+                for (int c = 0; c < kT; ++c) {
+                    if (X0 + c >= g.vp) continue;
+                    const float2 r = acc[0][c >> 1], i = acc[1][c >> 1];
+                    float2 o = (c & 1) ? make_float2(-sy * r.y, -sy * i.y) : make_float2(sy * r.x, sy * i.x);
+                    if (seg > 0) {  // this thread's own earlier store
+                        const float2 q = dst[c * 16];
+                        o = make_float2(o.x + q.x, o.y + q.y);
+                    }
+                    dst[c * 16] = o;
                 }
             }
-#pragma unroll
-            for (int c = 0; c < 8; ++c) acc[c][0] = acc[c][1] = dup(0.f);
         }
     }
     if (!ok && lane == 0) atomicAdd(err, 1);
@@ -486,11 +567,14 @@ void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev 
     if (zb > gd.demix_slices) throw Error(1, "adjoint direction mixing buffer too small");
     const int npl = vec_planes(g, zb), npz = npl / g.jg, nh = g.n / 2;
     if (npl > 32767) throw Error(1, "too many spectrum planes");  // plane ranges are packed in 16 bits
-    const dim3 gm((nh + kMThr / 8 - 1) / (kMThr / 8), gd.ndir, npz);
+    // the mix: up to eight planes per block while there are blocks for ten waves
+    const int qb = (nh + kMThr / 8 - 1) / (kMThr / 8);
+    const int per = (int)std::max<long long>(1, std::min<long long>(8, (long long)qb * gd.ndir * npz / 10000));
+    const dim3 gm(qb, gd.ndir, (npz + per - 1) / per);
     const int kstride = g.jg > 1 ? 16 * g.jg : g.tg;
     for (int jg = 0; jg < g.jg; ++jg) {
         k_adj_mix<<<gm, kMThr, 0, s>>>(gd.demix, rowsc, gd.dray_start, gd.drays, gd.dtau, gd.dkmat, gd.shiftadj, g, zb,
-                                       gd.ndir, jg, kstride);
+                                       gd.ndir, npz, per, jg, kstride);
         LAUNCH_CHECK("k_adj_mix");
         k_scatter_dir<<<gd.n_adj_items, kSThr, sizeof(ScatSmem), s>>>(gd.demix, reinterpret_cast<float4 *>(spec),
                                                                      gd.adj_pts, gd.adj_items, gd.sincos, g, gd.ndir,

@@ -166,7 +166,7 @@ int rectv_get_directions(rectv_handle *h, int *ndir, int *nrays);
  * (the per-ray kernels then run); *max_rays = the most rays grouped into one
  * direction.  tol_cells <= 0 and min_group <= 0 take the defaults of geometry
  * set-up (2e-3 grid cells, 2.5 rays); the environment switches are not read,
- * and a handle also needs the tensor-core adjoint (M >= 8) for the path.
+ * and odd detector widths or n < 32 keep the per-ray kernels.
  * Measured angles with a calibration factor (a scan that does not return to
  * its angles after each half-turn) are not grouped.  No reference
  * counterpart. */

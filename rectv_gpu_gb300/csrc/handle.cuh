@@ -79,7 +79,8 @@ struct Layout {
     bool tc_scatter = false;  // time samples mixed on the tensor cores in the adjoint (k_scatter_tc)
     bool pad_fft = false;     // hand-written padded-grid 2D FFTs
     bool fused_rows = false;  // fused residual rows (k_resid_rows)
-    bool iter_plans = false;  // the outer iteration runs cuFFT plans
+    bool dirs = false;        // the direction path may run (a geometry decides)
+    bool iter_plans = false;  // the outer iteration runs cuFFT plans (per-ray path)
     int tg = 1, zs = 1, jg = 1;  // vector layout of the direction path (UsGeo)
     long long slab = 0, gp = 0, img_spec = 0;
     size_t spec_elems = 0;
@@ -97,8 +98,9 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     // adjoint: tensor-core time-sample mixing (k_scatter_tc) from 8 time
     // samples up; RECTV_SCATTER=direct forces the FP32 scatter
     L.tc_scatter = m >= 8 && ntheta < 65536;  // ray index packed in 16 bits
+    L.dirs = true;
     if (const char *e = std::getenv("RECTV_SCATTER"))
-        if (!std::strcmp(e, "direct")) L.tc_scatter = false;
+        if (!std::strcmp(e, "direct")) L.tc_scatter = L.dirs = false;
     {
         const char *e = std::getenv("RECTV_CUFFT");
         L.pad_fft = pad_fft_supported(L.P) && !(e && std::atoi(e) != 0);
@@ -137,7 +139,7 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     const long long vec_pl = L.jg > 1 ? (long long)L.zb * L.jg : (L.zb + L.zs - 1) / L.zs;
     const long long vec_plane = (P + 2 * kVH) * (n + 1 + 2 * kVH) * 16;
     L.spec_elems = std::max<size_t>(std::max<size_t>((size_t)L.zb * m * (size_t)L.img_spec,
-                                                     L.tc_scatter ? (size_t)(vec_pl * vec_plane) : 0),
+                                                     L.dirs ? (size_t)(vec_pl * vec_plane) : 0),
                                     (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
@@ -543,15 +545,15 @@ struct Handle {
         // several half-turns share its sample positions, so the USFFT
         // interpolates once per position.  Used when the rays average at least
         // 2.5 per direction (RECTV_DIRS=1: whenever it can run, RECTV_DIRS=0:
-        // never) and the adjoint fills Hermitian half planes; rays are grouped
-        // when their samples agree within RECTV_DIR_TOL grid cells (2e-3).
+        // never) and no FP32 scatter is asked for; rays are grouped when their
+        // samples agree within RECTV_DIR_TOL grid cells (2e-3).
         double dir_min = kDirMinGroup, dir_tol = kDirTolCells;
         if (const char *e = std::getenv("RECTV_DIRS")) {
             if (!std::strcmp(e, "0")) dir_min = -1.0;
             if (!std::strcmp(e, "1")) dir_min = 1.0;
         }
         if (const char *e = std::getenv("RECTV_DIR_TOL")) dir_tol = std::max(0.0, std::atof(e));
-        if (!tc_scatter) dir_min = -1.0;
+        if (!lay.dirs) dir_min = -1.0;
         const size_t nphi = phi_h ? (size_t)2 * m * ntheta : 0;
         if (geo_valid && center == geo_center && tc_min_spr == geo_tc_spr && tc_scatter == geo_tc_scatter &&
             dir_min == geo_dir_min && dir_tol == geo_dir_tol &&
@@ -916,7 +918,7 @@ struct Handle {
         if (titer_ < 0) throw Error(RECTV_ERR_ARG, "rectv: titer must be >= 0");
         if (!phi_h) throw Error(RECTV_ERR_ARG, "rectv: phi is required");
         const bool rebuilt = set_geometry(theta_h, phi_h, center);
-        if (lay.iter_plans) ensure_plans();
+        if (!(pad_fft && fused_rows && (gd.dirs || gd.tc_scatter))) ensure_plans();
         lambda0 = lambda0_;
         set_lambda1(lambda1_);
         titer = titer_;
@@ -1164,7 +1166,7 @@ struct Handle {
         const int ng = jgroups();
         // the padded-grid FFTs replace deapodise/pad (crop) and the 2D cuFFT
         // executions by a row and a column kernel each
-        const bool own2d = pad_fft && gd.tc_scatter;
+        const bool own2d = pad_fft && (gd.dirs || gd.tc_scatter);
         // forward: [rows + columns | deapodise/pad], halo, zeroing of the k = 0
         // samples, per group of 16 time samples the tensor-core gather (8+ time
         // samples) and the direct one (items with few samples per ray), then the
@@ -1179,7 +1181,7 @@ struct Handle {
         // adjoint: [row preparation], the zeroing of split tiles (direct scatter),
         // one scatter per group, then [columns + rows | crop]
         // (direction path: mixing and scatter per group, the fold of the border)
-        const int adj_k = (fused_rows ? 0 : 1) + ((!gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
+        const int adj_k = (fused_rows ? 0 : 1) + ((!gd.dirs && !gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
                           (gd.dirs ? 2 * ng + 1 : ng) + (own2d ? 2 : (gd.dirs ? 2 * vcalls : 1));
         const int adj_f = (fused_rows ? 0 : 1) + (own2d ? 0 : (gd.dirs ? vcalls : f2));
         // per outer iteration: titer inner steps per batch (forward, graddiv,
@@ -1199,7 +1201,7 @@ struct Handle {
                 break;
             case 1:  // scatter: half row spectra in; Hermitian half planes out (tensor-core path), else full planes
                 *bytes = (double)zb * ntheta * (n / 2 + 1) * 8.0 +
-                         (gd.tc_scatter ? (double)zb * m * P * (P / 2 + 1) * 8.0 : (double)zb * m * P * P * 8.0);
+                         (gd.dirs || gd.tc_scatter ? (double)zb * m * P * (P / 2 + 1) * 8.0 : (double)zb * m * P * P * 8.0);
                 *flops = npts * (81.0 * 2.0 * m * 2.0 + 8.0 * m + 18.0 * 4.0);
                 break;
             case 2:  // graddiv after the first inner step: u in, u out, w in (psi and mu when titer = 1)

@@ -78,6 +78,8 @@ struct Layout {
     int P = 0, nchunks = 0, nzc = 0, zb = 0, nbatch = 0;
     bool tc_scatter = false;  // time samples mixed on the tensor cores in the adjoint (k_scatter_tc)
     bool pad_fft = false;     // hand-written padded-grid 2D FFTs
+    bool gen_fft = false;     // mixed-radix ones on the direction path
+    bool gen_rows = false;    // mixed-radix fused residual rows on the direction path
     bool fused_rows = false;  // fused residual rows (k_resid_rows)
     bool dirs = false;        // the direction path may run (a geometry decides)
     bool iter_plans = false;  // the outer iteration runs cuFFT plans (per-ray path)
@@ -104,8 +106,15 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     {
         const char *e = std::getenv("RECTV_CUFFT");
         L.pad_fft = pad_fft_supported(L.P) && !(e && std::atoi(e) != 0);
+        L.gen_fft = !pad_fft_supported(L.P) && !(e && std::atoi(e) != 0);
     }
     L.fused_rows = L.pad_fft && resid_rows_supported(n);
+    {
+        GenPlan p;
+        const char *e = std::getenv("RECTV_CUFFT");
+        L.gen_fft = L.gen_fft && L.dirs && gen_fft_plan(L.P, &p);
+        L.gen_rows = !L.fused_rows && L.dirs && !(e && std::atoi(e) != 0) && gen_fft_plan(n, &p);
+    }
     L.iter_plans = !(L.pad_fft && L.fused_rows && L.tc_scatter);
     const long long qp = n + 2 * kHalo + (n & 1);
     const long long img_fwd = (P + 2 * kHalo) * qp;
@@ -144,7 +153,7 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
     b += (double)L.zb * nt * 4 + L.spec_elems * 8.0 + (double)L.zb * ntheta * std::max(n, n / 2 + 1) * 8.0;
-    if (L.fused_rows) b += (double)L.zb * ntheta * (n / 2 + 1) * 8.0;
+    if (L.fused_rows || L.gen_rows) b += (double)L.zb * ntheta * (n / 2 + 1) * 8.0;
     b += 3.0 * 8 * (double)((n + 32) / 32) * ((n + 8) / 8) * d * (nzp + 1) * L.nbatch + (4 << 20);
     // geometry: angle plan, adjoint entries (about 2.25 tiles per sample) and records
     b += nt * (4 + 2.5 * 4 + (L.tc_scatter ? 2.5 * 144 + 12 : 0)) + 8.0 * ntheta * m + (1 << 20);
@@ -226,6 +235,15 @@ struct Handle {
     float2 *fft_tw_n = nullptr;  // twiddles of the n-point row transforms
     float2 *rows_adj = nullptr;  // the adjoint's row spectra [zb][ntheta][n/2+1]
     CUtensorMap fft_fwd_map, fft_inv_map;  // TMA tiles of the column passes
+    // direction path: mixed-radix passes where 2n is no power of two
+    bool gen_fft = false;
+    GenPlan gen_plan{};
+    float2 *gen_tw = nullptr;
+    bool gen_rows = false;  // residual rows, length n
+    GenPlan gen_rplan{};
+    float2 *gen_rtw = nullptr;
+    bool own_rows() const { return fused_rows || (gd.dirs && gen_rows); }
+    bool vec_cufft() const { return !pad_fft && !gen_fft; }  // cuFFT and a layout change instead
 
     // session
     bool session = false;
@@ -275,6 +293,8 @@ struct Handle {
         gather_dir_prepare();
         scatter_dir_prepare();
         pad_fft_prepare();
+        gen_fft_fwd_prepare();
+        gen_fft_inv_prepare();
         const int P = 2 * n;
         ug.n = n;
         ug.ntheta = ntheta;
@@ -373,6 +393,22 @@ struct Handle {
                 }
             }
         }
+        auto gen_table = [&](const GenPlan &p) {
+            const std::vector<float2> w = gen_fft_twiddles(p);
+            float2 *d = alloc<float2>(w.size());
+            CUDA_CHECK(cudaMemcpyAsync(d, w.data(), sizeof(float2) * w.size(), cudaMemcpyHostToDevice, stream));
+            CUDA_CHECK(cudaStreamSynchronize(stream));
+            return d;
+        };
+        if (lay.gen_fft && gen_fft_plan(P, &gen_plan)) {
+            gen_fft = true;
+            gen_tw = gen_table(gen_plan);
+        }
+        if (lay.gen_rows && gen_fft_plan(n, &gen_rplan)) {
+            gen_rows = true;
+            gen_rtw = gen_table(gen_rplan);
+            rows_adj = alloc<float2>((size_t)zb * ntheta * (size_t)(n / 2 + 1));
+        }
         CUDA_CHECK(cudaStreamSynchronize(stream));
     }
 
@@ -384,11 +420,13 @@ struct Handle {
         bool need[kNPlans] = {};
         need[kRowsR2C] = true;
         need[gd.dirs ? kRowsC2R : kRowsC2C] = true;
-        if (!pad_fft) need[gd.dirs ? kVecR2C : kR2C2D] = true;
-        if (!gd.dirs && !gd.tc_scatter)
-            need[kC2C2D] = true;
-        else if (!pad_fft)
-            need[gd.dirs ? kVecC2R : kC2R2D] = true;
+        if (gd.dirs) {
+            need[kVecR2C] = need[kVecC2R] = vec_cufft();
+        } else {
+            need[kR2C2D] = !pad_fft;
+            need[kC2C2D] = !gd.tc_scatter;
+            need[kC2R2D] = gd.tc_scatter && !pad_fft;
+        }
         make_fft_plans(need);
     }
 
@@ -694,7 +732,7 @@ struct Handle {
                 std::copy(kmat.begin() + th * m, kmat.begin() + (th + 1) * m, dk.begin() + (size_t)r * ks);
             }
             gd.dkmat = (float2 *)up(dk.data(), dk.size() * sizeof(float2));
-            if (!pad_fft) {
+            if (vec_cufft()) {
                 const size_t bytes = (size_t)vec_slices * m * ug.P * (n + 2) * sizeof(float2);
                 void *p = nullptr;
                 CUDA_CHECK(cudaMallocAsync(&p, bytes, stream));
@@ -760,6 +798,8 @@ struct Handle {
         if (gd.dirs) {
             if (pad_fft) {
                 launch_pad_fft_fwd_vec(u, spec, zb, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+            } else if (gen_fft) {
+                launch_gen_fft_fwd(u, spec, zb, gd.deapod, gen_tw, gen_plan, ug, stream);
             } else {
                 UsGeo gp2 = ug;  // planar images of rows of n + 2 complex
                 gp2.qp = n + 2;
@@ -807,6 +847,10 @@ struct Handle {
             launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
             if (pad_fft) {
                 launch_pad_fft_inv_accum_vec(spec, u, zb, tau, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+                return;
+            }
+            if (gen_fft) {
+                launch_gen_fft_inv_accum(spec, u, zb, tau, gd.deapod, gen_tw, gen_plan, ug, stream);
                 return;
             }
             for (int z = 0; z < zb; z += vec_slices) {
@@ -857,16 +901,19 @@ struct Handle {
             for (int bb = 0; bb < nbatch; ++bb) {
                 const long long z0 = (long long)bb * zb;
                 const int c0 = bb * dpb;
-                if (fused_rows) {  // residual rows straight into the adjoint's row spectra
+                if (own_rows()) {  // residual rows straight into the adjoint's row spectra
                     forward_rows(U[src] + z0 * slab);
-                    launch_resid_rows(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, zb, gd.dirs, ug, stream);
+                    if (fused_rows)
+                        launch_resid_rows(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, zb, gd.dirs, ug, stream);
+                    else
+                        launch_gen_resid(rows, gdata + z0 * ntheta * n, rows_adj, gen_rtw, gen_rplan, zb, ug, stream);
                 } else {
                     forward(U[src] + z0 * slab, gdata + z0 * ntheta * n, h1, 1.0f, 1);
                 }
                 // first inner step: psi, mu in, w = mu - rho psi out; later steps: w in
                 const int gmode = titer > 1 ? (k == 0 ? 1 : 2) : 0;
                 launch_graddiv(U[src], U[old], U[dst], psi, mu, wdual, gmode, rho_d, c0, nchunks, tv, stream);
-                if (fused_rows)
+                if (own_rows())
                     adjoint_rows(rows_adj, U[dst] + z0 * slab, -0.5f);
                 else
                     adjoint(h1, U[dst] + z0 * slab, -0.5f);
@@ -918,7 +965,7 @@ struct Handle {
         if (titer_ < 0) throw Error(RECTV_ERR_ARG, "rectv: titer must be >= 0");
         if (!phi_h) throw Error(RECTV_ERR_ARG, "rectv: phi is required");
         const bool rebuilt = set_geometry(theta_h, phi_h, center);
-        if (!(pad_fft && fused_rows && (gd.dirs || gd.tc_scatter))) ensure_plans();
+        if (!(own_rows() && (gd.dirs ? !vec_cufft() : pad_fft && gd.tc_scatter))) ensure_plans();
         lambda0 = lambda0_;
         set_lambda1(lambda1_);
         titer = titer_;
@@ -1166,7 +1213,8 @@ struct Handle {
         const int ng = jgroups();
         // the padded-grid FFTs replace deapodise/pad (crop) and the 2D cuFFT
         // executions by a row and a column kernel each
-        const bool own2d = pad_fft && (gd.dirs || gd.tc_scatter);
+        const bool own2d = gd.dirs ? !vec_cufft() : pad_fft && gd.tc_scatter;
+        const bool ownf = gd.dirs ? !vec_cufft() : pad_fft;
         // forward: [rows + columns | deapodise/pad], halo, zeroing of the k = 0
         // samples, per group of 16 time samples the tensor-core gather (8+ time
         // samples) and the direct one (items with few samples per ray), then the
@@ -1176,14 +1224,14 @@ struct Handle {
         const int gather_k =
             gd.dirs ? (gd.n_dfwd_items > 0 ? ng : 0)
                     : 1 + ng * (((m >= 8 && gd.n_fwd_tc_items > 0) ? 1 : 0) + (gd.n_fwd_items > 0 ? 1 : 0));
-        const int fwd_k = (pad_fft ? 2 : (gd.dirs ? 2 * vcalls : 1)) + 1 + gather_k + 1;
-        const int fwd_f = (pad_fft ? 0 : (gd.dirs ? vcalls : f2)) + (fused_rows ? 0 : 1);
+        const int fwd_k = (ownf ? 2 : (gd.dirs ? 2 * vcalls : 1)) + 1 + gather_k + 1;
+        const int fwd_f = (ownf ? 0 : (gd.dirs ? vcalls : f2)) + (own_rows() ? 0 : 1);
         // adjoint: [row preparation], the zeroing of split tiles (direct scatter),
         // one scatter per group, then [columns + rows | crop]
         // (direction path: mixing and scatter per group, the fold of the border)
-        const int adj_k = (fused_rows ? 0 : 1) + ((!gd.dirs && !gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
+        const int adj_k = (own_rows() ? 0 : 1) + ((!gd.dirs && !gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
                           (gd.dirs ? 2 * ng + 1 : ng) + (own2d ? 2 : (gd.dirs ? 2 * vcalls : 1));
-        const int adj_f = (fused_rows ? 0 : 1) + (own2d ? 0 : (gd.dirs ? vcalls : f2));
+        const int adj_f = (own_rows() ? 0 : 1) + (own2d ? 0 : (gd.dirs ? vcalls : f2));
         // per outer iteration: titer inner steps per batch (forward, graddiv,
         // adjoint), one shrink per batch, the two-stage rho reduction
         *kern = titer * nbatch * (fwd_k + 1 + adj_k) + nbatch + 2;
@@ -1240,7 +1288,7 @@ struct Handle {
         for (int r = 0; r < reps; ++r) {
             switch (which) {
                 case 0: launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &vec_tmap : &spec_tmap, stream); break;
-                case 1: launch_scatter_adj(fused_rows ? rows_adj : rows, spec, zb, gd, ug, stream); break;
+                case 1: launch_scatter_adj(own_rows() ? rows_adj : rows, spec, zb, gd, ug, stream); break;
                 case 2:  // the inner steps after the first (w = mu - rho psi as stored by the last iteration)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 2 : 0, rho_d, 0,
                                    nchunks, tv, stream);

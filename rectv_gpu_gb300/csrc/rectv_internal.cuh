@@ -283,6 +283,31 @@ void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const f
 // the same from half planes in the vector layout (make_vec_fft_map)
 void launch_pad_fft_inv_accum_vec(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                                   const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
+// mixed-radix passes for grid sides that are no power of two (fft_general.cuh,
+// fft_general_fwd.cu, fft_general_inv.cu): even lengths 32 .. 2048 with prime
+// factors up to 13
+struct GenPlan {
+    int P, np;           // length, passes
+    int R[6], Ns[6];     // radix of a pass, product of the radices before it
+    uint32_t magic[6];   // ceil(2^32 / Ns): j / Ns = mulhi(j, magic) for j < 2^16
+    int toff[6];         // first twiddle of a pass: exp(-2 pi i r k / (Ns R)) at toff + (r - 1) Ns + k
+};
+bool gen_fft_plan(int P, GenPlan *p);
+std::vector<float2> gen_fft_twiddles(const GenPlan &p);
+void gen_fft_fwd_prepare();
+void gen_fft_inv_prepare();
+size_t gen_rows_smem(int P, int C);
+size_t gen_cols_smem(int P, int C);
+int gen_width(int P);
+int gen_live_groups(const UsGeo &g, int C);
+int gen_resident(size_t smem, int threads);
+void launch_gen_fft_fwd(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const GenPlan &p,
+                        const UsGeo &g, cudaStream_t s);
+void launch_gen_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
+                              const GenPlan &p, const UsGeo &g, cudaStream_t s);
+// launch_resid_rows on Hermitian half rows, p and tw of length n
+void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
+                      const UsGeo &g, cudaStream_t s);
 // fused residual rows of the inner step (fft_kernels.cu), n a power of two in
 // [256, 1024]: gathered rows [z][theta][n] and data g -> the adjoint's row
 // spectra [z][theta][n/2+1] (inverse row FFT, residual, fftshift, R2C)

@@ -40,6 +40,15 @@ CASES = [
     (48, 90, 8, 1, 6, 0.0),
     (128, 96, 9, 1, 4, 0.0),     # nine of 16 values live
     (36, 64, 17, 2, 4, 0.0),     # two planes per slice, one sample in the second
+    # mixed-radix grids: every radix of the passes (2n = 100, 88, 104, 84, 120, 144, 196, 960)
+    (50, 40, 4, 2, 4, 0.0),
+    (44, 40, 16, 1, 4, 0.5),
+    (52, 40, 8, 3, 4, 0.0),
+    (42, 40, 4, 3, 4, 0.0),
+    (60, 40, 12, 1, 4, 0.0),
+    (72, 40, 2, 5, 4, -1.5),
+    (98, 40, 8, 2, 4, 0.0),
+    (480, 24, 3, 1, 4, 0.0),
     (64, 256, 16, 1, 2, 0.0),    # 128 directions: tiles with several weight tables, split over blocks
 ]
 
@@ -71,6 +80,29 @@ def test_operators_match_oracle(lib_built, torch_cuda, monkeypatch, case):
     obj.free()
     e = rel(fw, ops.radonapr(f.astype(np.float64), 1.0)), rel(ad, ops.radonapradj(g.astype(np.float64), 1.0))
     assert max(e) < OP_TOL, e
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", [
+    # n, ntheta, m, nz, nzp, nrot: mixed-radix grids and residual rows, an odd number of rows
+    (50, 45, 5, 1, 1, 3),
+    (84, 36, 16, 3, 1, 4),
+])
+def test_reconstruction_matches_oracle(lib_built, torch_cuda, case):
+    from rectv_gpu_gb300 import Solver
+    from rectv_gpu_gb300.phantom import add_noise, phantom4d
+    n, ntheta, m, nz, nzp, nrot = case
+    theta, phi = scan_angles(ntheta, nrot), _phi(ntheta, m, 2)
+    ops = orc.Operators(n, ntheta, m, theta, phi, n / 2)
+    g = add_noise(ops.radonapr(phantom4d(n, nz, m, ntheta, seed=1).astype(np.float64)), 0.01, 1)
+    ref, hist = orc.run(g, theta, phi, n / 2, 4e-3, 4.0, 3, 3, nzp, return_history=True)
+    with Solver(n, ntheta, m, nz, nzp, 1) as slv:
+        slv.set_verbose(False)
+        got = slv.recon(g, theta, phi, lambda0=1e-3, lambda1=4.0, niter=3, titer=3)
+        assert slv.directions() > 0
+        h = slv.history()
+    assert rel(got, ref) < 1e-4, rel(got, ref)
+    assert np.allclose(h["rho"], [x["rho"] for x in hist])
 
 
 @pytest.mark.gpu

@@ -1,4 +1,4 @@
-// Forward padded-grid FFT of the direction path for grid sides 2n that are no
+// Forward padded-grid FFT for grid sides 2n that are no
 // power of two in [256, 2048] but a product of radices up to 16 (detector
 // widths such as 480 and 504), in the vector layout: the passes of
 // fft_kernels.cu (rows of value pairs as one complex transform, only the n

@@ -1,4 +1,4 @@
-// Inverse padded-grid FFT of the direction path for grid sides that are no
+// Inverse padded-grid FFT for grid sides that are no
 // power of two (fft_general_fwd.cu): inverse columns of the Hermitian half
 // planes, then rows, added into the volume.
 #include <cuda_runtime.h>
@@ -98,10 +98,11 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
 
 // ---------------------------------------------------------------------------
 // Residual rows of the inner step (k_resid_rows of fft_kernels.cu on the
-// mixed-radix core, Hermitian half rows in and out): two rows are one complex
-// transform, C pairs per block.
+// mixed-radix core): two rows are one complex transform, C pairs per block.
+// HALF: the rows hold their Hermitian half (direction path), else the whole
+// row, of which the Hermitian part counts.
 // ---------------------------------------------------------------------------
-template <int C>
+template <int C, bool HALF>
 __global__ void __launch_bounds__(kThr, 3)
     k_gen_resid(const float2 *__restrict__ rows, const float *__restrict__ gdata, float2 *__restrict__ out,
                 const __grid_constant__ GenPlan p, const float2 *__restrict__ tw, long long nrows, float scale) {
@@ -111,15 +112,22 @@ __global__ void __launch_bounds__(kThr, 3)
     constexpr int js = kThr / C;
     const long long ra = 2 * ((long long)blockIdx.x * C + c), rb = ra + 1;
     const bool oka = ra < nrows, okb = rb < nrows;
-    const float2 *ga = rows + (oka ? ra : 0) * hn, *gb = rows + (okb ? rb : 0) * hn;
+    const int rn = HALF ? hn : n;  // values per row
+    const float2 *ga = rows + (oka ? ra : 0) * rn, *gb = rows + (okb ? rb : 0) * rn;
     const float2 zero = make_float2(0.f, 0.f);
+    auto load = [&](const float2 *r, int k) {
+        const float2 v = __ldg(r + k);
+        if (HALF) return v;
+        const float2 w = __ldg(r + (k ? n - k : 0));
+        return make_float2(0.5f * (v.x + w.x), 0.5f * (v.y - w.y));
+    };
     for (int kb = j0; kb < hn; kb += 2 * js) {
         float2 a[2], b[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int k = kb + i * js;
-            a[i] = oka && k < hn ? __ldg(ga + k) : zero;
-            b[i] = okb && k < hn ? __ldg(gb + k) : zero;
+            a[i] = oka && k < hn ? load(ga, k) : zero;
+            b[i] = okb && k < hn ? load(gb, k) : zero;
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -167,18 +175,23 @@ __global__ void __launch_bounds__(kThr, 3)
 }  // namespace
 
 void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
-                      const UsGeo &g, cudaStream_t s) {
+                      bool half, const UsGeo &g, cudaStream_t s) {
     constexpr int C = 4;
     const long long nrows = (long long)zb * g.ntheta, nblk = (nrows + 2 * C - 1) / (2 * C);
     if (nblk > 2147483647LL) throw Error(1, "residual rows: too many rows");
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
-    k_gen_resid<C><<<(unsigned)nblk, kThr, gen_rows_smem(g.n, C), s>>>(rows, gdata, out, p, tw, nrows, scale);
+    const size_t smem = gen_rows_smem(g.n, C);
+    if (half)
+        k_gen_resid<C, true><<<(unsigned)nblk, kThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
+    else
+        k_gen_resid<C, false><<<(unsigned)nblk, kThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
     LAUNCH_CHECK("k_gen_resid");
 }
 
 void gen_fft_inv_prepare() {
     constexpr int most = 227 * 1024;
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));

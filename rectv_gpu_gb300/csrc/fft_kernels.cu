@@ -8,7 +8,7 @@
 // Three quarters of the forward input and of the adjoint output are padding,
 // so the passes here touch only what is not:
 //
-//  forward  rows    n/2 row pairs per image: the pair's two deapodised real
+//  forward  rows    the n rows of two images at a time: their deapodised real
 //                   rows are one complex P-point FFT (a + i b, split after the
 //                   transform), input read straight from the volume; writes
 //                   the n+1 half-plane columns of rows [n/2, 3n/2)
@@ -16,9 +16,12 @@
 //                   [n/2, 3n/2) are zero (not read); writes all P rows
 //  adjoint  columns n+1 inverse P-point FFTs of the Hermitian half planes;
 //                   writes only rows [n/2, 3n/2) (in place)
-//           rows    n/2 row pairs: the Hermitian extension of two half rows
-//                   as one complex inverse FFT (Re -> first row, Im -> second),
+//           rows    two images at a time: the Hermitian extension of their half
+//                   rows as one complex inverse FFT (Re -> first, Im -> second),
 //                   only the n centre outputs, deapodised and added into u
+//
+// The spectra are in the vector layout (UsGeo): the two images of a transform
+// are neighbouring values of a cell.
 //
 // The same transform core also runs the n-point row transforms between the
 // gather and the scatter (k_resid_rows: inverse row FFT, residual, fftshift
@@ -53,7 +56,6 @@ __device__ __forceinline__ float2 operator-(float2 a, float2 b) { return make_fl
 __device__ __forceinline__ float2 cmul_(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ float2 conj_(float2 a) { return make_float2(a.x, -a.y); }
 
 // a * exp(DIR * i pi / 2): DIR = -1 (forward) multiplies by -i, DIR = +1 by +i
 template <int DIR>
@@ -222,62 +224,8 @@ __device__ __forceinline__ void fft_core(float2 *v, float2 *sh, int c, int t, co
 }
 
 constexpr int kRowThreads = 512;  // threads per block of the row kernels
-// values per tile of the vector layout's column passes (32- to 128-byte runs; 512 threads but for P = 256)
+// values per tile of the column passes (32- to 128-byte runs; 512 threads but for P = 256)
 constexpr int vec_col_c(int N) { return N >= 2048 ? 4 : (N == 1024 ? 8 : 16); }
-constexpr int kColC = 4;          // columns per block of the column kernels (32-byte row runs, two blocks per SM)
-
-// ---------------------------------------------------------------------------
-// Forward rows: deapodise, pad and modulate two rows of u (rows 2 pr, 2 pr+1
-// of image img), FFT as a + i b, split into the two half spectra and store
-// them at rows Y = y + n/2 of the halo-padded forward spectra, columns 0..n.
-// ---------------------------------------------------------------------------
-template <int N>
-__global__ void __launch_bounds__(kRowThreads, 2)
-    k_fft_rows_fwd(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp,
-                   const float2 *__restrict__ tw, UsGeo g, float inv4n2) {
-    constexpr int N1 = N / 16, RP = kRowThreads / N1;
-    using L = FftLayout<N, false, RP>;
-    extern __shared__ float2 fft_sh[];
-    const int n = N / 2;
-    const int t = threadIdx.x % N1, c = threadIdx.x / N1;
-    const int pr = blockIdx.x * RP + c;  // row pair
-    const long long img = blockIdx.y;
-    const bool ok = pr < n / 2;
-    const int ya = 2 * pr, yb = ya + 1;
-    float2 v[16];
-    {
-        const float *ua = u + (img * n + (ok ? ya : 0)) * (long long)n;
-        const float *ub = ua + n;
-        const int Ya = ya + n / 2;
-        const float sa = ok ? ((Ya & 1) ? -dp[ya] : dp[ya]) * inv4n2 : 0.f;
-        const float sb = ok ? ((Ya & 1) ? dp[yb] : -dp[yb]) * inv4n2 : 0.f;
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            v[r] = make_float2(0.f, 0.f);
-            if (r >= 4 && r < 12) {  // X = t + N1 r in [n/2, 3n/2)
-                const int x = t + N1 * (r - 4), X = x + n / 2;
-                const float w = (X & 1) ? -__ldg(dp + x) : __ldg(dp + x);
-                v[r] = make_float2(__ldg(ua + x) * w * sa, __ldg(ub + x) * w * sb);
-            }
-        }
-    }
-    fft_core<N, -1, L>(v, fft_sh, c, t, tw);
-    // Z in natural order, then A(k) = (Z(k) + conj Z(-k))/2, B(k) = (Z(k) - conj Z(-k))/(2i)
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < 16 / L::R3; ++q)
-#pragma unroll
-        for (int j1 = 0; j1 < L::R3; ++j1) fft_sh[c * L::S + t + N1 * q + 256 * j1] = v[q * L::R3 + j1];
-    __syncthreads();
-    if (!ok) return;
-    float2 *ra = spec + img * g.img_fwd + g.qoff + (long long)(ya + n / 2) * g.qp;
-    float2 *rb = ra + g.qp;
-    for (int k = t; k <= n; k += N1) {
-        const float2 zk = fft_sh[c * L::S + k], zm = fft_sh[c * L::S + ((N - k) & (N - 1))];
-        ra[k] = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
-        rb[k] = make_float2(0.5f * (zk.y + zm.y), 0.5f * (zm.x - zk.x));
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Forward rows into the vector layout (UsGeo): one row y of the images of one
@@ -311,7 +259,7 @@ struct VecRows {
 
 template <int N>
 __global__ void __launch_bounds__(kRowThreads, 2)
-    k_fft_rows_fwd_vec(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp,
+    k_fft_rows_fwd(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp,
                        const float2 *__restrict__ tw, UsGeo g, int zb, float inv4n2) {
     using V = VecRows<N>;
     using L = typename V::L;
@@ -383,42 +331,31 @@ __device__ __forceinline__ void mbar_expect(void *bar, uint32_t bytes) {
 
 
 // ---------------------------------------------------------------------------
-// Column passes.  Persistent blocks (one per SM) take tiles of 4 columns of
-// one image round-robin, column groups fastest; the tile after the current
-// one is loaded by TMA into the second landing buffer while the current one
-// is transformed, and each output tile leaves by TMA stores from the exchange
-// buffer, which the next tile reuses once those stores have read it.
+// Column passes.  Persistent blocks take tiles of C values of one column's
+// cells (C x 8 contiguous bytes), round-robin, the values of a cell fastest so
+// that the blocks in flight share the cells' 128-byte lines; the tile after
+// the current one is loaded by TMA into the second landing buffer while the
+// current one is transformed, and each output tile leaves by TMA stores from
+// the exchange buffer, which the next tile reuses once those stores have read
+// it.
 //
-// Forward: columns kx .. kx+3 of the row pass output (rows [n/2, 3n/2); the
-// others are zero and not read), P-point FFT, all P rows written back in
-// place (window coordinates of the halo-padded spectra: x = 2 (kHalo + kx)
-// floats, y = kHalo + row; columns past n are halo cells, rewritten by the
-// halo pass afterwards).
-// Inverse: inverse P-point FFT of columns kx .. kx+3 of the Hermitian half
-// planes [img][P][hpitch]; only rows [n/2, 3n/2) are written back (columns
-// past the row pitch read as zeros and are not stored).
-//
-// VEC: the vector layout.  A tile is C values of one column's cells (C x 8
-// contiguous bytes), tiles of a cell's values fastest, so that the blocks in
-// flight share the cells' 128-byte lines.
+// Forward: the row pass's output (rows [n/2, 3n/2); the others are zero and
+// not read), P-point FFT, all P rows written back in place.
+// Inverse: inverse P-point FFT of the columns of the Hermitian half planes;
+// only rows [n/2, 3n/2) are written back.
 // ---------------------------------------------------------------------------
-template <int N, int C, int DIR, bool VEC>
+template <int N, int C, int DIR>
 struct ColPass {
     static constexpr int n = N / 2;
-    static constexpr int BR = n < 256 ? n : 256;                // rows per TMA box
-    static constexpr int IN_ROWS = DIR < 0 ? n : N;              // rows loaded per tile
-    static constexpr int OUT_ROWS = DIR < 0 ? N : n;             // rows stored per tile
-    static constexpr int Y0 = VEC ? kVH : (DIR < 0 ? kHalo : 0);  // row 0 in map coordinates
-    static constexpr int IN_Y0 = DIR < 0 ? Y0 + n / 2 : Y0;       // first loaded row
-    static constexpr int OUT_Y0 = DIR < 0 ? Y0 : Y0 + n / 2;      // first stored row
-    // first float of tile group gr of an image; VEC: nlv groups of values per cell
+    static constexpr int BR = n < 256 ? n : 256;                  // rows per TMA box
+    static constexpr int IN_ROWS = DIR < 0 ? n : N;               // rows loaded per tile
+    static constexpr int OUT_ROWS = DIR < 0 ? N : n;              // rows stored per tile
+    static constexpr int IN_Y0 = DIR < 0 ? kVH + n / 2 : kVH;     // first loaded row (window coordinates)
+    static constexpr int OUT_Y0 = DIR < 0 ? kVH : kVH + n / 2;    // first stored row
+    // first float of tile group gr of a plane, nlv groups of values per cell
     __device__ static __forceinline__ int x0(int gr, int nlv) {
-        if constexpr (VEC) {
-            const int k = gr / nlv;
-            return 32 * (kVH + k) + 2 * C * (gr - k * nlv);
-        } else {
-            return 2 * ((DIR < 0 ? kHalo : 0) + gr * C);  // column offset of the planar map window
-        }
+        const int k = gr / nlv;
+        return 32 * (kVH + k) + 2 * C * (gr - k * nlv);
     }
     using L = FftLayout<N, true, C>;
     static constexpr size_t EX = (size_t)L::S * C > (size_t)OUT_ROWS * C ? (size_t)L::S * C : (size_t)OUT_ROWS * C;
@@ -426,11 +363,11 @@ struct ColPass {
     static constexpr size_t SMEM = sizeof(float2) * (EX + 2 * LAND);
 };
 
-template <int N, int C, int DIR, bool VEC>
+template <int N, int C, int DIR>
 __global__ void __launch_bounds__(C *(N / 16), 1)
     k_fft_cols(const __grid_constant__ CUtensorMap tmap, const float2 *__restrict__ tw, int ngroups, int nlv,
                int ntiles, int *__restrict__ err) {
-    using CP = ColPass<N, C, DIR, VEC>;
+    using CP = ColPass<N, C, DIR>;
     using L = typename CP::L;
     constexpr int N1 = N / 16, n = N / 2, BR = CP::BR;
     extern __shared__ __align__(1024) float2 fft_sh[];
@@ -497,71 +434,14 @@ __global__ void __launch_bounds__(C *(N / 16), 1)
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint rows: rows Ya = n/2 + 2 pr and Ya + 1 of the column pass output
-// (row pitch hp complex), Hermitian-extended to P points, one inverse FFT as
-// A + i B; the centre outputs X in [n/2, 3n/2) are modulated, deapodised,
-// scaled by c and added into rows 2 pr, 2 pr + 1 of u.
-// ---------------------------------------------------------------------------
-template <int N>
-__global__ void __launch_bounds__(kRowThreads, 2)
-    k_fft_rows_inv(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp,
-                   const float2 *__restrict__ tw, float cscale, int hp) {
-    constexpr int N1 = N / 16, RP = kRowThreads / N1;
-    using L = FftLayout<N, false, RP>;
-    extern __shared__ float2 fft_sh[];
-    const int n = N / 2;
-    const int t = threadIdx.x % N1, c = threadIdx.x / N1;
-    const int pr = blockIdx.x * RP + c;
-    const long long img = blockIdx.y;
-    const bool ok = pr < n / 2;
-    const int ya = 2 * pr, yb = ya + 1, Ya = ya + n / 2;
-    const float2 *ha = spec + img * N * hp + (long long)(ok ? Ya : n / 2) * hp;
-    const float2 *hb = ha + hp;
-    float2 v[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const int k = t + N1 * r;
-        float2 a, b;
-        if (k <= n) {
-            a = ha[k];
-            b = hb[k];
-            if (k == 0 || k == n) a.y = b.y = 0.f;
-        } else {
-            a = conj_(ha[N - k]);
-            b = conj_(hb[N - k]);
-        }
-        v[r] = make_float2(a.x - b.y, a.y + b.x);  // A + i B
-    }
-    fft_core<N, 1, L>(v, fft_sh, c, t, tw);
-    if (!ok) return;
-    float *ua = u + (img * n + ya) * (long long)n;
-    float *ub = ua + n;
-    const float sa = ((Ya & 1) ? -dp[ya] : dp[ya]) * cscale;
-    const float sb = ((Ya & 1) ? dp[yb] : -dp[yb]) * cscale;
-#pragma unroll
-    for (int q = 0; q < 16 / L::R3; ++q)
-#pragma unroll
-        for (int j1 = 0; j1 < L::R3; ++j1) {
-            const int X = t + N1 * q + 256 * j1;
-            const int x = X - n / 2;
-            if (x >= 0 && x < n) {
-                const float w = (X & 1) ? -__ldg(dp + x) : __ldg(dp + x);
-                const float2 z = v[q * L::R3 + j1];
-                ua[x] += z.x * w * sa;
-                ub[x] += z.y * w * sb;
-            }
-        }
-}
-
-// ---------------------------------------------------------------------------
 // Adjoint rows from the vector layout: the two images of a value pair are the
-// real and imaginary part of one inverse FFT (as k_fft_rows_fwd_vec); the
+// real and imaginary part of one inverse FFT (as k_fft_rows_fwd); the
 // centre outputs pass through shared memory once more so that the rows of u
 // are read and written as whole lines.
 // ---------------------------------------------------------------------------
 template <int N>
 __global__ void __launch_bounds__(kRowThreads, 2)
-    k_fft_rows_inv_vec(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp,
+    k_fft_rows_inv(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp,
                        const float2 *__restrict__ tw, UsGeo g, int zb, float cscale) {
     using V = VecRows<N>;
     using L = typename V::L;
@@ -740,20 +620,14 @@ void resid_n(const float2 *rows, const float *gdata, float2 *out, const float2 *
 
 template <int N>
 void set_attrs_n() {
-    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd_vec<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VecRows<N>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv_vec<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)VecRows<N>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, vec_col_c(N), 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, vec_col_c(N), 1, true>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, vec_col_c(N), -1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, vec_col_c(N), -1, true>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, -1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, kColC, -1, false>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, kColC, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)ColPass<N, kColC, 1, false>::SMEM));
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    constexpr int C = vec_col_c(N);
+    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, false>, attr, (int)rows_smem<N>()));
+    CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, true>, attr, (int)rows_smem<N>()));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, C, -1>, attr, (int)ColPass<N, C, -1>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, C, 1>, attr, (int)ColPass<N, C, 1>::SMEM));
 }
 
 int sm_count() {
@@ -766,74 +640,40 @@ int sm_count() {
     return nsm;
 }
 
-template <int N, int C, int DIR, bool VEC>
-void launch_cols(const CUtensorMap &map, const float2 *tw, int nimg, int ngroups, int nlv, int *err, cudaStream_t s) {
-    const long long ntiles = (long long)ngroups * nimg;
+template <int N, int DIR>
+void launch_cols(const CUtensorMap &map, const float2 *tw, int zb, int *err, const UsGeo &g, cudaStream_t s) {
+    constexpr int C = vec_col_c(N), thr = C * (N / 16);
+    constexpr size_t smem = ColPass<N, C, DIR>::SMEM;
+    // value groups of a cell that hold data (fewer than all with 9 .. 15 time samples)
+    const int nlv = g.tg == 16 && g.jg == 1 ? (g.m + C - 1) / C : 16 / C, ngroups = (N / 2 + 1) * nlv;
+    const long long ntiles = (long long)ngroups * vec_planes(g, zb);
     if (ntiles > 2147483647LL - 65536) throw Error(1, "pad FFT: too many column tiles");
-    constexpr int thr = C * (N / 16);
-    constexpr size_t smem = ColPass<N, C, DIR, VEC>::SMEM;
     // persistent: as many blocks per SM as shared memory and 1024 threads allow
     const int per_sm = std::max(1, std::min((int)((size_t)227 * 1024 / (smem + 1024)), 1024 / thr));
     const int grid = (int)std::min<long long>(ntiles, (long long)per_sm * sm_count());
-    k_fft_cols<N, C, DIR, VEC><<<grid, thr, smem, s>>>(map, tw, ngroups, nlv, (int)ntiles, err);
+    k_fft_cols<N, C, DIR><<<grid, thr, smem, s>>>(map, tw, ngroups, nlv, (int)ntiles, err);
     LAUNCH_CHECK(DIR < 0 ? "k_fft_cols (forward)" : "k_fft_cols (inverse)");
 }
 
-template <int N, int DIR>
-void launch_cols_planar(const CUtensorMap &map, const float2 *tw, int nimg, int *err, cudaStream_t s) {
-    launch_cols<N, kColC, DIR, false>(map, tw, nimg, (N / 2 + 1 + kColC - 1) / kColC, 1, err, s);
-}
-
-template <int N, int DIR>
-void launch_cols_vec(const CUtensorMap &map, const float2 *tw, int zb, int *err, const UsGeo &g, cudaStream_t s) {
-    constexpr int C = vec_col_c(N);
-    // value groups of a cell that hold data (fewer than all with 9 .. 15 time samples)
-    const int nlv = g.tg == 16 && g.jg == 1 ? (g.m + C - 1) / C : 16 / C;
-    launch_cols<N, C, DIR, true>(map, tw, vec_planes(g, zb), (N / 2 + 1) * nlv, nlv, err, s);
-}
-
 template <int N>
-void fwd_vec_n(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const CUtensorMap &map,
-               int *err, const UsGeo &g, cudaStream_t s) {
+void fwd_n(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const CUtensorMap &map,
+           int *err, const UsGeo &g, cudaStream_t s) {
     using V = VecRows<N>;
     const int n = N / 2;
     const float inv4n2 = (float)(1.0 / (4.0 * n * (double)n));
     const dim3 gr(n / V::R * (8 / V::C), vec_planes(g, zb));
-    k_fft_rows_fwd_vec<N><<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g, zb, inv4n2);
-    LAUNCH_CHECK("k_fft_rows_fwd_vec");
-    launch_cols_vec<N, -1>(map, tw, zb, err, g, s);
-}
-
-template <int N>
-void inv_vec_n(float2 *spec, float *u, int zb, float cscale, const float *deapod, const float2 *tw,
-               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
-    using V = VecRows<N>;
-    launch_cols_vec<N, 1>(map, tw, zb, err, g, s);
-    const dim3 gr(N / 2 / V::R * (8 / V::C), vec_planes(g, zb));
-    k_fft_rows_inv_vec<N><<<gr, kRowThreads, V::SMEM, s>>>(spec, u, deapod, tw, g, zb, cscale);
-    LAUNCH_CHECK("k_fft_rows_inv_vec");
-}
-
-template <int N>
-void fwd_n(const float *u, float2 *spec, int nimg, const float *deapod, const float2 *tw, const CUtensorMap &map,
-           int *err, const UsGeo &g, cudaStream_t s) {
-    constexpr int N1 = N / 16, RP = kRowThreads / N1;
-    const int n = N / 2;
-    const float inv4n2 = (float)(1.0 / (4.0 * n * (double)n));
-    dim3 gr((n / 2 + RP - 1) / RP, nimg);
-    k_fft_rows_fwd<N><<<gr, kRowThreads, rows_smem<N>(), s>>>(u, spec, deapod, tw, g, inv4n2);
+    k_fft_rows_fwd<N><<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g, zb, inv4n2);
     LAUNCH_CHECK("k_fft_rows_fwd");
-    launch_cols_planar<N, -1>(map, tw, nimg, err, s);
+    launch_cols<N, -1>(map, tw, zb, err, g, s);
 }
 
 template <int N>
-void inv_n(float2 *spec, float *u, int nimg, float cscale, const float *deapod, const float2 *tw,
-           const CUtensorMap &map, int *err, int hpitch, cudaStream_t s) {
-    constexpr int N1 = N / 16, RP = kRowThreads / N1;
-    const int n = N / 2;
-    launch_cols_planar<N, 1>(map, tw, nimg, err, s);
-    dim3 gr((n / 2 + RP - 1) / RP, nimg);
-    k_fft_rows_inv<N><<<gr, kRowThreads, rows_smem<N>(), s>>>(spec, u, deapod, tw, cscale, hpitch);
+void inv_n(float2 *spec, float *u, int zb, float cscale, const float *deapod, const float2 *tw, const CUtensorMap &map,
+           int *err, const UsGeo &g, cudaStream_t s) {
+    using V = VecRows<N>;
+    launch_cols<N, 1>(map, tw, zb, err, g, s);
+    const dim3 gr(N / 2 / V::R * (8 / V::C), vec_planes(g, zb));
+    k_fft_rows_inv<N><<<gr, kRowThreads, V::SMEM, s>>>(spec, u, deapod, tw, g, zb, cscale);
     LAUNCH_CHECK("k_fft_rows_inv");
 }
 
@@ -846,20 +686,6 @@ PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
         if (q != cudaDriverEntryPointSuccess || !encode) throw Error(1, "cuTensorMapEncodeTiled unavailable");
     }
     return encode;
-}
-
-// float view [nimg][rows][row_floats] (pitches in bytes), boxes of 2 c floats x
-// min(n, 256) rows x 1 image
-void encode_cols_map(CUtensorMap *map, void *base, long long row_floats, long long rows, long long nimg,
-                     long long row_pitch, long long img_pitch, int n, const char *what, int c = kColC) {
-    const cuuint64_t dims[3] = {(cuuint64_t)row_floats, (cuuint64_t)rows, (cuuint64_t)nimg};
-    const cuuint64_t strides[2] = {(cuuint64_t)row_pitch, (cuuint64_t)img_pitch};
-    const cuuint32_t box[3] = {(cuuint32_t)(2 * c), (cuuint32_t)(n < 256 ? n : 256), 1};
-    const cuuint32_t es[3] = {1, 1, 1};
-    const CUresult r = tmap_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, es,
-                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error(1, std::string("cuTensorMapEncodeTiled failed for ") + what);
 }
 
 }  // namespace
@@ -890,40 +716,26 @@ std::vector<float2> pad_fft_twiddles(int P) {
     return w;
 }
 
-void make_pad_fft_maps(CUtensorMap *fwd, CUtensorMap *inv, float2 *spec, int nimg, const UsGeo &g) {
-    // forward: the halo-padded window [P + 2 kHalo rows][2 qp floats]
-    encode_cols_map(fwd, spec, 2LL * g.qp, g.P + 2LL * kHalo, nimg, 8LL * g.qp, 8LL * g.img_fwd, g.n,
-                    "the forward column FFT");
-    // inverse: Hermitian half planes [P rows][2 hpitch floats]
-    encode_cols_map(inv, spec, 2LL * g.hpitch, g.P, nimg, 8LL * g.hpitch, 8LL * g.P * g.hpitch, g.n,
-                    "the inverse column FFT");
-}
-
+// float view [planes][rows][32 cells], boxes of one tile's values x min(n, 256) rows
 void make_vec_fft_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g) {
-    encode_cols_map(map, spec, 32LL * g.vp, g.vrows, npl, 128LL * g.vp, 8LL * g.vplane, g.n,
-                    "the vector layout's column FFT", vec_col_c(g.P));
+    const cuuint64_t dims[3] = {(cuuint64_t)32 * g.vp, (cuuint64_t)g.vrows, (cuuint64_t)npl};
+    const cuuint64_t strides[2] = {(cuuint64_t)128 * g.vp, (cuuint64_t)8 * g.vplane};
+    const cuuint32_t box[3] = {(cuuint32_t)(2 * vec_col_c(g.P)), (cuuint32_t)(g.n < 256 ? g.n : 256), 1};
+    const cuuint32_t es[3] = {1, 1, 1};
+    const CUresult r = tmap_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, spec, dims, strides, box, es,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw Error(1, "cuTensorMapEncodeTiled failed for the column FFT");
 }
 
-void launch_pad_fft_fwd_vec(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
-                            const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
+void launch_pad_fft_fwd(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
+                        const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
     if (vec_planes(g, zb) > 65535) throw Error(1, "pad FFT: too many planes per batch");
     switch (g.P) {
-        case 256: fwd_vec_n<256>(u, spec, zb, deapod, tw, map, err, g, s); break;
-        case 512: fwd_vec_n<512>(u, spec, zb, deapod, tw, map, err, g, s); break;
-        case 1024: fwd_vec_n<1024>(u, spec, zb, deapod, tw, map, err, g, s); break;
-        case 2048: fwd_vec_n<2048>(u, spec, zb, deapod, tw, map, err, g, s); break;
-        default: throw Error(1, "pad FFT: unsupported grid size");
-    }
-}
-
-void launch_pad_fft_fwd(const float *u, float2 *spec, int nimg, const float *deapod, const float2 *tw,
-                        const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
-    if (nimg > 65535) throw Error(1, "pad FFT: too many images per batch");
-    switch (g.P) {
-        case 256: fwd_n<256>(u, spec, nimg, deapod, tw, map, err, g, s); break;
-        case 512: fwd_n<512>(u, spec, nimg, deapod, tw, map, err, g, s); break;
-        case 1024: fwd_n<1024>(u, spec, nimg, deapod, tw, map, err, g, s); break;
-        case 2048: fwd_n<2048>(u, spec, nimg, deapod, tw, map, err, g, s); break;
+        case 256: fwd_n<256>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 512: fwd_n<512>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 1024: fwd_n<1024>(u, spec, zb, deapod, tw, map, err, g, s); break;
+        case 2048: fwd_n<2048>(u, spec, zb, deapod, tw, map, err, g, s); break;
         default: throw Error(1, "pad FFT: unsupported grid size");
     }
 }
@@ -945,30 +757,14 @@ void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, cons
 
 void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
-    const int nimg = zb * g.m;
-    if (nimg > 65535) throw Error(1, "pad FFT: too many images per batch");
-    // the scale of the C2R path's crop (1/sqrt(n ntheta) / (4 n^2)) times tau
-    const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
-    const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
-    switch (g.P) {
-        case 256: inv_n<256>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
-        case 512: inv_n<512>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
-        case 1024: inv_n<1024>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
-        case 2048: inv_n<2048>(spec, u, nimg, c, deapod, tw, map, err, g.hpitch, s); break;
-        default: throw Error(1, "pad FFT: unsupported grid size");
-    }
-}
-
-void launch_pad_fft_inv_accum_vec(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
-                                  const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s) {
     if (vec_planes(g, zb) > 65535) throw Error(1, "pad FFT: too many planes per batch");
     const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
     const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
     switch (g.P) {
-        case 256: inv_vec_n<256>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
-        case 512: inv_vec_n<512>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
-        case 1024: inv_vec_n<1024>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
-        case 2048: inv_vec_n<2048>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 256: inv_n<256>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 512: inv_n<512>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 1024: inv_n<1024>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
+        case 2048: inv_n<2048>(spec, u, zb, c, deapod, tw, map, err, g, s); break;
         default: throw Error(1, "pad FFT: unsupported grid size");
     }
 }

@@ -330,18 +330,19 @@ void make_vec_gather_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g
 }
 
 // ---------------------------------------------------------------------------
-// Halo of the spectra in the vector layout: the ring of cells a joint window
-// can reach (4 before, 5 after the half plane) gets the periodic spectrum's
-// values, through the Hermitian symmetry F(a, b) = conj F(-a, -b) outside the
-// stored columns.  One thread per 16 bytes (two values of a cell).
+// Halo of the spectra in the vector layout: the ring of cells that stencils
+// and footprints can reach (4 rows and columns before, 5 rows and `right`
+// columns after the half plane) gets the periodic spectrum's values, through
+// the Hermitian symmetry F(a, b) = conj F(-a, -b) outside the stored columns.
+// One thread per 16 bytes (two values of a cell).
 // ---------------------------------------------------------------------------
-__global__ void k_vec_halo(float4 *__restrict__ spec, UsGeo g) {
+__global__ void k_vec_halo(float4 *__restrict__ spec, int right, UsGeo g) {
     constexpr int H0 = kR, H1 = kR + 1, HS = H0 + H1;
-    const int P = g.P, n = g.n;
+    const int P = g.P, n = g.n, side = H0 + right;
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int ci = (int)(i & 7);
     const long long e = i >> 3;
-    const int wide = n + 1 + HS;  // cells of a full halo row
+    const int wide = n + 1 + side;  // cells of a full halo row
     int y, x;
     if (e < (long long)HS * wide) {
         const int r = (int)(e / wide);
@@ -349,14 +350,14 @@ __global__ void k_vec_halo(float4 *__restrict__ spec, UsGeo g) {
         y = r < H0 ? r - H0 : P + r - H0;
     } else {
         const long long e2 = e - (long long)HS * wide;
-        if (e2 >= (long long)P * HS) return;
-        y = (int)(e2 / HS);
-        const int c = (int)(e2 - (long long)y * HS);
+        if (e2 >= (long long)P * side) return;
+        y = (int)(e2 / side);
+        const int c = (int)(e2 - (long long)y * side);
         x = c < H0 ? c - H0 : n + 1 + c - H0;
     }
     float4 *pl = spec + blockIdx.y * (g.vplane / 2);
     auto at = [&](int yy, int xx) { return pl + ((long long)(yy + kVH) * g.vp + xx + kVH) * 8 + ci; };
-    const int a = y < 0 ? y + P : (y >= P ? y - P : y), b = x < 0 ? x + P : x;
+    const int a = (y % P + P) % P, b = (x % P + P) % P;
     float4 v;
     if (b <= n) {
         v = *at(a, b);
@@ -368,16 +369,16 @@ __global__ void k_vec_halo(float4 *__restrict__ spec, UsGeo g) {
     *at(y, x) = v;
 }
 
-void launch_vec_halo(float2 *spec, int npl, const UsGeo &g, cudaStream_t s) {
-    constexpr int HS = 2 * kR + 1;
-    const long long thr = 8 * ((long long)HS * (g.n + 1 + HS) + (long long)g.P * HS);
+void launch_vec_halo(float2 *spec, int npl, int right, const UsGeo &g, cudaStream_t s) {
+    const int side = kR + right;
+    const long long thr = 8 * ((long long)(2 * kR + 1) * (g.n + 1 + side) + (long long)g.P * side);
     if (npl > 65535) throw Error(1, "too many spectrum planes");
-    k_vec_halo<<<dim3((unsigned)((thr + 255) / 256), npl), 256, 0, s>>>(reinterpret_cast<float4 *>(spec), g);
+    k_vec_halo<<<dim3((unsigned)((thr + 255) / 256), npl), 256, 0, s>>>(reinterpret_cast<float4 *>(spec), right, g);
     LAUNCH_CHECK("k_vec_halo");
 }
 
 // ---------------------------------------------------------------------------
-// Planar half planes [image][P][n + 2] (cuFFT's output for slices z0 .. z0 +
+// Planar half planes [image][P][planar_pitch] (cuFFT's output for slices z0 .. z0 +
 // nz - 1, image (z - z0) m + t) into the vector layout: one block per 32
 // cells of a row, transposed through shared memory.
 // ---------------------------------------------------------------------------
@@ -385,13 +386,14 @@ __global__ void __launch_bounds__(256)
     k_planar_to_vec(const float2 *__restrict__ planar, float4 *__restrict__ spec, UsGeo g, int z0, int nz, int pl0) {
     __shared__ float2 sh[32][17];
     const int pl = pl0 + blockIdx.z, y = blockIdx.y, x0 = blockIdx.x * 32;
-    const long long img = (long long)g.P * (g.n + 2);
+    const int pitch = planar_pitch(g.n);
+    const long long img = (long long)g.P * pitch;
     const int lane = threadIdx.x & 31;
     for (int v = threadIdx.x >> 5; v < 16; v += 8) {
         const int z = vec_slice(g, pl, v), t = vec_time(g, pl, v), x = x0 + lane;
         float2 f = make_float2(0.f, 0.f);
         if (x <= g.n && z < z0 + nz && t < g.m)
-            f = __ldg(planar + ((long long)(z - z0) * g.m + t) * img + (long long)y * (g.n + 2) + x);
+            f = __ldg(planar + ((long long)(z - z0) * g.m + t) * img + (long long)y * pitch + x);
         sh[lane][v] = f;
     }
     __syncthreads();

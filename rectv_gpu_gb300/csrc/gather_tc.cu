@@ -22,11 +22,14 @@
 //  * once: the sample table (stencil origin, separable Gaussian weights with
 //    the fftshift signs, row factor) and the item's rays; the B operands
 //    (K' rows) when the item has at most two chunks of rays;
-//  * per slice: one TMA box load brings the 24x24-cell footprint of the
-//    16x16 floor tile, 16 time samples, from the halo-padded spectra into
-//    shared memory (the next slice's box is loaded while this slice is
+//  * per plane of the vector layout (16 time samples of a slice, or 8 of two):
+//    one TMA box load brings the 24x24-cell footprint of the 16x16 floor tile
+//    into shared memory (the next plane's box is loaded while this one is
 //    computed); threads convert it (Hermitian-mirrored tiles read the mirrored
 //    box, conjugated) into the A operand in tensor memory, hi and lo parts;
+//    (one aligned 128-byte line per cell, against 16 boxes of one sample's
+//    plane each: 1.07 instead of 1.10 ms at 8 slices of 1440 angles, width 480,
+//    16 samples, 1.91 instead of 1.95 at 3 slices of 2880, width 1024)
 //  * per chunk of 16 rays: 60 MMAs into the accumulator, issued by five
 //    threads (one per M tile of 128 cells: its own accumulation chain);
 //    the block moves G to shared memory, the next chunk's MMAs are issued,
@@ -35,6 +38,8 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "rectv_internal.cuh"
 #include "tcgen05.cuh"
@@ -46,7 +51,6 @@ namespace {
 
 constexpr int kT = 16;                       // floor tile side
 constexpr int kFW = kT + 2 * kR;             // footprint side (24)
-constexpr int kBoxW = kFW + 2;               // box width: even start column of a mirrored footprint
 constexpr int kCells = kFW * kFW;            // 576
 constexpr int kGP = kFW + 1;                 // row pitch of G in shared memory (25: the four threads
                                              // of a sample read rows 8 B x 25 apart, on distinct banks)
@@ -62,7 +66,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColAhi = 0;              // TMEM columns: A hi [mt*32, +32)
 constexpr uint32_t kColAlo = kMT * kK;       //               A lo
 constexpr uint32_t kColD = 2 * kMT * kK;     //               D    [mt*32, +32)
-constexpr uint32_t kBoxBytes = 16 * kFW * kBoxW * 8;
+constexpr uint32_t kBoxBytes = kCells * 128;
 
 // Core-matrix offset (floats) of element (row, kk) of a K-major FP32 operand
 // with 32 K values per row (LBO 128 B, SBO 1024 B).
@@ -71,7 +75,8 @@ __device__ __forceinline__ int off32(int row, int kk) {
 }
 
 struct TcSmem {
-    float2 box[16][kFW][kBoxW];          // TMA destination: 16 time samples x 24 rows x 26 cells
+    float4 box[kCells][8];               // TMA destination: 24 x 24 cells x 16 values, 16-byte chunk i of
+                                         // cell c at i ^ (c & 7) (128-byte swizzle)
     float2 g[kRays][kFW * kGP];          // G of the current chunk's rays, cell (row, col) at row * kGP + col
     float bhi[2][kN * kK];               // B = K' rows, FP32 (double-buffered)
     float blo[2][kN * kK];               // B - trunc(B)
@@ -118,22 +123,23 @@ __global__ void __launch_bounds__(kThr, 1)
     k_gather_tc(float2 *__restrict__ rows, const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
                 const float2 *__restrict__ sincos, const float2 *__restrict__ kmat,
                 const float2 *__restrict__ shiftf, const __grid_constant__ CUtensorMap tmap, UsGeo g, int zb,
-                int jbase, int accumulate, int *__restrict__ err) {
+                int npz, int per, int jgrp, int *__restrict__ err) {
+    const int jbase = 16 * jgrp;
     extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
     TcSmem &sm = *reinterpret_cast<TcSmem *>(tc_smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int4 it = items[blockIdx.x];
-    const int zper = g.zper;
-    const int z0 = blockIdx.y * zper, z1 = min(zb, z0 + zper);
+    const int z0 = blockIdx.y * per, z1 = min(npz, z0 + per);  // planes (of zs slices) of this block
+    const int zsh = g.zs >> 1;  // 16 time samples of one slice, or 8 of two
     const int tyi = it.x / g.NT, txi = it.x - tyi * g.NT;
     const int P = g.P;
     const int cnt = min(it.z, kTab);
-    // Footprint box in the halo-padded spectra (window origin (-kHalo, -kHalo)):
-    // tiles left of the Nyquist column read the direct box, the others the
-    // box of the mirrored cells (P - KY, P - KX), conjugated.
-    const bool mirrored = txi * kT > g.n + 2;
-    const int bx = mirrored ? 2 * (P - txi * kT - kR - kT + kHalo) : 2 * (txi * kT - kR + kHalo);
-    const int by = mirrored ? P - tyi * kT - (kT + kR - 1) + kHalo : tyi * kT - kR + kHalo;
+    // Footprint box in the vector layout's window: tiles left of the Nyquist
+    // column read the direct box, the others the box of the mirrored cells
+    // (P - KY, P - KX), conjugated.
+    const bool mirrored = txi * kT > g.n - 3;
+    const int bx = (mirrored ? P - txi * kT - (kT + kR - 1) : txi * kT - kR) + kVH;
+    const int by = (mirrored ? P - tyi * kT - (kT + kR - 1) : tyi * kT - kR) + kVH;
 
     if (wid == 0) tc::alloc(&sm.tslot, kTmemCols);
     if (tid == 0) {
@@ -141,14 +147,14 @@ __global__ void __launch_bounds__(kThr, 1)
         tc::mbar_init(&sm.bar_tma, 1);
         tc::fence_mbar_init();
     }
-    auto tma_issue = [&](int z) {  // one thread: box of slice z, time samples [jbase, jbase + 16)
+    auto tma_issue = [&](int z) {  // one thread: box of plane group z (plane z jg + jgrp)
         const uint32_t bar = tc::smem_addr(&sm.bar_tma);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(kBoxBytes)
                      : "memory");
         asm volatile(
-            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
-            "%4}], [%5];\n" ::"r"(tc::smem_addr(&sm.box[0][0][0])),
-            "l"((unsigned long long)&tmap), "r"(bx), "r"(by), "r"(z * g.m + jbase), "r"(bar)
+            "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, "
+            "%4, %5}], [%6];\n" ::"r"(tc::smem_addr(&sm.box[0][0])),
+            "l"((unsigned long long)&tmap), "r"(0), "r"(bx), "r"(by), "r"(z * g.jg + jgrp), "r"(bar)
             : "memory");
     };
     __syncthreads();  // barriers initialised
@@ -213,23 +219,26 @@ __global__ void __launch_bounds__(kThr, 1)
         if (tid == 0) sm.seg_first[nseg] = cnt;
     }
     __syncthreads();
-    const int nch = (nseg + kRays - 1) / kRays;
+    // a plane holds zs slices: ray r of slice s is the virtual ray r zs + s,
+    // whose K' row is zero at the other slices' values
+    const int nvs = nseg << zsh, rc = kRays >> zsh;  // virtual rays; rays per chunk
+    const int nch = (nvs + kRays - 1) / kRays;
 
     // B rows of chunk ch into buffer buf: row 2r gives Re G, row 2r+1 Im G of
-    // ray r; K index 2j (Re F_j) and 2j+1 (Im F_j).  Threads 0..255 = (row, 4 K values).
+    // virtual ray r; K index 2v (Re F_v) and 2v+1 (Im F_v).  Threads 0..255 = (row, 4 K values).
     auto stage_b = [&](int ch, int buf) {
         if (tid >= kN * kK / 4) return;
         const int nrow = tid >> 3, q4 = tid & 7;
         const int r = nrow >> 1, o = nrow & 1;
         const int s = ch * kRays + r;
         float bv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (s < nseg) {
-            const int th = sm.th[sm.seg_first[s]];
+        if (s < nvs) {
+            const int th = sm.th[sm.seg_first[s >> zsh]];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
-                const int j = 2 * q4 + i;
+                const int v = 2 * q4 + i, j = zsh ? v & 7 : v;
                 float2 kv = make_float2(0.f, 0.f);
-                if (jbase + j < g.m) kv = __ldg(kmat + (long long)th * g.m + jbase + j);
+                if ((v >> 3) * zsh == (s & zsh) && jbase + j < g.m) kv = __ldg(kmat + (long long)th * g.m + jbase + j);
                 if (o == 0) {
                     bv[2 * i] = kv.x;
                     bv[2 * i + 1] = -kv.y;
@@ -249,7 +258,7 @@ __global__ void __launch_bounds__(kThr, 1)
     // G = A B^T for chunk ch (B in buffer buf), M tile mt, into the
     // accumulator; N = 16 when the chunk has at most 8 rays.
     auto issue = [&](uint32_t tbase, int ch, int buf, int mt) {
-        const int nr = min(kRays, nseg - ch * kRays);
+        const int nr = min(kRays, nvs - ch * kRays);
         const uint32_t IT = nr > 8 ? tc::idesc(tc::kFmtTF32, 128, 32) : tc::idesc(tc::kFmtTF32, 128, 16);
         const uint64_t dh = tc::sdesc(tc::smem_addr(sm.bhi[buf]), 128, 1024);
         const uint64_t dl = tc::sdesc(tc::smem_addr(sm.blo[buf]), 128, 1024);
@@ -282,20 +291,31 @@ __global__ void __launch_bounds__(kThr, 1)
     const int issuer = kThr - 32;
     const int imt = (lane == 0 && wid >= kWarps - kMT) ? wid - (kWarps - kMT) : -1;
 
-    // footprint box of slice z -> A operand in tensor memory (thread = cell)
+    // footprint box of plane group z -> A operand in tensor memory (thread = cell)
     auto convert = [&](int z) {
         ok = tc::mbar_wait(&sm.bar_tma, (uint32_t)((z - z0) & 1), ok) && ok;
+        // values of the plane that hold data (the others are not written)
+        const int nt = min(zsh ? 8 : 16, g.m - jbase);
+        uint32_t live = (1u << nt) - 1u;
+        if (zsh && 2 * z + 1 < zb) live |= live << 8;
         for (int mt = wid >> 2; mt < kMT; mt += kWarps / 4) {
             const int cell = mt * 128 + 32 * q + lane;
             float hi[32], lo[32];
             if (cell < kCells) {
-                const int row = cell / kFW, col = cell - row * kFW;
-                const int br = mirrored ? kFW - 1 - row : row, bc = mirrored ? kFW - col : col;
+                const int bc = mirrored ? kCells - 1 - cell : cell;  // both axes reversed
+                const float4 *b = sm.box[bc];
+                const float sg = mirrored ? -1.f : 1.f;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float2 v = sm.box[j][br][bc];
-                    hi[2 * j] = v.x;
-                    hi[2 * j + 1] = mirrored ? -v.y : v.y;
+                for (int i = 0; i < 8; ++i) {
+                    const float4 f = b[i ^ (bc & 7)];
+                    hi[4 * i] = f.x;
+                    hi[4 * i + 1] = sg * f.y;
+                    hi[4 * i + 2] = f.z;
+                    hi[4 * i + 3] = sg * f.w;
+                }
+                if (live != 0xffffu) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) hi[i] = (live >> (i >> 1)) & 1 ? hi[i] : 0.f;
                 }
             } else {
 #pragma unroll
@@ -329,7 +349,7 @@ __global__ void __launch_bounds__(kThr, 1)
     }
     for (int z = z0; z < z1 && nch > 0; ++z) {
         for (int ch = 0; ch < nch; ++ch) {
-            const int nr = min(kRays, nseg - ch * kRays);
+            const int nr = min(kRays, nvs - ch * kRays);
             ok = tc::mbar_wait(&sm.bar_mma, mma_par, ok) && ok;
             mma_par ^= 1u;
             tc::fence_after();
@@ -373,13 +393,13 @@ __global__ void __launch_bounds__(kThr, 1)
             }
             // ---- samples of this chunk: four threads per sample (rows p, p+4, p+8) ----
             {
-                const int e0 = sm.seg_first[ch * kRays];
-                const int e1 = sm.seg_first[min((ch + 1) * kRays, nseg)];
+                const int e0 = sm.seg_first[ch * rc];
+                const int e1 = sm.seg_first[min((ch + 1) * rc, nseg)];
                 const int part = tid & 3;
-                for (int t = tid >> 2; e0 + t < e1; t += kThr / 4) {
-                    const int e = e0 + t;
+                for (int t = tid >> 2; t < (e1 - e0) << zsh; t += kThr / 4) {
+                    const int e = e0 + (t >> zsh), sl = t & zsh;  // sample and slice of the plane
                     const int pos = sm.pos[e];
-                    const float2 *gp = sm.g[sm.seg_of[e] - ch * kRays] + (pos < 0 ? 0 : pos);
+                    const float2 *gp = sm.g[((sm.seg_of[e] - ch * rc) << zsh) + sl] + (pos < 0 ? 0 : pos);
                     float ex[kTaps];
 #pragma unroll
                     for (int b = 0; b < kTaps; ++b) ex[b] = sm.wx[e][b];
@@ -401,11 +421,12 @@ __global__ void __launch_bounds__(kThr, 1)
                     ay += __shfl_xor_sync(gm, ay, 1);
                     ax += __shfl_xor_sync(gm, ax, 2);
                     ay += __shfl_xor_sync(gm, ay, 2);
-                    if (part == 0 && pos >= 0) {
+                    const int zr = (z << zsh) + sl;
+                    if (part == 0 && pos >= 0 && zr < zb) {
                         const int th = sm.th[e], k = sm.k[e];
                         float2 r = cmul(make_float2(ax, ay), sm.f[e]);
-                        float2 *dst = rows + ((long long)z * g.ntheta + th) * g.n + k;
-                        if (accumulate) {
+                        float2 *dst = rows + ((long long)zr * g.ntheta + th) * g.n + k;
+                        if (jgrp > 0) {
                             const float2 o = *dst;
                             r.x += o.x;
                             r.y += o.y;
@@ -430,33 +451,33 @@ void gather_tc_prepare() {
                                     (int)sizeof(TcSmem)));
 }
 
-void make_spec_tensor_map(CUtensorMap *map, float2 *spec, int nimg, const UsGeo &g) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
-        cudaDriverEntryPointQueryResult q;
-        CUDA_CHECK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&encode, 12000,
-                                                    cudaEnableDefault, &q));
-        if (q != cudaDriverEntryPointSuccess || !encode) throw Error(1, "cuTensorMapEncodeTiled unavailable");
-    }
-    // float view: [images][P + 2 kHalo rows][2 qp floats]
-    const cuuint64_t dims[3] = {(cuuint64_t)2 * g.qp, (cuuint64_t)(g.P + 2 * kHalo), (cuuint64_t)nimg};
-    const cuuint64_t strides[2] = {(cuuint64_t)g.qp * 8, (cuuint64_t)g.img_fwd * 8};
-    const cuuint32_t box[3] = {2 * kBoxW, kFW, 16};
-    const cuuint32_t es[3] = {1, 1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, spec, dims, strides, box, es,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+void make_vec_gather_tc_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g) {
+    PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    CUDA_CHECK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&encode, 12000, cudaEnableDefault,
+                                                &q));
+    if (q != cudaDriverEntryPointSuccess || !encode) throw Error(1, "cuTensorMapEncodeTiled unavailable");
+    // float view: [planes][rows][cells][32]
+    const cuuint64_t dims[4] = {32, (cuuint64_t)g.vp, (cuuint64_t)g.vrows, (cuuint64_t)npl};
+    const cuuint64_t strides[3] = {128, 128ull * g.vp, 8ull * g.vplane};
+    const cuuint32_t box[4] = {32, kFW, kFW, 1};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, spec, dims, strides, box, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error(1, "cuTensorMapEncodeTiled failed for the forward spectra");
+    if (r != CUDA_SUCCESS) throw Error(1, "cuTensorMapEncodeTiled failed for the tensor-core gather's footprints");
 }
 
-void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &tmap, int jbase,
-                      int accumulate, cudaStream_t s) {
+void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &tmap, int jgrp,
+                      cudaStream_t s) {
     if (gd.n_fwd_tc_items == 0) return;
     if (g.T != kT) throw Error(1, "tile size must be 16");
     if (g.zper < 1 || g.zper > kZPer) throw Error(1, "gather slices per block must be in [1, 64]");
-    dim3 gs(gd.n_fwd_tc_items, (zb + g.zper - 1) / g.zper);
+    if (g.zs > 2) throw Error(1, "the tensor-core gather takes at least 8 time samples");
+    const int npz = vec_planes(g, zb) / g.jg, per = std::max(1, g.zper / g.zs);
+    dim3 gs(gd.n_fwd_tc_items, (npz + per - 1) / per);
     k_gather_tc<<<gs, kThr, sizeof(TcSmem), s>>>(rows, gd.fwd_pts, gd.fwd_tc_items, gd.sincos, gd.kmat, gd.shiftfwd,
-                                                 tmap, g, zb, jbase, accumulate, gd.err);
+                                                 tmap, g, zb, npz, per, jgrp, gd.err);
     LAUNCH_CHECK("k_gather_tc");
 }
 

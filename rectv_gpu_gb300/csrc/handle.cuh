@@ -77,14 +77,13 @@ inline int usfft_radius(int n, float *mu_out) {
 struct Layout {
     int P = 0, nchunks = 0, nzc = 0, zb = 0, nbatch = 0;
     bool tc_scatter = false;  // time samples mixed on the tensor cores in the adjoint (k_scatter_tc)
-    bool pad_fft = false;     // hand-written padded-grid 2D FFTs
-    bool gen_fft = false;     // mixed-radix ones on the direction path
-    bool gen_rows = false;    // mixed-radix fused residual rows on the direction path
+    bool pad_fft = false;     // hand-written padded-grid 2D FFTs, 2n a power of two
+    bool gen_fft = false;     // mixed-radix ones
     bool fused_rows = false;  // fused residual rows (k_resid_rows)
+    bool gen_rows = false;    // mixed-radix ones (k_gen_resid)
     bool dirs = false;        // the direction path may run (a geometry decides)
-    bool iter_plans = false;  // the outer iteration runs cuFFT plans (per-ray path)
     int tg = 1, zs = 1, jg = 1;  // vector layout of the direction path (UsGeo)
-    long long slab = 0, gp = 0, img_spec = 0;
+    long long slab = 0, gp = 0;
     size_t spec_elems = 0;
     double bytes = 0;         // estimate of all device memory, geometry included
 };
@@ -105,29 +104,28 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
         if (!std::strcmp(e, "direct")) L.tc_scatter = L.dirs = false;
     {
         const char *e = std::getenv("RECTV_CUFFT");
-        L.pad_fft = pad_fft_supported(L.P) && !(e && std::atoi(e) != 0);
-        L.gen_fft = !pad_fft_supported(L.P) && !(e && std::atoi(e) != 0);
-    }
-    L.fused_rows = L.pad_fft && resid_rows_supported(n);
-    {
+        const bool own = !(e && std::atoi(e) != 0);
         GenPlan p;
-        const char *e = std::getenv("RECTV_CUFFT");
-        L.gen_fft = L.gen_fft && L.dirs && gen_fft_plan(L.P, &p);
-        L.gen_rows = !L.fused_rows && L.dirs && !(e && std::atoi(e) != 0) && gen_fft_plan(n, &p);
+        L.pad_fft = own && pad_fft_supported(L.P);
+        L.gen_fft = own && !L.pad_fft && gen_fft_plan(L.P, &p);
+        L.fused_rows = own && resid_rows_supported(n);
+        L.gen_rows = own && !L.fused_rows && gen_fft_plan(n, &p);
     }
-    L.iter_plans = !(L.pad_fft && L.fused_rows && L.tc_scatter);
-    const long long qp = n + 2 * kHalo + (n & 1);
-    const long long img_fwd = (P + 2 * kHalo) * qp;
-    // the tensor-core scatter fills Hermitian half planes (row pitch P/2+2),
-    // the FP32 scatter full periodic planes
-    L.img_spec = L.tc_scatter ? std::max(img_fwd, P * (P / 2 + 2)) : std::max(img_fwd, P * P);
+    if (m > 16) {
+        L.tg = 16;
+        L.jg = (m + 15) / 16;
+    } else {
+        while (L.tg < m) L.tg *= 2;
+        L.zs = 16 / L.tg;
+    }
+    const long long vec_plane = (P + 2 * kVH) * (n + 1 + kVH + kVR) * 16;
     // batch size: largest zb = nzp*d, d | nchunks, with per-batch scratch under budget
     double budget = batch_bytes;
     if (budget <= 0) {
         budget = 40.0 * (1ull << 30);
         if (const char *e = std::getenv("RECTV_BATCH_BYTES")) budget = std::atof(e);
     }
-    const double per_slice = (double)m * L.img_spec * 8.0 + (double)ntheta * n * 12.0;
+    const double per_slice = (double)vec_plane * L.jg / L.zs * 8.0 + (double)ntheta * n * 12.0;
     int d = 1;
     for (int cand = L.nchunks; cand >= 1; --cand) {
         if (L.nchunks % cand) continue;
@@ -138,18 +136,8 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     }
     L.zb = nzp * d;
     L.nbatch = L.nchunks / d;
-    if (m > 16) {
-        L.tg = 16;
-        L.jg = (m + 15) / 16;
-    } else {
-        while (L.tg < m) L.tg *= 2;
-        L.zs = 16 / L.tg;
-    }
     const long long vec_pl = L.jg > 1 ? (long long)L.zb * L.jg : (L.zb + L.zs - 1) / L.zs;
-    const long long vec_plane = (P + 2 * kVH) * (n + 1 + 2 * kVH) * 16;
-    L.spec_elems = std::max<size_t>(std::max<size_t>((size_t)L.zb * m * (size_t)L.img_spec,
-                                                     L.dirs ? (size_t)(vec_pl * vec_plane) : 0),
-                                    (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
+    L.spec_elems = std::max<size_t>((size_t)(vec_pl * vec_plane), (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
     b += (double)L.zb * nt * 4 + L.spec_elems * 8.0 + (double)L.zb * ntheta * std::max(n, n / 2 + 1) * 8.0;
@@ -158,8 +146,8 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     // geometry: angle plan, adjoint entries (about 2.25 tiles per sample) and records
     b += nt * (4 + 2.5 * 4 + (L.tc_scatter ? 2.5 * 144 + 12 : 0)) + 8.0 * ntheta * m + (1 << 20);
     if (L.pad_fft) b += 16.0 * P * 8;
-    // cuFFT work area when the iteration runs cuFFT (about one batch of 2D planes, at most 8 GiB)
-    if (L.iter_plans) b += std::min(8.0 * (1ull << 30), (double)L.zb * m * P * P * 8.0);
+    // cuFFT's planar images and work area
+    if (!L.pad_fft && !L.gen_fft) b += 3.0 * 64e6;
     L.bytes = b;
     return L;
 }
@@ -208,14 +196,13 @@ struct Handle {
     std::vector<void *> geo_owned;
 
     // cuFFT plans, made as a geometry's path needs them (ensure_plans)
-    enum { kR2C2D, kC2C2D, kC2R2D, kRowsC2C, kRowsR2C, kRowsC2R, kVecR2C, kVecC2R, kNPlans };
+    enum { kR2C2D, kC2R2D, kRowsC2C, kRowsR2C, kRowsC2R, kNPlans };
     cufftHandle plan[kNPlans] = {};
     bool plan_made[kNPlans] = {};
     size_t fft_work_bytes = 0;
-    int vec_slices = 1;          // slices per cuFFT call of the direction path without the hand-written FFTs
-    float2 *planar = nullptr;    // its planar images [vec_slices m][P][n + 2] (geometry)
-    CUtensorMap spec_tmap;  // TMA boxes of the forward spectra (tensor-core gather)
-    CUtensorMap vec_tmap, vec_fft_map;  // vector layout: gather footprints, column FFT tiles
+    int vec_slices = 1;          // slices per 2D cuFFT call (without the hand-written FFTs)
+    float2 *planar = nullptr;    // their planar images [vec_slices m][P][planar_pitch]
+    CUtensorMap dir_tmap, tc_tmap;  // footprint boxes of the direction gather and the tensor-core gather
     // key of the geometry on the device (set_geometry)
     bool geo_valid = false, geo_has_phi = false, geo_tc_scatter = false;
     float geo_center = 0.f, geo_tc_spr = 0.f;
@@ -224,26 +211,22 @@ struct Handle {
     // key of the captured graphs besides the geometry (setup)
     int graph_titer = -1;
     float graph_lambda0 = 0.f, graph_lambda1 = 0.f;
-    int img_per_fft = 0;
     void *fft_work = nullptr;
-    // hand-written padded-grid FFTs (P a power of two in [256, 2048]) instead
-    // of cuFFT + deapodise/pad + crop passes; RECTV_CUFFT=1 selects cuFFT
-    bool pad_fft = false;
-    float2 *fft_tw = nullptr;  // twiddle tables (pad_fft_twiddles)
-    // fused residual rows (inverse row FFT, residual, R2C in one kernel)
-    bool fused_rows = false;
-    float2 *fft_tw_n = nullptr;  // twiddles of the n-point row transforms
-    float2 *rows_adj = nullptr;  // the adjoint's row spectra [zb][ntheta][n/2+1]
-    CUtensorMap fft_fwd_map, fft_inv_map;  // TMA tiles of the column passes
-    // direction path: mixed-radix passes where 2n is no power of two
-    bool gen_fft = false;
+    // padded-grid FFTs: hand-written ones for P a power of two in [256, 2048],
+    // mixed-radix ones for other lengths, else cuFFT with pad, crop and layout
+    // passes (RECTV_CUFFT=1 selects cuFFT)
+    bool pad_fft = false, gen_fft = false;
+    float2 *fft_tw = nullptr;  // twiddle tables (pad_fft_twiddles, gen_fft_twiddles)
     GenPlan gen_plan{};
-    float2 *gen_tw = nullptr;
-    bool gen_rows = false;  // residual rows, length n
+    CUtensorMap fft_map;       // TMA tiles of the column passes (pad_fft)
+    // fused residual rows (inverse row FFT, residual, R2C in one kernel), n a
+    // power of two in [256, 1024] or mixed-radix
+    bool fused_rows = false, gen_rows = false;
+    float2 *fft_tw_n = nullptr;  // twiddles of the n-point row transforms
     GenPlan gen_rplan{};
-    float2 *gen_rtw = nullptr;
-    bool own_rows() const { return fused_rows || (gd.dirs && gen_rows); }
-    bool vec_cufft() const { return !pad_fft && !gen_fft; }  // cuFFT and a layout change instead
+    float2 *rows_adj = nullptr;  // the adjoint's row spectra [zb][ntheta][n/2+1]
+    bool own_rows() const { return fused_rows || gen_rows; }
+    bool own_fft() const { return pad_fft || gen_fft; }
 
     // session
     bool session = false;
@@ -301,11 +284,6 @@ struct Handle {
         ug.m = m;
         ug.P = P;
         ug.hp = P / 2 + 1;
-        ug.hpitch = P / 2 + 1;
-        ug.qp = n + 2 * kHalo + (n & 1);
-        ug.qoff = (long long)kHalo * ug.qp + kHalo;
-        ug.img_fwd = (long long)(P + 2 * kHalo) * ug.qp;
-        ug.img_adj = (long long)P * P;
         ug.tn = (float)(2 * n);
         ug.inv2n = (float)(1.0 / (2.0 * n));
         ug.wexp = (float)(kPiUsfft * kPiUsfft / (double)mu_us);
@@ -319,7 +297,7 @@ struct Handle {
         ug.tg = lay.tg;
         ug.zs = lay.zs;
         ug.jg = lay.jg;
-        ug.vp = n + 1 + 2 * kVH;
+        ug.vp = n + 1 + kVH + kVR;
         ug.vrows = P + 2 * kVH;
         ug.vplane = (long long)ug.vrows * ug.vp * 16;
         slab = lay.slab;
@@ -335,23 +313,11 @@ struct Handle {
         wdual = alloc<float>((size_t)4 * nchunks * gp);
         CUDA_CHECK(cudaMemsetAsync(wdual, 0, sizeof(float) * (size_t)4 * nchunks * gp, stream));
         h1 = alloc<float>((size_t)zb * ntheta * n);
-        // spectra (forward images and the adjoint's half or full planes); also
-        // the float4 gradient scratch of check_adjoints
+        // spectra (forward and the adjoint's half planes); also the float4
+        // gradient scratch of check_adjoints
         spec = alloc<float2>(lay.spec_elems);
-        make_spec_tensor_map(&spec_tmap, spec, zb * m, ug);
-        make_vec_gather_map(&vec_tmap, spec, vec_planes(ug, zb), ug);
-        {  // cuFFT calls of the direction path: as many slices as keep its images near the L2
-            const double img = (double)m * P * (n + 2) * 8.0;
-            vec_slices = (int)std::max(1.0, std::min((double)zb, 64e6 / img));
-            vec_slices = std::max(lay.zs, vec_slices / lay.zs * lay.zs);
-            img_per_fft = zb * m;
-            const double cap = 8.0 * (1ull << 30), one = (double)P * P * 8.0;
-            while (img_per_fft > 1 && img_per_fft * one > cap) {
-                int nx = img_per_fft - 1;
-                while (nx > 1 && (zb * m) % nx) --nx;
-                img_per_fft = nx;
-            }
-        }
+        make_vec_gather_map(&dir_tmap, spec, vec_planes(ug, zb), ug);
+        make_vec_gather_tc_map(&tc_tmap, spec, vec_planes(ug, zb), ug);
         rows = alloc<float2>((size_t)zb * ntheta * (size_t)std::max(n, n / 2 + 1));
 
         tv.n = n;
@@ -371,62 +337,43 @@ struct Handle {
         iter_ctr = alloc<int>(1);
         gd.err = alloc<int>(1);
         CUDA_CHECK(cudaMemsetAsync(gd.err, 0, sizeof(int), stream));
-        {
-            pad_fft = lay.pad_fft;
-            if (pad_fft) {
-                const std::vector<float2> w = pad_fft_twiddles(P);
-                fft_tw = alloc<float2>(w.size());
-                CUDA_CHECK(cudaMemcpyAsync(fft_tw, w.data(), sizeof(float2) * w.size(), cudaMemcpyHostToDevice,
-                                           stream));
-                CUDA_CHECK(cudaStreamSynchronize(stream));
-                ug.hpitch = P / 2 + 2;  // 16-byte half-plane rows for the TMA tiles
-                make_pad_fft_maps(&fft_fwd_map, &fft_inv_map, spec, zb * m, ug);
-                make_vec_fft_map(&vec_fft_map, spec, vec_planes(ug, zb), ug);
-                fused_rows = lay.fused_rows;
-                if (fused_rows) {
-                    const std::vector<float2> wn = pad_fft_twiddles(n);
-                    fft_tw_n = alloc<float2>(wn.size());
-                    CUDA_CHECK(cudaMemcpyAsync(fft_tw_n, wn.data(), sizeof(float2) * wn.size(),
-                                               cudaMemcpyHostToDevice, stream));
-                    rows_adj = alloc<float2>((size_t)zb * ntheta * (size_t)(n / 2 + 1));
-                    CUDA_CHECK(cudaStreamSynchronize(stream));
-                }
-            }
-        }
-        auto gen_table = [&](const GenPlan &p) {
-            const std::vector<float2> w = gen_fft_twiddles(p);
+        auto table = [&](const std::vector<float2> &w) {
             float2 *d = alloc<float2>(w.size());
             CUDA_CHECK(cudaMemcpyAsync(d, w.data(), sizeof(float2) * w.size(), cudaMemcpyHostToDevice, stream));
             CUDA_CHECK(cudaStreamSynchronize(stream));
             return d;
         };
-        if (lay.gen_fft && gen_fft_plan(P, &gen_plan)) {
-            gen_fft = true;
-            gen_tw = gen_table(gen_plan);
+        pad_fft = lay.pad_fft;
+        gen_fft = lay.gen_fft && gen_fft_plan(P, &gen_plan);
+        if (pad_fft) {
+            fft_tw = table(pad_fft_twiddles(P));
+            make_vec_fft_map(&fft_map, spec, vec_planes(ug, zb), ug);
+        } else if (gen_fft) {
+            fft_tw = table(gen_fft_twiddles(gen_plan));
+        } else {  // 2D cuFFT calls: as many slices as keep the planar images near the L2
+            const double img = (double)m * P * planar_pitch(n) * 8.0;
+            vec_slices = (int)std::max(1.0, std::min((double)zb, 64e6 / img));
+            vec_slices = std::max(lay.zs, vec_slices / lay.zs * lay.zs);
+            planar = alloc<float2>((size_t)vec_slices * m * P * planar_pitch(n));
         }
-        if (lay.gen_rows && gen_fft_plan(n, &gen_rplan)) {
-            gen_rows = true;
-            gen_rtw = gen_table(gen_rplan);
+        fused_rows = lay.fused_rows;
+        gen_rows = lay.gen_rows && gen_fft_plan(n, &gen_rplan);
+        if (own_rows()) {
+            fft_tw_n = table(fused_rows ? pad_fft_twiddles(n) : gen_fft_twiddles(gen_rplan));
             rows_adj = alloc<float2>((size_t)zb * ntheta * (size_t)(n / 2 + 1));
         }
         CUDA_CHECK(cudaStreamSynchronize(stream));
     }
 
     // cuFFT plans are made on first need (never during stream capture): the
-    // outer iteration needs them only off the hand-written path
-    // (lay.iter_plans), the operator API, check_adjoints and FBP always.  The
-    // geometry must be set: its path decides which plans run.
+    // outer iteration needs them only where the hand-written transforms do not
+    // run, the operator API, check_adjoints and FBP always (rows).  The geometry
+    // must be set: its path decides which plans run.
     void ensure_plans() {
         bool need[kNPlans] = {};
         need[kRowsR2C] = true;
         need[gd.dirs ? kRowsC2R : kRowsC2C] = true;
-        if (gd.dirs) {
-            need[kVecR2C] = need[kVecC2R] = vec_cufft();
-        } else {
-            need[kR2C2D] = !pad_fft;
-            need[kC2C2D] = !gd.tc_scatter;
-            need[kC2R2D] = gd.tc_scatter && !pad_fft;
-        }
+        need[kR2C2D] = need[kC2R2D] = !own_fft();
         make_fft_plans(need);
     }
 
@@ -448,7 +395,7 @@ struct Handle {
     }
 
     void make_fft_plans(const bool (&need)[kNPlans]) {
-        const int P = 2 * n, per = img_per_fft, nrows = zb * ntheta, hn = n / 2 + 1;
+        const int P = 2 * n, nrows = zb * ntheta, hn = n / 2 + 1, pp = planar_pitch(n);
         size_t ws = fft_work_bytes;
         bool any = false;
         for (int i = 0; i < kNPlans; ++i) {
@@ -468,19 +415,10 @@ struct Handle {
                 CUFFT_CHECK(cufftMakePlanMany(plan[i], rank, nn, in, 1, idist, on, 1, odist, type, batch, &w1));
             };
             switch (i) {
-                case kR2C2D:  // in place inside the padded forward images
-                    make(2, P, 2 * ug.qp, (int)(2 * ug.img_fwd), ug.qp, (int)ug.img_fwd, CUFFT_R2C, per);
+                case kR2C2D:  // in place in the planar images
+                    make(2, P, 2 * pp, 2 * pp * P, pp, pp * P, CUFFT_R2C, vec_slices * m);
                     break;
-                case kC2R2D:  // in place: Hermitian half planes of P/2+1 complex -> real rows of P+2 floats
-                    make(2, P, P / 2 + 1, P * (P / 2 + 1), P + 2, P * (P + 2), CUFFT_C2R, per);
-                    break;
-                case kC2C2D: make(2, P, P, P * P, P, P * P, CUFFT_C2C, per); break;  // full planes
-                case kVecR2C:  // in place, rows of n + 2 complex
-                    make(2, P, 2 * (n + 2), 2 * (n + 2) * P, n + 2, (n + 2) * P, CUFFT_R2C, vec_slices * m);
-                    break;
-                case kVecC2R:
-                    make(2, P, n + 2, (n + 2) * P, 2 * (n + 2), 2 * (n + 2) * P, CUFFT_C2R, vec_slices * m);
-                    break;
+                case kC2R2D: make(2, P, pp, pp * P, 2 * pp, 2 * pp * P, CUFFT_C2R, vec_slices * m); break;
                 case kRowsC2C: make(1, n, n, n, n, n, CUFFT_C2C, nrows); break;
                 case kRowsR2C: make(1, n, 2 * hn, 2 * hn, hn, hn, CUFFT_R2C, nrows); break;  // in place (adjoint)
                 case kRowsC2R: make(1, n, hn, hn, 2 * hn, 2 * hn, CUFFT_C2R, nrows); break;  // in place (forward)
@@ -516,7 +454,6 @@ struct Handle {
         for (void *p : geo_owned) cudaFreeAsync(p, stream);
         geo_owned.clear();
         geo_bytes = 0;
-        planar = nullptr;
         int *err = gd.err;
         gd = GeoDev();
         gd.err = err;
@@ -609,7 +546,7 @@ struct Handle {
             hp.adj_pts = std::move(dplan.adj_pos);
             hp.adj_items = dir_adj_work(dplan.adj_items, vec_planes(ug, zb) / ug.jg);
         } else {
-            hp = build_plan(theta_h, n, ntheta, ug.T, table_capacity(), 1 << 30, tc_min_spr);
+            hp = build_plan(theta_h, n, ntheta, ug.T, table_capacity(), tc_min_spr);
         }
         auto up = [&](const void *src, size_t bytes) -> void * {
             void *p = nullptr;
@@ -630,8 +567,6 @@ struct Handle {
         gd.n_adj_items = (int)hp.adj_items.size();
         gd.n_adj_busy = 0;
         while (gd.n_adj_busy < gd.n_adj_items && hp.adj_items[gd.n_adj_busy].z > 0) ++gd.n_adj_busy;
-        gd.split_tiles = (int *)up(hp.split_tiles.data(), hp.split_tiles.size() * 4);
-        gd.n_split_tiles = (int)hp.split_tiles.size();
         gd.tc_scatter = tc_scatter;
         if (dirs) {
             gd.dirs = true;
@@ -732,14 +667,6 @@ struct Handle {
                 std::copy(kmat.begin() + th * m, kmat.begin() + (th + 1) * m, dk.begin() + (size_t)r * ks);
             }
             gd.dkmat = (float2 *)up(dk.data(), dk.size() * sizeof(float2));
-            if (vec_cufft()) {
-                const size_t bytes = (size_t)vec_slices * m * ug.P * (n + 2) * sizeof(float2);
-                void *p = nullptr;
-                CUDA_CHECK(cudaMallocAsync(&p, bytes, stream));
-                geo_owned.push_back(p);
-                geo_bytes += bytes;
-                planar = (float2 *)p;
-            }
         }
         // set_center (radonusfft.cu:70-75, takeshift kernels_radonusfft.cuh:191-198)
         std::vector<float2> sf(n), sa(n);
@@ -794,41 +721,22 @@ struct Handle {
     // the gathered row spectra of R_apr u (before the inverse row FFT) in rows:
     // whole rows, or their Hermitian halves on the direction path
     void forward_rows(const float *u) {
-        const int nimg = zb * m;
-        if (gd.dirs) {
-            if (pad_fft) {
-                launch_pad_fft_fwd_vec(u, spec, zb, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
-            } else if (gen_fft) {
-                launch_gen_fft_fwd(u, spec, zb, gd.deapod, gen_tw, gen_plan, ug, stream);
-            } else {
-                UsGeo gp2 = ug;  // planar images of rows of n + 2 complex
-                gp2.qp = n + 2;
-                gp2.qoff = 0;
-                gp2.img_fwd = (long long)ug.P * (n + 2);
-                for (int z = 0; z < zb; z += vec_slices) {
-                    const int nzg = std::min(vec_slices, zb - z);
-                    launch_deapod_pad(u + (long long)z * slab, reinterpret_cast<float *>(planar), nzg * m, gd.deapod,
-                                      gp2, stream);
-                    CUFFT_CHECK(cufftExecR2C(plan[kVecR2C], reinterpret_cast<cufftReal *>(planar),
-                                             reinterpret_cast<cufftComplex *>(planar)));
-                    launch_planar_to_vec(planar, spec, z, nzg, ug, stream);
-                }
-            }
-            launch_vec_halo(spec, vec_planes(ug, zb), ug, stream);
-            launch_gather_fwd(spec, rows, zb, gd, ug, &vec_tmap, stream);
-            return;
-        }
         if (pad_fft) {
-            launch_pad_fft_fwd(u, spec, nimg, gd.deapod, fft_tw, fft_fwd_map, gd.err, ug, stream);
+            launch_pad_fft_fwd(u, spec, zb, gd.deapod, fft_tw, fft_map, gd.err, ug, stream);
+        } else if (gen_fft) {
+            launch_gen_fft_fwd(u, spec, zb, gd.deapod, fft_tw, gen_plan, ug, stream);
         } else {
-            launch_deapod_pad(u, reinterpret_cast<float *>(spec), nimg, gd.deapod, ug, stream);
-            for (int i = 0; i < nimg; i += img_per_fft) {
-                cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * ug.img_fwd + ug.qoff);
-                CUFFT_CHECK(cufftExecR2C(plan[kR2C2D], reinterpret_cast<cufftReal *>(p), p));
+            for (int z = 0; z < zb; z += vec_slices) {
+                const int nzg = std::min(vec_slices, zb - z);
+                launch_deapod_pad(u + (long long)z * slab, reinterpret_cast<float *>(planar), nzg * m, gd.deapod, ug,
+                                  stream);
+                CUFFT_CHECK(cufftExecR2C(plan[kR2C2D], reinterpret_cast<cufftReal *>(planar),
+                                         reinterpret_cast<cufftComplex *>(planar)));
+                launch_planar_to_vec(planar, spec, z, nzg, ug, stream);
             }
         }
-        launch_spec_halo(spec, nimg, ug, stream);
-        launch_gather_fwd(spec, rows, zb, gd, ug, &spec_tmap, stream);
+        launch_vec_halo(spec, vec_planes(ug, zb), gd.dirs ? kR + 1 : kVR, ug, stream);
+        launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &dir_tmap : &tc_tmap, stream);
     }
 
     // u += tau R_apr^T h
@@ -842,53 +750,22 @@ struct Handle {
 
     // u += tau R_apr^T of the row spectra rowsc [zb][ntheta][n/2+1]
     void adjoint_rows(const float2 *rowsc, float *u, float tau) {
-        const int nimg = zb * m;
-        if (gd.dirs) {  // Hermitian half planes in the vector layout
-            launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
-            if (pad_fft) {
-                launch_pad_fft_inv_accum_vec(spec, u, zb, tau, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
-                return;
-            }
-            if (gen_fft) {
-                launch_gen_fft_inv_accum(spec, u, zb, tau, gd.deapod, gen_tw, gen_plan, ug, stream);
-                return;
-            }
+        // Re IFFT2 of the scattered grids as a C2R of their Hermitian part
+        launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
+        if (pad_fft) {
+            launch_pad_fft_inv_accum(spec, u, zb, tau, gd.deapod, fft_tw, fft_map, gd.err, ug, stream);
+        } else if (gen_fft) {
+            launch_gen_fft_inv_accum(spec, u, zb, tau, gd.deapod, fft_tw, gen_plan, ug, stream);
+        } else {
             for (int z = 0; z < zb; z += vec_slices) {
                 const int nzg = std::min(vec_slices, zb - z);
                 launch_vec_to_planar(spec, planar, z, nzg, ug, stream);
-                CUFFT_CHECK(cufftExecC2R(plan[kVecC2R], reinterpret_cast<cufftComplex *>(planar),
+                CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], reinterpret_cast<cufftComplex *>(planar),
                                          reinterpret_cast<cufftReal *>(planar)));
                 launch_crop_accum_real(reinterpret_cast<const float *>(planar), u + (long long)z * slab, nzg, tau,
-                                       gd.deapod, 2 * (n + 2), ug, stream);
+                                       gd.deapod, ug, stream);
             }
-            return;
         }
-        if (gd.tc_scatter) {
-            // Re IFFT2 of the scattered grids as a C2R of their Hermitian part,
-            // which the tensor-core scatter adds into zeroed half planes
-            const long long img_half = (long long)ug.P * ug.hpitch;
-            CUDA_CHECK(cudaMemsetAsync(spec, 0, sizeof(float2) * (size_t)nimg * img_half, stream));
-            launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
-            if (pad_fft) {
-                launch_pad_fft_inv_accum(spec, u, zb, tau, gd.deapod, fft_tw, fft_inv_map, gd.err, ug, stream);
-                return;
-            }
-            for (int i = 0; i < nimg; i += img_per_fft) {
-                cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * img_half);
-                CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], p, reinterpret_cast<cufftReal *>(p)));
-            }
-            launch_crop_accum_real(reinterpret_cast<const float *>(spec), u, zb, tau, gd.deapod, ug.P + 2, ug, stream);
-            return;
-        }
-        if (lay.img_spec < (long long)ug.P * ug.P)
-            throw Error(RECTV_ERR_STATE, "rectv: spectra buffer sized for half planes, FP32 scatter needs full planes");
-        launch_zero_split(spec, zb, gd, ug, stream);
-        launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
-        for (int i = 0; i < nimg; i += img_per_fft) {
-            cufftComplex *p = reinterpret_cast<cufftComplex *>(spec + (size_t)i * ug.img_adj);
-            CUFFT_CHECK(cufftExecC2C(plan[kC2C2D], p, p, CUFFT_INVERSE));
-        }
-        launch_crop_accum(spec, u, zb, tau, gd.deapod, ug, stream);
     }
 
     // ---- one outer ADMM iteration (rectv.cu:140-245 for all chunks) ----
@@ -906,7 +783,8 @@ struct Handle {
                     if (fused_rows)
                         launch_resid_rows(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, zb, gd.dirs, ug, stream);
                     else
-                        launch_gen_resid(rows, gdata + z0 * ntheta * n, rows_adj, gen_rtw, gen_rplan, zb, ug, stream);
+                        launch_gen_resid(rows, gdata + z0 * ntheta * n, rows_adj, fft_tw_n, gen_rplan, zb, gd.dirs, ug,
+                                         stream);
                 } else {
                     forward(U[src] + z0 * slab, gdata + z0 * ntheta * n, h1, 1.0f, 1);
                 }
@@ -965,7 +843,7 @@ struct Handle {
         if (titer_ < 0) throw Error(RECTV_ERR_ARG, "rectv: titer must be >= 0");
         if (!phi_h) throw Error(RECTV_ERR_ARG, "rectv: phi is required");
         const bool rebuilt = set_geometry(theta_h, phi_h, center);
-        if (!(own_rows() && (gd.dirs ? !vec_cufft() : pad_fft && gd.tc_scatter))) ensure_plans();
+        if (!own_rows() || !own_fft()) ensure_plans();
         lambda0 = lambda0_;
         set_lambda1(lambda1_);
         titer = titer_;
@@ -1208,30 +1086,23 @@ struct Handle {
     // ---- instrumentation ----
     int jgroups() const { return (m + 15) / 16; }
     void launch_counts(int *kern, int *ffts) const {
-        const int nimg = zb * m;
-        const int f2 = img_per_fft > 0 ? (nimg + img_per_fft - 1) / img_per_fft : 0;
         const int ng = jgroups();
-        // the padded-grid FFTs replace deapodise/pad (crop) and the 2D cuFFT
-        // executions by a row and a column kernel each
-        const bool own2d = gd.dirs ? !vec_cufft() : pad_fft && gd.tc_scatter;
-        const bool ownf = gd.dirs ? !vec_cufft() : pad_fft;
-        // forward: [rows + columns | deapodise/pad], halo, zeroing of the k = 0
-        // samples, per group of 16 time samples the tensor-core gather (8+ time
-        // samples) and the direct one (items with few samples per ray), then the
-        // fused residual rows or the forward epilogue
-        // (direction path: deapodise/pad and the layout change per cuFFT call, no zeroing)
-        const int vcalls = (zb + vec_slices - 1) / vec_slices;
+        const int calls = (zb + vec_slices - 1) / vec_slices;  // 2D cuFFT calls without the hand-written FFTs
+        // forward: rows and columns (deapodise/pad and the layout change per
+        // cuFFT call), halo, then per group of 16 time samples the direction
+        // gather, or after the zeroing of the k = 0 samples the tensor-core
+        // gather (8+ time samples) and the direct one (items with few samples
+        // per ray), then the residual rows or the forward epilogue
         const int gather_k =
             gd.dirs ? (gd.n_dfwd_items > 0 ? ng : 0)
                     : 1 + ng * (((m >= 8 && gd.n_fwd_tc_items > 0) ? 1 : 0) + (gd.n_fwd_items > 0 ? 1 : 0));
-        const int fwd_k = (ownf ? 2 : (gd.dirs ? 2 * vcalls : 1)) + 1 + gather_k + 1;
-        const int fwd_f = (ownf ? 0 : (gd.dirs ? vcalls : f2)) + (own_rows() ? 0 : 1);
-        // adjoint: [row preparation], the zeroing of split tiles (direct scatter),
-        // one scatter per group, then [columns + rows | crop]
-        // (direction path: mixing and scatter per group, the fold of the border)
-        const int adj_k = (own_rows() ? 0 : 1) + ((!gd.dirs && !gd.tc_scatter && gd.n_split_tiles > 0) ? 1 : 0) +
-                          (gd.dirs ? 2 * ng + 1 : ng) + (own2d ? 2 : (gd.dirs ? 2 * vcalls : 1));
-        const int adj_f = (own_rows() ? 0 : 1) + (own2d ? 0 : (gd.dirs ? vcalls : f2));
+        const int fwd_k = (own_fft() ? 2 : 2 * calls) + 1 + gather_k + 1;
+        const int fwd_f = (own_fft() ? 0 : calls) + (own_rows() ? 0 : 1);
+        // adjoint: [row preparation], one scatter per group (direction path: the
+        // mixing and the scatter, and the fold of the border), then columns and
+        // rows (the layout change and the crop per cuFFT call)
+        const int adj_k = (own_rows() ? 0 : 1) + (gd.dirs ? 2 * ng + 1 : ng) + (own_fft() ? 2 : 2 * calls);
+        const int adj_f = (own_rows() ? 0 : 1) + (own_fft() ? 0 : calls);
         // per outer iteration: titer inner steps per batch (forward, graddiv,
         // adjoint), one shrink per batch, the two-stage rho reduction
         *kern = titer * nbatch * (fwd_k + 1 + adj_k) + nbatch + 2;
@@ -1247,9 +1118,9 @@ struct Handle {
                 *bytes = (double)zb * m * P * (P / 2 + 1) * 8.0 + (double)zb * ntheta * n * 8.0;
                 *flops = npts * (81.0 * 2.0 * m * 2.0 + 8.0 * m + 18.0 * 4.0);
                 break;
-            case 1:  // scatter: half row spectra in; Hermitian half planes out (tensor-core path), else full planes
+            case 1:  // scatter: half row spectra in, Hermitian half planes out
                 *bytes = (double)zb * ntheta * (n / 2 + 1) * 8.0 +
-                         (gd.dirs || gd.tc_scatter ? (double)zb * m * P * (P / 2 + 1) * 8.0 : (double)zb * m * P * P * 8.0);
+                         (double)zb * m * P * (P / 2 + 1) * 8.0;
                 *flops = npts * (81.0 * 2.0 * m * 2.0 + 8.0 * m + 18.0 * 4.0);
                 break;
             case 2:  // graddiv after the first inner step: u in, u out, w in (psi and mu when titer = 1)
@@ -1283,11 +1154,11 @@ struct Handle {
         check_live();
         if (!session) throw Error(RECTV_ERR_STATE, "rectv_launch_kernel: needs a set-up session");
         if (which < 0 || which > 6) throw Error(RECTV_ERR_ARG, "rectv_launch_kernel: unknown kernel id");
-        if ((which == 4 || which == 5) && !pad_fft)
+        if ((which == 4 || which == 5) && !own_fft())
             throw Error(RECTV_ERR_ARG, "rectv_launch_kernel: no padded-grid FFT at this size");
         for (int r = 0; r < reps; ++r) {
             switch (which) {
-                case 0: launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &vec_tmap : &spec_tmap, stream); break;
+                case 0: launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &dir_tmap : &tc_tmap, stream); break;
                 case 1: launch_scatter_adj(own_rows() ? rows_adj : rows, spec, zb, gd, ug, stream); break;
                 case 2:  // the inner steps after the first (w = mu - rho psi as stored by the last iteration)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 2 : 0, rho_d, 0,
@@ -1297,22 +1168,22 @@ struct Handle {
                     launch_shrink(U[cur], U[cur], psi, mu, rho_d, lambda0, 0, nchunks, tv, partials, stream);
                     break;
                 case 4:  // padded-grid forward FFT of the batch (rows + columns)
-                    if (gd.dirs)
-                        launch_pad_fft_fwd_vec(U[cur], spec, zb, gd.deapod, fft_tw, vec_fft_map, gd.err, ug, stream);
+                    if (pad_fft)
+                        launch_pad_fft_fwd(U[cur], spec, zb, gd.deapod, fft_tw, fft_map, gd.err, ug, stream);
                     else
-                        launch_pad_fft_fwd(U[cur], spec, zb * m, gd.deapod, fft_tw, fft_fwd_map, gd.err, ug, stream);
+                        launch_gen_fft_fwd(U[cur], spec, zb, gd.deapod, fft_tw, gen_plan, ug, stream);
                     break;
                 case 6:  // the first inner step (psi, mu in; stores w = mu - rho psi, unchanged values)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 1 : 0, rho_d, 0,
                                    nchunks, tv, stream);
                     break;
                 case 5:  // padded-grid inverse FFT (columns + rows), added into the scratch iterate
-                    if (gd.dirs)
-                        launch_pad_fft_inv_accum_vec(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, vec_fft_map,
-                                                     gd.err, ug, stream);
+                    if (pad_fft)
+                        launch_pad_fft_inv_accum(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, fft_map, gd.err, ug,
+                                                 stream);
                     else
-                        launch_pad_fft_inv_accum(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, fft_inv_map,
-                                                 gd.err, ug, stream);
+                        launch_gen_fft_inv_accum(spec, U[(cur + 1) % 3], zb, 0.f, gd.deapod, fft_tw, gen_plan, ug,
+                                                 stream);
                     break;
                 default: throw Error(RECTV_ERR_ARG, "rectv_launch_kernel: unknown kernel id");
             }

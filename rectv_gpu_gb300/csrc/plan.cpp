@@ -58,7 +58,7 @@ void parallel_for(int nthr, F &&fn) {
 }
 }  // namespace
 
-HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, int adj_cap, float tc_min_spr) {
+HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, float tc_min_spr) {
     HostPlan p;
     const int P = 2 * n;
     const int NT = (P + T - 1) / T;
@@ -182,18 +182,7 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, i
             i = j;
         }
     }
-    for (int t = 0; t < ntiles; ++t) {
-        const int c = acnt[t];
-        if (c == 0) {
-            p.adj_items.push_back(make_int4(t, (int)aoff[t], 0, 0));
-            continue;
-        }
-        const int nit = (c + adj_cap - 1) / adj_cap;
-        const int split = nit > 1 ? 1 : 0;
-        if (split) p.split_tiles.push_back(t);
-        for (int st = 0; st < c; st += adj_cap)
-            p.adj_items.push_back(make_int4(t, (int)(aoff[t] + st), std::min(adj_cap, c - st), split));
-    }
+    for (int t = 0; t < ntiles; ++t) p.adj_items.push_back(make_int4(t, (int)aoff[t], acnt[t], 0));
     // heaviest tiles first, so that they do not finish last
     std::stable_sort(p.adj_items.begin(), p.adj_items.end(),
                      [](const int4 &a, const int4 &b) { return a.z > b.z; });
@@ -272,7 +261,7 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
     // starts kVH cells before cell 0, so they never leave it), direction-major
     // inside a tile
     const int P = 2 * n, nh = n / 2;
-    const int NT = (P + T - 1) / T, WX = (n + 1 + 2 * kVH + T - 1) / T, WY = (P + 2 * kVH + T - 1) / T;
+    const int NT = (P + T - 1) / T, WX = (n + 1 + kVH + kVR + T - 1) / T, WY = (P + 2 * kVH + T - 1) / T;
     const int ntiles = NT * NT, nwin = WX * WY;
     const float tn = (float)(2 * n);
     std::vector<float> qk(n);

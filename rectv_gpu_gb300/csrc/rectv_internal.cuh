@@ -4,8 +4,8 @@
 //   volume  u  [z][t][y][x]            z < nz, t < m (time samples), y,x < n
 //   data    g  [z][theta][s]           s < n (detector)
 //   dual    psi, mu: SoA [4][chunk][qz][qt][qy][qx], qz<=nzp, qt<=m, qy,qx<=n
-//   spectra half-plane R2C images [z][t][P][P/2+1] complex (forward) or full
-//           periodic planes [z][t][P][P] complex (adjoint), P = 2n
+//   spectra half planes of P x (n+1) complex, P = 2n, 16 (slice, time sample)
+//           values per cell (UsGeo)
 //   rows    [z][theta][n] complex (forward), [z][theta][n+2] real / n/2+1
 //           complex in-place R2C (adjoint)
 #pragma once
@@ -24,8 +24,6 @@ namespace rectv {
 // kernels are specialised for it and the host checks the formula.
 constexpr int kR = 4;
 constexpr int kTaps = 2 * kR + 1;
-// halo of the stored forward spectra (see UsGeo::qp)
-constexpr int kHalo = 24;
 // The USFFT kernels of the reference use this truncated value of pi
 // (kernels_radonusfft.cuh:1).
 constexpr double kPiUsfft = 3.1415926535;
@@ -46,16 +44,6 @@ struct UsGeo {
     int n, ntheta, m;   // detector width, projections, time samples
     int P;              // oversampled grid side 2n
     int hp;             // half-plane row length P/2+1 (complex)
-    int hpitch;         // row pitch of the adjoint's Hermitian half planes (complex):
-                        // P/2+1, or P/2+2 (16-byte rows for TMA) with the padded-grid FFTs
-    // Forward spectra are stored as the window rows [-kHalo, P+kHalo) x
-    // columns [-kHalo, n+kHalo) of the periodic full spectrum: the R2C output
-    // (rows [0,P), columns [0,n]) plus a halo of wrapped / Hermitian-mirrored
-    // cells, so that every tile footprint is one rectangular box.
-    int qp;             // row pitch of a forward image (complex), even
-    long long qoff;     // offset of cell (0, 0) in a forward image
-    long long img_fwd;  // complex elements per forward image ((P + 2 kHalo) qp)
-    long long img_adj;  // complex elements per adjoint image (P*P)
     float tn;           // (float)(2n)
     float inv2n;        // 1/(2n)
     float wexp;         // pi^2/mu
@@ -67,24 +55,34 @@ struct UsGeo {
     // scatter (0: one per SM)
     int zper;
     int sc_grid;
-    // Vector layout of the direction path (scatter_dir.cu): the spectra of 16
-    // (slice, time sample) pairs are stored together, cell by cell:
-    // [plane][row][column][16] complex over the window rows [-kVH, P + kVH) x
-    // columns [-kVH, n + kVH] of the half plane.  One plane holds tg time
-    // samples (1, 2, 4, 8 or 16, at least m) of zs = 16 / tg slices; with
-    // m > 16 a slice takes jg = ceil(m / 16) planes of 16 samples.
+    // Vector layout of the spectra: the half planes of 16 (slice, time sample)
+    // pairs are stored together, cell by cell: [plane][row][column][16] complex
+    // over the window rows [-kVH, P + kVH) x columns [-kVH, n + kVR].  One plane
+    // holds tg time samples (1, 2, 4, 8 or 16, at least m) of zs = 16 / tg
+    // slices; with m > 16 a slice takes jg = ceil(m / 16) planes of 16 samples.
+    // The halo around rows [0, P) x columns [0, n] holds the periodic
+    // spectrum's wrapped and Hermitian-mirrored cells, so that every tile's
+    // footprint is one rectangular box.
     int tg, zs, jg;
-    int vp;             // row pitch in cells: n + 1 + 2 kVH
+    int vp;             // row pitch in cells: n + 1 + kVH + kVR
     int vrows;          // P + 2 kVH
     long long vplane;   // complex elements per plane
 };
 
-// halo cells of the vector layout (a stencil and its mirror image reach from
-// 4 cells before to 5 cells after the origin)
-constexpr int kVH = 8;
+// halo cells of the vector layout: a stencil and its mirror image reach from 4
+// cells before to 5 cells after the origin; the per-ray gather's footprints
+// read up to 16 columns past the half plane
+constexpr int kVH = 8, kVR = 16;
 __host__ __device__ inline int vec_planes(const UsGeo &g, int zb) {  // planes of zb slices
     return g.jg > 1 ? zb * g.jg : (zb + g.zs - 1) / g.zs;
 }
+// planes of slice z, group jgrp of 16 time samples, and the slice's first entry there
+__host__ __device__ inline long long vec_plane_of(const UsGeo &g, int z, int jgrp) {
+    return g.jg > 1 ? (long long)z * g.jg + jgrp : z / g.zs;
+}
+__host__ __device__ inline int vec_entry(const UsGeo &g, int z) { return g.jg > 1 ? 0 : (z % g.zs) * g.tg; }
+// floats per row of the planar images cuFFT transforms (even: 16-byte rows), in complex
+__host__ __device__ inline int planar_pitch(int n) { return n + 2 + (n & 1); }
 // slice and time sample of entry v of plane pl
 __host__ __device__ inline int vec_slice(const UsGeo &g, int pl, int v) {
     return g.jg > 1 ? pl / g.jg : pl * g.zs + v / g.tg;
@@ -118,10 +116,8 @@ struct GeoDev {
     int4 *fwd_tc_items = nullptr; // (tile, start, count, rays): tensor-core gather (k_gather_tc)
     int n_fwd_tc_items = 0;
     uint32_t *adj_pts = nullptr; // point ids, one entry per tile a stencil touches
-    int4 *adj_items = nullptr;   // (tile, start, count, split)
+    int4 *adj_items = nullptr;   // (tile, start, count, 0), whole tiles
     int n_adj_items = 0;
-    int *split_tiles = nullptr;  // tiles with more than one adjoint item
-    int n_split_tiles = 0;
     int *err = nullptr;          // device counter of host/device bin disagreements
     bool tc_scatter = false;     // adjoint time-sample mixing on the tensor cores (k_scatter_tc)
     AdjRec *adj_recs = nullptr;  // geometry records of adj_pts (tensor-core scatter only)
@@ -159,13 +155,12 @@ struct HostPlan {
     std::vector<int4> fwd_tc_items;
     std::vector<uint32_t> adj_pts;
     std::vector<int4> adj_items;
-    std::vector<int> split_tiles;
 };
 
 // Forward work items hold whole rays of one tile and at most fwd_cap samples;
 // an item with at least tc_min_spr samples per ray goes to the tensor-core
 // gather (tc_min_spr < 0: none does).
-HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, int adj_cap, float tc_min_spr);
+HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, float tc_min_spr);
 
 // Rays grouped by direction (theta modulo pi), for scans that revisit their
 // angles over several half-turns: the rays of one direction sample the same
@@ -200,10 +195,9 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
 __host__ __device__ constexpr int adj_info_words(int nseg) { return (4 + 8 * nseg + (nseg + 2) / 2 + 3) & ~3; }
 
 // ---- USFFT kernel launchers (usfft_kernels.cu) ----
-void launch_deapod_pad(const float *u, float *spec, int nimg, const float *deapod, const UsGeo &g,
+// deapodised, padded and modulated images for cuFFT's R2C (planar_pitch)
+void launch_deapod_pad(const float *u, float *planar, int nimg, const float *deapod, const UsGeo &g,
                        cudaStream_t s);
-// fill the halo of nimg forward spectra after the R2C transform
-void launch_spec_halo(float2 *spec, int nimg, const UsGeo &g, cudaStream_t s);
 void launch_gather_fwd(const float2 *spec, float2 *rows, int zb, const GeoDev &gd, const UsGeo &g,
                        const CUtensorMap *tmap, cudaStream_t s);
 void launch_finish_fwd(const float2 *rows, const float *gdata, float *out, int zb, float tau,
@@ -212,26 +206,19 @@ void launch_finish_fwd(const float2 *rows, const float *gdata, float *out, int z
 void launch_finish_fwd_real(const float *rows, const float *gdata, float *out, int zb, float tau, int residual,
                             const UsGeo &g, cudaStream_t s);
 void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaStream_t s);
-void launch_zero_split(float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
 void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
                         const UsGeo &g, cudaStream_t s);
-void launch_crop_accum(const float2 *spec, float *u, int zb, float tau, const float *deapod,
-                       const UsGeo &g, cudaStream_t s);
-// the same from the real output of the C2R inverse (rows of 2 (P/2+1) floats)
-// (rowf: floats per row, 2 (P/2+1), or 2 (n+2) on the direction path)
-void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, int rowf,
-                            const UsGeo &g, cudaStream_t s);
+// cropped, deapodised and added into u, from cuFFT's C2R output (rows of 2 planar_pitch floats)
+void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, const UsGeo &g,
+                            cudaStream_t s);
 // tensor-core gather (gather_tc.cu): items of fwd_tc_items, time samples
-// [jbase, jbase + 16)
-void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &tmap, int jbase,
-                      int accumulate, cudaStream_t s);
-// TMA descriptor of the forward spectra of a batch (zb*m images), boxes of
-// 16 images x 24 rows x 26 cells
-void make_spec_tensor_map(CUtensorMap *map, float2 *spec, int nimg, const UsGeo &g);
+// [16 jgrp, 16 jgrp + 16)
+void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &tmap, int jgrp,
+                      cudaStream_t s);
 void gather_tc_prepare();
-// tensor-core scatter (scatter_tc.cu): all adjoint items, time samples [jbase, jbase + 16),
-// added into the zeroed Hermitian half planes [z][t][P][P/2+1] of the C2R inverse
-void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jbase,
+// tensor-core scatter (scatter_tc.cu): all adjoint items, time samples [16 jgrp, 16 jgrp + 16),
+// added into the zeroed Hermitian half planes of the C2R inverse
+void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jgrp,
                        cudaStream_t s);
 void scatter_tc_prepare();
 void launch_adj_records(AdjRec *recs, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
@@ -248,12 +235,16 @@ void launch_adj_tabinfo(const GeoDev &gd, cudaStream_t s);
 void launch_gather_dir(float2 *hrows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &vmap,
                        cudaStream_t s);
 void launch_scatter_dir(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
-// TMA descriptor of the gather's footprints in the vector layout (npl planes)
+// TMA descriptors of the gathers' footprints in the vector layout (npl planes):
+// the direction path's 25x25 cells, the per-ray tensor-core gather's 24x24
+// cells with 128-byte swizzle
 void make_vec_gather_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
-// fills the halo of the forward spectra in the vector layout
-void launch_vec_halo(float2 *spec, int npl, const UsGeo &g, cudaStream_t s);
-// cuFFT's spectra of slices z0 .. z0 + nz - 1 (planar, rows of n + 2 complex,
-// image (z - z0) m + t) into the vector layout, and back
+void make_vec_gather_tc_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
+// fills the halo of the forward spectra (right: columns past the half plane, 5
+// on the direction path, kVR per ray)
+void launch_vec_halo(float2 *spec, int npl, int right, const UsGeo &g, cudaStream_t s);
+// cuFFT's spectra of slices z0 .. z0 + nz - 1 (planar, rows of planar_pitch
+// complex, image (z - z0) m + t) into the vector layout, and back
 void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, const UsGeo &g, cudaStream_t s);
 void launch_vec_to_planar(const float2 *spec, float2 *planar, int z0, int nz, const UsGeo &g, cudaStream_t s);
 void gather_dir_prepare();    // kernel attributes; once, outside stream capture
@@ -263,26 +254,19 @@ int dir_fwd_capacity();       // position pairs per forward item
 // end plane << 16) of a plan's (tile, start, count), the most work first
 std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz);
 size_t dir_mix_bytes(const UsGeo &g, int zb, int ndir);  // the adjoint's per-position mixing buffer
-// hand-written 2D FFTs of the zero-padded grids (fft_kernels.cu), P = 2n a
-// power of two in [256, 2048]: forward = deapodise/pad/modulate + R2C into
-// the halo-padded spectra (halo not filled); inverse = C2R of the Hermitian
-// half planes [img][P][hpitch] (overwritten) + crop/deapodise, u += tau * ...
+// hand-written 2D FFTs of the zero-padded grids in the vector layout
+// (fft_kernels.cu), P = 2n a power of two in [256, 2048]: forward =
+// deapodise/pad/modulate + R2C (halo not filled); inverse = C2R of the
+// Hermitian half planes (overwritten) + crop/deapodise, u += tau * ...
 bool pad_fft_supported(int P);
 void pad_fft_prepare();
 std::vector<float2> pad_fft_twiddles(int P);
-// TMA descriptors of the column passes over the spectra buffer (nimg images)
-void make_pad_fft_maps(CUtensorMap *fwd, CUtensorMap *inv, float2 *spec, int nimg, const UsGeo &g);
-void launch_pad_fft_fwd(const float *u, float2 *spec, int nimg, const float *deapod, const float2 *tw,
-                        const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
-// the forward pass into the vector layout (halo not filled)
+// TMA descriptor of the column passes over the spectra (npl planes)
 void make_vec_fft_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g);
-void launch_pad_fft_fwd_vec(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
-                            const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
+void launch_pad_fft_fwd(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw,
+                        const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
-// the same from half planes in the vector layout (make_vec_fft_map)
-void launch_pad_fft_inv_accum_vec(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
-                                  const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 // mixed-radix passes for grid sides that are no power of two (fft_general.cuh,
 // fft_general_fwd.cu, fft_general_inv.cu): even lengths 32 .. 2048 with prime
 // factors up to 13
@@ -305,9 +289,9 @@ void launch_gen_fft_fwd(const float *u, float2 *spec, int zb, const float *deapo
                         const UsGeo &g, cudaStream_t s);
 void launch_gen_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,
                               const GenPlan &p, const UsGeo &g, cudaStream_t s);
-// launch_resid_rows on Hermitian half rows, p and tw of length n
+// launch_resid_rows, p and tw of length n
 void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
-                      const UsGeo &g, cudaStream_t s);
+                      bool half, const UsGeo &g, cudaStream_t s);
 // fused residual rows of the inner step (fft_kernels.cu), n a power of two in
 // [256, 1024]: gathered rows [z][theta][n] and data g -> the adjoint's row
 // spectra [z][theta][n/2+1] (inverse row FFT, residual, fftshift, R2C)
@@ -317,8 +301,6 @@ void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, cons
                        const UsGeo &g, cudaStream_t s);
 size_t gather_tc_smem();
 int gather_tc_table_capacity();
-size_t gather_fwd_smem(const UsGeo &g);
-size_t scatter_adj_smem(const UsGeo &g);
 void usfft_prepare();  // kernel attributes; call once, outside stream capture
 int table_capacity();  // samples per gather work item
 

@@ -524,7 +524,7 @@ __global__ void k_vec_fold(float4 *__restrict__ spec, UsGeo g) {
 
 // ---------------------------------------------------------------------------
 // The vector layout's half planes of slices z0 .. z0 + nz - 1 into planar ones
-// (rows of n + 2 complex) for cuFFT's C2R: k_planar_to_vec reversed.
+// (rows of planar_pitch complex) for cuFFT's C2R: k_planar_to_vec reversed.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     k_vec_to_planar(const float4 *__restrict__ spec, float2 *__restrict__ planar, UsGeo g, int z0, int nz, int pl0) {
@@ -537,12 +537,13 @@ __global__ void __launch_bounds__(256)
         sh[cell][2 * ci + 1] = hi2(f);
     }
     __syncthreads();
-    const long long img = (long long)g.P * (g.n + 2);
+    const int pitch = planar_pitch(g.n);
+    const long long img = (long long)g.P * pitch;
     const int lane = threadIdx.x & 31, x = x0 + lane;
     for (int v = threadIdx.x >> 5; v < 16; v += 8) {
         const int z = vec_slice(g, pl, v), t = vec_time(g, pl, v);
         if (x <= g.n && z < z0 + nz && t < g.m)
-            planar[((long long)(z - z0) * g.m + t) * img + (long long)y * (g.n + 2) + x] = sh[lane][v];
+            planar[((long long)(z - z0) * g.m + t) * img + (long long)y * pitch + x] = sh[lane][v];
     }
 }
 

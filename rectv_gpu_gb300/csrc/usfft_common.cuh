@@ -47,4 +47,24 @@ __device__ __forceinline__ void tap_weights(int f, float p0, const UsGeo &g, flo
     for (int i = 0; i < kTaps; ++i) e[i] = tap_weight(f, i, p0, g);
 }
 
+// Adds samples (j, j + 1) of cell (KX, KY)'s sum X(k) to the zeroed Hermitian half
+// planes of the C2R inverse (base: the slice's entry of its plane): the adjoint
+// only needs Re IFFT2(X), the C2R of H(k) = (X(k) + conj X(-k)) / 2 on kx <= n,
+// so X(k)/2 goes to H(k) and conj(X(k))/2 to H(-k) where they lie in the half
+// plane (at most two adds per value, onto zeros: the sum does not depend on
+// their order).  v is X / 2 with the pre-IFFT fftshift sign.  ONE: sample j alone.
+template <bool ONE>
+__device__ __forceinline__ void add_hermitian(float2 *__restrict__ base, const UsGeo &g, int KX, int KY, int j,
+                                              const float4 &v) {
+    const int P = g.P, half = P / 2;
+    if (KY >= P || KX >= P) return;
+    auto add = [&](int X, int Y, const float4 &a) {
+        float2 *d = base + ((long long)(Y + kVH) * g.vp + X + kVH) * 16 + j;
+        if constexpr (ONE) atomicAdd(d, make_float2(a.x, a.y));
+        else atomicAdd(reinterpret_cast<float4 *>(d), a);
+    };
+    if (KX <= half) add(KX, KY, v);
+    if (KX >= half || KX == 0) add(KX ? P - KX : 0, KY ? P - KY : 0, make_float4(v.x, -v.y, v.z, -v.w));
+}
+
 }  // namespace rectv

@@ -30,6 +30,11 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
 }
 
+__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
@@ -37,19 +42,18 @@ __device__ __forceinline__ void cp_async_wait_all() {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Forward: deapodise, zero-pad to P x P and modulate by (-1)^(X+Y)
-// (divphi + fftshift, kernels_radonusfft.cuh:4-38), writing the real input of
-// the in-place R2C transform: row Y of image img starts at complex element
-// img_fwd*img + qoff + Y*qp (2*qp floats per row; the P reals are written).
-// One block per row, 16-byte stores; rows outside the image are zeros.
+// Forward without the hand-written FFTs: deapodise, zero-pad to P x P and
+// modulate by (-1)^(X+Y) (divphi + fftshift, kernels_radonusfft.cuh:4-38),
+// writing the real input of cuFFT's in-place R2C: rows of 2 planar_pitch(n)
+// floats.  One block per row, 16-byte stores; rows outside the image are zeros.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-    k_deapod_pad(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp, UsGeo g,
+    k_deapod_pad(const float *__restrict__ u, float2 *__restrict__ planar, const float *__restrict__ dp, UsGeo g,
                  float inv4n2) {
     const int Y = blockIdx.x;
     const long long img = blockIdx.y;
     const int n = g.n;
-    float2 *row = spec + img * g.img_fwd + g.qoff + (long long)Y * g.qp;  // 16-byte aligned (qp, qoff even)
+    float2 *row = planar + (img * g.P + Y) * planar_pitch(n);  // 16-byte aligned
     float4 *row4 = reinterpret_cast<float4 *>(row);
     const int n4 = n / 2;  // float4 stores: reals 4i .. 4i+3
     const int y = Y - n / 2;
@@ -73,56 +77,12 @@ __global__ void __launch_bounds__(256)
     if ((n & 1) && threadIdx.x == 0) row[n - 1] = make_float2(val(2 * n - 2), val(2 * n - 1));
 }
 
-void launch_deapod_pad(const float *u, float *spec, int nimg, const float *deapod, const UsGeo &g,
+void launch_deapod_pad(const float *u, float *planar, int nimg, const float *deapod, const UsGeo &g,
                        cudaStream_t s) {
     dim3 gs(g.P, nimg);
     const float inv4n2 = (float)(1.0 / (4.0 * g.n * (double)g.n));
-    k_deapod_pad<<<gs, 256, 0, s>>>(u, reinterpret_cast<float2 *>(spec), deapod, g, inv4n2);
+    k_deapod_pad<<<gs, 256, 0, s>>>(u, reinterpret_cast<float2 *>(planar), deapod, g, inv4n2);
     LAUNCH_CHECK("k_deapod_pad");
-}
-
-// ---------------------------------------------------------------------------
-// Halo of the stored forward spectra: cell (y, x) of the window rows
-// [-kHalo, P+kHalo) x columns [-kHalo, n+kHalo) outside the R2C output gets
-// the periodic full-spectrum value F(y mod P, x mod P), read through the
-// Hermitian symmetry F(a, b) = conj F(-a, -b) of a real input when b > n.
-// One thread per halo cell: 2 kHalo full rows, then 2 kHalo - 1 columns of
-// every interior row.
-// ---------------------------------------------------------------------------
-__global__ void k_spec_halo(float2 *__restrict__ spec, UsGeo g) {
-    const int P = g.P, n = g.n;
-    const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    const long long wide = (long long)(2 * kHalo) * g.qp;  // cells of the full halo rows
-    const int side = g.qp - (n + 1);                        // halo columns of an interior row
-    if (e >= wide + (long long)P * side) return;
-    int y, x;
-    if (e < wide) {
-        const int r = (int)(e / g.qp);
-        x = (int)(e - (long long)r * g.qp) - kHalo;
-        y = (r < kHalo) ? r - kHalo : P + (r - kHalo);
-    } else {
-        const long long e2 = e - wide;
-        y = (int)(e2 / side);
-        const int c = (int)(e2 - (long long)y * side);
-        x = (c < kHalo) ? c - kHalo : n + 1 + (c - kHalo);
-    }
-    float2 *img = spec + (long long)blockIdx.y * g.img_fwd + g.qoff;
-    const int a = ((y % P) + P) % P, b = ((x % P) + P) % P;
-    float2 v;
-    if (b <= n) {
-        v = img[(long long)a * g.qp + b];
-    } else {
-        v = img[(long long)((P - a) % P) * g.qp + (P - b)];
-        v.y = -v.y;
-    }
-    img[(long long)y * g.qp + x] = v;
-}
-
-void launch_spec_halo(float2 *spec, int nimg, const UsGeo &g, cudaStream_t s) {
-    const long long cells = (long long)(2 * kHalo) * g.qp + (long long)g.P * (g.qp - (g.n + 1));
-    dim3 gs((unsigned)((cells + 255) / 256), nimg);
-    k_spec_halo<<<gs, 256, 0, s>>>(spec, g);
-    LAUNCH_CHECK("k_spec_halo");
 }
 
 // ---------------------------------------------------------------------------
@@ -175,8 +135,8 @@ __global__ void __launch_bounds__(kThreads)
     k_gather_fwd(const float2 *__restrict__ spec, float2 *__restrict__ rows,
                  const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
                  const float2 *__restrict__ sincos, const float2 *__restrict__ kmat,
-                 const float2 *__restrict__ shiftf, UsGeo g, int jbase, int accumulate,
-                 int *__restrict__ err) {
+                 const float2 *__restrict__ shiftf, UsGeo g, int jgrp, int *__restrict__ err) {
+    const int jbase = 16 * jgrp;
     constexpr int TW = T + 2 * kR;
     constexpr int EPW = 32 / MP;  // samples per warp
     extern __shared__ float4 smraw[];
@@ -187,19 +147,21 @@ __global__ void __launch_bounds__(kThreads)
     const int tyi = it.x / g.NT, txi = it.x - tyi * g.NT;
     const int P = g.P, half = P / 2;
     const int count = it.z;
-    const float2 *img0 = spec + (long long)z * g.m * g.img_fwd;
+    const float2 *img0 = spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
 
-    // ---- stage the tile with asynchronous copies, one time-sample plane at
-    // a time with consecutive threads on consecutive cells (coalesced reads).
-    // Cell c, time sample j sits at float2 c*MP + (j ^ (column & (MP-1))): the
-    // XOR swizzle keeps both these stores and the compute loop's 128-byte rows
-    // free of bank conflicts.  The post-FFT fftshift sign (-1)^(X+Y) of a cell
+    // ---- stage the tile with asynchronous copies (a cell's MP time samples
+    // are contiguous; consecutive threads copy consecutive pairs of samples).
+    // Cell c, time sample j sits at float2 c*MP + j, so the MP lanes of a sample
+    // read one contiguous run at constant offsets from the stencil origin (8 slices of
+    // 720 angles, width 256, 4 samples: 0.277 ms; 8-byte copies by cell and swizzled
+    // slots 0.322).  The post-FFT fftshift sign (-1)^(X+Y) of a cell
     // is (-1)^(column+row) of its tile position, and cells right of the
     // Nyquist column are read through the Hermitian symmetry of the real-input
     // FFT (conjugated); both signs are folded into the tap weights. ----
     {
-        constexpr int NC = TW * TW;
-        for (int cell = threadIdx.x; cell < NC; cell += blockDim.x) {
+        constexpr int W = MP > 1 ? 2 : 1, NC = TW * TW * (MP / W);
+        for (int i = threadIdx.x; i < NC; i += blockDim.x) {
+            const int cell = i / (MP / W), j = W * (i - cell * (MP / W));
             const int row = cell / TW, col = cell - row * TW;
             int KY = tyi * T - kR + row;
             KY += (KY < 0) ? P : 0;
@@ -207,15 +169,15 @@ __global__ void __launch_bounds__(kThreads)
             int KX = txi * T - kR + col;
             KX += (KX < 0) ? P : 0;
             KX -= (KX >= P) ? P : 0;
-            const long long so = g.qoff + ((KX <= half) ? (long long)KY * g.qp + KX
-                                                        : (long long)(KY ? P - KY : 0) * g.qp + (P - KX));
-            const float2 *src = img0 + (long long)jbase * g.img_fwd + so;
-            float2 *dst = tile + cell * MP;
-            const int sw = col & (MP - 1);
-#pragma unroll 4
-            for (int j = 0; j < MP; ++j) {
-                if (jbase + j < g.m) cp_async8(dst + (j ^ sw), src + (long long)j * g.img_fwd);
-                else dst[j ^ sw] = make_float2(0.f, 0.f);
+            const int sy = KX <= half ? KY : (KY ? P - KY : 0), sx = KX <= half ? KX : P - KX;
+            const float2 *src = img0 + ((long long)(sy + kVH) * g.vp + sx + kVH) * 16 + j;
+            float2 *dst = tile + cell * MP + j;
+            if (jbase + j + W <= g.m) {
+                if constexpr (W == 2) cp_async16(dst, src);
+                else cp_async8(dst, src);
+            } else {
+                dst[0] = jbase + j < g.m ? __ldg(src) : make_float2(0.f, 0.f);
+                if constexpr (W == 2) dst[1] = make_float2(0.f, 0.f);
             }
         }
         cp_async_wait_all();
@@ -247,7 +209,7 @@ __global__ void __launch_bounds__(kThreads)
             atomicAdd(err, 1);
             tab.cb[e] = -1;
         } else {
-            tab.cb[e] = ((ly0 * TW + lx0) * MP) | (lx0 << 20);
+            tab.cb[e] = (ly0 * TW + lx0) * MP;
         }
         tab.th[e] = th;
         tab.k[e] = k;
@@ -264,16 +226,9 @@ __global__ void __launch_bounds__(kThreads)
     const unsigned full = 0xffffffffu;
     for (int e0 = wid * EPW; e0 < count; e0 += nw * EPW) {
         const int e = e0 + grp;
-        bool valid = e < count;
-        const int ee = valid ? e : e0;
-        int cb = tab.cb[ee];
-        int lx0 = cb >> 20;
-        cb &= (1 << 20) - 1;
-        if (tab.cb[ee] < 0) {
-            valid = false;
-            cb = 0;
-            lx0 = 0;
-        }
+        const int ee = e < count ? e : e0;
+        const int cb = tab.cb[ee];
+        const bool valid = e < count && cb >= 0;
         float w[kWS];
         {
             const float4 *wr = reinterpret_cast<const float4 *>(tab.w[ee]);
@@ -288,16 +243,14 @@ __global__ void __launch_bounds__(kThreads)
         }
         const int th = tab.th[ee];
         const float2 kv = (jg < g.m) ? __ldg(kmat + (long long)th * g.m + jg) : make_float2(0.f, 0.f);
-        const float2 *bcol[kTaps];  // per tap column: swizzled slot of time sample j
-#pragma unroll
-        for (int b = 0; b < kTaps; ++b) bcol[b] = tile + cb + b * MP + (j ^ ((lx0 + b) & (MP - 1)));
+        const float2 *c0 = tile + max(cb, 0) + j;
         float ax = 0.f, ay = 0.f;
 #pragma unroll
         for (int a = 0; a < kTaps; ++a) {
             float rx = 0.f, ry = 0.f;
 #pragma unroll
             for (int b = 0; b < kTaps; ++b) {
-                const float2 v = bcol[b][a * TW * MP];
+                const float2 v = c0[(a * TW + b) * MP];
                 rx = fmaf(w[b], v.x, rx);
                 ry = fmaf(w[2 * kTaps + b], v.y, ry);
             }
@@ -315,7 +268,7 @@ __global__ void __launch_bounds__(kThreads)
         if (valid && j == 0) {
             float2 r = cmul(make_float2(px, py), tab.f[ee]);
             float2 *dst = rows + ((long long)z * g.ntheta + th) * g.n + tab.k[ee];
-            if (accumulate) {
+            if (jgrp > 0) {
                 const float2 o = *dst;
                 r.x += o.x;
                 r.y += o.y;
@@ -331,19 +284,15 @@ static int mp_for(int m) {
     return mp;
 }
 
-size_t gather_fwd_smem(const UsGeo &g) {
-    return (size_t)(g.T + 2 * kR) * (g.T + 2 * kR) * mp_for(g.m) * sizeof(float2) + sizeof(EntryTab);
-}
-size_t scatter_adj_smem(const UsGeo &g) { return sizeof(ScatterSmem<16>); }
 int table_capacity() { return kCH; }
 
 template <int MP, int T>
 static void gather_fwd_t(const float2 *spec, float2 *rows, int zb, const GeoDev &gd, const UsGeo &g,
-                         int jbase, int accumulate, int *err, cudaStream_t s) {
+                         int jgrp, cudaStream_t s) {
     const size_t smem = (size_t)(T + 2 * kR) * (T + 2 * kR) * MP * sizeof(float2) + sizeof(EntryTab);
     dim3 gs(gd.n_fwd_items, zb);
     k_gather_fwd<MP, T><<<gs, kThreads, smem, s>>>(spec, rows, gd.fwd_pts, gd.fwd_items, gd.sincos, gd.kmat,
-                                              gd.shiftfwd, g, jbase, accumulate, err);
+                                              gd.shiftfwd, g, jgrp, gd.err);
     LAUNCH_CHECK("k_gather_fwd");
 }
 
@@ -365,18 +314,17 @@ void launch_gather_fwd(const float2 *spec, float2 *rows, int zb, const GeoDev &g
     k_zero_k0<<<(unsigned)((nrows + 255) / 256), 256, 0, s>>>(rows, nrows, g.n);
     LAUNCH_CHECK("k_zero_k0");
     const int mp = mp_for(g.m);
-    for (int jb = 0; jb < g.m; jb += 16) {
-        const int acc = jb > 0;
+    for (int jg = 0; jg < g.jg; ++jg) {
         // the plan gives items with several samples per ray to the tensor-core
         // gather from 8 time samples up (any group size: missing samples are zero)
-        if (gd.n_fwd_tc_items > 0) launch_gather_tc(rows, zb, gd, g, *tmap, jb, acc, s);
+        if (gd.n_fwd_tc_items > 0) launch_gather_tc(rows, zb, gd, g, *tmap, jg, s);
         if (gd.n_fwd_items == 0) continue;
         switch (mp) {
-            case 1: gather_fwd_t<1, 16>(spec, rows, zb, gd, g, jb, acc, gd.err, s); break;
-            case 2: gather_fwd_t<2, 16>(spec, rows, zb, gd, g, jb, acc, gd.err, s); break;
-            case 4: gather_fwd_t<4, 16>(spec, rows, zb, gd, g, jb, acc, gd.err, s); break;
-            case 8: gather_fwd_t<8, 16>(spec, rows, zb, gd, g, jb, acc, gd.err, s); break;
-            default: gather_fwd_t<16, 16>(spec, rows, zb, gd, g, jb, acc, gd.err, s); break;
+            case 1: gather_fwd_t<1, 16>(spec, rows, zb, gd, g, jg, s); break;
+            case 2: gather_fwd_t<2, 16>(spec, rows, zb, gd, g, jg, s); break;
+            case 4: gather_fwd_t<4, 16>(spec, rows, zb, gd, g, jg, s); break;
+            case 8: gather_fwd_t<8, 16>(spec, rows, zb, gd, g, jg, s); break;
+            default: gather_fwd_t<16, 16>(spec, rows, zb, gd, g, jg, s); break;
         }
     }
 }
@@ -457,26 +405,6 @@ void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaS
     LAUNCH_CHECK("k_adj_prep");
 }
 
-// Zero the core cells of tiles that several scatter blocks accumulate into.
-__global__ void k_zero_split(float2 *spec, const int *__restrict__ tiles, int T, int NT, int P,
-                             long long img_adj) {
-    const int t = tiles[blockIdx.x];
-    const long long img = blockIdx.y;
-    const int tyi = t / NT, txi = t - tyi * NT;
-    for (int c = threadIdx.x; c < T * T; c += blockDim.x) {
-        const int ly = c / T, lx = c - ly * T;
-        const int KY = tyi * T + ly, KX = txi * T + lx;
-        if (KY < P && KX < P) spec[img * img_adj + (long long)KY * P + KX] = make_float2(0.f, 0.f);
-    }
-}
-
-void launch_zero_split(float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, cudaStream_t s) {
-    if (gd.n_split_tiles == 0) return;
-    dim3 gs(gd.n_split_tiles, zb * g.m);
-    k_zero_split<<<gs, 256, 0, s>>>(spec, gd.split_tiles, g.T, g.NT, g.P, g.img_adj);
-    LAUNCH_CHECK("k_zero_split");
-}
-
 // ---------------------------------------------------------------------------
 // Adjoint scatter (gather TOMO_ADJ + wrap TOMO_ADJ, kernels_radonusfft.cuh:
 // 40-64,81-144, fused with shift/fftshift of radonusfft.cu:115-121, the basis
@@ -490,14 +418,15 @@ void launch_zero_split(float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, c
 //     ray's single-complex grid V_ray (shared memory);
 //  2. thread = cell adds conj(K'(theta, j)) V_ray(cell) to the cell's MP
 //     complex time-sample accumulators, held in registers.
-// The tile is stored once at the end (added, for a tile split over blocks).
+// The tile is added once at the end into the zeroed Hermitian half planes.
 // ---------------------------------------------------------------------------
 template <int MP, int T>
 __global__ void __launch_bounds__(T * T, 3)
     k_scatter_adj(const float2 *__restrict__ rowsc, float2 *__restrict__ spec,
                   const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
                   const float2 *__restrict__ sincos, const float2 *__restrict__ kmat,
-                  const float2 *__restrict__ shifta, UsGeo g, int jbase) {
+                  const float2 *__restrict__ shifta, UsGeo g, int jgrp) {
+    const int jbase = 16 * jgrp;
     static_assert(T == 16, "one thread per cell of a 16x16 tile");
     extern __shared__ float4 smraw[];
     ScatterSmem<T> &sm = *reinterpret_cast<ScatterSmem<T> *>(smraw);
@@ -633,34 +562,25 @@ __global__ void __launch_bounds__(T * T, 3)
             }
         }
     }
-    // ---- store the cell (pre-IFFT fftshift sign); split tiles add ----
+    // ---- the cell's sums into the half planes ----
     const int ly = tid / T, lx = tid - (tid / T) * T;
-    const int KY = tyi * T + ly, KX = txi * T + lx;
-    if (KY < P && KX < P) {
-        const float sg = ((KX + KY) & 1) ? -1.f : 1.f;
-        float2 *dst = spec + ((long long)z * g.m + jbase) * g.img_adj + (long long)KY * P + KX;
+    float2 *base = spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
+    const float sg = ((lx + ly) & 1) ? -0.5f : 0.5f;
 #pragma unroll
-        for (int j = 0; j < MP; ++j) {
-            if (jbase + j >= g.m) break;
-            const float2 v = make_float2(sg * ar[j], sg * ai[j]);
-            float2 *d = dst + (long long)j * g.img_adj;
-            if (it.w) {
-                atomicAdd(&d->x, v.x);
-                atomicAdd(&d->y, v.y);
-            } else {
-                *d = v;
-            }
-        }
+    for (int j = 0; j < MP; j += 2) {  // (the sample after an odd last one adds zeros)
+        if (jbase + j >= g.m) break;
+        const int i = MP > 1 ? j + 1 : 0;
+        add_hermitian<MP == 1>(base, g, txi * T + lx, tyi * T + ly, j, make_float4(sg * ar[j], sg * ai[j], sg * ar[i], sg * ai[i]));
     }
 }
 
 template <int MP, int T>
 static void scatter_adj_t(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
-                          const UsGeo &g, int jbase, cudaStream_t s) {
+                          const UsGeo &g, int jgrp, cudaStream_t s) {
     const size_t smem = sizeof(ScatterSmem<T>);
     dim3 gs(gd.n_adj_items, zb);
     k_scatter_adj<MP, T><<<gs, T * T, smem, s>>>(rowsc, spec, gd.adj_pts, gd.adj_items, gd.sincos, gd.kmat,
-                                               gd.shiftadj, g, jbase);
+                                               gd.shiftadj, g, jgrp);
     LAUNCH_CHECK("k_scatter_adj");
 }
 
@@ -671,52 +591,29 @@ void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev 
         launch_scatter_dir(rowsc, spec, zb, gd, g, s);
         return;
     }
+    // the per-ray kernels add into zeroed half planes
+    CUDA_CHECK(cudaMemsetAsync(spec, 0, sizeof(float2) * (size_t)vec_planes(g, zb) * g.vplane, s));
     const int mp = mp_for(g.m);
-    for (int jb = 0; jb < g.m; jb += 16) {
-        // the tensor-core scatter fills the Hermitian half planes the spectra
-        // buffer is sized for (from 8 time samples up)
-        if (gd.tc_scatter) {
-            launch_scatter_tc(rowsc, spec, zb, gd, g, jb, s);
+    for (int jg = 0; jg < g.jg; ++jg) {
+        if (gd.tc_scatter) {  // from 8 time samples up
+            launch_scatter_tc(rowsc, spec, zb, gd, g, jg, s);
             continue;
         }
         switch (mp) {
-            case 1: scatter_adj_t<1, 16>(rowsc, spec, zb, gd, g, jb, s); break;
-            case 2: scatter_adj_t<2, 16>(rowsc, spec, zb, gd, g, jb, s); break;
-            case 4: scatter_adj_t<4, 16>(rowsc, spec, zb, gd, g, jb, s); break;
-            case 8: scatter_adj_t<8, 16>(rowsc, spec, zb, gd, g, jb, s); break;
-            default: scatter_adj_t<16, 16>(rowsc, spec, zb, gd, g, jb, s); break;
+            case 1: scatter_adj_t<1, 16>(rowsc, spec, zb, gd, g, jg, s); break;
+            case 2: scatter_adj_t<2, 16>(rowsc, spec, zb, gd, g, jg, s); break;
+            case 4: scatter_adj_t<4, 16>(rowsc, spec, zb, gd, g, jg, s); break;
+            case 8: scatter_adj_t<8, 16>(rowsc, spec, zb, gd, g, jg, s); break;
+            default: scatter_adj_t<16, 16>(rowsc, spec, zb, gd, g, jg, s); break;
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint epilogue after the inverse 2D FFT: post-FFT fftshift, crop and
-// deapodisation (divphi TOMO_ADJ), 1/sqrt(n ntheta) (radonusfft.cu:129-132),
-// real part accumulated with tau (addreal, operators.cu:178).
+// Adjoint without the hand-written FFTs, after cuFFT's C2R: post-FFT fftshift,
+// crop and deapodisation (divphi TOMO_ADJ), 1/sqrt(n ntheta)
+// (radonusfft.cu:129-132), accumulated with tau (addreal, operators.cu:178).
 // ---------------------------------------------------------------------------
-__global__ void k_crop_accum(const float2 *__restrict__ spec, float *__restrict__ u,
-                             const float *__restrict__ dp, int n, int P, long long img_adj, float c) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y;
-    const long long img = blockIdx.z;
-    if (x >= n) return;
-    const int X = x + n / 2, Y = y + n / 2;
-    float v = spec[img * img_adj + (long long)Y * P + X].x;
-    v = ((X + Y) & 1) ? -v : v;
-    u[(img * n + y) * n + x] += c * v * dp[x] * dp[y];
-}
-
-void launch_crop_accum(const float2 *spec, float *u, int zb, float tau, const float *deapod,
-                       const UsGeo &g, cudaStream_t s) {
-    dim3 gs((g.n + 255) / 256, g.n, zb * g.m);
-    const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
-    const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
-    k_crop_accum<<<gs, 256, 0, s>>>(spec, u, deapod, g.n, g.P, g.img_adj, c);
-    LAUNCH_CHECK("k_crop_accum");
-}
-
-// Same epilogue after the C2R inverse of the Hermitian half planes: real
-// images with rows of rowf floats.
 __global__ void k_crop_accum_real(const float *__restrict__ out, float *__restrict__ u,
                                   const float *__restrict__ dp, int n, int rowf, long long img_real, float c) {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -729,13 +626,13 @@ __global__ void k_crop_accum_real(const float *__restrict__ out, float *__restri
     u[(img * n + y) * n + x] += c * v * dp[x] * dp[y];
 }
 
-void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, int rowf,
-                            const UsGeo &g, cudaStream_t s) {
+void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, const UsGeo &g,
+                            cudaStream_t s) {
     dim3 gs((g.n + 255) / 256, g.n, zb * g.m);
     const double scale = 1.0 / std::sqrt((double)g.n * (double)g.ntheta);
     const float c = (float)(tau * scale / (4.0 * g.n * (double)g.n));
-    const long long img_real = (long long)g.P * rowf;
-    k_crop_accum_real<<<gs, 256, 0, s>>>(out, u, deapod, g.n, rowf, img_real, c);
+    const int rowf = 2 * planar_pitch(g.n);
+    k_crop_accum_real<<<gs, 256, 0, s>>>(out, u, deapod, g.n, rowf, (long long)g.P * rowf, c);
     LAUNCH_CHECK("k_crop_accum_real");
 }
 

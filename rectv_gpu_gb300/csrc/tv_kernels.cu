@@ -16,6 +16,9 @@
 // (n+1)^2 (m+1)(nzp+1) points whose point q sees voxel q-1 (clamped).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstdint>
+
 #include "rectv_internal.cuh"
 
 namespace rectv {
@@ -26,6 +29,24 @@ __device__ __forceinline__ int clampi(int a, int lo, int hi) { return a < lo ? l
 
 __device__ __forceinline__ void prefetch_l2(const void *p) {
     asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p));
+}
+
+// the value d bytes from p
+__device__ __forceinline__ const float &at(const float *p, long long d) {
+    return *reinterpret_cast<const float *>(reinterpret_cast<const char *>(p) + d);
+}
+template <int V>
+__device__ __forceinline__ void ldv(const float *p, float (&v)[V]) {
+    if constexpr (V == 2) {
+        const float2 a = *reinterpret_cast<const float2 *>(p);
+        v[0] = a.x;
+        v[1] = a.y;
+    } else {
+        v[0] = *p;
+    }
+}
+__device__ __forceinline__ void put(float *p, long long d, float v) {
+    *reinterpret_cast<float *>(reinterpret_cast<char *>(p) + d) = v;
 }
 
 template <int NW>
@@ -67,156 +88,186 @@ __device__ __forceinline__ void block_reduce3(double a, double b, double c, doub
 // inner step (MODE 1) reads psi and mu and also stores w for every dual point
 // the step reads, and the later ones (MODE 2) read w alone (half the dual
 // bytes); MODE 0 reads psi and mu only.
-// One thread per (x, y, slice), marching along t: h_t(q - e_t) is the previous
-// time point's h_t(q), kept in a register, and the loads of time point t+1
-// are issued before t is computed.  Blocks of 256 x-voxels; the grid runs
-// over (x blocks, slices, rows) in that order, so the blocks that read a
-// block's z-1 and y-1 dual neighbours run at the same time (L2 hits rather
-// than second HBM reads).
+// One thread per (V neighbouring x, y, slice), marching along t: h_t(q - e_t) is
+// the previous time point's h_t(q), kept in a register.  The grid runs over (x
+// blocks, slices, rows) in that order, so the blocks that read a block's z-1 and
+// y-1 dual neighbours run at the same time (L2 hits rather than second HBM reads).
+// Bound by HBM (24 bytes a voxel in MODE 2, 56 in MODE 1) as far as enough loads
+// are in flight: 512 x 512 x 16 x 16 voxels take 0.283 ms in MODE 2 (5.7 TB/s)
+// and 0.705 in MODE 1.  Two voxels per thread share the loads' addresses and the
+// h_x between them (110 instead of 152 instructions a voxel), and 40 warps per SM
+// with the next time point's lines prefetched into L2 hide more latency than 32
+// (24) warps that hold the next point's loads in registers: 0.397 (0.781) ms.
 // ---------------------------------------------------------------------------
-template <int MODE>
-__global__ void __launch_bounds__(256, MODE == 2 ? 4 : 3)  // MODE 2 loads less: 32 warps per SM
+template <int MODE, int V>
+__global__ void __launch_bounds__(256, V == 2 ? (MODE == 2 ? 5 : 3) : (MODE == 2 ? 6 : 4))
     k_graddiv(const float *__restrict__ uin, const float *__restrict__ uold, float *__restrict__ uout,
               const float *__restrict__ psi, const float *__restrict__ mu, float *__restrict__ w,
               const float *__restrict__ rhop, TvGeo t, int c0, int nch_total, float tau) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    const int x = V * (blockIdx.x * blockDim.x + threadIdx.x);
     const int zr = blockIdx.y;
-    const int y = blockIdx.z;
-    if (x >= t.n) return;
+    const int y = blockIdx.z * blockDim.y + threadIdx.y;
+    if (x >= t.n || y >= t.n) return;
     const int n = t.n, m = t.m, nzp = t.nzp;
     const int c = c0 + zr / nzp, zl = zr % nzp;
     const long long slab = t.vol_slab, nn = (long long)n * n;
     const long long v0 = ((long long)c * nzp + zl) * slab + (long long)y * n + x;  // voxel (x, y, t = 0)
-    const float *u = uin + v0;
-    // z neighbours: inside the chunk, else the previous outer iterate, else replicated
-    const float *uzp = (zl < nzp - 1) ? uin + v0 + slab : ((c < nch_total - 1) ? uold + v0 + slab : u);
-    const float *uzm = (zl > 0) ? uin + v0 - slab : ((c > 0) ? uold + v0 - slab : u);
-    const int dxp = x < n - 1 ? 1 : 0, dxm = x > 0 ? 1 : 0;
-    const int dyp = y < n - 1 ? n : 0, dym = y > 0 ? n : 0;
     const float rho = *rhop;
-    const long long sx = 1, sy = n + 1, st = (long long)(n + 1) * (n + 1), sz = st * (m + 1);
+    const long long sy = n + 1, st = (long long)(n + 1) * (n + 1), sz = st * (m + 1);
     const long long cs = t.comp_stride;
     const long long q0 = (long long)c * t.gp + (zl + 1) * sz + st + (y + 1) * sy + (x + 1);  // q of t = 0
     const float sg = t.sg, sgt = t.sg * t.lambda1;
-    // a[]: u at x+1, x-1, y+1, y-1, z+1, z-1, t+1; then the dual values: at q
-    // (4 components) and of component x at q-sx, y at q-sy, z at q-sz, as
-    // (psi, mu) pairs (MODE 0, 1: a[7..10] psi, a[11..14] mu, a[15..20]
-    // psi/mu pairs) or w alone (MODE 2: a[7..10] w, a[15], a[17], a[19])
-    auto load = [&](int tt, float(&a)[21]) {
-        const long long o = (long long)tt * nn;
-        const long long q = q0 + (long long)tt * st;
-        a[0] = u[o + dxp];
-        a[1] = u[o - dxm];
-        a[2] = u[o + dyp];
-        a[3] = u[o - dym];
-        a[4] = uzp[o];
-        a[5] = uzm[o];
-        a[6] = u[o + (tt < m - 1 ? nn : 0)];
-        if constexpr (MODE == 2) {
+    // Everything a time point reads lies at block-uniform byte distances from
+    // the thread's voxel and from its dual point: a thread carries two pointers along t.
+    const float *u = uin + v0;  // the voxel at the time point the next load() is for
+    const bool xp = x + V < n, xm = x > 0, yp = y < n - 1, ym = y > 0;
+    // z neighbours: inside the chunk, else the previous outer iterate, else replicated
+    const long long alt = reinterpret_cast<const char *>(uold) - reinterpret_cast<const char *>(uin);
+    const long long dzp = zl < nzp - 1 ? 4 * slab : (c < nch_total - 1 ? alt + 4 * slab : 0);
+    const long long dzm = zl > 0 ? -4 * slab : (c > 0 ? alt - 4 * slab : 0);
+    float *out = uout + v0;
+    const float *pq = (MODE == 2 ? w : psi) + q0;  // its dual point
+    const long long dmu = reinterpret_cast<const char *>(mu) - reinterpret_cast<const char *>(psi);
+    float *pw = w + q0;
+    const long long ci[4] = {0, 4 * cs, 8 * cs, 12 * cs}, cy = 4 * (cs - sy), cz = 4 * (3 * cs - sz);
+    // one time point: u at y+1, y-1, z+1, z-1, t+1 and right and left of the
+    // V voxels; the dual values (psi and mu, or w) at q (4 components) and of
+    // component x at q-1, y at q-sy, z at q-sz
+    constexpr int S = MODE == 2 ? 1 : 2;
+    struct Pt {
+        float up[V], um[V], uzp[V], uzm[V], ut[V], xr, xl;
+        float p[S][4][V], py[S][V], pz[S][V], px[S];
+    };
+    auto load = [&](int tt, const float(&f)[V], Pt &a) {
+        a.xr = xp ? u[V] : f[V - 1];
+        a.xl = xm ? u[-1] : f[0];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[7 + i] = w[i * cs + q];
-            a[15] = w[q - sx];
-            a[17] = w[cs + q - sy];
-            a[19] = w[3 * cs + q - sz];
-        } else {
+        for (int v = 0; v < V; ++v) a.up[v] = a.um[v] = a.ut[v] = f[v];
+        if (yp) ldv<V>(u + n, a.up);
+        if (ym) ldv<V>(u - n, a.um);
+        ldv<V>(&at(u, dzp), a.uzp);
+        ldv<V>(&at(u, dzm), a.uzm);
+        if (tt < m - 1) ldv<V>(u + nn, a.ut);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[7 + i] = psi[i * cs + q];
-                a[11 + i] = mu[i * cs + q];
+        for (int s = 0; s < S; ++s) {
+            const long long d = s ? dmu : 0;
+            a.px[s] = at(pq, d - 4);
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) a.p[s][i][v] = at(pq + v, d + ci[i]);
+                a.py[s][v] = at(pq + v, d + cy);
+                a.pz[s][v] = at(pq + v, d + cz);
             }
-            a[15] = psi[q - sx];
-            a[16] = mu[q - sx];
-            a[17] = psi[cs + q - sy];
-            a[18] = mu[cs + q - sy];
-            a[19] = psi[3 * cs + q - sz];
-            a[20] = mu[3 * cs + q - sz];
         }
     };
     // h of one component from the gradient term g and the dual values
-    auto hval = [&](float g, const float(&a)[21], int ip, int im) {
+    auto hval = [&](float g, float p, float mv) {
         if constexpr (MODE == 2)
-            return rho * g + a[ip];
+            return rho * g + p;
         else
-            return rho * (g - a[ip]) + a[im];
+            return rho * (g - p) + mv;
     };
-    float cur[21];
-    load(0, cur);
-    float f0 = u[0];
-    // h_t at q - st for t = 0: the clamped backward difference is zero
-    float hmt;
-    if constexpr (MODE == 2) {
-        hmt = rho * (sgt * (f0 - f0)) + w[2 * cs + q0 - st];
-    } else {
-        const float p0 = psi[2 * cs + q0 - st], m0 = mu[2 * cs + q0 - st];
-        hmt = rho * (sgt * (f0 - f0) - p0) + m0;
-        if constexpr (MODE == 1) w[2 * cs + q0 - st] = m0 - rho * p0;
+    float f0[V], hmt[V];  // hmt: h_t at q - st; for t = 0 the clamped backward difference is zero
+    ldv<V>(u, f0);
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const float p0 = at(pq + v, ci[2] - 4 * st), m0 = MODE == 2 ? 0.f : at(pq + v, dmu + ci[2] - 4 * st);
+        hmt[v] = hval(sgt * (f0[v] - f0[v]), p0, m0);
+        if constexpr (MODE == 1) put(pw + v, ci[2] - 4 * st, m0 - rho * p0);
     }
-    const float *wpf = w + q0 + 3 * st;  // MODE 2: w of time point tt + 3
+#pragma unroll 1
     for (int tt = 0; tt < m; ++tt) {
-        float nxt[21];
-        if constexpr (MODE == 2) {
-            // the dual lines only this thread's column brings from HBM (its own
-            // w, 16 of the 20 new bytes per voxel; the neighbours' are other
-            // threads' own), into L2 two time points before load() asks for
-            // them: registers hold only one point ahead
-            if (tt + 3 < m) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) prefetch_l2(wpf + i * cs);
-            }
-            wpf += st;
-        }
-        if (tt + 1 < m) load(tt + 1, nxt);
-        if constexpr (MODE == 1) {  // w at q, and at the lower boundary planes this voxel reads
-            const long long q = q0 + (long long)tt * st;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) w[i * cs + q] = cur[11 + i] - rho * cur[7 + i];
-            if (x == 0) w[q - sx] = cur[16] - rho * cur[15];
-            if (y == 0) w[cs + q - sy] = cur[18] - rho * cur[17];
-            if (zl == 0) w[3 * cs + q - sz] = cur[20] - rho * cur[19];
-        }
-        float d;
-        {  // x
-            const float hq = hval(sg * (cur[0] - f0), cur, 7, 11);
-            const float hm = hval(sg * (f0 - cur[1]), cur, 15, 16);
-            d = hm - hq;
-        }
-        {  // y
-            const float hq = hval(sg * (cur[2] - f0), cur, 8, 12);
-            const float hm = hval(sg * (f0 - cur[3]), cur, 17, 18);
-            d += hm - hq;
-        }
-        {  // t (scaled by lambda1 in both gradient and divergence)
-            const float hq = hval(sgt * (cur[6] - f0), cur, 9, 13);
-            d += t.lambda1 * (hmt - hq);
-            hmt = hq;
-        }
-        {  // z
-            const float hq = hval(sg * (cur[4] - f0), cur, 10, 14);
-            const float hm = hval(sg * (f0 - cur[5]), cur, 19, 20);
-            d += hm - hq;
-        }
-        uout[v0 + (long long)tt * nn] = f0 + tau * t.sd * d;
-        f0 = cur[6];  // u at t+1
+        // the lines only this thread's column brings from HBM (its own dual
+        // values and u at the next time point; the neighbours' are other
+        // threads' own), into L2 two time points ahead of their load
         if (tt + 1 < m) {
 #pragma unroll
-            for (int i = 0; i < 21; ++i) cur[i] = nxt[i];
+            for (int i = 0; i < 4; ++i) {
+                prefetch_l2(&at(pq, 4 * st + ci[i]));
+                if constexpr (MODE != 2) prefetch_l2(&at(pq, dmu + 4 * st + ci[i]));
+            }
         }
+        if (tt + 2 < m) prefetch_l2(u + 2 * nn);
+        Pt cur;
+        load(tt, f0, cur);
+        if constexpr (MODE == 1) {  // w at q, and at the lower boundary planes these voxels read
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) put(pw + v, ci[i], cur.p[S - 1][i][v] - rho * cur.p[0][i][v]);
+                if (v == 0 && x == 0) put(pw, -4, cur.px[S - 1] - rho * cur.px[0]);
+                if (y == 0) put(pw + v, cy, cur.py[S - 1][v] - rho * cur.py[0][v]);
+                if (zl == 0) put(pw + v, cz, cur.pz[S - 1][v] - rho * cur.pz[0][v]);
+            }
+        }
+        u += nn;
+        pq += st;
+        pw += st;
+        float r[V], hx = hval(sg * (f0[0] - cur.xl), cur.px[0], cur.px[S - 1]);  // h_x left of the voxel
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            float d;
+            {  // x
+                const float hq = hval(sg * ((v < V - 1 ? f0[v + 1 < V ? v + 1 : v] : cur.xr) - f0[v]), cur.p[0][0][v],
+                                      cur.p[S - 1][0][v]);
+                d = hx - hq;
+                hx = hq;
+            }
+            {  // y
+                const float hq = hval(sg * (cur.up[v] - f0[v]), cur.p[0][1][v], cur.p[S - 1][1][v]);
+                const float hm = hval(sg * (f0[v] - cur.um[v]), cur.py[0][v], cur.py[S - 1][v]);
+                d += hm - hq;
+            }
+            {  // t (scaled by lambda1 in both gradient and divergence)
+                const float hq = hval(sgt * (cur.ut[v] - f0[v]), cur.p[0][2][v], cur.p[S - 1][2][v]);
+                d += t.lambda1 * (hmt[v] - hq);
+                hmt[v] = hq;
+            }
+            {  // z
+                const float hq = hval(sg * (cur.uzp[v] - f0[v]), cur.p[0][3][v], cur.p[S - 1][3][v]);
+                const float hm = hval(sg * (f0[v] - cur.uzm[v]), cur.pz[0][v], cur.pz[S - 1][v]);
+                d += hm - hq;
+            }
+            r[v] = f0[v] + tau * t.sd * d;
+        }
+        if constexpr (V == 2)
+            *reinterpret_cast<float2 *>(out) = make_float2(r[0], r[1]);
+        else
+            *out = r[0];
+        out += nn;
+#pragma unroll
+        for (int v = 0; v < V; ++v) f0[v] = cur.ut[v];  // u at t+1
     }
+}
+
+template <int V>
+static void graddiv_v(const float *u_in, const float *u_old, float *u_out, const float *psi, const float *mu, float *w,
+                      int mode, const float *rho, int c0, int nch, const TvGeo &t, cudaStream_t s) {
+    const int bx = std::min(256, ((t.n + V - 1) / V + 31) / 32 * 32);
+    const dim3 bs(bx, 256 / bx), gs((t.n + V * bx - 1) / (V * bx), t.nchunks * t.nzp, (t.n + bs.y - 1) / bs.y);
+    if (gs.y > 65535u || gs.z > 65535u) throw Error(1, "graddiv: grid too large");
+    if (mode == 1)
+        k_graddiv<1, V><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nch, -0.5f);
+    else if (mode == 2)
+        k_graddiv<2, V><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nch, -0.5f);
+    else
+        k_graddiv<0, V><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nch, -0.5f);
+    LAUNCH_CHECK("k_graddiv");
 }
 
 void launch_graddiv(const float *u_in, const float *u_old, float *u_out, const float *psi,
                     const float *mu, float *w, int mode, const float *rho, int c0, int nchunks_total,
                     const TvGeo &t, cudaStream_t s) {
-    dim3 bs(256, 1), gs((t.n + 255) / 256, t.nchunks * t.nzp, t.n);
-    if (gs.y > 65535u || gs.z > 65535u) throw Error(1, "graddiv: grid too large");
     if (mode != 0 && !w) throw Error(1, "graddiv: no w buffer");
-    if (mode == 1)
-        k_graddiv<1><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nchunks_total, -0.5f);
-    else if (mode == 2)
-        k_graddiv<2><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nchunks_total, -0.5f);
+    // two voxels per thread where the rows' voxels come in aligned pairs and the
+    // threads still fill the chip
+    const bool even = t.n % 2 == 0 && t.vol_slab % 2 == 0 && (long long)t.n * t.n * t.nchunks * t.nzp >= 152 * 2048 &&
+                      ((uintptr_t)u_in | (uintptr_t)u_old | (uintptr_t)u_out) % 8 == 0;
+    if (even)
+        graddiv_v<2>(u_in, u_old, u_out, psi, mu, w, mode, rho, c0, nchunks_total, t, s);
     else
-        k_graddiv<0><<<gs, bs, 0, s>>>(u_in, u_old, u_out, psi, mu, w, rho, t, c0, nchunks_total, -0.5f);
-    LAUNCH_CHECK("k_graddiv");
+        graddiv_v<1>(u_in, u_old, u_out, psi, mu, w, mode, rho, c0, nchunks_total, t, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -224,22 +275,28 @@ void launch_graddiv(const float *u_in, const float *u_old, float *u_out, const f
 //   h = G u_cur, ho = G u_old (the reference's h2stored),
 //   psi = shrink(h + mu/rho, lambda0/rho), mu += rho h - rho psi,
 //   sums of |h-psi|^2, |ho-h|^2 and, for q >= 1, (u_cur-u_old)^2.
-// One thread per (qx, qy, qz) marching along qt; the squares along its qt
-// column are summed in FP32 (at most m+1 = 17 terms for m = 16) and the
-// thread sums are accumulated in FP64 in a fixed order; one FP64 partial
-// triple per block.  Blocks of 32x8 over (qx, qy), grid.z over (chunk, qz).
+// One thread per (qx, qy, qz) marching along qt; the squares along its qt column
+// are summed in FP32 (at most m+1 = 17 terms for m = 16) and the column sums
+// are accumulated in FP64 in a fixed order; one FP64 partial triple per block.
+// Blocks of 256 threads over a plane's (qy, qx) in that order, the planes
+// (chunk, qz) fastest, so that the blocks reading a slice twice run together.
+// At 17 x 17 x 513 x 513 points per chunk, two chunks of 8 slices: 0.83 ms
+// (the planes slowest 0.92; the next time point's values held in registers in
+// place of the L2 prefetch, blocks of 32 x 8 points: 1.00; two points per
+// thread 1.06).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256, 4)
     k_shrink(const float *__restrict__ ucur, const float *__restrict__ uold, float *__restrict__ psi,
              float *__restrict__ mu, const float *__restrict__ rhop, float lambda0, TvGeo t, int c0,
              int nch_total, double *__restrict__ partials) {
-    const int qx = blockIdx.x * blockDim.x + threadIdx.x;
-    const int qy = blockIdx.y * blockDim.y + threadIdx.y;
     const int n = t.n, m = t.m, nzp = t.nzp;
-    const int qz = blockIdx.z % (nzp + 1);
-    const int c = c0 + blockIdx.z / (nzp + 1);
+    const int planes = t.nchunks * (nzp + 1), pl = blockIdx.x % planes;  // the block's (chunk, qz)
+    const int e = blockIdx.x / planes * 256 + threadIdx.x;
+    const int qy = e / (n + 1), qx = e - qy * (n + 1);
+    const int qz = pl % (nzp + 1);
+    const int c = c0 + pl / (nzp + 1);
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    if (qx <= n && qy <= n) {
+    if (qy <= n) {
         const long long slab = t.vol_slab, nn = (long long)n * n;
         const long long zc = (long long)c * nzp;
         // extended-chunk slabs at z0 = qz-1 and z1 = qz (extendf, kernels_operators.cuh:14-19)
@@ -248,50 +305,51 @@ __global__ void __launch_bounds__(256, 4)
             if (zl >= nzp) return (c < nch_total - 1) ? uold + (zc + nzp) * slab : u + (zc + nzp - 1) * slab;
             return u + (zc + zl) * slab;
         };
-        const float *c0p = slab_of(ucur, qz - 1), *c1p = slab_of(ucur, qz);
-        const float *o0p = slab_of(uold, qz - 1), *o1p = slab_of(uold, qz);
-        const int x0 = clampi(qx - 1, 0, n - 1), x1 = clampi(qx, 0, n - 1);
-        const int y0 = clampi(qy - 1, 0, n - 1), y1 = clampi(qy, 0, n - 1);
-        const long long p00 = (long long)y0 * n + x0, px = (long long)y0 * n + x1, py = (long long)y1 * n + x0;
-        const bool inner_xyz = (qx >= 1 && qy >= 1 && qz >= 1);
+        // as in k_graddiv: block-uniform byte distances from the thread's
+        // lower voxel (x0, y0, z0) in the new iterate
+        const char *b0 = reinterpret_cast<const char *>(slab_of(ucur, qz - 1));
+        const long long dz[2] = {reinterpret_cast<const char *>(slab_of(ucur, qz)) - b0,
+                                 reinterpret_cast<const char *>(slab_of(uold, qz)) - b0};
+        const long long du[2] = {0, reinterpret_cast<const char *>(slab_of(uold, qz - 1)) - b0};
+        const int x0 = clampi(qx - 1, 0, n - 1), y0 = clampi(qy - 1, 0, n - 1);
+        const bool xin = qx > 0 && qx < n, yin = qy > 0 && qy < n;  // the upper neighbour is another voxel
+        const float *u = reinterpret_cast<const float *>(b0) + (long long)y0 * n + x0;  // at t0 = clamp(qt-1)
         const float sg = t.sg, sgt = t.sg * t.lambda1;
         const float rho = *rhop;
         const float thr = lambda0 / rho, rinv = 1.0f / rho;
-        const long long cs = t.comp_stride;
-        long long q = (long long)c * t.gp + ((long long)qz * (m + 1)) * (n + 1) * (n + 1) + (long long)qy * (n + 1) + qx;
+        const long long ci[4] = {0, 4 * t.comp_stride, 8 * t.comp_stride, 12 * t.comp_stride};
         const long long st = (long long)(n + 1) * (n + 1);
-        float fc = c0p[p00], fo = o0p[p00];  // values at (x0, y0, t0 = clamp(qt-1) = 0, z0)
-        // loads of time point qt + 1 are issued before qt is computed and
-        // stored (two time points of loads in flight per thread)
-        float lu[8], lm[4];
-        auto load = [&](int qt, long long qq) {
-            const long long o0 = (long long)(qt > 0 ? qt - 1 : 0) * nn;  // t0 = clamp(qt-1)
-            const long long o1 = (long long)(qt < m ? qt : m - 1) * nn;  // t1 = clamp(qt)
-            lu[0] = c0p[o0 + px];
-            lu[1] = c0p[o0 + py];
-            lu[2] = c0p[o1 + p00];
-            lu[3] = c1p[o0 + p00];
-            lu[4] = o0p[o0 + px];
-            lu[5] = o0p[o0 + py];
-            lu[6] = o0p[o1 + p00];
-            lu[7] = o1p[o0 + p00];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) lm[i] = mu[i * cs + qq];
-        };
-        load(0, q);
+        float *pm = mu + (long long)c * t.gp + ((long long)qz * (m + 1)) * st + (long long)qy * (n + 1) + qx;
+        float *pp = psi + (pm - mu);
+        float f[2] = {u[0], at(u, du[1])};  // values at t0 of the new and the old iterate
+#pragma unroll 1
         for (int qt = 0; qt <= m; ++qt) {
-            const float fcx = lu[0], fcy = lu[1], fct = lu[2], fcz = lu[3];
-            const float fox = lu[4], foy = lu[5], fot = lu[6], foz = lu[7];
-            float mv[4], ps[4];
+            // the lines only this thread's column brings from HBM, into L2 ahead of their loads
+            if (qt + 2 <= m) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) mv[i] = lm[i];
-            if (qt < m) load(qt + 1, q + st);
-            const float h[4] = {sg * (fcx - fc), sg * (fcy - fc), sgt * (fct - fc), sg * (fcz - fc)};
-            const float ho[4] = {sg * (fox - fo), sg * (foy - fo), sgt * (fot - fo), sg * (foz - fo)};
-            float za2 = 0.f;
+                for (int i = 0; i < 4; ++i) prefetch_l2(&at(pm, ci[i] + 8 * st));
+                if (qt > 0 && qt + 2 < m) {
+                    prefetch_l2(u + 3 * nn);
+                    prefetch_l2(&at(u, du[1] + 12 * nn));
+                }
+            }
+            float mv[4], g[2][4], ft[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) mv[i] = at(pm, ci[i]);
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+                const float *us = &at(u, du[s]);
+                const float fx = xin ? us[1] : f[s], fy = yin ? us[n] : f[s], fz = at(u, dz[s]);
+                ft[s] = qt > 0 && qt < m ? us[nn] : f[s];
+                g[s][0] = sg * (fx - f[s]);
+                g[s][1] = sg * (fy - f[s]);
+                g[s][2] = sgt * (ft[s] - f[s]);
+                g[s][3] = sg * (fz - f[s]);
+            }
+            float ps[4], za2 = 0.f;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                ps[i] = h[i] + mv[i] * rinv;  // solve_reg_ker, admm.cu:49-52
+                ps[i] = g[0][i] + mv[i] * rinv;  // solve_reg_ker, admm.cu:49-52
                 za2 += ps[i] * ps[i];
             }
             const float za = sqrtf(za2);
@@ -299,39 +357,41 @@ __global__ void __launch_bounds__(256, 4)
             float r2 = 0.f, s2 = 0.f;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
+                const float h = g[0][i];
                 ps[i] = ps[i] * shr;
-                psi[i * cs + q] = ps[i];
-                mu[i * cs + q] = mv[i] + rho * h[i] - rho * ps[i];  // lin4(mu,h2,psi,1,rho,-rho)
-                const float dr = h[i] - ps[i], ds = ho[i] - h[i];
+                put(pp, ci[i], ps[i]);
+                put(pm, ci[i], mv[i] + rho * h - rho * ps[i]);  // lin4(mu,h2,psi,1,rho,-rho)
+                const float dr = h - ps[i], ds = g[1][i] - h;
                 r2 += dr * dr;
                 s2 += ds * ds;
             }
             a0 += r2;
             a1 += s2;
-            if (inner_xyz && qt >= 1) {  // voxel q-1 = (x0, y0, t0, z0) inside the chunk
-                const float dd = fc - fo;
+            if (qt >= 1 && qx >= 1 && qy >= 1 && qz >= 1) {  // voxel q-1 = (x0, y0, t0, z0) inside the chunk
+                const float dd = f[0] - f[1];
                 a2 = fmaf(dd, dd, a2);
             }
-            fc = fct;
-            fo = fot;
-            q += st;
+            f[0] = ft[0];
+            f[1] = ft[1];
+            if (qt > 0) u += nn;
+            pm += st;
+            pp += st;
         }
     }
-    const long long bid = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    block_reduce3<8>((double)a0, (double)a1, (double)a2, partials + 3 * bid);
+    block_reduce3<8>((double)a0, (double)a1, (double)a2, partials + 3LL * blockIdx.x);
 }
 
 int shrink_blocks(const TvGeo &t, int nchunks) {
-    return ((t.n + 1 + 31) / 32) * ((t.n + 1 + 7) / 8) * nchunks * (t.nzp + 1);
+    return (int)(((long long)(t.n + 1) * (t.n + 1) + 255) / 256) * nchunks * (t.nzp + 1);
 }
 
 int launch_shrink(const float *u_cur, const float *u_old, float *psi, float *mu, const float *rho,
                   float lambda0, int c0, int nchunks_total, const TvGeo &t, double *partials,
                   cudaStream_t s) {
-    dim3 bs(32, 8), gs((t.n + 1 + 31) / 32, (t.n + 1 + 7) / 8, t.nchunks * (t.nzp + 1));
-    k_shrink<<<gs, bs, 0, s>>>(u_cur, u_old, psi, mu, rho, lambda0, t, c0, nchunks_total, partials);
+    const int nb = shrink_blocks(t, t.nchunks);
+    k_shrink<<<nb, 256, 0, s>>>(u_cur, u_old, psi, mu, rho, lambda0, t, c0, nchunks_total, partials);
     LAUNCH_CHECK("k_shrink");
-    return (int)(gs.x * gs.y * gs.z);
+    return nb;
 }
 
 // ---------------------------------------------------------------------------

@@ -799,7 +799,7 @@ struct Handle {
             src = dst;
         }
         for (int bb = 0; bb < nbatch; ++bb) {
-            launch_shrink(U[src], U[old], psi, mu, rho_d, lambda0, bb * dpb, nchunks, tv,
+            launch_shrink(U[src], U[old], psi, mu, rho_d, 0.f, lambda0, bb * dpb, nchunks, tv,
                           partials + (size_t)3 * nparts_batch * bb, stream);
         }
         launch_reduce_rho(partials, nparts_batch * nbatch, stage1, rho_d, stats, iter_ctr, stats_cap, stream);
@@ -1165,7 +1165,7 @@ struct Handle {
                                    nchunks, tv, stream);
                     break;
                 case 3:  // overwrites the session's dual variables
-                    launch_shrink(U[cur], U[cur], psi, mu, rho_d, lambda0, 0, nchunks, tv, partials, stream);
+                    launch_shrink(U[cur], U[cur], psi, mu, rho_d, 0.f, lambda0, 0, nchunks, tv, partials, stream);
                     break;
                 case 4:  // padded-grid forward FFT of the batch (rows + columns)
                     if (pad_fft)

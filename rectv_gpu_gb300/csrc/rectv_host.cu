@@ -502,8 +502,7 @@ namespace {
 
 // At most this many thread blocks per call: 3 doubles of partial sums each.
 constexpr int kNoAllocMaxBlocks = 65536;
-constexpr int kNoAllocRhoSlot = 3 * kNoAllocMaxBlocks;  // one double slot holds rho
-static __device__ __align__(256) double g_noalloc_scratch[3 * kNoAllocMaxBlocks + 2];
+static __device__ __align__(256) double g_noalloc_scratch[3 * kNoAllocMaxBlocks];
 
 constexpr int kNoAllocMaxDevices = 256;
 std::mutex g_noalloc_mu;
@@ -539,38 +538,23 @@ double *noalloc_scratch(cudaStream_t s) {
     return g_noalloc_ptr[dev];
 }
 
-__global__ void k_noalloc_set_rho(float *dst, float rho) { *dst = rho; }
-
-// Fixed-order FP64 sum of the partials: one block, each thread sums a strided
-// share, then a tree over the threads.  The order differs from rectv_iterate's
-// two-stage reduction (k_sum_stage1 over contiguous shares, then
-// k_reduce_rho), so the sums agree with its history to FP64 rounding, not
-// bit for bit.
-__global__ void k_noalloc_sum3(const double *__restrict__ partials, int nparts, double *out) {
-    __shared__ double sh[3][256];
-    double a = 0, b = 0, c = 0;
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-        a += partials[3 * i];
-        b += partials[3 * i + 1];
-        c += partials[3 * i + 2];
-    }
-    sh[0][threadIdx.x] = a;
-    sh[1][threadIdx.x] = b;
-    sh[2][threadIdx.x] = c;
+// Fixed-order FP64 sum of the partials: two warps per sum, each lane a strided
+// share, then shuffles (one FP64 addition of a warp takes 16 cycles of the SM,
+// so a few warps with long shares are faster than a block's tree).  The order
+// differs from rectv_iterate's two-stage reduction (k_sum_stage1 over
+// contiguous shares, then k_reduce_rho), so the sums agree with its history to
+// FP64 rounding, not bit for bit.
+__global__ void __launch_bounds__(192) k_noalloc_sum3(const double *__restrict__ partials, int nparts, double *out) {
+    __shared__ double sh[6];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = w >> 1;
+    double a = 0;
+#pragma unroll 4
+    for (int i = 32 * (w & 1) + lane; i < nparts; i += 64) a += partials[3 * i + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+    if (lane == 0) sh[w] = a;
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            sh[0][threadIdx.x] += sh[0][threadIdx.x + o];
-            sh[1][threadIdx.x] += sh[1][threadIdx.x + o];
-            sh[2][threadIdx.x] += sh[2][threadIdx.x + o];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        out[0] = sh[0][0];
-        out[1] = sh[1][0];
-        out[2] = sh[2][0];
-    }
+    if (threadIdx.x < 3) out[threadIdx.x] = sh[2 * threadIdx.x] + sh[2 * threadIdx.x + 1];
 }
 
 }  // namespace
@@ -609,12 +593,9 @@ extern "C" int rectv_shrink_noalloc(const float *d_u_cur, const float *d_u_old, 
                                    " (ceil((n+1)/32)*ceil((n+1)/8)*nchunks*(nzp+1))");
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         double *scratch = rectv::noalloc_scratch(s);
-        float *rho_d = reinterpret_cast<float *>(scratch + rectv::kNoAllocRhoSlot);
-        rectv::k_noalloc_set_rho<<<1, 1, 0, s>>>(rho_d, rho);
-        LAUNCH_CHECK("k_noalloc_set_rho");
-        const int nparts = rectv::launch_shrink(d_u_cur, d_u_old, d_psi, d_mu, rho_d, lambda0, 0, nchunks, t,
+        const int nparts = rectv::launch_shrink(d_u_cur, d_u_old, d_psi, d_mu, nullptr, rho, lambda0, 0, nchunks, t,
                                                 scratch, s);
-        rectv::k_noalloc_sum3<<<1, 256, 0, s>>>(scratch, nparts, d_sums);
+        rectv::k_noalloc_sum3<<<1, 192, 0, s>>>(scratch, nparts, d_sums);
         LAUNCH_CHECK("k_noalloc_sum3");
     });
 }

@@ -322,7 +322,8 @@ void launch_graddiv(const float *u_in, const float *u_old, float *u_out, const f
                     const float *mu, float *w, int mode, const float *rho, int c0, int nchunks_total,
                     const TvGeo &t, cudaStream_t s);
 // shrink + dual update + residual sums into per-block partials
-int launch_shrink(const float *u_cur, const float *u_old, float *psi, float *mu, const float *rho,
+// (rho is read from rho_d, or is the argument where rho_d is null)
+int launch_shrink(const float *u_cur, const float *u_old, float *psi, float *mu, const float *rho_d, float rho,
                   float lambda0, int c0, int nchunks_total, const TvGeo &t, double *partials,
                   cudaStream_t s);
 int shrink_blocks(const TvGeo &t, int nchunks);

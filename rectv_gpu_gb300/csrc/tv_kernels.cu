@@ -49,33 +49,20 @@ __device__ __forceinline__ void put(float *p, long long d, float v) {
     *reinterpret_cast<float *>(reinterpret_cast<char *>(p) + d) = v;
 }
 
-template <int NW>
-__device__ __forceinline__ void block_reduce3(double a, double b, double c, double *out) {
-    __shared__ double sh[3][NW];
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_down_sync(0xffffffffu, a, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-        c += __shfl_down_sync(0xffffffffu, c, o);
-    }
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;  // 2D blocks
-    const int lane = tid & 31, w = tid >> 5;
-    if (lane == 0) {
-        sh[0][w] = a;
-        sh[1][w] = b;
-        sh[2][w] = c;
-    }
+// FP64 sums of the first cnt floats of each of sm's three rows, in a fixed order:
+// warp w sums row w, a lane every 32nd value.  (One FP64 addition of a warp takes
+// 16 cycles of the SM: all warps reducing their threads' doubles by shuffles
+// cost 18 of them per warp, this 20 + cnt / 16 per block and row.)
+template <int CAP>
+__device__ __forceinline__ void block_sums3(const float (&sm)[3][CAP], int cnt, double *out) {
     __syncthreads();
-    if (tid == 0) {
-        double s0 = 0, s1 = 0, s2 = 0;
-        for (int i = 0; i < NW; ++i) {
-            s0 += sh[0][i];
-            s1 += sh[1][i];
-            s2 += sh[2][i];
-        }
-        out[0] = s0;
-        out[1] = s1;
-        out[2] = s2;
-    }
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w >= 3) return;
+    double s = 0.;
+    for (int i = lane; i < cnt; i += 32) s += (double)sm[w][i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) out[w] = s;
 }
 
 }  // namespace
@@ -280,116 +267,226 @@ void launch_graddiv(const float *u_in, const float *u_old, float *u_out, const f
 // are accumulated in FP64 in a fixed order; one FP64 partial triple per block.
 // Blocks of 256 threads over a plane's (qy, qx) in that order, the planes
 // (chunk, qz) fastest, so that the blocks reading a slice twice run together.
-// At 17 x 17 x 513 x 513 points per chunk, two chunks of 8 slices: 0.83 ms
-// (the planes slowest 0.92; the next time point's values held in registers in
-// place of the L2 prefetch, blocks of 32 x 8 points: 1.00; two points per
-// thread 1.06).
+// At 9 x 17 x 513 x 513 points per chunk, two chunks: 0.83 ms (the planes slowest
+// 0.92; the next time point's values held in registers in place of the L2
+// prefetch, blocks of 32 x 8 points: 1.00; two points per thread 1.06).
 // ---------------------------------------------------------------------------
+// What a thread's column of points (qx, qy, qz) reads: the extended chunk's slabs
+// at z0 = qz-1 and z1 = qz (extendf, kernels_operators.cuh:14-19) and, as in
+// k_graddiv, block-uniform byte distances from its lower voxel (x0, y0, z0) in
+// the new iterate.
+struct ShrinkCol {
+    const float *u;          // (x0, y0, t = 0, z0) of the new iterate
+    float *pm, *pp;          // mu and psi at qt = 0
+    long long dz[2], du[2];  // z1 of the new and the old iterate; z0 of the same
+    long long nn, st, ci[4];
+    bool xin, yin, inner;    // the upper neighbour is another voxel; q - 1 is inside the chunk
+    float sg, sgt, rho, thr, rinv;
+    __device__ __forceinline__ void init(const float *ucur, const float *uold, float *psi, float *mu, float r,
+                                         float lambda0, const TvGeo &t, int c, int nch_total, int qx, int qy, int qz) {
+        const int n = t.n, nzp = t.nzp;
+        const long long slab = t.vol_slab, zc = (long long)c * nzp;
+        auto slab_of = [&](const float *v, int zl) -> const char * {
+            const float *p;
+            if (zl < 0) p = (c > 0) ? uold + (zc - 1) * slab : v + zc * slab;
+            else if (zl >= nzp) p = (c < nch_total - 1) ? uold + (zc + nzp) * slab : v + (zc + nzp - 1) * slab;
+            else p = v + (zc + zl) * slab;
+            return reinterpret_cast<const char *>(p);
+        };
+        const char *b0 = slab_of(ucur, qz - 1);
+        dz[0] = slab_of(ucur, qz) - b0;
+        dz[1] = slab_of(uold, qz) - b0;
+        du[0] = 0;
+        du[1] = slab_of(uold, qz - 1) - b0;
+        nn = (long long)n * n;
+        st = (long long)(n + 1) * (n + 1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ci[i] = 4 * i * t.comp_stride;
+        u = reinterpret_cast<const float *>(b0) + (long long)clampi(qy - 1, 0, n - 1) * n + clampi(qx - 1, 0, n - 1);
+        const long long q = (long long)c * t.gp + (long long)qz * (t.m + 1) * st + (long long)qy * (n + 1) + qx;
+        pm = mu + q;
+        pp = psi + q;
+        xin = qx > 0 && qx < n;
+        yin = qy > 0 && qy < n;
+        inner = qx >= 1 && qy >= 1 && qz >= 1;
+        sg = t.sg;
+        sgt = t.sg * t.lambda1;
+        rho = r;
+        thr = lambda0 / rho;
+        rinv = 1.0f / rho;
+    }
+    __device__ __forceinline__ void grad(float f, float fx, float fy, float fz, float ft, float (&g)[4]) const {
+        g[0] = sg * (fx - f);
+        g[1] = sg * (fy - f);
+        g[2] = sgt * (ft - f);
+        g[3] = sg * (fz - f);
+    }
+};
+
+// One point: g = (G u_new, G u_old); stores psi and mu, returns its squares.
+__device__ __forceinline__ void shrink_point(const float (&g)[2][4], float *pm, float *pp, const ShrinkCol &k,
+                                             const float (&mv)[4], float &r2, float &s2) {
+    float ps[4], za2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        ps[i] = g[0][i] + mv[i] * k.rinv;  // solve_reg_ker, admm.cu:49-52
+        za2 += ps[i] * ps[i];
+    }
+    const float za = sqrtf(za2);
+    const float shr = (za <= k.thr) ? 0.f : 1.0f - k.thr / za;  // shrink factor of the 4-vector
+    r2 = s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float h = g[0][i];
+        ps[i] = ps[i] * shr;
+        put(pp, k.ci[i], ps[i]);
+        put(pm, k.ci[i], mv[i] + k.rho * h - k.rho * ps[i]);  // lin4(mu,h2,psi,1,rho,-rho)
+        const float dr = h - ps[i], ds = g[1][i] - h;
+        r2 += dr * dr;
+        s2 += ds * ds;
+    }
+}
+
 __global__ void __launch_bounds__(256, 4)
     k_shrink(const float *__restrict__ ucur, const float *__restrict__ uold, float *__restrict__ psi,
-             float *__restrict__ mu, const float *__restrict__ rhop, float lambda0, TvGeo t, int c0,
+             float *__restrict__ mu, const float *__restrict__ rhop, float rho, float lambda0, TvGeo t, int c0,
              int nch_total, double *__restrict__ partials) {
-    const int n = t.n, m = t.m, nzp = t.nzp;
-    const int planes = t.nchunks * (nzp + 1), pl = blockIdx.x % planes;  // the block's (chunk, qz)
+    __shared__ float cs[3][256];
+    const int n = t.n, m = t.m;
+    const int planes = t.nchunks * (t.nzp + 1), pl = blockIdx.x % planes;  // the block's (chunk, qz)
     const int e = blockIdx.x / planes * 256 + threadIdx.x;
-    const int qy = e / (n + 1), qx = e - qy * (n + 1);
-    const int qz = pl % (nzp + 1);
-    const int c = c0 + pl / (nzp + 1);
+    const int qy = e / (n + 1);
     float a0 = 0.f, a1 = 0.f, a2 = 0.f;
     if (qy <= n) {
-        const long long slab = t.vol_slab, nn = (long long)n * n;
-        const long long zc = (long long)c * nzp;
-        // extended-chunk slabs at z0 = qz-1 and z1 = qz (extendf, kernels_operators.cuh:14-19)
-        auto slab_of = [&](const float *u, int zl) -> const float * {
-            if (zl < 0) return (c > 0) ? uold + (zc - 1) * slab : u + zc * slab;
-            if (zl >= nzp) return (c < nch_total - 1) ? uold + (zc + nzp) * slab : u + (zc + nzp - 1) * slab;
-            return u + (zc + zl) * slab;
-        };
-        // as in k_graddiv: block-uniform byte distances from the thread's
-        // lower voxel (x0, y0, z0) in the new iterate
-        const char *b0 = reinterpret_cast<const char *>(slab_of(ucur, qz - 1));
-        const long long dz[2] = {reinterpret_cast<const char *>(slab_of(ucur, qz)) - b0,
-                                 reinterpret_cast<const char *>(slab_of(uold, qz)) - b0};
-        const long long du[2] = {0, reinterpret_cast<const char *>(slab_of(uold, qz - 1)) - b0};
-        const int x0 = clampi(qx - 1, 0, n - 1), y0 = clampi(qy - 1, 0, n - 1);
-        const bool xin = qx > 0 && qx < n, yin = qy > 0 && qy < n;  // the upper neighbour is another voxel
-        const float *u = reinterpret_cast<const float *>(b0) + (long long)y0 * n + x0;  // at t0 = clamp(qt-1)
-        const float sg = t.sg, sgt = t.sg * t.lambda1;
-        const float rho = *rhop;
-        const float thr = lambda0 / rho, rinv = 1.0f / rho;
-        const long long ci[4] = {0, 4 * t.comp_stride, 8 * t.comp_stride, 12 * t.comp_stride};
-        const long long st = (long long)(n + 1) * (n + 1);
-        float *pm = mu + (long long)c * t.gp + ((long long)qz * (m + 1)) * st + (long long)qy * (n + 1) + qx;
-        float *pp = psi + (pm - mu);
-        float f[2] = {u[0], at(u, du[1])};  // values at t0 of the new and the old iterate
+        ShrinkCol k;
+        k.init(ucur, uold, psi, mu, rhop ? *rhop : rho, lambda0, t, c0 + pl / (t.nzp + 1), nch_total, e - qy * (n + 1),
+               qy, pl % (t.nzp + 1));
+        const float *u = k.u;  // at t0 = clamp(qt-1)
+        float *pm = k.pm, *pp = k.pp;
+        float f[2] = {u[0], at(u, k.du[1])};  // values at t0 of the new and the old iterate
 #pragma unroll 1
         for (int qt = 0; qt <= m; ++qt) {
             // the lines only this thread's column brings from HBM, into L2 ahead of their loads
             if (qt + 2 <= m) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) prefetch_l2(&at(pm, ci[i] + 8 * st));
+                for (int i = 0; i < 4; ++i) prefetch_l2(&at(pm, k.ci[i] + 8 * k.st));
                 if (qt > 0 && qt + 2 < m) {
-                    prefetch_l2(u + 3 * nn);
-                    prefetch_l2(&at(u, du[1] + 12 * nn));
+                    prefetch_l2(u + 3 * k.nn);
+                    prefetch_l2(&at(u, k.du[1] + 12 * k.nn));
                 }
             }
-            float mv[4], g[2][4], ft[2];
+            float mv[4], g[2][4], ft[2], r2, s2;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) mv[i] = at(pm, ci[i]);
+            for (int i = 0; i < 4; ++i) mv[i] = at(pm, k.ci[i]);
 #pragma unroll
             for (int s = 0; s < 2; ++s) {
-                const float *us = &at(u, du[s]);
-                const float fx = xin ? us[1] : f[s], fy = yin ? us[n] : f[s], fz = at(u, dz[s]);
-                ft[s] = qt > 0 && qt < m ? us[nn] : f[s];
-                g[s][0] = sg * (fx - f[s]);
-                g[s][1] = sg * (fy - f[s]);
-                g[s][2] = sgt * (ft[s] - f[s]);
-                g[s][3] = sg * (fz - f[s]);
+                const float *us = &at(u, k.du[s]);
+                const float fx = k.xin ? us[1] : f[s], fy = k.yin ? us[n] : f[s], fz = at(u, k.dz[s]);
+                ft[s] = qt > 0 && qt < m ? us[k.nn] : f[s];
+                k.grad(f[s], fx, fy, fz, ft[s], g[s]);
             }
-            float ps[4], za2 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                ps[i] = g[0][i] + mv[i] * rinv;  // solve_reg_ker, admm.cu:49-52
-                za2 += ps[i] * ps[i];
-            }
-            const float za = sqrtf(za2);
-            const float shr = (za <= thr) ? 0.f : 1.0f - thr / za;  // shrink factor of the 4-vector
-            float r2 = 0.f, s2 = 0.f;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float h = g[0][i];
-                ps[i] = ps[i] * shr;
-                put(pp, ci[i], ps[i]);
-                put(pm, ci[i], mv[i] + rho * h - rho * ps[i]);  // lin4(mu,h2,psi,1,rho,-rho)
-                const float dr = h - ps[i], ds = g[1][i] - h;
-                r2 += dr * dr;
-                s2 += ds * ds;
-            }
+            shrink_point(g, pm, pp, k, mv, r2, s2);
             a0 += r2;
             a1 += s2;
-            if (qt >= 1 && qx >= 1 && qy >= 1 && qz >= 1) {  // voxel q-1 = (x0, y0, t0, z0) inside the chunk
+            if (qt >= 1 && k.inner) {  // voxel q-1 = (x0, y0, t0, z0)
                 const float dd = f[0] - f[1];
                 a2 = fmaf(dd, dd, a2);
             }
             f[0] = ft[0];
             f[1] = ft[1];
-            if (qt > 0) u += nn;
-            pm += st;
-            pp += st;
+            if (qt > 0) u += k.nn;
+            pm += k.st;
+            pp += k.st;
         }
     }
-    block_reduce3<8>((double)a0, (double)a1, (double)a2, partials + 3LL * blockIdx.x);
+    cs[0][threadIdx.x] = a0;
+    cs[1][threadIdx.x] = a1;
+    cs[2][threadIdx.x] = a2;
+    block_sums3(cs, 256, partials + 3LL * blockIdx.x);
+}
+
+// Grids of at most two blocks per SM, where a column costs m+1 memory latencies:
+// the same with the loads of five points at a time in flight (a grid this small
+// leaves the registers for it).  9 x 9 x 65 x 65 points: 7.4 us, 10.6 one point at a time.
+__global__ void __launch_bounds__(256, 2)
+    k_shrink_few(const float *__restrict__ ucur, const float *__restrict__ uold, float *__restrict__ psi,
+                 float *__restrict__ mu, const float *__restrict__ rhop, float rho, float lambda0, TvGeo t, int c0,
+                 int nch_total, double *__restrict__ partials) {
+    constexpr int G = 5;
+    __shared__ float cs[3][256];
+    const int n = t.n, m = t.m;
+    const int planes = t.nchunks * (t.nzp + 1), pl = blockIdx.x % planes;
+    const int e = blockIdx.x / planes * 256 + threadIdx.x;
+    const int qy = e / (n + 1);
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+    if (qy <= n) {
+        ShrinkCol k;
+        k.init(ucur, uold, psi, mu, rhop ? *rhop : rho, lambda0, t, c0 + pl / (t.nzp + 1), nch_total, e - qy * (n + 1),
+               qy, pl % (t.nzp + 1));
+        const float *u = k.u;
+        float *pm = k.pm, *pp = k.pp;
+        float f[2] = {u[0], at(u, k.du[1])};
+#pragma unroll 1
+        for (int q0 = 0; q0 <= m; q0 += G) {
+            float mv[G][4], fx[G][2], fy[G][2], fz[G][2], ft[G][2];
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if (q0 + j > m) break;
+                const float *v = u;  // (x0, y0, t0, z0) of the point
+                if (j > 0) v += (j - (q0 == 0 ? 1 : 0)) * k.nn;
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {  // (neighbours a clamp maps to the voxel itself stay unset)
+                    const float *us = &at(v, k.du[s]);
+                    if (k.xin) fx[j][s] = us[1];
+                    if (k.yin) fy[j][s] = us[n];
+                    fz[j][s] = at(v, k.dz[s]);
+                    if (q0 + j > 0 && q0 + j < m) ft[j][s] = us[k.nn];
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) mv[j][i] = at(pm + j * k.st, k.ci[i]);
+            }
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                if (q0 + j > m) break;
+                float g[2][4], r2, s2;
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    if (q0 + j == 0 || q0 + j == m) ft[j][s] = f[s];
+                    k.grad(f[s], k.xin ? fx[j][s] : f[s], k.yin ? fy[j][s] : f[s], fz[j][s], ft[j][s], g[s]);
+                }
+                shrink_point(g, pm, pp, k, mv[j], r2, s2);
+                a0 += r2;
+                a1 += s2;
+                if (q0 + j >= 1 && k.inner) {
+                    const float dd = f[0] - f[1];
+                    a2 = fmaf(dd, dd, a2);
+                }
+                f[0] = ft[j][0];
+                f[1] = ft[j][1];
+                if (q0 + j > 0) u += k.nn;
+                pm += k.st;
+                pp += k.st;
+            }
+        }
+    }
+    cs[0][threadIdx.x] = a0;
+    cs[1][threadIdx.x] = a1;
+    cs[2][threadIdx.x] = a2;
+    block_sums3(cs, 256, partials + 3LL * blockIdx.x);
 }
 
 int shrink_blocks(const TvGeo &t, int nchunks) {
     return (int)(((long long)(t.n + 1) * (t.n + 1) + 255) / 256) * nchunks * (t.nzp + 1);
 }
 
-int launch_shrink(const float *u_cur, const float *u_old, float *psi, float *mu, const float *rho,
+int launch_shrink(const float *u_cur, const float *u_old, float *psi, float *mu, const float *rho_d, float rho,
                   float lambda0, int c0, int nchunks_total, const TvGeo &t, double *partials,
                   cudaStream_t s) {
     const int nb = shrink_blocks(t, t.nchunks);
-    k_shrink<<<nb, 256, 0, s>>>(u_cur, u_old, psi, mu, rho, lambda0, t, c0, nchunks_total, partials);
+    if (nb <= 152 * 2)
+        k_shrink_few<<<nb, 256, 0, s>>>(u_cur, u_old, psi, mu, rho_d, rho, lambda0, t, c0, nchunks_total, partials);
+    else
+        k_shrink<<<nb, 256, 0, s>>>(u_cur, u_old, psi, mu, rho_d, rho, lambda0, t, c0, nchunks_total, partials);
     LAUNCH_CHECK("k_shrink");
     return nb;
 }

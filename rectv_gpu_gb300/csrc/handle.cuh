@@ -545,6 +545,7 @@ struct Handle {
             hp.sincos = dplan.sincos;
             hp.adj_pts = std::move(dplan.adj_pos);
             hp.adj_items = dir_adj_work(dplan.adj_items, vec_planes(ug, zb) / ug.jg);
+            dplan.fwd_items = dir_fwd_work(dplan.fwd_items, vec_planes(ug, zb) / ug.jg);
         } else {
             hp = build_plan(theta_h, n, ntheta, ug.T, table_capacity(), tc_min_spr);
         }

@@ -318,7 +318,12 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
 // pairs, the others tens), but no block has fewer than 256 pairs x planes.  A
 // tile with more than half a resident block's whole share of the work (small
 // problems: few tiles, most of them dense) goes to four blocks per plane, one
-// per four rows (item.x = 5 tile + 1 + row group; 5 tile for whole tiles).
+// per four rows, from 256 pairs and two whole shares up to eight, one per two
+// rows (item.x = 16 tile + 1 + group of four rows, + 5 + pair of rows, or 16
+// tile for whole tiles).  A pair costs a warp about 1000 cycles, so it is the
+// densest tiles' pairs per warp that a small problem waits for: a launch at 64
+// directions of width 64 (8 slices, 8 samples) 33 us, 42 in four at most; 180
+// directions of width 256 (8 slices, 4 samples) 92 us, 123 in four at most.
 std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz) {
     constexpr long long kBlocks = 456;  // resident blocks: three per SM
     long long total = 0;
@@ -327,14 +332,30 @@ std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz) {
     std::vector<int4> work;
     for (const int4 &t : tiles) {
         const bool split = t.z >= 32 && 2LL * t.z > share;
+        const int ways = !split ? 1 : (t.z >= 256 && t.z > 2 * share ? 8 : 4);
         const int per =
             split ? 1 : (int)std::max<long long>(1, std::min<long long>(npz, budget / std::max(1, t.z)));
         for (int p = 0; p < npz; p += per)
-            for (int r = 0; r < (split ? 4 : 1); ++r)
-                work.push_back(make_int4(5 * t.x + (split ? 1 + r : 0), t.y, t.z, p | std::min(npz, p + per) << 16));
+            for (int r = 0; r < ways; ++r)
+                work.push_back(make_int4(16 * t.x + (ways == 1 ? 0 : ways == 4 ? 1 + r : 5 + r), t.y, t.z,
+                                         p | std::min(npz, p + per) << 16));
     }
-    auto cost = [](const int4 &a) { return (long long)a.z * ((a.w >> 16) - (a.w & 0xffff)) * (a.x % 5 ? 1 : 4); };
+    auto cost = [](const int4 &a) { return (long long)a.z * ((a.w >> 16) - (a.w & 0xffff)) * 8 / ((a.x & 15) == 0 ? 1 : (a.x & 15) < 5 ? 4 : 8); };
     std::stable_sort(work.begin(), work.end(), [&](const int4 &a, const int4 &b) { return cost(a) > cost(b); });
+    return work;
+}
+
+// A gather block takes its item's pairs eight at a time, so a problem with less
+// than two waves of blocks (two per SM) has its items halved, down to 16 pairs:
+// a launch at 64 directions of width 64 (4 planes) 11 us, 16 with 64 pairs.
+std::vector<int4> dir_fwd_work(const std::vector<int4> &items, int npz) {
+    std::vector<int4> work = items;
+    for (int cap = 32; cap >= 16 && (long long)work.size() * npz < 608; cap /= 2) {
+        std::vector<int4> half;
+        for (const int4 &it : work)
+            for (int i = 0; i < it.z; i += cap) half.push_back(make_int4(it.x, it.y + i, std::min(cap, it.z - i), it.w));
+        work.swap(half);
+    }
     return work;
 }
 

@@ -253,6 +253,7 @@ int dir_fwd_capacity();       // position pairs per forward item
 // work items of the adjoint over npz planes: (tile, start, count, first plane |
 // end plane << 16) of a plan's (tile, start, count), the most work first
 std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz);
+std::vector<int4> dir_fwd_work(const std::vector<int4> &items, int npz);  // and of the forward gather
 size_t dir_mix_bytes(const UsGeo &g, int zb, int ndir);  // the adjoint's per-position mixing buffer
 // hand-written 2D FFTs of the zero-padded grids in the vector layout
 // (fft_kernels.cu), P = 2n a power of two in [256, 2048]: forward =

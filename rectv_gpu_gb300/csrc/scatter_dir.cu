@@ -221,9 +221,10 @@ __global__ void __launch_bounds__(kMThr)
 // the left and the right eight cells each only if the window reaches them.
 // Warps wait for copies only, never for each other.  All sums run in entry
 // order; the cells leave as full 128-byte lines.
-// Split items (item.x % 5 > 0): a block has four rows of the tile, its warps
-// take every fourth entry each and add up at the end in warp order: four times
-// the blocks for problems whose tiles would leave SMs idle (dir_adj_work).
+// Split items (item.x % 16 > 0): a block has four (two) rows of the tile, its
+// warps take every fourth (eighth) entry each and add up at the end in warp
+// order: four (eight) times the blocks for problems whose tiles would leave SMs
+// idle (dir_adj_work).
 // Measured at n = 1024, 360 directions, 16 time samples, 16 slices: 3.47 ms a
 // launch (a scatter of every position with float2 atomics into cleared half
 // planes: 6.4 ms).  Bound by instruction issue (59 % active; 105 instructions
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(kSThr, 3)
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int4 it = items[blockIdx.x];
     const int ntx = (g.vp + kT - 1) / kT;
-    const int tile = it.x / 5, sub = it.x - 5 * tile;  // sub > 0: row group sub - 1 alone
+    const int tile = it.x >> 4, sub = it.x & 15;  // sub 1..4: rows 4 (sub - 1) .. alone; 5..12: rows 2 (sub - 5) ..
     const int ty = tile / ntx, Y0 = ty * kT, X0 = (tile - ty * ntx) * kT;  // window cell (0, 0) of the tile
     const int p0 = it.w & 0xffff, p1 = it.w >> 16;
     const int nh = g.n / 2, nseg = (it.z + kSCap - 1) / kSCap;
@@ -320,8 +321,10 @@ __global__ void __launch_bounds__(kSThr, 3)
             }
         }
     };
-    const int rg = sub ? 2 * (sub - 1) + (wid & 1) : wid & 7;  // this warp's pair of rows
-    const uint32_t part = sub ? 0x11111111u << ((wid >> 1) & 3) : 0xffffffffu;
+    // this warp's pair of rows and its entries; the first nl warps sum a pair's warps
+    const int nl = sub == 0 ? kSWarps : (sub < 5 ? 2 : 1);
+    const int rg = sub == 0 ? wid & 7 : (sub < 5 ? 2 * (sub - 1) + (wid & 1) : sub - 5);
+    const uint32_t part = sub == 0 ? 0xffffffffu : (sub < 5 ? 0x11111111u << ((wid >> 1) & 3) : 0x01010101u << (wid & 7));
     const int vi = lane & 15, ry = 2 * rg + (lane >> 4);
     float2 acc[2][8];  // [re, im][cell pair]
     bool ok = true;
@@ -436,17 +439,17 @@ __global__ void __launch_bounds__(kSThr, 3)
                                      : "memory");
                 }
             }
-            if (sub) {  // add the four warps' sums, in warp order, through the (idle) stages
+            if (sub) {  // add the four or eight warps' sums, in warp order, through the (idle) stages
                 __syncthreads();
                 float2 *red = reinterpret_cast<float2 *>(sm.m);
-                static_assert(sizeof(sm.m) >= 6 * 16 * 32 * sizeof(float2), "six warps' sums");
-                if (wid > 1 && wid < kSWarps) {
+                static_assert(sizeof(sm.m) >= 7 * 16 * 32 * sizeof(float2), "seven warps' sums");
+                if (wid >= nl && wid < kSWarps) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) red[((wid - 2) * 16 + i) * 32 + lane] = acc[i >> 3][i & 7];
+                    for (int i = 0; i < 16; ++i) red[((wid - nl) * 16 + i) * 32 + lane] = acc[i >> 3][i & 7];
                 }
                 __syncthreads();
-                if (wid < 2) {
-                    for (int w = wid; w < 6; w += 2)
+                if (wid < nl) {
+                    for (int w = wid; w < kSWarps - nl; w += nl)
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
                             const float2 o = red[(w * 16 + i) * 32 + lane];
@@ -457,7 +460,7 @@ __global__ void __launch_bounds__(kSThr, 3)
                 tc::fence_proxy_async();  // before the next copies into the stages
                 __syncthreads();
             }
-            if (wid < (sub ? 2 : kSWarps) && Y0 + ry < g.vrows) {  // the pre-IFFT fftshift sign is applied here
+            if (wid < nl && Y0 + ry < g.vrows) {  // the pre-IFFT fftshift sign is applied here
                 const float sy = ((X0 + Y0 + ry) & 1) ? -1.f : 1.f;
 #pragma unroll
                 for (int c = 0; c < kT; ++c) {

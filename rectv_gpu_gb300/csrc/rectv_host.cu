@@ -27,6 +27,7 @@
 
 #include "rectv_gb300.h"
 #include "handle.cuh"
+#include "host_pages.h"
 #include "rectv_internal.cuh"
 #include "tcgen05.cuh"
 
@@ -115,11 +116,13 @@ int rectv_run(rectv_handle *h, float *fres, const float *g, const float *theta, 
     return rectv::guarded([&] {
         rectv::Handle *H = live(h);
         if (!fres || !g || !theta || !phi) throw rectv::Error(RECTV_ERR_ARG, "rectv_run: null pointer");
+        const size_t nf = (size_t)H->nzc * H->slab;
+        rectv::ResultPages pages(fres, sizeof(float) * nf);
         CUDA_CHECK(cudaMemcpyAsync(H->gdata, g, sizeof(float) * (size_t)H->nz * H->ntheta * H->n,
                                    cudaMemcpyHostToDevice, H->stream));
         H->setup(theta, phi, center, lambda0, lambda1, titer);
         H->iterate(niter);
-        const size_t nf = (size_t)H->nzc * H->slab;
+        pages.wait();
         CUDA_CHECK(cudaMemcpyAsync(fres, H->U[H->cur], sizeof(float) * nf, cudaMemcpyDeviceToHost, H->stream));
         CUDA_CHECK(cudaStreamSynchronize(H->stream));
         const size_t total = (size_t)H->nz * H->slab;
@@ -296,11 +299,13 @@ int rectv_run_init(rectv_handle *h, float *fres, const float *g, const float *th
     return rectv::guarded([&] {
         rectv::Handle *H = live(h);
         if (!fres || !g || !theta || !phi) throw rectv::Error(RECTV_ERR_ARG, "rectv_run_init: null pointer");
+        const size_t nf = (size_t)H->nzc * H->slab;
+        rectv::ResultPages pages(fres, sizeof(float) * nf);
         CUDA_CHECK(cudaMemcpyAsync(H->gdata, g, sizeof(float) * (size_t)H->nz * H->ntheta * H->n,
                                    cudaMemcpyHostToDevice, H->stream));
         H->setup(theta, phi, center, lambda0, lambda1, titer, finit);
         H->iterate(niter);
-        const size_t nf = (size_t)H->nzc * H->slab;
+        pages.wait();
         CUDA_CHECK(cudaMemcpyAsync(fres, H->U[H->cur], sizeof(float) * nf, cudaMemcpyDeviceToHost, H->stream));
         CUDA_CHECK(cudaStreamSynchronize(H->stream));
         const size_t total = (size_t)H->nz * H->slab;

@@ -12,10 +12,15 @@ namespace rectv {
 
 namespace {
 
-constexpr int kThr = 256, kColThr = 256;
+// Threads per block.  Columns: 192 in three blocks per SM (four where a tile has eight
+// values): the radix passes have P / R x C items, few more than the threads, and
+// wider blocks left half of a last round idle (8 planes of 505 columns of 1008
+// points 0.279 ms, 0.291 with 256, 0.332 with 352; 4 planes of 65 x 128 points 4.6
+// us, 7.3 with 256).  Residual rows: 128 in six blocks (0.107 ms, 0.116 with 256 in three).
+constexpr int kThr = 256, kColThr = 192, kResThr = 128;
 
 template <int C>
-__global__ void __launch_bounds__(kColThr, 3)
+__global__ void __launch_bounds__(kColThr, C == 8 ? 4 : 3)
     k_gen_cols_inv(float2 *__restrict__ spec, const __grid_constant__ GenPlan p, const float2 *__restrict__ tw, UsGeo g, int nlv, int ntiles) {
     gen::cols<C, 1>(spec, p, tw, g, nlv, ntiles);
 }
@@ -103,13 +108,13 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
 // row, of which the Hermitian part counts.
 // ---------------------------------------------------------------------------
 template <int C, bool HALF>
-__global__ void __launch_bounds__(kThr, 3)
+__global__ void __launch_bounds__(kResThr, 6)
     k_gen_resid(const float2 *__restrict__ rows, const float *__restrict__ gdata, float2 *__restrict__ out,
                 const __grid_constant__ GenPlan p, const float2 *__restrict__ tw, long long nrows, float scale) {
     using gen::gen_sh;
     const int n = p.P, hn = n / 2 + 1;
     const int c = threadIdx.x % C, j0 = threadIdx.x / C;
-    constexpr int js = kThr / C;
+    constexpr int js = kResThr / C;
     const long long ra = 2 * ((long long)blockIdx.x * C + c), rb = ra + 1;
     const bool oka = ra < nrows, okb = rb < nrows;
     const int rn = HALF ? hn : n;  // values per row
@@ -182,9 +187,9 @@ void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
     const size_t smem = gen_rows_smem(g.n, C);
     if (half)
-        k_gen_resid<C, true><<<(unsigned)nblk, kThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
+        k_gen_resid<C, true><<<(unsigned)nblk, kResThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
     else
-        k_gen_resid<C, false><<<(unsigned)nblk, kThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
+        k_gen_resid<C, false><<<(unsigned)nblk, kResThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
     LAUNCH_CHECK("k_gen_resid");
 }
 

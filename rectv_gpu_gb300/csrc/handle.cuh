@@ -336,6 +336,7 @@ struct Handle {
         rho_d = alloc<float>(1);
         iter_ctr = alloc<int>(1);
         gd.err = alloc<int>(1);
+        gd.sc_next = alloc<int>(1);
         CUDA_CHECK(cudaMemsetAsync(gd.err, 0, sizeof(int), stream));
         auto table = [&](const std::vector<float2> &w) {
             float2 *d = alloc<float2>(w.size());
@@ -454,9 +455,10 @@ struct Handle {
         for (void *p : geo_owned) cudaFreeAsync(p, stream);
         geo_owned.clear();
         geo_bytes = 0;
-        int *err = gd.err;
+        int *err = gd.err, *next = gd.sc_next;
         gd = GeoDev();
         gd.err = err;
+        gd.sc_next = next;
     }
 
     // Queue this handle's work on s (a stream of the same device) from now on;

@@ -119,6 +119,7 @@ struct GeoDev {
     int4 *adj_items = nullptr;   // (tile, start, count, 0), whole tiles
     int n_adj_items = 0;
     int *err = nullptr;          // device counter of host/device bin disagreements
+    int *sc_next = nullptr;      // unit counter of the tensor-core scatter, zeroed by each launch
     bool tc_scatter = false;     // adjoint time-sample mixing on the tensor cores (k_scatter_tc)
     AdjRec *adj_recs = nullptr;  // geometry records of adj_pts (tensor-core scatter only)
     int n_adj_busy = 0;          // leading adj_items with samples (items are sorted by count)

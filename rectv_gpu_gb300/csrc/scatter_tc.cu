@@ -21,7 +21,9 @@
 // by k_adj_tabinfo.
 //
 // Persistent blocks of 512 threads, one per SM, take the (tile, slice pair)
-// units with samples round-robin; each block half (256 threads, thread =
+// units with samples one after another from a counter, the fullest tiles first
+// (8 slices, 1440 angles, width 480: 1.30 ms; 1.54 in a fixed round-robin, where the
+// blocks with the centre tiles finished a fifth later than the others); each block half (256 threads, thread =
 // cell) works on one slice of the pair, and the halves share what does not
 // depend on the slice: the records, the segmentation, K' (the MMA's B) and
 // the barriers.  The records and segmentation of the next table are
@@ -96,6 +98,7 @@ struct ScTcSmem {
     float blo[kN * kK];           // B - trunc(B): rows 32..63 (contiguous with bhi)
     unsigned long long bar;      // MMA batch done (both slices)
     unsigned long long rbar[2];  // record buffer landed
+    int uq[4];                   // the block's coming units
     uint32_t tslot;
 };
 
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(kThr, 1)
                  const int4 *__restrict__ items, const int4 *__restrict__ tabs, const int *__restrict__ tab_base,
                  const uint32_t *__restrict__ info, const float2 *__restrict__ kmat,
                  const float2 *__restrict__ shifta, UsGeo g, int zb, int npairs, int nunits, int jgrp,
-                 int *__restrict__ err) {
+                 int *__restrict__ next, int *__restrict__ err) {
     const int jbase = 16 * jgrp;
     extern __shared__ __align__(1024) unsigned char sc_smem_raw[];
     ScTcSmem &sm = *reinterpret_cast<ScTcSmem *>(sc_smem_raw);
@@ -291,7 +294,11 @@ __global__ void __launch_bounds__(kThr, 1)
     // Thread 0's copy cursor: the next table (unit, first entry) to fetch, in
     // the order the tables are consumed; a table is fetched while the one
     // before it is processed.
-    int fu = blockIdx.x, ft = 0;
+    // The cursor takes the block's next unit when the last table of one has been
+    // fetched, and leaves it for the others in uq: unit k of the block in slot k % 4
+    // (the cursor is at most two units ahead of them).  The unit after that is
+    // claimed one step early, so that no step waits for the counter.
+    int fu = blockIdx.x, ft = 0, fk = 0, claimed = tid == 0 ? atomicAdd(next, 1) : 0;
     auto fetch = [&](int slot) {  // records and segmentation of table ft of unit fu
         if (fu >= nunits) return;
         const int item = fu / npairs;
@@ -311,17 +318,20 @@ __global__ void __launch_bounds__(kThr, 1)
                      : "memory");
         if (++ft >= tb1 - tb0) {
             ft = 0;
-            fu += gridDim.x;
+            fu = min(nunits, (int)gridDim.x + claimed);
+            sm.uq[++fk & 3] = fu;
+            claimed = atomicAdd(next, 1);
         }
     };
     if (tid == 0) fetch(0);
     bool have_next = false;  // rnext holds the current table's row spectrum values (both slices)
 
-    // persistent: units (tile item, slice pair) round-robin, pairs fastest, so
-    // the blocks in flight share their items' records in L2; all units hold
-    // samples.  The two halves share the records, ray starts, sample ranges and
-    // K' (B); each has its slice's E, T, A, accumulator and sums.
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
+    // persistent: units (tile item, slice pair) as blocks come free, the most
+    // samples first and pairs fastest, so that the blocks in flight share their
+    // items' records in L2; all units hold samples.  The two halves share the
+    // records, ray starts, sample ranges and K' (B); each has its slice's E, T, A,
+    // accumulator and sums.
+    for (int u = blockIdx.x, nxt = 1; u < nunits; u = sm.uq[nxt & 3], ++nxt) {
         const int z = 2 * (u % npairs) + h;
         const bool zok = z < zb;  // the last pair of an odd batch has one slice
         const int4 it = __ldg(items + u / npairs);
@@ -434,7 +444,7 @@ __global__ void __launch_bounds__(kThr, 1)
                 if (sb == 0) {
                     int nti = ti + 1, nu = u;
                     if (nti >= tb1) {
-                        nu = u + gridDim.x;
+                        nu = sm.uq[nxt & 3];
                         nti = nu < nunits ? __ldg(tab_base + nu / npairs) : 0;
                     }
                     have_next = nu < nunits;
@@ -543,7 +553,8 @@ __global__ void __launch_bounds__(kThr, 1)
         }
         // ---- the cell's sums into the half planes, from its own lane: swapping
         // the chunks first, so that 4 or 8 lanes add to one cell, measured slower
-        // (8 slices, 1440 angles, width 480, 16 samples: 1.99 and 1.72 ms, this form 1.55) ----
+        // (8 slices, 1440 angles, width 480, 16 samples: 1.99 and 1.72 ms, this form
+        // 1.55, all with units in fixed order) ----
         if (zok) {
             float2 *base = spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
             const float sg = ((cx + cy) & 1) ? -0.5f : 0.5f;
@@ -578,7 +589,7 @@ void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &
     const int npairs = (zb + kZ - 1) / kZ;
     const long long nunits = (long long)npairs * gd.n_adj_busy;
     if (nunits == 0) return;
-    if (nunits > 2147483647LL) throw Error(1, "adjoint grid too large");
+    if (nunits > 2147483647LL - 262144) throw Error(1, "adjoint grid too large");
     static int nsm = 0;
     if (nsm == 0) {
         int dev = 0;
@@ -587,9 +598,10 @@ void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &
     }
     const int grid = (int)std::min<long long>(nunits, g.sc_grid > 0 ? g.sc_grid : nsm);
     if (!gd.adj_tabs || !gd.adj_info) throw Error(1, "adjoint table segmentation missing");
+    CUDA_CHECK(cudaMemsetAsync(gd.sc_next, 0, sizeof(int), s));
     k_scatter_tc<<<grid, kThr, kScSmemBytes, s>>>(rowsc, spec, gd.adj_recs, gd.adj_items, gd.adj_tabs,
                                                   gd.adj_tab_base, gd.adj_info, gd.kmat, gd.shiftadj, g, zb, npairs,
-                                                  (int)nunits, jgrp, gd.err);
+                                                  (int)nunits, jgrp, gd.sc_next, gd.err);
     LAUNCH_CHECK("k_scatter_tc");
 }
 

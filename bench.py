@@ -713,22 +713,17 @@ def run_ours(args, rank, world, local_rank):
     peak, peak_kind = measured_peaks()
     achieved = bytes_.value / (ktimes[dom] * 1e-3) / 1e9
     limiter = {
-        "k_adj_mix+k_scatter_dir": "k_scatter_dir (~90% of the pair): per-cell FP32 sums of w E + w_perp E_perp "
-                                   "over the entries touching each 4x4-cell block (two lanes per cell) -- latency of "
-                                   "the shared-memory loads of E and of the packed-FMA chains with 16 warps per SM "
-                                   "(two 8-warp blocks at 128 registers; issue ~54% active, L1/shared ~73% busy, FMA "
-                                   "pipe ~38%); float2 atomics into the Hermitian half planes; DRAM ~20% of peak, so "
-                                   "not DRAM-bound",
-        "k_gather_dir": "latency of the footprint loads and block barriers (two 8-warp blocks per SM at 121 "
-                        "registers, ~30 positions per tile and slice) and shared-memory bandwidth of the 81-tap "
-                        "reads (L1/shared pipe ~70% busy); DRAM ~14% of peak",
-        "k_scatter_tc": "block barriers and the per-cell ray sums on the CUDA cores (shared-memory loads), "
-                        "the tcgen05 time-sample GEMM (3xTF32) at ~14% of the tensor pipe; DRAM traffic 4.0x "
-                        "the algorithmic bytes (float2 atomics read and write every Hermitian half-plane cell "
-                        "twice), about 1.7 TB/s (25% of the DRAM peak) at full size, so not DRAM-bound",
+        "k_adj_mix+k_scatter_dir": "instruction issue of k_scatter_dir (88% of the pair; 62% active, ~100 instructions "
+                                   "per position pair and two tile rows, 24 warps per SM at 72 registers) and the "
+                                   "latency of its shared loads; FMA pipe 41%, DRAM 18% of peak, so not DRAM-bound",
+        "k_gather_dir": "shared-memory bandwidth of the 10x10-cell reads of a position pair (L1/shared pipe ~58% busy) "
+                        "and the latency of the footprint loads (two 8-warp blocks per SM at 122 registers); DRAM "
+                        "~20% of peak",
+        "k_scatter_tc": "block barriers and the per-cell ray sums on the CUDA cores (shared-memory loads; issue ~46%), "
+                        "the tcgen05 time-sample GEMM (3xTF32); float4 atomics into the Hermitian half planes; DRAM "
+                        "~10% of peak",
         "k_gather_tc": "shared-memory bandwidth of the per-sample 81-tap sums and of the TMEM -> shared "
-                       "read-out of G, block barriers; TMA-staged footprints, DRAM traffic 3.0x the spectra "
-                       "(overlapping footprints) at 8% of the DRAM peak",
+                       "read-out of G (L1/shared pipe ~57% busy), block barriers; DRAM ~9% of peak",
         "k_graddiv": "HBM bandwidth", "k_shrink": "HBM bandwidth",
         KERNEL_NAMES[4]: "HBM bandwidth", KERNEL_NAMES[5]: "HBM bandwidth"}[names[dom]]
     fma = ctypes.c_double()

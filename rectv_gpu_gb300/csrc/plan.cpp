@@ -315,7 +315,9 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
 
 // A tile's planes are split so that a block has about an eighth of a wave's
 // share of the work (the tiles at the centre of the spectrum hold thousands of
-// pairs, the others tens), but no block has fewer than 256 pairs x planes.  A
+// pairs, the others tens), but no block has fewer than 256 pairs x planes, or than
+// half a share (32 at least) where the whole problem has few: 12 directions of
+// width 64, 8 planes, 15 us a launch, 33 with 256.  A
 // tile with more than half a resident block's whole share of the work (small
 // problems: few tiles, most of them dense) goes to four blocks per plane, one
 // per four rows, from 256 pairs and two whole shares up to eight, one per two
@@ -328,13 +330,14 @@ std::vector<int4> dir_adj_work(const std::vector<int4> &tiles, int npz) {
     constexpr long long kBlocks = 456;  // resident blocks: three per SM
     long long total = 0;
     for (const int4 &t : tiles) total += (long long)t.z * npz;
-    const long long budget = std::max<long long>(256, total / (8 * kBlocks)), share = total / kBlocks;
+    const long long share = total / kBlocks;
+    const long long part = std::max(total / (8 * kBlocks), std::min<long long>(256, std::max<long long>(32, share / 2)));
     std::vector<int4> work;
     for (const int4 &t : tiles) {
         const bool split = t.z >= 32 && 2LL * t.z > share;
         const int ways = !split ? 1 : (t.z >= 256 && t.z > 2 * share ? 8 : 4);
         const int per =
-            split ? 1 : (int)std::max<long long>(1, std::min<long long>(npz, budget / std::max(1, t.z)));
+            split ? 1 : (int)std::max<long long>(1, std::min<long long>(npz, part / std::max(1, t.z)));
         for (int p = 0; p < npz; p += per)
             for (int r = 0; r < ways; ++r)
                 work.push_back(make_int4(16 * t.x + (ways == 1 ? 0 : ways == 4 ? 1 + r : 5 + r), t.y, t.z,

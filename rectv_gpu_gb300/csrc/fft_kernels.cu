@@ -337,13 +337,7 @@ __device__ __forceinline__ void mbar_expect(void *bar, uint32_t bytes) {
 // the current one is loaded by TMA into the second landing buffer while the
 // current one is transformed, and each output tile leaves by TMA stores from
 // the exchange buffer, which the next tile reuses once those stores have read
-// it.  Forward tiles from P = 1024 up have half as many rows as the exchange
-// buffer, so with one landing buffer (free as soon as the tile is in registers)
-// two blocks of 64 registers fit an SM and hide each other's barriers: 256
-// images of P = 2048 1.42 ms (1.46 with one block), of P = 1024 0.314 (0.354).
-// At P = 512 (0.104 against 0.091) and for the inverse, whose tiles would have to
-// land in the exchange buffer (P = 2048 1.46 against 1.36, P = 1024 0.357 against
-// 0.306), one block with two landing buffers is the faster.
+// it.
 //
 // Forward: the row pass's output (rows [n/2, 3n/2); the others are zero and
 // not read), P-point FFT, all P rows written back in place.
@@ -366,12 +360,11 @@ struct ColPass {
     using L = FftLayout<N, true, C>;
     static constexpr size_t EX = (size_t)L::S * C > (size_t)OUT_ROWS * C ? (size_t)L::S * C : (size_t)OUT_ROWS * C;
     static constexpr size_t LAND = (size_t)IN_ROWS * C;          // float2 per landing buffer
-    static constexpr int NL = DIR < 0 && N >= 1024 ? 1 : 2;       // landing buffers
-    static constexpr size_t SMEM = sizeof(float2) * (EX + NL * LAND);
+    static constexpr size_t SMEM = sizeof(float2) * (EX + 2 * LAND);
 };
 
 template <int N, int C, int DIR>
-__global__ void __launch_bounds__(C *(N / 16), 3 - ColPass<N, C, DIR>::NL)
+__global__ void __launch_bounds__(C *(N / 16), 1)
     k_fft_cols(const __grid_constant__ CUtensorMap tmap, const float2 *__restrict__ tw, int ngroups, int nlv,
                int ntiles, int *__restrict__ err) {
     using CP = ColPass<N, C, DIR>;
@@ -379,11 +372,11 @@ __global__ void __launch_bounds__(C *(N / 16), 3 - ColPass<N, C, DIR>::NL)
     constexpr int N1 = N / 16, n = N / 2, BR = CP::BR;
     extern __shared__ __align__(1024) float2 fft_sh[];
     float2 *ex = fft_sh;  // exchange buffer / output tile; landing buffers follow it
-    constexpr int NL = CP::NL;
-    __shared__ uint64_t bar[NL];
+    __shared__ uint64_t bar[2];
     const int c = threadIdx.x % C, t = threadIdx.x / C;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < NL; ++i) tc::mbar_init(&bar[i], 1);
+        tc::mbar_init(&bar[0], 1);
+        tc::mbar_init(&bar[1], 1);
         tc::fence_mbar_init();
     }
     __syncthreads();
@@ -397,12 +390,11 @@ __global__ void __launch_bounds__(C *(N / 16), 3 - ColPass<N, C, DIR>::NL)
     bool ok = true;
     int it = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
-        const int buf = it % NL;
-        const bool more = threadIdx.x == 0 && tile + (int)gridDim.x < ntiles;
+        const int buf = it & 1;
         // the other landing buffer was read in the previous iteration, before
         // at least one block barrier: it takes the next tile
-        if (NL == 2 && more) fetch(tile + gridDim.x, buf ^ 1);
-        ok = tc::mbar_wait(&bar[buf], (uint32_t)((it / NL) & 1), ok) && ok;
+        if (threadIdx.x == 0 && tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x, buf ^ 1);
+        ok = tc::mbar_wait(&bar[buf], (uint32_t)((it >> 1) & 1), ok) && ok;
         float2 v[16];
         const float2 *in = fft_sh + CP::EX + buf * CP::LAND;
 #pragma unroll
@@ -414,7 +406,6 @@ __global__ void __launch_bounds__(C *(N / 16), 3 - ColPass<N, C, DIR>::NL)
         }
         if (threadIdx.x == 0) tma_store_wait_read();  // the previous output tile has left the exchange buffer
         __syncthreads();
-        if (NL == 1 && more) fetch(tile + gridDim.x, 0);  // the tile is in registers
         fft_core<N, DIR, L>(v, ex, c, t, tw);
         __syncthreads();
 #pragma unroll

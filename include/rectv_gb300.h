@@ -130,7 +130,7 @@ int rectv_set_graphs(rectv_handle *h, int enable);
  *   divergence step, 3 shrink + dual update + residual sums, 4 forward
  *   padded-grid 2D FFT (row and column kernels), 5 inverse padded-grid 2D FFT
  *   (column and row kernels; 4 and 5 exist where the hand-written FFTs
- *   run: 2n at most 2048 with prime factors up to 13), 6 fused gradient-divergence step of the first inner
+ *   run: 2n at most 2048 with prime factors up to 19), 6 fused gradient-divergence step of the first inner
  *   iteration (2 is then the step of the later inner iterations).
  * ------------------------------------------------------------------------- */
 

@@ -1,6 +1,6 @@
 // Mixed-radix FFT passes in shared memory for transform lengths that are no
 // power of two (fft_general_fwd.cu, fft_general_inv.cu): Stockham passes of
-// radix 2 .. 16, at most four for the lengths in use, C transforms interleaved
+// radix 2 .. 16, 17 and 19, at most four for the lengths in use, C transforms interleaved
 // (element i of transform c at i C + c).
 #pragma once
 
@@ -237,6 +237,8 @@ __device__ __forceinline__ void any_pass(int so, int d0, const GenPlan &g, int p
         RECTV_PASS(13)
         RECTV_PASS(15)
         RECTV_PASS(16)
+        RECTV_PASS(17)
+        RECTV_PASS(19)
 #undef RECTV_PASS
     }
 }

@@ -1,5 +1,5 @@
 // Forward padded-grid FFT for grid sides 2n that are no
-// power of two in [256, 2048] but a product of radices up to 16 (detector
+// power of two in [256, 2048] but a product of radices up to 19 (detector
 // widths such as 480 and 504), in the vector layout: the passes of
 // fft_kernels.cu (rows of value pairs as one complex transform, only the n
 // non-zero rows; columns with the padding not read) on the mixed-radix core
@@ -98,12 +98,12 @@ void gen_fft_fwd_prepare() {
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 }
 
-// Radices of P, at most six of 2 .. 13, 15, 16, as few as possible and then as
+// Radices of P, at most six of 2 .. 13, 15, 16, 17, 19, as few as possible and then as
 // even as possible; an odd one first where there is one (the first pass
 // writes with the stride of its radix: odd strides are free of bank
 // conflicts).  False when P has a larger prime factor or does not fit.
 bool gen_fft_plan(int P, GenPlan *p) {
-    static const int radix[] = {16, 15, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    static const int radix[] = {19, 17, 16, 15, 13, 12, 11, 10, 9, 8, 7, 6, 5, 4, 3, 2};
     if (P < 32 || P > 2048 || P % 2) return false;
     int best[6], nbest = 7, cur[6];
     long long cost = 0;
@@ -121,7 +121,7 @@ bool gen_fft_plan(int P, GenPlan *p) {
                 return;
             }
             if (depth == 6) return;
-            for (int i = from; i < 14; ++i)
+            for (int i = from; i < 16; ++i)
                 if (rest % radix[i] == 0) {
                     cur[depth] = radix[i];
                     go(rest / radix[i], i, depth + 1, cur, best, nbest, cost);

@@ -271,7 +271,7 @@ void launch_pad_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const f
                               const CUtensorMap &map, int *err, const UsGeo &g, cudaStream_t s);
 // mixed-radix passes for grid sides that are no power of two (fft_general.cuh,
 // fft_general_fwd.cu, fft_general_inv.cu): even lengths 32 .. 2048 with prime
-// factors up to 13
+// factors up to 13, 17 or 19
 struct GenPlan {
     int P, np;           // length, passes
     int R[6], Ns[6];     // radix of a pass, product of the radices before it

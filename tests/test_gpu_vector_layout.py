@@ -31,7 +31,7 @@ def _phi(ntheta, m, seed):
 CASES = [
     # n, ntheta, m, nz, nrot, centre offset
     (32, 32, 1, 3, 4, 0.0),      # one time sample: 16 slices per plane, three of them live
-    (34, 48, 2, 9, 4, 0.5),      # 2n = 68: partial tiles; eight slices per plane, two planes
+    (38, 48, 2, 9, 4, 0.5),      # 2n = 76: partial tiles; eight slices per plane, two planes
     (46, 60, 3, 5, 4, -1.0),     # three of four samples live
     (64, 96, 4, 4, 4, 0.0),
     (40, 72, 5, 3, 8, 0.0),      # five of eight samples, an odd slice
@@ -40,14 +40,15 @@ CASES = [
     (48, 90, 8, 1, 6, 0.0),
     (128, 96, 9, 1, 4, 0.0),     # nine of 16 values live
     (36, 64, 17, 2, 4, 0.0),     # two planes per slice, one sample in the second
-    # mixed-radix grids: every radix of the passes (2n = 100, 88, 104, 84, 120, 144, 196, 960)
-    (50, 40, 4, 2, 4, 0.0),
+    # mixed-radix grids: every radix of the passes (2n = 108, 88, 104, 140, 120, 144, 200, 272, 76, 960)
+    (54, 40, 4, 2, 4, 0.0),
     (44, 40, 16, 1, 4, 0.5),
     (52, 40, 8, 3, 4, 0.0),
-    (42, 40, 4, 3, 4, 0.0),
+    (70, 40, 4, 3, 4, 0.0),
     (60, 40, 12, 1, 4, 0.0),
     (72, 40, 2, 5, 4, -1.5),
-    (98, 40, 8, 2, 4, 0.0),
+    (100, 40, 8, 2, 4, 0.0),
+    (136, 40, 8, 2, 4, 0.0),
     (480, 24, 3, 1, 4, 0.0),
     (64, 256, 16, 1, 2, 0.0),    # 128 directions: tiles with several weight tables, split over blocks
 ]
@@ -85,7 +86,7 @@ def test_operators_match_oracle(lib_built, torch_cuda, monkeypatch, case):
 @pytest.mark.gpu
 @pytest.mark.parametrize("case", [
     # n, ntheta, m, nz, nzp, nrot: mixed-radix grids and residual rows, an odd number of rows
-    (50, 45, 5, 1, 1, 3),
+    (54, 45, 5, 1, 1, 3),
     (84, 36, 16, 3, 1, 4),
 ])
 def test_reconstruction_matches_oracle(lib_built, torch_cuda, case):

@@ -69,12 +69,26 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
         p.sincos[th] = make_float2((float)std::sin(t), (float)std::cos(t));
     }
     const long long npts = (long long)ntheta * (n - 1);
-    std::vector<int> ftile(npts);
-    std::vector<int4> atiles(npts);  // up to 4 tiles, -1 = none
+    std::vector<int2> cell(npts);  // cell (KX, KY) of each sample's stencil origin
     const float tn = (float)(2 * n);
     std::vector<float> qk(n);
     for (int k = 1; k < n; ++k) qk[k] = (float)(k - n / 2) / (float)n;
     if (T < kTaps) throw Error(1, "tile smaller than the interpolation stencil");
+    // Tiles holding any cell of the nine of a stencil's axis (cells wrap modulo P):
+    // those from its first cell's to its last one's.  There are three where the
+    // last tile is narrower than eight cells and the stencil reaches from the tile
+    // before it to the one behind the wrap.
+    auto axis_tiles = [&](int K, int *out) {
+        const int lo = wrapi(K - kR, P), hi = wrapi(K + kR, P), first = lo / T, last = hi / T;
+        int k = 0;
+        out[k++] = first;
+        // (on a grid below 2T cells a wrapped stencil may end in the tile it starts in)
+        for (int t = first; t != last || (k == 1 && lo > hi && NT > 1);) {
+            t = t + 1 < NT ? t + 1 : 0;
+            if (t != first) out[k++] = t;
+        }
+        return k;
+    };
     // Angles are split into contiguous ranges, one per host thread; each
     // thread counts its samples per tile and later places them at its own
     // offsets, so every tile keeps the theta-major sample order.
@@ -96,21 +110,12 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
                 const int fx = (int)std::floor(tn * x0);
                 const int fy = (int)std::floor(tn * y0);
                 const int KX = n + fx, KY = n + fy;  // in [0, P)
-                const int t = (KY / T) * NT + (KX / T);
-                ftile[ip] = t;
-                fcnt[t]++;
-                // tiles holding any cell of the 9x9 stencil (cells wrap modulo P):
-                // a stencil row spans 9 < T cells, so it touches the tiles of its
-                // first and last cell and none between
-                const int xa = wrapi(KX - kR, P) / T, xb = wrapi(KX + kR, P) / T;
-                const int ya = wrapi(KY - kR, P) / T, yb = wrapi(KY + kR, P) / T;
-                const int nx = (xa == xb) ? 1 : 2, ny = (ya == yb) ? 1 : 2;
-                const int xs[2] = {xa, xb}, ys[2] = {ya, yb};
-                int tl[4] = {-1, -1, -1, -1}, nt = 0;
+                cell[ip] = make_int2(KX, KY);
+                fcnt[(KY / T) * NT + KX / T]++;
+                int xs[3], ys[3];
+                const int nx = axis_tiles(KX, xs), ny = axis_tiles(KY, ys);
                 for (int a = 0; a < ny; ++a)
-                    for (int b = 0; b < nx; ++b) tl[nt++] = ys[a] * NT + xs[b];
-                atiles[ip] = make_int4(tl[0], tl[1], tl[2], tl[3]);
-                for (int i = 0; i < nt; ++i) acnt[tl[i]]++;
+                    for (int b = 0; b < nx; ++b) acnt[ys[a] * NT + xs[b]]++;
             }
         }
     };
@@ -148,11 +153,12 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
             for (int th = rg.first; th < rg.second; ++th)
                 for (int k = 1; k < n; ++k, ++ip) {
                     const uint32_t id = (uint32_t)th * (uint32_t)n + (uint32_t)k;
-                    p.fwd_pts[fp[ftile[ip]]++] = id;
-                    const int4 a = atiles[ip];
-                    const int tl[4] = {a.x, a.y, a.z, a.w};
-                    for (int i = 0; i < 4; ++i)
-                        if (tl[i] >= 0) p.adj_pts[ap[tl[i]]++] = id;
+                    const int2 c = cell[ip];
+                    p.fwd_pts[fp[(c.y / T) * NT + c.x / T]++] = id;
+                    int xs[3], ys[3];
+                    const int nx = axis_tiles(c.x, xs), ny = axis_tiles(c.y, ys);
+                    for (int a = 0; a < ny; ++a)
+                        for (int b = 0; b < nx; ++b) p.adj_pts[ap[ys[a] * NT + xs[b]]++] = id;
                 }
         };
         parallel_for(nthr, place);
@@ -204,10 +210,6 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
     // sample k of a ray mirrors sample n - k for an even detector width only (and the border cells that
     // fold into each other must be distinct)
     if (n % 2 || n < 32) return false;
-    // n = 2 mod 8: the last column and row of tiles are four cells wide, and the per-ray adjoint leaves
-    // them out for stencils that reach from the tile before to the one behind the wrap (4e-4 of the
-    // result); such widths stay on the per-ray kernels, so that their results do not depend on the angles
-    if (n % 8 == 2) return false;
     const double pi = 3.14159265358979323846;
     const double tol = tol_cells / (double)n;
     std::vector<double> alpha(ntheta);

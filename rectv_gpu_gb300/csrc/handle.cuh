@@ -82,10 +82,12 @@ struct Layout {
     bool fused_rows = false;  // fused residual rows (k_resid_rows)
     bool gen_rows = false;    // mixed-radix ones (k_gen_resid)
     bool dirs = false;        // the direction path may run (a geometry decides)
-    int tg = 1, zs = 1, jg = 1;  // vector layout of the direction path (UsGeo)
+    int tg = 1, zs = 1, jg = 1;  // vector layout of the spectra (UsGeo)
+    int vec_slices = 0;       // slices per 2D cuFFT call (without the hand-written FFTs)
     long long slab = 0, gp = 0;
-    size_t spec_elems = 0;
+    size_t spec_elems = 0, planar_elems = 0;
     double bytes = 0;         // estimate of all device memory, geometry included
+    int planes() const { return (jg > 1 ? zb * jg : (zb + zs - 1) / zs); }
 };
 
 inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batch_bytes) {
@@ -136,8 +138,16 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     }
     L.zb = nzp * d;
     L.nbatch = L.nchunks / d;
-    const long long vec_pl = L.jg > 1 ? (long long)L.zb * L.jg : (L.zb + L.zs - 1) / L.zs;
-    L.spec_elems = std::max<size_t>((size_t)(vec_pl * vec_plane), (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
+    L.spec_elems = std::max<size_t>((size_t)(L.planes() * vec_plane), (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
+    if (!L.pad_fft && !L.gen_fft) {
+        // 2D cuFFT calls over as many slices as keep the planar images near the L2 (whole planes
+        // of the vector layout, but never more slices than there are), of equal size
+        const double img = (double)m * P * planar_pitch(n) * 8.0;
+        const int most = (int)std::max(1.0, std::min((double)L.zb, 64e6 / img));
+        const int calls = (L.zb + most - 1) / most, even = (L.zb + calls - 1) / calls;
+        L.vec_slices = std::min(L.zb, (even + L.zs - 1) / L.zs * L.zs);
+        L.planar_elems = (size_t)L.vec_slices * m * P * planar_pitch(n);
+    }
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
     b += (double)L.zb * nt * 4 + L.spec_elems * 8.0 + (double)L.zb * ntheta * std::max(n, n / 2 + 1) * 8.0;
@@ -200,7 +210,7 @@ struct Handle {
     cufftHandle plan[kNPlans] = {};
     bool plan_made[kNPlans] = {};
     size_t fft_work_bytes = 0;
-    int vec_slices = 1;          // slices per 2D cuFFT call (without the hand-written FFTs)
+    int vec_slices = 1;          // slices per 2D cuFFT call (Layout)
     float2 *planar = nullptr;    // their planar images [vec_slices m][P][planar_pitch]
     CUtensorMap dir_tmap, tc_tmap;  // footprint boxes of the direction gather and the tensor-core gather
     // key of the geometry on the device (set_geometry)
@@ -351,11 +361,9 @@ struct Handle {
             make_vec_fft_map(&fft_map, spec, vec_planes(ug, zb), ug);
         } else if (gen_fft) {
             fft_tw = table(gen_fft_twiddles(gen_plan));
-        } else {  // 2D cuFFT calls: as many slices as keep the planar images near the L2
-            const double img = (double)m * P * planar_pitch(n) * 8.0;
-            vec_slices = (int)std::max(1.0, std::min((double)zb, 64e6 / img));
-            vec_slices = std::max(lay.zs, vec_slices / lay.zs * lay.zs);
-            planar = alloc<float2>((size_t)vec_slices * m * P * planar_pitch(n));
+        } else {
+            vec_slices = lay.vec_slices;
+            planar = alloc<float2>(lay.planar_elems);
         }
         fused_rows = lay.fused_rows;
         gen_rows = lay.gen_rows && gen_fft_plan(n, &gen_rplan);

@@ -201,7 +201,10 @@ int rectv_autotune(rectv_handle *h, int force, int *zper, int *sc_grid);
 int rectv_get_device_bytes(rectv_handle *h, double *bytes);
 
 /* Estimated device memory of a handle with these dimensions (before creating
- * it), in bytes: the figure the engine admits jobs by. */
+ * it), in bytes.  A geometry whose rays share directions holds the mixing
+ * buffer besides: for each plane of 16 (slice, time sample) values of a batch
+ * 192 n bytes per direction (the engine, which knows its jobs' angles, admits
+ * them by the sum). */
 int rectv_estimate_bytes(int n, int ntheta, int m, int nz, int nzp, double *bytes);
 
 /* ---------------------------------------------------------------------------

@@ -151,7 +151,8 @@ struct Job {
     const float *g = nullptr, *theta = nullptr, *phi = nullptr;
     float *fres = nullptr;
     double arrival = 0, admitted = -1, done = -1;
-    double est_bytes = 0, bytes = 0;
+    double est_bytes = 0, bytes = 0;  // estimated (with the angles' path from admission on), allocated
+    bool sized = false;
     int state = kWaiting;
     std::string error;
     std::unique_ptr<Handle> h;
@@ -235,6 +236,17 @@ struct Engine {
         return jobs.back()->id;
     }
 
+    // The estimate of a job from its dimensions, and the direction path's
+    // buffers where its angles take it.
+    static double job_bytes(const Job &j) {
+        const Layout L = make_layout(j.n, j.ntheta, j.m, j.nz, j.nzp, -1);
+        double dir_min = 0.0, dir_tol = 0.0;
+        direction_rule(L, &dir_min, &dir_tol);
+        DirPlan dp;
+        const bool dirs = dir_min > 0 && group_directions(j.theta, j.n, j.ntheta, dir_tol, dir_min, dp);
+        return L.bytes + direction_bytes(L, j.n, j.ntheta, dirs ? dp.ndir : 0);
+    }
+
     static bool same_dims(const Handle &h, const Job &j) {
         return h.n == j.n && h.ntheta == j.ntheta && h.m == j.m && h.nz == j.nz && h.nzp == j.nzp;
     }
@@ -251,6 +263,10 @@ struct Engine {
     // Admits job j if it fits; false when it has to wait.  Throws on errors
     // that make the job fail.
     bool admit(Job &j, const std::vector<Job *> &active) {
+        if (!j.sized) {
+            j.est_bytes = job_bytes(j);
+            j.sized = true;
+        }
         std::unique_ptr<Handle> h;
         bool fresh = false;
         for (size_t i = 0; i < idle.size(); ++i)

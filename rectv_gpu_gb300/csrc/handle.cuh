@@ -86,7 +86,9 @@ struct Layout {
     int vec_slices = 0;       // slices per 2D cuFFT call (without the hand-written FFTs)
     long long slab = 0, gp = 0;
     size_t spec_elems = 0, planar_elems = 0;
-    double bytes = 0;         // estimate of all device memory, geometry included
+    // estimate of all device memory, geometry included, for a geometry on the
+    // per-ray kernels; direction_bytes() more where rays share directions
+    double bytes = 0;
     int planes() const { return (jg > 1 ? zb * jg : (zb + zs - 1) / zs); }
 };
 
@@ -156,10 +158,40 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     // geometry: angle plan, adjoint entries (about 2.25 tiles per sample) and records
     b += nt * (4 + 2.5 * 4 + (L.tc_scatter ? 2.5 * 144 + 12 : 0)) + 8.0 * ntheta * m + (1 << 20);
     if (L.pad_fft) b += 16.0 * P * 8;
-    // cuFFT's planar images and work area
-    if (!L.pad_fft && !L.gen_fft) b += 3.0 * 64e6;
+    // cuFFT's planar images, and the work area that its plans share: as large as the images (twice
+    // for small ones) and as the batch's rows at most
+    const bool own_fft = L.pad_fft || L.gen_fft, own_rows = L.fused_rows || L.gen_rows;
+    b += L.planar_elems * 8.0;
+    if (!own_fft || !own_rows)
+        b += std::max((n < 32 ? 2.0 : 1.0) * L.planar_elems * 8.0, (double)L.zb * nt * 8.0) * 1.01 + (1 << 20);
     L.bytes = b;
     return L;
+}
+
+// When a geometry may take the direction path: rays per direction at least
+// *min_group (<= 0: never), rays grouped within *tol grid cells.  Used when the
+// rays average at least 2.5 per direction (RECTV_DIRS=1: whenever it can run,
+// RECTV_DIRS=0: never) and no FP32 scatter is asked for; RECTV_DIR_TOL sets the
+// tolerance (2e-3).
+inline void direction_rule(const Layout &L, double *min_group, double *tol) {
+    *min_group = kDirMinGroup;
+    *tol = kDirTolCells;
+    if (const char *e = std::getenv("RECTV_DIRS")) {
+        if (!std::strcmp(e, "0")) *min_group = -1.0;
+        if (!std::strcmp(e, "1")) *min_group = 1.0;
+    }
+    if (const char *e = std::getenv("RECTV_DIR_TOL")) *tol = std::max(0.0, std::atof(e));
+    if (!L.dirs) *min_group = -1.0;
+}
+
+// Device memory of a geometry of ndir directions: the mixing buffer, the
+// position pairs (about 2.6 tiles each), their work items and K'.
+inline double direction_bytes(const Layout &L, int n, int ntheta, int ndir) {
+    if (ndir <= 0) return 0.0;
+    const double npz = L.planes() / L.jg, pairs = (double)ndir * (n / 2);
+    const double tiles = ((n + 1 + kVH + kVR) / 16 + 1.0) * ((L.P + 2 * kVH) / 16 + 1.0);
+    return npz * pairs * 384.0 + pairs * 4 * 3.6 + tiles * npz * 16 * 2 +
+           (double)ntheta * (L.jg > 1 ? 16.0 * L.jg : L.tg) * 8 + ntheta * 8.0 + (1 << 20);
 }
 
 struct Handle {
@@ -528,17 +560,9 @@ struct Handle {
         const bool tc_scatter = lay.tc_scatter;
         // direction path (scatter_dir.cu): rays that revisit a direction over
         // several half-turns share its sample positions, so the USFFT
-        // interpolates once per position.  Used when the rays average at least
-        // 2.5 per direction (RECTV_DIRS=1: whenever it can run, RECTV_DIRS=0:
-        // never) and no FP32 scatter is asked for; rays are grouped when their
-        // samples agree within RECTV_DIR_TOL grid cells (2e-3).
-        double dir_min = kDirMinGroup, dir_tol = kDirTolCells;
-        if (const char *e = std::getenv("RECTV_DIRS")) {
-            if (!std::strcmp(e, "0")) dir_min = -1.0;
-            if (!std::strcmp(e, "1")) dir_min = 1.0;
-        }
-        if (const char *e = std::getenv("RECTV_DIR_TOL")) dir_tol = std::max(0.0, std::atof(e));
-        if (!lay.dirs) dir_min = -1.0;
+        // interpolates once per position
+        double dir_min = 0.0, dir_tol = 0.0;
+        direction_rule(lay, &dir_min, &dir_tol);
         const size_t nphi = phi_h ? (size_t)2 * m * ntheta : 0;
         if (geo_valid && center == geo_center && tc_min_spr == geo_tc_spr && tc_scatter == geo_tc_scatter &&
             dir_min == geo_dir_min && dir_tol == geo_dir_tol &&

@@ -204,8 +204,7 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
 // positions of one representative ray, the group member of median angle; a
 // ray's own samples lie (q-n/2)/n * tau_r cells across the direction from the
 // shared positions (the kernels correct for it to first order).
-bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, double tol_cells, double min_group,
-                    DirPlan &dp) {
+bool group_directions(const float *theta, int n, int ntheta, double tol_cells, double min_group, DirPlan &dp) {
     dp = DirPlan();
     // sample k of a ray mirrors sample n - k for an even detector width only (and the border cells that
     // fold into each other must be distinct)
@@ -258,7 +257,12 @@ bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, d
         i = j;
     }
     dp.ndir = (int)dp.sincos.size();
-    if ((double)ntheta < min_group * dp.ndir || dp.ndir >= 65536) return false;
+    return (double)ntheta >= min_group * dp.ndir && dp.ndir < 65536;
+}
+
+bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, double tol_cells, double min_group,
+                    DirPlan &dp) {
+    if (!group_directions(theta, n, ntheta, tol_cells, min_group, dp)) return false;
 
     // position pairs (d, q), 1 <= q <= n/2 (sample n - q is the mirror image):
     // the same float sequence as the kernels (sample_pos), binned by the tile

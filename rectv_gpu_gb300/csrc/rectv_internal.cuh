@@ -188,6 +188,8 @@ constexpr double kDirMinGroup = 2.5;
 // direction or there are 65536 directions or more.
 bool build_dir_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, double tol_cells, double min_group,
                     DirPlan &dp);
+// its first step, the rays of each direction (no positions)
+bool group_directions(const float *theta, int n, int ntheta, double tol_cells, double min_group, DirPlan &dp);
 
 // 32-bit words of an adjoint table's ray segmentation with nseg rays: [0]
 // nseg, [4 + 8 s + w] the table rows [lo, hi) of ray s that cover rows 2w,

@@ -26,8 +26,9 @@ __global__ void __launch_bounds__(kColThr, C == 8 ? 4 : 3)
 }
 
 // One row y of C value pairs of a plane: the pair's two real rows are one
-// complex transform, split into the two half spectra.
-template <int C>
+// complex transform, split into the two half spectra (YP, one time sample per
+// slice: the rows y and y + 1 of C values, so that slices stay apart).
+template <int C, bool YP>
 __global__ void __launch_bounds__(kThr, 3)
     k_gen_rows_fwd(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp, const __grid_constant__ GenPlan p,
                    const float2 *__restrict__ tw, UsGeo g, int zb, float inv4n2) {
@@ -36,13 +37,16 @@ __global__ void __launch_bounds__(kThr, 3)
     const int X = 0, Y = P * C;
     const int c = threadIdx.x % C, j0 = threadIdx.x / C;
     constexpr int js = kThr / C;
-    const int y = blockIdx.x / (8 / C), pl = blockIdx.y, v0 = 2 * ((blockIdx.x % (8 / C)) * C + c);
+    constexpr int G = YP ? 16 / C : 8 / C;  // blocks per row (pair)
+    const int y = (YP ? 2 : 1) * (blockIdx.x / G), y1 = YP ? min(y + 1, n - 1) : y, pl = blockIdx.y;
+    const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
-    const int zc = vec_slice(g, pl, v0 + 1), tb = vec_time(g, pl, v0 + 1);
-    const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m;
+    const int zc = vec_slice(g, pl, v1), tb = vec_time(g, pl, v1);
+    const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m && !(YP && y + 1 >= n);
     const float *ua = u + (((long long)(oka ? za : 0) * g.m + (oka ? ta : 0)) * n + y) * n;
-    const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y) * n;
+    const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y1) * n;
     const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * inv4n2;
+    const float sy1 = YP ? (((y1 + n / 2) & 1) ? -dp[y1] : dp[y1]) * inv4n2 : sy;
     for (int xb = j0; xb < n; xb += 4 * js) {  // deapodised, times (-1)^(X+Y); eight loads in flight
         float va[4], vb[4];
 #pragma unroll
@@ -55,8 +59,8 @@ __global__ void __launch_bounds__(kThr, 3)
         for (int i = 0; i < 4; ++i) {
             const int x = xb + i * js;
             if (x >= n) break;
-            const float w = (((x + n / 2) & 1) ? -__ldg(dp + x) : __ldg(dp + x)) * sy;
-            gen_sh[Y + x * C + c] = make_float2(va[i] * w, vb[i] * w);
+            const float d = ((x + n / 2) & 1) ? -__ldg(dp + x) : __ldg(dp + x);
+            gen_sh[Y + x * C + c] = make_float2(va[i] * (d * sy), vb[i] * (d * sy1));
         }
     }
     __syncthreads();
@@ -64,11 +68,17 @@ __global__ void __launch_bounds__(kThr, 3)
     __syncthreads();
     const float2 *a = gen_sh + gen::passes<-1, C>(X, Y, 1, p, tw, c, j0, js) + c;
     if (!oka && !okb) return;
-    float4 *row = reinterpret_cast<float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0);
+    float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0;
     for (int k = j0; k <= n; k += js) {
         const float2 zk = a[k * C], zm = a[(k ? P - k : 0) * C];
-        row[(long long)k * 8] = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y),
-                                            0.5f * (zm.x - zk.x));
+        const float4 o = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y),
+                                     0.5f * (zm.x - zk.x));
+        if constexpr (YP) {
+            row[(long long)k * 16] = make_float2(o.x, o.y);
+            if (okb) row[((long long)g.vp + k) * 16] = make_float2(o.z, o.w);
+        } else {
+            *reinterpret_cast<float4 *>(row + (long long)k * 16) = o;
+        }
     }
 }
 
@@ -77,7 +87,12 @@ void run_fwd(const float *u, float2 *spec, int zb, const float *deapod, const fl
              const UsGeo &g, cudaStream_t s) {
     const int n = g.n, npl = vec_planes(g, zb);
     const float inv4n2 = (float)(1.0 / (4.0 * n * (double)n));
-    k_gen_rows_fwd<C><<<dim3(n * (8 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(u, spec, deapod, p, tw, g, zb, inv4n2);
+    if (g.tg == 1)
+        k_gen_rows_fwd<C, true><<<dim3((n + 1) / 2 * (16 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(u, spec, deapod, p,
+                                                                                                 tw, g, zb, inv4n2);
+    else
+        k_gen_rows_fwd<C, false><<<dim3(n * (8 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(u, spec, deapod, p, tw, g, zb,
+                                                                                       inv4n2);
     LAUNCH_CHECK("k_gen_rows_fwd");
     const size_t smem = gen_cols_smem(g.P, C);
     const int nlv = gen_live_groups(g, C);
@@ -94,8 +109,10 @@ void gen_fft_fwd_prepare() {
     constexpr int most = 227 * 1024;
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_fwd<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_fwd<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 }
 
 // Radices of P, at most six of 2 .. 13, 15, 16, 17, 19, as few as possible and then as

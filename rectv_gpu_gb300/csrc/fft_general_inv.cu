@@ -27,8 +27,8 @@ __global__ void __launch_bounds__(kColThr, C == 8 ? 4 : 3)
 
 // One row y of C value pairs of a plane: the Hermitian extension of the two
 // half rows as one complex inverse transform A + i B, the centre outputs
-// modulated, deapodised, scaled and added into u.
-template <int C>
+// modulated, deapodised, scaled and added into u (YP: as the forward's).
+template <int C, bool YP>
 __global__ void __launch_bounds__(kThr, 3)
     k_gen_rows_inv(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp, const __grid_constant__ GenPlan p,
                    const float2 *__restrict__ tw, UsGeo g, int zb, float cscale) {
@@ -36,15 +36,24 @@ __global__ void __launch_bounds__(kThr, 3)
     const int n = g.n, P = g.P;
     const int c = threadIdx.x % C, j0 = threadIdx.x / C;
     constexpr int js = kThr / C;
-    const int y = blockIdx.x / (8 / C), pl = blockIdx.y, v0 = 2 * ((blockIdx.x % (8 / C)) * C + c);
-    const float4 *row =
-        reinterpret_cast<const float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0);
+    constexpr int G = YP ? 16 / C : 8 / C;  // blocks per row (pair)
+    const int y = (YP ? 2 : 1) * (blockIdx.x / G), y1 = YP ? min(y + 1, n - 1) : y, pl = blockIdx.y;
+    const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
+    const float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0;
+    auto load = [&](int k) {  // column k of the pair's two half rows
+        if constexpr (YP) {
+            const float2 a = __ldg(row + (long long)k * 16), b = __ldg(row + ((long long)(y1 - y) * g.vp + k) * 16);
+            return make_float4(a.x, a.y, b.x, b.y);
+        } else {
+            return __ldg(reinterpret_cast<const float4 *>(row + (long long)k * 16));
+        }
+    };
     for (int kb = j0; kb <= n; kb += 4 * js) {  // four loads in flight
         float4 f[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int k = kb + i * js;
-            if (k <= n) f[i] = __ldg(row + (long long)k * 8);
+            if (k <= n) f[i] = load(k);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -61,11 +70,12 @@ __global__ void __launch_bounds__(kThr, 3)
     __syncthreads();
     const float2 *a = gen_sh + gen::passes<1, C>(0, P * C, 0, p, tw, c, j0, js) + c;
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
-    const int zc = vec_slice(g, pl, v0 + 1), tb = vec_time(g, pl, v0 + 1);
-    const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m;
+    const int zc = vec_slice(g, pl, v1), tb = vec_time(g, pl, v1);
+    const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m && !(YP && y + 1 >= n);
     float *ua = u + (((long long)(oka ? za : 0) * g.m + (oka ? ta : 0)) * n + y) * n;
-    float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y) * n;
+    float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y1) * n;
     const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * cscale;
+    const float sy1 = YP ? (((y1 + n / 2) & 1) ? -dp[y1] : dp[y1]) * cscale : sy;
     for (int xb = j0; xb < n; xb += 4 * js) {
         float va[4], vb[4];
 #pragma unroll
@@ -78,10 +88,10 @@ __global__ void __launch_bounds__(kThr, 3)
         for (int i = 0; i < 4; ++i) {
             const int x = xb + i * js;
             if (x >= n) break;
-            const float w = (((x + n / 2) & 1) ? -__ldg(dp + x) : __ldg(dp + x)) * sy;
+            const float d = ((x + n / 2) & 1) ? -__ldg(dp + x) : __ldg(dp + x);
             const float2 o = a[(x + n / 2) * C];
-            if (oka) ua[x] = va[i] + o.x * w;
-            if (okb) ub[x] = vb[i] + o.y * w;
+            if (oka) ua[x] = va[i] + o.x * (d * sy);
+            if (okb) ub[x] = vb[i] + o.y * (d * sy1);
         }
     }
 }
@@ -97,7 +107,12 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
     const int grid = (int)std::min<long long>(ntiles, gen_resident(smem, kColThr));
     k_gen_cols_inv<C><<<grid, kColThr, smem, s>>>(spec, p, tw, g, nlv, (int)ntiles);
     LAUNCH_CHECK("k_gen_cols_inv");
-    k_gen_rows_inv<C><<<dim3(n * (8 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(spec, u, deapod, p, tw, g, zb, cscale);
+    if (g.tg == 1)
+        k_gen_rows_inv<C, true><<<dim3((n + 1) / 2 * (16 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(spec, u, deapod, p,
+                                                                                                 tw, g, zb, cscale);
+    else
+        k_gen_rows_inv<C, false><<<dim3(n * (8 / C), npl), kThr, gen_rows_smem(g.P, C), s>>>(spec, u, deapod, p, tw, g, zb,
+                                                                                       cscale);
     LAUNCH_CHECK("k_gen_rows_inv");
 }
 
@@ -199,8 +214,10 @@ void gen_fft_inv_prepare() {
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
 }
 
 void launch_gen_fft_inv_accum(float2 *spec, float *u, int zb, float tau, const float *deapod, const float2 *tw,

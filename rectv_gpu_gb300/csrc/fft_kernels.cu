@@ -234,6 +234,9 @@ constexpr int vec_col_c(int N) { return N >= 2048 ? 4 : (N == 1024 ? 8 : 16); }
 // stores and the C pairs of a block as C x 16 contiguous bytes per cell
 // (64-128 bytes).  Thread = (pair c, point t) with c fastest: C transforms
 // interleaved in shared memory as in the column kernels, R rows per block.
+// With one time sample per slice the two values would be two slices, and a NaN
+// or the rounding of a bright slice would reach its neighbour: there (YP) a
+// transform takes the rows y and y + 1 of one image, a block C images.
 // ---------------------------------------------------------------------------
 template <int N>
 struct VecRows {
@@ -257,7 +260,7 @@ struct VecRows {
     }
 };
 
-template <int N>
+template <int N, bool YP>
 __global__ void __launch_bounds__(kRowThreads, 2)
     k_fft_rows_fwd(const float *__restrict__ u, float2 *__restrict__ spec, const float *__restrict__ dp,
                        const float2 *__restrict__ tw, UsGeo g, int zb, float inv4n2) {
@@ -267,25 +270,29 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     extern __shared__ float2 fft_sh[];
     const int n = N / 2;
     const int c = threadIdx.x % C, t = (threadIdx.x / C) % N1, rr = threadIdx.x / (C * N1);
-    const int y = (blockIdx.x / (8 / C)) * R + rr, pl = blockIdx.y;
-    const int v0 = 2 * ((blockIdx.x % (8 / C)) * C + c);  // the pair's values v0, v0 + 1 of the plane
+    constexpr int G = YP ? 16 / C : 8 / C;  // blocks per row (pair)
+    const int ry = (blockIdx.x / G) * R + rr, pl = blockIdx.y;
+    const int y = YP ? 2 * ry : ry, y1 = YP ? y + 1 : y;
+    // the pair's values v0, v0 + 1 of the plane (YP: value v0, rows y and y + 1)
+    const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
     float2 *sh = fft_sh + rr * (L::S * C);
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
-    const int zc = vec_slice(g, pl, v0 + 1), tb = vec_time(g, pl, v0 + 1);
+    const int zc = vec_slice(g, pl, v1), tb = vec_time(g, pl, v1);
     const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m;
     float2 v[16];
     {
         const float *ua = u + (((long long)(oka ? za : 0) * g.m + (oka ? ta : 0)) * n + y) * n;
-        const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y) * n;
+        const float *ub = u + (((long long)(okb ? zc : 0) * g.m + (okb ? tb : 0)) * n + y1) * n;
         const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * inv4n2;
+        const float sy1 = YP ? (((y1 + n / 2) & 1) ? -dp[y1] : dp[y1]) * inv4n2 : sy;
 #pragma unroll
         for (int r = 0; r < 16; ++r) {
             v[r] = make_float2(0.f, 0.f);
             if (r >= 4 && r < 12) {  // X = t + N1 r in [n/2, 3n/2)
                 const int x = t + N1 * (r - 4), X = x + n / 2;
-                const float w = ((X & 1) ? -__ldg(dp + x) : __ldg(dp + x)) * sy;
-                if (oka) v[r].x = __ldg(ua + x) * w;
-                if (okb) v[r].y = __ldg(ub + x) * w;
+                const float d = (X & 1) ? -__ldg(dp + x) : __ldg(dp + x);
+                if (oka) v[r].x = __ldg(ua + x) * (d * sy);
+                if (okb) v[r].y = __ldg(ub + x) * (d * sy1);
             }
         }
     }
@@ -298,11 +305,17 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         for (int j1 = 0; j1 < L::R3; ++j1) sh[(t + N1 * q + 256 * j1) * C + c] = v[q * L::R3 + j1];
     __syncthreads();
     if (!oka && !okb) return;
-    float4 *row = reinterpret_cast<float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0);
+    float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0;
     for (int k = t; k <= n; k += N1) {
         const float2 zk = sh[k * C + c], zm = sh[((N - k) & (N - 1)) * C + c];
-        row[(long long)k * 8] = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y),
-                                            0.5f * (zm.x - zk.x));
+        const float4 o = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y),
+                                     0.5f * (zm.x - zk.x));
+        if constexpr (YP) {
+            row[(long long)k * 16] = make_float2(o.x, o.y);
+            row[((long long)g.vp + k) * 16] = make_float2(o.z, o.w);
+        } else {
+            *reinterpret_cast<float4 *>(row + (long long)k * 16) = o;
+        }
     }
 }
 
@@ -439,7 +452,7 @@ __global__ void __launch_bounds__(C *(N / 16), 1)
 // centre outputs pass through shared memory once more so that the rows of u
 // are read and written as whole lines.
 // ---------------------------------------------------------------------------
-template <int N>
+template <int N, bool YP>
 __global__ void __launch_bounds__(kRowThreads, 2)
     k_fft_rows_inv(const float2 *__restrict__ spec, float *__restrict__ u, const float *__restrict__ dp,
                        const float2 *__restrict__ tw, UsGeo g, int zb, float cscale) {
@@ -448,19 +461,27 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     constexpr int N1 = V::N1, C = V::C, R = V::R, n = N / 2;
     extern __shared__ float2 fft_sh[];
     const int c = threadIdx.x % C, t = (threadIdx.x / C) % N1, rr = threadIdx.x / (C * N1);
-    const int y = (blockIdx.x / (8 / C)) * R + rr, pl = blockIdx.y;
-    const int vb = 2 * (blockIdx.x % (8 / C)) * C;  // the block's first value
+    constexpr int G = YP ? 16 / C : 8 / C;
+    const int ry = (blockIdx.x / G) * R + rr, pl = blockIdx.y, y = YP ? 2 * ry : ry;
+    const int vb = (YP ? 1 : 2) * (blockIdx.x % G) * C;  // the block's first value
     float2 *sh = fft_sh + rr * (L::S * C);
-    const float4 *row =
-        reinterpret_cast<const float4 *>(spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + vb) + c;
+    const float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + vb + (YP ? 1 : 2) * c;
+    auto load = [&](int k) {  // column k of the pair's two half rows
+        if constexpr (YP) {
+            const float2 a = row[(long long)k * 16], b = row[((long long)g.vp + k) * 16];
+            return make_float4(a.x, a.y, b.x, b.y);
+        } else {
+            return *reinterpret_cast<const float4 *>(row + (long long)k * 16);
+        }
+    };
     // A + i B at k = t + N1 r: the stored half k <= n is read once; its mirror
     // image at N - k belongs to thread N1 - t and goes there through shared memory
     float2 v[16];
     {
         float4 f[9];
 #pragma unroll
-        for (int r = 0; r < 8; ++r) f[r] = row[(long long)(t + N1 * r) * 8];
-        f[8] = t == 0 ? row[(long long)n * 8] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int r = 0; r < 8; ++r) f[r] = load(t + N1 * r);
+        f[8] = t == 0 ? load(n) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (t == 0) f[0].y = f[0].w = f[8].y = f[8].w = 0.f;  // columns 0 and n of a real image's spectrum
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
@@ -488,14 +509,16 @@ __global__ void __launch_bounds__(kRowThreads, 2)
             }
         }
     const float sy = (((y + n / 2) & 1) ? -dp[y] : dp[y]) * cscale;
+    const float sy1 = YP ? (((y + 1 + n / 2) & 1) ? -dp[y + 1] : dp[y + 1]) * cscale : sy;
     float4 *up[V::PER], f[V::PER];
     const int tr = threadIdx.x % (C * N1);
 #pragma unroll
     for (int i = 0; i < V::PER; ++i) {  // the rows of u are on their way during the barrier
         int j, x;
         V::piece(i, tr, j, x);
-        const int vj = vb + 2 * (j % C) + j / C, z = vec_slice(g, pl, vj), tt = vec_time(g, pl, vj);
-        up[i] = z < zb && tt < g.m ? reinterpret_cast<float4 *>(u + (((long long)z * g.m + tt) * n + y) * n + x) : nullptr;
+        const int vj = YP ? vb + j % C : vb + 2 * (j % C) + j / C, yj = YP ? y + j / C : y;
+        const int z = vec_slice(g, pl, vj), tt = vec_time(g, pl, vj);
+        up[i] = z < zb && tt < g.m ? reinterpret_cast<float4 *>(u + (((long long)z * g.m + tt) * n + yj) * n + x) : nullptr;
         if (up[i]) f[i] = *up[i];
     }
     __syncthreads();
@@ -506,7 +529,8 @@ __global__ void __launch_bounds__(kRowThreads, 2)
         V::piece(i, tr, j, x);
         const float4 o = *reinterpret_cast<const float4 *>(rows + j * V::RP + x);
         const float4 d = __ldg(reinterpret_cast<const float4 *>(dp + x));
-        const float s0 = ((x + n / 2) & 1) ? -sy : sy;  // (-1)^X of column x; the next ones alternate
+        const float syj = YP && j >= C ? sy1 : sy;
+        const float s0 = ((x + n / 2) & 1) ? -syj : syj;  // (-1)^X of column x; the next ones alternate
         f[i].x += o.x * d.x * s0;
         f[i].y -= o.y * d.y * s0;
         f[i].z += o.z * d.z * s0;
@@ -624,8 +648,10 @@ void set_attrs_n() {
     constexpr int C = vec_col_c(N);
     CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, false>, attr, (int)rows_smem<N>()));
     CUDA_CHECK(cudaFuncSetAttribute(k_resid_rows<N, true>, attr, (int)rows_smem<N>()));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N>, attr, (int)VecRows<N>::SMEM));
-    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N, false>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_fwd<N, true>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N, false>, attr, (int)VecRows<N>::SMEM));
+    CUDA_CHECK(cudaFuncSetAttribute(k_fft_rows_inv<N, true>, attr, (int)VecRows<N>::SMEM));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, C, -1>, attr, (int)ColPass<N, C, -1>::SMEM));
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, C, 1>, attr, (int)ColPass<N, C, 1>::SMEM));
 }
@@ -662,7 +688,8 @@ void fwd_n(const float *u, float2 *spec, int zb, const float *deapod, const floa
     const int n = N / 2;
     const float inv4n2 = (float)(1.0 / (4.0 * n * (double)n));
     const dim3 gr(n / V::R * (8 / V::C), vec_planes(g, zb));
-    k_fft_rows_fwd<N><<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g, zb, inv4n2);
+    (g.tg == 1 ? k_fft_rows_fwd<N, true> : k_fft_rows_fwd<N, false>)<<<gr, kRowThreads, V::SMEM, s>>>(u, spec, deapod, tw, g,
+                                                                                               zb, inv4n2);
     LAUNCH_CHECK("k_fft_rows_fwd");
     launch_cols<N, -1>(map, tw, zb, err, g, s);
 }
@@ -673,7 +700,8 @@ void inv_n(float2 *spec, float *u, int zb, float cscale, const float *deapod, co
     using V = VecRows<N>;
     launch_cols<N, 1>(map, tw, zb, err, g, s);
     const dim3 gr(N / 2 / V::R * (8 / V::C), vec_planes(g, zb));
-    k_fft_rows_inv<N><<<gr, kRowThreads, V::SMEM, s>>>(spec, u, deapod, tw, g, zb, cscale);
+    (g.tg == 1 ? k_fft_rows_inv<N, true> : k_fft_rows_inv<N, false>)<<<gr, kRowThreads, V::SMEM, s>>>(spec, u, deapod, tw, g,
+                                                                                               zb, cscale);
     LAUNCH_CHECK("k_fft_rows_inv");
 }
 

@@ -118,7 +118,8 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
 
 // ---------------------------------------------------------------------------
 // Residual rows of the inner step (k_resid_rows of fft_kernels.cu on the
-// mixed-radix core): two rows are one complex transform, C pairs per block.
+// mixed-radix core): two rows are one complex transform, C pairs per block;
+// blockIdx.y: runs of nrows rows (launch_resid_rows).
 // HALF: the rows hold their Hermitian half (direction path), else the whole
 // row, of which the Hermitian part counts.
 // ---------------------------------------------------------------------------
@@ -133,6 +134,9 @@ __global__ void __launch_bounds__(kResThr, 6)
     const long long ra = 2 * ((long long)blockIdx.x * C + c), rb = ra + 1;
     const bool oka = ra < nrows, okb = rb < nrows;
     const int rn = HALF ? hn : n;  // values per row
+    rows += blockIdx.y * nrows * rn;
+    gdata += blockIdx.y * nrows * n;
+    out += blockIdx.y * nrows * hn;
     const float2 *ga = rows + (oka ? ra : 0) * rn, *gb = rows + (okb ? rb : 0) * rn;
     const float2 zero = make_float2(0.f, 0.f);
     auto load = [&](const float2 *r, int k) {
@@ -197,15 +201,19 @@ __global__ void __launch_bounds__(kResThr, 6)
 void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
                       bool half, const UsGeo &g, cudaStream_t s) {
     constexpr int C = 4;
-    const long long nrows = (long long)zb * g.ntheta, nblk = (nrows + 2 * C - 1) / (2 * C);
+    const int runs = resid_runs(zb, g.ntheta);
+    const long long nrows = (long long)zb * g.ntheta / runs, nblk = (nrows + 2 * C - 1) / (2 * C);
     if (nblk > 2147483647LL) throw Error(1, "residual rows: too many rows");
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
     const size_t smem = gen_rows_smem(g.n, C);
-    if (half)
-        k_gen_resid<C, true><<<(unsigned)nblk, kResThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
-    else
-        k_gen_resid<C, false><<<(unsigned)nblk, kResThr, smem, s>>>(rows, gdata, out, p, tw, nrows, scale);
-    LAUNCH_CHECK("k_gen_resid");
+    const long long rn = half ? g.n / 2 + 1 : g.n;
+    for (int y = 0; y < runs; y += 65535) {
+        const long long r0 = y * nrows;
+        const dim3 gr((unsigned)nblk, std::min(65535, runs - y));
+        (half ? k_gen_resid<C, true> : k_gen_resid<C, false>)<<<gr, kResThr, smem, s>>>(
+            rows + r0 * rn, gdata + r0 * g.n, out + r0 * (g.n / 2 + 1), p, tw, nrows, scale);
+        LAUNCH_CHECK("k_gen_resid");
+    }
 }
 
 void gen_fft_inv_prepare() {

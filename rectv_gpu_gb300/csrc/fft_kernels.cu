@@ -554,7 +554,8 @@ size_t rows_smem() {
 // Re IFFT(a) + i Re IFFT(b) is the inverse FFT of Ha + i Hb (H = Hermitian
 // part), and FFT(wa + i wb) splits into the two half spectra, so a row pair
 // costs one inverse and one forward n-point FFT; the residual never goes to
-// memory.  Rows are the flattened (slice, angle) index; N = n.
+// memory.  Rows are the flattened (slice, angle) index, in runs of nrows
+// (blockIdx.y); N = n.
 // ---------------------------------------------------------------------------
 // HALF: the rows hold H(k) itself, k = 0 .. n/2 (direction path).
 template <int N, bool HALF>
@@ -568,6 +569,9 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     const long long ra = 2 * ((long long)blockIdx.x * RP + c), rb = ra + 1;
     const bool oka = ra < nrows, okb = rb < nrows;
     constexpr int RN = HALF ? N / 2 + 1 : N;  // values per row
+    rows += blockIdx.y * nrows * RN;
+    gdata += blockIdx.y * nrows * N;
+    out += blockIdx.y * nrows * (N / 2 + 1);
     const float2 *ga = rows + (oka ? ra : 0) * RN, *gb = rows + (okb ? rb : 0) * RN;
     float2 v[16];
 #pragma unroll
@@ -632,14 +636,18 @@ __global__ void __launch_bounds__(kRowThreads, 2)
 }
 
 template <int N, bool HALF>
-void resid_n(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, long long nrows, float scale,
-             cudaStream_t s) {
+void resid_n(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, long long nrows, int runs,
+             float scale, cudaStream_t s) {
     constexpr int N1 = N / 16, RP = kRowThreads / N1;
     const long long npairs = (nrows + 1) / 2;
     const long long nblk = (npairs + RP - 1) / RP;
     if (nblk > 2147483647LL) throw Error(1, "residual rows: too many rows");
-    k_resid_rows<N, HALF><<<(unsigned)nblk, kRowThreads, rows_smem<N>(), s>>>(rows, gdata, out, tw, nrows, scale);
-    LAUNCH_CHECK("k_resid_rows");
+    for (int y = 0; y < runs; y += 65535) {
+        const long long r0 = y * nrows;
+        k_resid_rows<N, HALF><<<dim3((unsigned)nblk, std::min(65535, runs - y)), kRowThreads, rows_smem<N>(), s>>>(
+            rows + r0 * (HALF ? N / 2 + 1 : N), gdata + r0 * N, out + r0 * (N / 2 + 1), tw, nrows, scale);
+        LAUNCH_CHECK("k_resid_rows");
+    }
 }
 
 template <int N>
@@ -770,15 +778,21 @@ void launch_pad_fft_fwd(const float *u, float2 *spec, int zb, const float *deapo
 
 bool resid_rows_supported(int n) { return n >= 256 && n <= 1024 && (n & (n - 1)) == 0; }
 
+// A pair of rows must not lie in two slices (a NaN or the rounding of a bright
+// slice would reach the other): one run of all rows where a slice has an even
+// number, else one run per slice, whose last row has no partner.
+int resid_runs(int zb, int ntheta) { return ntheta % 2 == 0 ? 1 : zb; }
+
 // tw_n: the twiddle table of the n-point transforms, pad_fft_twiddles(n)
 void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb, bool half,
                        const UsGeo &g, cudaStream_t s) {
-    const long long nrows = (long long)zb * g.ntheta;
+    const int runs = resid_runs(zb, g.ntheta);
+    const long long nrows = (long long)zb * g.ntheta / runs;
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
     switch (g.n) {
-        case 256: (half ? resid_n<256, true> : resid_n<256, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
-        case 512: (half ? resid_n<512, true> : resid_n<512, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
-        case 1024: (half ? resid_n<1024, true> : resid_n<1024, false>)(rows, gdata, out, tw_n, nrows, scale, s); break;
+        case 256: (half ? resid_n<256, true> : resid_n<256, false>)(rows, gdata, out, tw_n, nrows, runs, scale, s); break;
+        case 512: (half ? resid_n<512, true> : resid_n<512, false>)(rows, gdata, out, tw_n, nrows, runs, scale, s); break;
+        case 1024: (half ? resid_n<1024, true> : resid_n<1024, false>)(rows, gdata, out, tw_n, nrows, runs, scale, s); break;
         default: throw Error(1, "residual rows: unsupported detector width");
     }
 }

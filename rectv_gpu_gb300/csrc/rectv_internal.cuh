@@ -300,6 +300,7 @@ void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const
 // [256, 1024]: gathered rows [z][theta][n] and data g -> the adjoint's row
 // spectra [z][theta][n/2+1] (inverse row FFT, residual, fftshift, R2C)
 bool resid_rows_supported(int n);
+int resid_runs(int zb, int ntheta);  // runs of rows that are paired among themselves
 // half: the rows hold the Hermitian half k = 0 .. n/2 (direction path)
 void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb, bool half,
                        const UsGeo &g, cudaStream_t s);

@@ -2,7 +2,8 @@
 10000 times brighter, or one value of it NaN, the other slices keep every bit.
 
 The operators act on each slice alone (radonapr / radonapradj of the
-reference, src/cuda/operators.cu)."""
+reference, src/cuda/operators.cu), and with one slice per chunk so does an
+outer iteration from zero (its halos are zero)."""
 
 import numpy as np
 import pytest
@@ -58,4 +59,37 @@ def test_operators(lib_built, torch_cuda, monkeypatch, n, m, dirs):
             for i in range(nz):
                 if i != z:
                     assert torch.equal(a[i], b[i]), i
+    obj.free()
+
+
+@pytest.mark.parametrize("ntheta", [45, 48])  # an odd count: a slice's last row has no partner
+@pytest.mark.parametrize("n,m", [(54, 5), (54, 1), (128, 16), (256, 16), (46, 4)])
+def test_outer_iteration_of_single_slice_chunks(lib_built, torch_cuda, n, m, ntheta):
+    torch = torch_cuda
+    from rectv_gpu_gb300 import rectv
+    nz, z = 3, 1
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    g = torch.randn((nz, ntheta, n), generator=gen, device="cuda")
+    theta, phi = torch.from_numpy(scan_angles(ntheta, 3)).cuda(), torch.from_numpy(_phi(ntheta, m)).cuda()
+    obj = rectv(n, ntheta, m, nz, 1, 1)
+    obj.set_verbose(False)
+
+    def run(gg):
+        f = torch.empty((nz, m, n, n), device="cuda")
+        torch.cuda.synchronize()
+        obj.setup_device(gg.data_ptr(), theta.data_ptr(), phi.data_ptr(), n / 2, 4e-3, 4.0, 3)
+        obj.iterate(1)
+        obj.result_device(f.data_ptr())
+        torch.cuda.synchronize()
+        return f
+
+    ref = run(g)
+    bright, nan = g.clone(), g.clone()
+    bright[z] *= 1e4
+    nan[z, -1] = float("nan")
+    nan[z, 0] = float("nan")
+    for gg in (bright, nan):
+        got = run(gg)
+        for i in (0, 2):
+            assert torch.equal(got[i], ref[i]), i
     obj.free()

@@ -119,6 +119,8 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d, uint32_t a, uint64_t b, 
 
 }  // namespace
 
+// zsh: 0, 16 time samples of one slice per plane, or 1, eight of two slices
+template <int zsh>
 __global__ void __launch_bounds__(kThr, 1)
     k_gather_tc(float2 *__restrict__ rows, const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
                 const float2 *__restrict__ sincos, const float2 *__restrict__ kmat,
@@ -130,7 +132,6 @@ __global__ void __launch_bounds__(kThr, 1)
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int4 it = items[blockIdx.x];
     const int z0 = blockIdx.y * per, z1 = min(npz, z0 + per);  // planes (of zs slices) of this block
-    const int zsh = g.zs >> 1;  // 16 time samples of one slice, or 8 of two
     const int tyi = it.x / g.NT, txi = it.x - tyi * g.NT;
     const int P = g.P;
     const int cnt = min(it.z, kTab);
@@ -219,10 +220,14 @@ __global__ void __launch_bounds__(kThr, 1)
         if (tid == 0) sm.seg_first[nseg] = cnt;
     }
     __syncthreads();
-    // a plane holds zs slices: ray r of slice s is the virtual ray r zs + s,
-    // whose K' row is zero at the other slices' values
-    const int nvs = nseg << zsh, rc = kRays >> zsh;  // virtual rays; rays per chunk
-    const int nch = (nvs + kRays - 1) / kRays;
+    // a chunk holds rc rays of each of the plane's zs slices: ray r of slice s is
+    // the chunk's virtual ray s rc + r, and its product takes the K values of slice
+    // s alone (a NaN in the other slice stays there)
+    constexpr int rc = kRays >> zsh;
+    const int nch = (nseg + rc - 1) / rc;
+
+    // (G in shared memory: ray by ray, so that the two slices of a sample lie on distinct banks)
+    auto slot = [](int r) { return zsh ? ((r & (rc - 1)) << 1) + r / rc : r; };
 
     // B rows of chunk ch into buffer buf: row 2r gives Re G, row 2r+1 Im G of
     // virtual ray r; K index 2v (Re F_v) and 2v+1 (Im F_v).  Threads 0..255 = (row, 4 K values).
@@ -230,15 +235,15 @@ __global__ void __launch_bounds__(kThr, 1)
         if (tid >= kN * kK / 4) return;
         const int nrow = tid >> 3, q4 = tid & 7;
         const int r = nrow >> 1, o = nrow & 1;
-        const int s = ch * kRays + r;
+        const int s = ch * rc + (r & (rc - 1));
         float bv[4] = {0.f, 0.f, 0.f, 0.f};
-        if (s < nvs) {
-            const int th = sm.th[sm.seg_first[s >> zsh]];
+        if (s < nseg) {
+            const int th = sm.th[sm.seg_first[s]];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int v = 2 * q4 + i, j = zsh ? v & 7 : v;
                 float2 kv = make_float2(0.f, 0.f);
-                if ((v >> 3) * zsh == (s & zsh) && jbase + j < g.m) kv = __ldg(kmat + (long long)th * g.m + jbase + j);
+                if (jbase + j < g.m) kv = __ldg(kmat + (long long)th * g.m + jbase + j);
                 if (o == 0) {
                     bv[2 * i] = kv.x;
                     bv[2 * i + 1] = -kv.y;
@@ -256,9 +261,10 @@ __global__ void __launch_bounds__(kThr, 1)
     };
 
     // G = A B^T for chunk ch (B in buffer buf), M tile mt, into the
-    // accumulator; N = 16 when the chunk has at most 8 rays.
+    // accumulator; N = 16 when the chunk has at most 8 rays.  With two slices
+    // slice s has B's rows 16 s .. and D's columns 16 s .., and K steps 2 s, 2 s + 1.
     auto issue = [&](uint32_t tbase, int ch, int buf, int mt) {
-        const int nr = min(kRays, nvs - ch * kRays);
+        const int nr = min(rc, nseg - ch * rc);
         const uint32_t IT = nr > 8 ? tc::idesc(tc::kFmtTF32, 128, 32) : tc::idesc(tc::kFmtTF32, 128, 16);
         const uint64_t dh = tc::sdesc(tc::smem_addr(sm.bhi[buf]), 128, 1024);
         const uint64_t dl = tc::sdesc(tc::smem_addr(sm.blo[buf]), 128, 1024);
@@ -266,9 +272,12 @@ __global__ void __launch_bounds__(kThr, 1)
 #pragma unroll
         for (int s = 0; s < kK / 8; ++s) {  // 8 K values per MMA; +256 B per K step
             const uint32_t ah = tbase + kColAhi + mt * kK + s * 8, al = tbase + kColAlo + mt * kK + s * 8;
-            mma_tf32_ts(d, ah, dh + (uint64_t)(16 * s), IT, s > 0 ? 1u : 0u);
-            mma_tf32_ts(d, ah, dl + (uint64_t)(16 * s), IT, 1u);
-            mma_tf32_ts(d, al, dh + (uint64_t)(16 * s), IT, 1u);
+            const int sl = zsh & (s >> 1);  // slice of the step
+            const uint32_t ds = d + 16 * sl;
+            const uint64_t o = 16 * s + 128 * sl;
+            mma_tf32_ts(ds, ah, dh + o, IT, s > 2 * sl ? 1u : 0u);
+            mma_tf32_ts(ds, ah, dl + o, IT, 1u);
+            mma_tf32_ts(ds, al, dh + o, IT, 1u);
         }
         tc::commit(&sm.bar_mma);
     };
@@ -349,7 +358,7 @@ __global__ void __launch_bounds__(kThr, 1)
     }
     for (int z = z0; z < z1 && nch > 0; ++z) {
         for (int ch = 0; ch < nch; ++ch) {
-            const int nr = min(kRays, nvs - ch * kRays);
+            const int nr = min(rc, nseg - ch * rc);  // rays of each slice
             ok = tc::mbar_wait(&sm.bar_mma, mma_par, ok) && ok;
             mma_par ^= 1u;
             tc::fence_after();
@@ -363,7 +372,7 @@ __global__ void __launch_bounds__(kThr, 1)
                 const int cell = mt * 128 + 32 * q + lane, gc = cell + cell / kFW;
 #pragma unroll
                 for (int r = 0; r < kRays; ++r)
-                    if (r < nr) sm.g[r][gc] = make_float2(v[2 * r], v[2 * r + 1]);
+                    if ((r & (rc - 1)) < nr) sm.g[slot(r)][gc] = make_float2(v[2 * r], v[2 * r + 1]);
             }
             static_assert(kMT == 5 && kCells - 4 * 128 <= 64 && kWarps == 16, "G read-out split");
             if (q < 2) {
@@ -373,7 +382,7 @@ __global__ void __launch_bounds__(kThr, 1)
                 const int cell = 4 * 128 + 32 * q + lane, gc = cell + cell / kFW;
 #pragma unroll
                 for (int r = 0; r < 4; ++r)
-                    if (r0 + r < nr) sm.g[r0 + r][gc] = make_float2(v[2 * r], v[2 * r + 1]);
+                    if (((r0 + r) & (rc - 1)) < nr) sm.g[slot(r0 + r)][gc] = make_float2(v[2 * r], v[2 * r + 1]);
             }
             tc::fence_before();
             __syncthreads();
@@ -447,8 +456,8 @@ __global__ void __launch_bounds__(kThr, 1)
 size_t gather_tc_smem() { return sizeof(TcSmem); }
 
 void gather_tc_prepare() {
-    CUDA_CHECK(cudaFuncSetAttribute(k_gather_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)sizeof(TcSmem)));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gather_tc<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gather_tc<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem)));
 }
 
 void make_vec_gather_tc_map(CUtensorMap *map, float2 *spec, int npl, const UsGeo &g) {
@@ -476,7 +485,7 @@ void launch_gather_tc(float2 *rows, int zb, const GeoDev &gd, const UsGeo &g, co
     if (g.zs > 2) throw Error(1, "the tensor-core gather takes at least 8 time samples");
     const int npz = vec_planes(g, zb) / g.jg, per = std::max(1, g.zper / g.zs);
     dim3 gs(gd.n_fwd_tc_items, (npz + per - 1) / per);
-    k_gather_tc<<<gs, kThr, sizeof(TcSmem), s>>>(rows, gd.fwd_pts, gd.fwd_tc_items, gd.sincos, gd.kmat, gd.shiftfwd,
+    (g.zs == 2 ? k_gather_tc<1> : k_gather_tc<0>)<<<gs, kThr, sizeof(TcSmem), s>>>(rows, gd.fwd_pts, gd.fwd_tc_items, gd.sincos, gd.kmat, gd.shiftfwd,
                                                  tmap, g, zb, npz, per, jgrp, gd.err);
     LAUNCH_CHECK("k_gather_tc");
 }

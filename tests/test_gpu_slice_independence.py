@@ -29,7 +29,7 @@ def _spoiled(a, z):
 
 
 @pytest.mark.parametrize("dirs", ["0", "1"])
-@pytest.mark.parametrize("m", [1, 2, 3, 16, 17])
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 16, 17])
 @pytest.mark.parametrize("n", WIDTHS)
 def test_operators(lib_built, torch_cuda, monkeypatch, n, m, dirs):
     torch = torch_cuda
@@ -63,7 +63,7 @@ def test_operators(lib_built, torch_cuda, monkeypatch, n, m, dirs):
 
 
 @pytest.mark.parametrize("ntheta", [45, 48])  # an odd count: a slice's last row has no partner
-@pytest.mark.parametrize("n,m", [(54, 5), (54, 1), (128, 16), (256, 16), (46, 4)])
+@pytest.mark.parametrize("n,m", [(54, 5), (54, 1), (128, 8), (256, 8), (46, 4)])
 def test_outer_iteration_of_single_slice_chunks(lib_built, torch_cuda, n, m, ntheta):
     torch = torch_cuda
     from rectv_gpu_gb300 import rectv

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(kThr, 3)
     constexpr int G = YP ? 16 / C : 8 / C;  // blocks per row (pair)
     const int y = (YP ? 2 : 1) * (blockIdx.x / G), y1 = YP ? min(y + 1, n - 1) : y, pl = blockIdx.y;
     const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
+    if (!vec_live(g, zb, pl, v0 - (YP ? 1 : 2) * c)) return;  // the block's values hold no data
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
     const int zc = vec_slice(g, pl, v1), tb = vec_time(g, pl, v1);
     const bool oka = za < zb && ta < g.m, okb = zc < zb && tb < g.m && !(YP && y + 1 >= n);
@@ -95,7 +96,7 @@ void run_fwd(const float *u, float2 *spec, int zb, const float *deapod, const fl
                                                                                        inv4n2);
     LAUNCH_CHECK("k_gen_rows_fwd");
     const size_t smem = gen_cols_smem(g.P, C);
-    const int nlv = gen_live_groups(g, C);
+    const int nlv = vec_groups(g, zb, C);
     const long long ntiles = (long long)npl * (n + 1) * nlv;
     if (ntiles > 2147483647LL - 65536) throw Error(1, "pad FFT: too many column tiles");
     const int grid = (int)std::min<long long>(ntiles, gen_resident(smem, kColThr));
@@ -179,8 +180,6 @@ size_t gen_rows_smem(int P, int C) { return (size_t)2 * P * C * sizeof(float2); 
 size_t gen_cols_smem(int P, int C) { return (size_t)2 * P * C * sizeof(float2); }
 // Eight values per tile (64-byte runs) while three blocks fit an SM, else four.
 int gen_width(int P) { return gen_cols_smem(P, 8) <= 74 * 1024 ? 8 : 4; }
-// values of a cell that hold data, in groups of C (fewer than all with 9 .. 15 time samples)
-int gen_live_groups(const UsGeo &g, int C) { return g.tg == 16 && g.jg == 1 ? (g.m + C - 1) / C : 16 / C; }
 int gen_resident(size_t smem, int threads) {
     static int nsm = 0;
     if (nsm == 0) {

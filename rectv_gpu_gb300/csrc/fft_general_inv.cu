@@ -39,6 +39,7 @@ __global__ void __launch_bounds__(kThr, 3)
     constexpr int G = YP ? 16 / C : 8 / C;  // blocks per row (pair)
     const int y = (YP ? 2 : 1) * (blockIdx.x / G), y1 = YP ? min(y + 1, n - 1) : y, pl = blockIdx.y;
     const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
+    if (!vec_live(g, zb, pl, v0 - (YP ? 1 : 2) * c)) return;  // the block's values hold no data
     const float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + v0;
     auto load = [&](int k) {  // column k of the pair's two half rows
         if constexpr (YP) {
@@ -101,7 +102,7 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
              const UsGeo &g, cudaStream_t s) {
     const int n = g.n, npl = vec_planes(g, zb);
     const size_t smem = gen_cols_smem(g.P, C);
-    const int nlv = gen_live_groups(g, C);
+    const int nlv = vec_groups(g, zb, C);
     const long long ntiles = (long long)npl * (n + 1) * nlv;
     if (ntiles > 2147483647LL - 65536) throw Error(1, "pad FFT: too many column tiles");
     const int grid = (int)std::min<long long>(ntiles, gen_resident(smem, kColThr));

@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     const int y = YP ? 2 * ry : ry, y1 = YP ? y + 1 : y;
     // the pair's values v0, v0 + 1 of the plane (YP: value v0, rows y and y + 1)
     const int v0 = (YP ? 1 : 2) * ((blockIdx.x % G) * C + c), v1 = YP ? v0 : v0 + 1;
+    if (!vec_live(g, zb, pl, v0 - (YP ? 1 : 2) * c)) return;  // the block's values hold no data
     float2 *sh = fft_sh + rr * (L::S * C);
     const int za = vec_slice(g, pl, v0), ta = vec_time(g, pl, v0);
     const int zc = vec_slice(g, pl, v1), tb = vec_time(g, pl, v1);
@@ -464,6 +465,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
     constexpr int G = YP ? 16 / C : 8 / C;
     const int ry = (blockIdx.x / G) * R + rr, pl = blockIdx.y, y = YP ? 2 * ry : ry;
     const int vb = (YP ? 1 : 2) * (blockIdx.x % G) * C;  // the block's first value
+    if (!vec_live(g, zb, pl, vb)) return;  // the block's values hold no data
     float2 *sh = fft_sh + rr * (L::S * C);
     const float2 *row = spec + pl * g.vplane + ((long long)(y + n / 2 + kVH) * g.vp + kVH) * 16 + vb + (YP ? 1 : 2) * c;
     auto load = [&](int k) {  // column k of the pair's two half rows
@@ -678,8 +680,7 @@ template <int N, int DIR>
 void launch_cols(const CUtensorMap &map, const float2 *tw, int zb, int *err, const UsGeo &g, cudaStream_t s) {
     constexpr int C = vec_col_c(N), thr = C * (N / 16);
     constexpr size_t smem = ColPass<N, C, DIR>::SMEM;
-    // value groups of a cell that hold data (fewer than all with 9 .. 15 time samples)
-    const int nlv = g.tg == 16 && g.jg == 1 ? (g.m + C - 1) / C : 16 / C, ngroups = (N / 2 + 1) * nlv;
+    const int nlv = vec_groups(g, zb, C), ngroups = (N / 2 + 1) * nlv;
     const long long ntiles = (long long)ngroups * vec_planes(g, zb);
     if (ntiles > 2147483647LL - 65536) throw Error(1, "pad FFT: too many column tiles");
     // persistent: as many blocks per SM as shared memory and 1024 threads allow

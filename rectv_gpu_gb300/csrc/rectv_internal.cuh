@@ -91,6 +91,17 @@ __host__ __device__ inline int vec_time(const UsGeo &g, int pl, int v) {
     return g.jg > 1 ? (pl % g.jg) * 16 + v : v & (g.tg - 1);
 }
 
+// whether entry v of plane pl holds data (of zb slices); a run of 2, 4, 8 or 16
+// entries from a multiple of its length on holds some where its first one does
+__host__ __device__ inline bool vec_live(const UsGeo &g, int zb, int pl, int v) {
+    return g.jg > 1 ? (pl % g.jg) * 16 + v < g.m : v < (zb - pl * g.zs) * g.tg && (v & (g.tg - 1)) < g.m;
+}
+// groups of C entries of a cell that hold data in any plane: fewer than all with
+// 9 .. 15 time samples, or with less than a plane's slices
+inline int vec_groups(const UsGeo &g, int zb, int C) {
+    return g.jg > 1 ? 16 / C : (((zb < g.zs ? zb : g.zs) - 1) * g.tg + g.m + C - 1) / C;
+}
+
 // Weights of one polar sample restricted to one 16x16 tile of the adjoint
 // plan (zero outside the sample's 9x9 stencil), with its ray and the mask of
 // tile rows its stencil covers (thm = theta << 16 | mask, theta < 65536),
@@ -287,7 +298,6 @@ void gen_fft_inv_prepare();
 size_t gen_rows_smem(int P, int C);
 size_t gen_cols_smem(int P, int C);
 int gen_width(int P);
-int gen_live_groups(const UsGeo &g, int C);
 int gen_resident(size_t smem, int threads);
 void launch_gen_fft_fwd(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const GenPlan &p,
                         const UsGeo &g, cudaStream_t s);

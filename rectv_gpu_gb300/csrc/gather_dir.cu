@@ -379,34 +379,44 @@ void launch_vec_halo(float2 *spec, int npl, int right, const UsGeo &g, cudaStrea
 
 // ---------------------------------------------------------------------------
 // Planar half planes [image][P][planar_pitch] (cuFFT's output for slices z0 .. z0 +
-// nz - 1, image (z - z0) m + t) into the vector layout: one block per 32
-// cells of a row, transposed through shared memory.
+// nz - 1, image (z - z0) m + t) into the vector layout: one block per 128
+// cells of a row, transposed through shared memory (eight loads of a thread in flight).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     k_planar_to_vec(const float2 *__restrict__ planar, float4 *__restrict__ spec, UsGeo g, int z0, int nz, int pl0) {
-    __shared__ float2 sh[32][17];
-    const int pl = pl0 + blockIdx.z, y = blockIdx.y, x0 = blockIdx.x * 32;
-    const int pitch = planar_pitch(g.n);
+    __shared__ float2 sh[kLayoutCells][17];
+    const int pl = pl0 + blockIdx.z, y = blockIdx.y, x0 = blockIdx.x * kLayoutCells;
+    const int pitch = planar_pitch(g.n), lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long img = (long long)g.P * pitch;
-    const int lane = threadIdx.x & 31;
-    for (int v = threadIdx.x >> 5; v < 16; v += 8) {
-        const int z = vec_slice(g, pl, v), t = vec_time(g, pl, v), x = x0 + lane;
-        float2 f = make_float2(0.f, 0.f);
-        if (x <= g.n && z < z0 + nz && t < g.m)
-            f = __ldg(planar + ((long long)(z - z0) * g.m + t) * img + (long long)y * pitch + x);
-        sh[lane][v] = f;
+    float2 f[2][kLayoutCells / 32];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {  // values w and w + 8
+        const int v = w + 8 * h;
+        const bool live = vec_live(g, z0 + nz, pl, v);
+        const long long im = live ? (long long)(vec_slice(g, pl, v) - z0) * g.m + vec_time(g, pl, v) : 0;
+        const float2 *src = planar + im * img + (long long)y * pitch + x0 + lane;
+#pragma unroll
+        for (int i = 0; i < kLayoutCells / 32; ++i)
+            f[h][i] = live && x0 + lane + 32 * i <= g.n ? __ldg(src + 32 * i) : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < kLayoutCells / 32; ++i) {
+        sh[lane + 32 * i][w] = f[0][i];
+        sh[lane + 32 * i][w + 8] = f[1][i];
     }
     __syncthreads();
-    const int cell = threadIdx.x >> 3, ci = threadIdx.x & 7, x = x0 + cell;
-    if (x <= g.n) {
-        const float2 a = sh[cell][2 * ci], b = sh[cell][2 * ci + 1];
-        spec[pl * (g.vplane / 2) + ((long long)(y + kVH) * g.vp + x + kVH) * 8 + ci] = make_float4(a.x, a.y, b.x, b.y);
+    const int cell = threadIdx.x >> 3, ci = threadIdx.x & 7;
+    float4 *dst = spec + pl * (g.vplane / 2) + ((long long)(y + kVH) * g.vp + kVH + x0 + cell) * 8 + ci;
+#pragma unroll
+    for (int i = 0; i < kLayoutCells / 32; ++i) {
+        const float2 a = sh[cell + 32 * i][2 * ci], b = sh[cell + 32 * i][2 * ci + 1];
+        if (x0 + cell + 32 * i <= g.n) dst[32 * 8 * i] = make_float4(a.x, a.y, b.x, b.y);
     }
 }
 
 void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, const UsGeo &g, cudaStream_t s) {
     const int pl0 = g.jg > 1 ? z0 * g.jg : z0 / g.zs, npl = vec_planes(g, nz);
-    k_planar_to_vec<<<dim3((g.n + 32) / 32, g.P, npl), 256, 0, s>>>(planar, reinterpret_cast<float4 *>(spec), g, z0, nz,
+    k_planar_to_vec<<<dim3(g.n / kLayoutCells + 1, g.P, npl), 256, 0, s>>>(planar, reinterpret_cast<float4 *>(spec), g, z0, nz,
                                                                     pl0);
     LAUNCH_CHECK("k_planar_to_vec");
 }

@@ -260,6 +260,7 @@ void launch_vec_halo(float2 *spec, int npl, int right, const UsGeo &g, cudaStrea
 // cuFFT's spectra of slices z0 .. z0 + nz - 1 (planar, rows of planar_pitch
 // complex, image (z - z0) m + t) into the vector layout, and back
 void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, const UsGeo &g, cudaStream_t s);
+constexpr int kLayoutCells = 128;  // cells of a row per block of either
 void launch_vec_to_planar(const float2 *spec, float2 *planar, int z0, int nz, const UsGeo &g, cudaStream_t s);
 void gather_dir_prepare();    // kernel attributes; once, outside stream capture
 void scatter_dir_prepare();

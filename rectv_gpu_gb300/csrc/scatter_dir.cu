@@ -533,28 +533,36 @@ __global__ void k_vec_fold(float4 *__restrict__ spec, UsGeo g) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     k_vec_to_planar(const float4 *__restrict__ spec, float2 *__restrict__ planar, UsGeo g, int z0, int nz, int pl0) {
-    __shared__ float2 sh[32][17];
-    const int pl = pl0 + blockIdx.z, y = blockIdx.y, x0 = blockIdx.x * 32;
+    __shared__ float2 sh[kLayoutCells][17];
+    const int pl = pl0 + blockIdx.z, y = blockIdx.y, x0 = blockIdx.x * kLayoutCells;
     const int cell = threadIdx.x >> 3, ci = threadIdx.x & 7;
-    if (x0 + cell <= g.n) {
-        const float4 f = spec[pl * (g.vplane / 2) + ((long long)(y + kVH) * g.vp + x0 + cell + kVH) * 8 + ci];
-        sh[cell][2 * ci] = lo2(f);
-        sh[cell][2 * ci + 1] = hi2(f);
+    const bool any = vec_live(g, z0 + nz, pl, 2 * ci);  // (or the pair holds no data)
+    const float4 *src = spec + pl * (g.vplane / 2) + ((long long)(y + kVH) * g.vp + kVH + x0 + cell) * 8 + ci;
+    float4 f[kLayoutCells / 32];
+#pragma unroll
+    for (int i = 0; i < kLayoutCells / 32; ++i)
+        f[i] = any && x0 + cell + 32 * i <= g.n ? __ldg(src + 32 * 8 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < kLayoutCells / 32; ++i) {
+        sh[cell + 32 * i][2 * ci] = lo2(f[i]);
+        sh[cell + 32 * i][2 * ci + 1] = hi2(f[i]);
     }
     __syncthreads();
-    const int pitch = planar_pitch(g.n);
+    const int pitch = planar_pitch(g.n), lane = threadIdx.x & 31;
     const long long img = (long long)g.P * pitch;
-    const int lane = threadIdx.x & 31, x = x0 + lane;
     for (int v = threadIdx.x >> 5; v < 16; v += 8) {
-        const int z = vec_slice(g, pl, v), t = vec_time(g, pl, v);
-        if (x <= g.n && z < z0 + nz && t < g.m)
-            planar[((long long)(z - z0) * g.m + t) * img + (long long)y * pitch + x] = sh[lane][v];
+        if (!vec_live(g, z0 + nz, pl, v)) continue;
+        float2 *dst = planar + ((long long)(vec_slice(g, pl, v) - z0) * g.m + vec_time(g, pl, v)) * img +
+                      (long long)y * pitch + x0 + lane;
+#pragma unroll
+        for (int i = 0; i < kLayoutCells / 32; ++i)
+            if (x0 + lane + 32 * i <= g.n) dst[32 * i] = sh[lane + 32 * i][v];
     }
 }
 
 void launch_vec_to_planar(const float2 *spec, float2 *planar, int z0, int nz, const UsGeo &g, cudaStream_t s) {
     const int pl0 = g.jg > 1 ? z0 * g.jg : z0 / g.zs, npl = vec_planes(g, nz);
-    k_vec_to_planar<<<dim3((g.n + 32) / 32, g.P, npl), 256, 0, s>>>(reinterpret_cast<const float4 *>(spec), planar, g,
+    k_vec_to_planar<<<dim3(g.n / kLayoutCells + 1, g.P, npl), 256, 0, s>>>(reinterpret_cast<const float4 *>(spec), planar, g,
                                                                     z0, nz, pl0);
     LAUNCH_CHECK("k_vec_to_planar");
 }

@@ -122,12 +122,14 @@ void run_inv(float2 *spec, float *u, int zb, float cscale, const float *deapod, 
 // mixed-radix core): two rows are one complex transform, C pairs per block;
 // blockIdx.y: runs of nrows rows (launch_resid_rows).
 // HALF: the rows hold their Hermitian half (direction path), else the whole
-// row, of which the Hermitian part counts.
+// row, of which the Hermitian part counts.  FWD: the forward operator of the
+// direction path, fout = tau R u (k_resid_rows).
 // ---------------------------------------------------------------------------
-template <int C, bool HALF>
+template <int C, bool HALF, bool FWD>
 __global__ void __launch_bounds__(kResThr, 6)
     k_gen_resid(const float2 *__restrict__ rows, const float *__restrict__ gdata, float2 *__restrict__ out,
-                const __grid_constant__ GenPlan p, const float2 *__restrict__ tw, long long nrows, float scale) {
+                const __grid_constant__ GenPlan p, const float2 *__restrict__ tw, long long nrows, float scale,
+                float *__restrict__ fout, float tau) {
     using gen::gen_sh;
     const int n = p.P, hn = n / 2 + 1;
     const int c = threadIdx.x % C, j0 = threadIdx.x / C;
@@ -136,8 +138,12 @@ __global__ void __launch_bounds__(kResThr, 6)
     const bool oka = ra < nrows, okb = rb < nrows;
     const int rn = HALF ? hn : n;  // values per row
     rows += blockIdx.y * nrows * rn;
-    gdata += blockIdx.y * nrows * n;
-    out += blockIdx.y * nrows * hn;
+    if constexpr (FWD) {
+        fout += blockIdx.y * nrows * n;
+    } else {
+        gdata += blockIdx.y * nrows * n;
+        out += blockIdx.y * nrows * hn;
+    }
     const float2 *ga = rows + (oka ? ra : 0) * rn, *gb = rows + (okb ? rb : 0) * rn;
     const float2 zero = make_float2(0.f, 0.f);
     auto load = [&](const float2 *r, int k) {
@@ -168,6 +174,15 @@ __global__ void __launch_bounds__(kResThr, 6)
     }
     __syncthreads();
     const int f = gen::passes<1, C>(0, n * C, 0, p, tw, c, j0, js);
+    if constexpr (FWD) {
+        for (int x = j0; x < n; x += js) {
+            const float2 v = gen_sh[f + x * C + c];
+            const float sc = (x & 1) ? scale : -scale;
+            if (oka) fout[ra * n + x] = tau * (v.x * sc);
+            if (okb) fout[rb * n + x] = tau * (v.y * sc);
+        }
+        return;
+    }
     const float *da = gdata + (oka ? ra : 0) * n, *db = gdata + (okb ? rb : 0) * n;
     for (int sb = j0; sb < n; sb += 2 * js) {
         float va[2], vb[2];
@@ -199,8 +214,8 @@ __global__ void __launch_bounds__(kResThr, 6)
 
 }  // namespace
 
-void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
-                      bool half, const UsGeo &g, cudaStream_t s) {
+static void gen_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
+                           bool half, const UsGeo &g, float *fout, float tau, cudaStream_t s) {
     constexpr int C = 4;
     const int runs = resid_runs(zb, g.ntheta);
     const long long nrows = (long long)zb * g.ntheta / runs, nblk = (nrows + 2 * C - 1) / (2 * C);
@@ -208,19 +223,32 @@ void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const
     const float scale = (float)(1.0 / std::sqrt((double)g.n * (double)g.ntheta));
     const size_t smem = gen_rows_smem(g.n, C);
     const long long rn = half ? g.n / 2 + 1 : g.n;
+    const auto kern = fout ? k_gen_resid<C, true, true> : half ? k_gen_resid<C, true, false> : k_gen_resid<C, false, false>;
     for (int y = 0; y < runs; y += 65535) {
         const long long r0 = y * nrows;
         const dim3 gr((unsigned)nblk, std::min(65535, runs - y));
-        (half ? k_gen_resid<C, true> : k_gen_resid<C, false>)<<<gr, kResThr, smem, s>>>(
-            rows + r0 * rn, gdata + r0 * g.n, out + r0 * (g.n / 2 + 1), p, tw, nrows, scale);
+        kern<<<gr, kResThr, smem, s>>>(rows + r0 * rn, fout ? nullptr : gdata + r0 * g.n,
+                                       fout ? nullptr : out + r0 * (g.n / 2 + 1), p, tw, nrows, scale,
+                                       fout ? fout + r0 * g.n : nullptr, tau);
         LAUNCH_CHECK("k_gen_resid");
     }
 }
 
+void launch_gen_resid(const float2 *rows, const float *gdata, float2 *out, const float2 *tw, const GenPlan &p, int zb,
+                      bool half, const UsGeo &g, cudaStream_t s) {
+    gen_resid_rows(rows, gdata, out, tw, p, zb, half, g, nullptr, 0.f, s);
+}
+
+void launch_gen_fwd_rows(const float2 *hrows, float *out, float tau, const float2 *tw, const GenPlan &p, int zb,
+                         const UsGeo &g, cudaStream_t s) {
+    gen_resid_rows(hrows, nullptr, nullptr, tw, p, zb, true, g, out, tau, s);
+}
+
 void gen_fft_inv_prepare() {
     constexpr int most = 227 * 1024;
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+    CUDA_CHECK(cudaFuncSetAttribute(k_gen_resid<4, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_cols_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
     CUDA_CHECK(cudaFuncSetAttribute(k_gen_rows_inv<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));

@@ -413,7 +413,7 @@ struct Handle {
     void ensure_plans() {
         bool need[kNPlans] = {};
         need[kRowsR2C] = true;
-        need[gd.dirs ? kRowsC2R : kRowsC2C] = true;
+        need[gd.dirs ? kRowsC2R : kRowsC2C] = !(gd.dirs && own_rows());
         need[kR2C2D] = need[kC2R2D] = !own_fft();
         make_fft_plans(need);
     }
@@ -742,7 +742,14 @@ struct Handle {
     // out = tau R_apr u  (residual: out = R_apr u - gb)
     void forward(const float *u, const float *gb, float *out, float tau, int residual) {
         forward_rows(u);
-        if (gd.dirs) {  // Hermitian half rows
+        if (gd.dirs && own_rows() && !residual) {  // Hermitian half rows, two per transform
+            if (fused_rows)
+                launch_fwd_rows(rows, out, tau, fft_tw_n, zb, ug, stream);
+            else
+                launch_gen_fwd_rows(rows, out, tau, fft_tw_n, gen_rplan, zb, ug, stream);
+            return;
+        }
+        if (gd.dirs) {
             CUFFT_CHECK(cufftExecC2R(plan[kRowsC2R], reinterpret_cast<cufftComplex *>(rows),
                                      reinterpret_cast<cufftReal *>(rows)));
             launch_finish_fwd_real(reinterpret_cast<const float *>(rows), gb, out, zb, tau, residual, ug, stream);

@@ -315,6 +315,11 @@ int resid_runs(int zb, int ntheta);  // runs of rows that are paired among thems
 // half: the rows hold the Hermitian half k = 0 .. n/2 (direction path)
 void launch_resid_rows(const float2 *rows, const float *gdata, float2 *out, const float2 *tw_n, int zb, bool half,
                        const UsGeo &g, cudaStream_t s);
+// out = tau R u from the Hermitian half rows, on the same transforms
+void launch_fwd_rows(const float2 *hrows, float *out, float tau, const float2 *tw_n, int zb, const UsGeo &g,
+                     cudaStream_t s);
+void launch_gen_fwd_rows(const float2 *hrows, float *out, float tau, const float2 *tw, const GenPlan &p, int zb,
+                         const UsGeo &g, cudaStream_t s);
 size_t gather_tc_smem();
 int gather_tc_table_capacity();
 void usfft_prepare();  // kernel attributes; call once, outside stream capture

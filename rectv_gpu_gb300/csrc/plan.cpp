@@ -74,21 +74,26 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
     std::vector<float> qk(n);
     for (int k = 1; k < n; ++k) qk[k] = (float)(k - n / 2) / (float)n;
     if (T < kTaps) throw Error(1, "tile smaller than the interpolation stencil");
-    // Tiles holding any cell of the nine of a stencil's axis (cells wrap modulo P):
-    // those from its first cell's to its last one's.  There are three where the
-    // last tile is narrower than eight cells and the stencil reaches from the tile
-    // before it to the one behind the wrap.
-    auto axis_tiles = [&](int K, int *out) {
-        const int lo = wrapi(K - kR, P), hi = wrapi(K + kR, P), first = lo / T, last = hi / T;
-        int k = 0;
-        out[k++] = first;
-        // (on a grid below 2T cells a wrapped stencil may end in the tile it starts in)
-        for (int t = first; t != last || (k == 1 && lo > hi && NT > 1);) {
-            t = t + 1 < NT ? t + 1 : 0;
-            if (t != first) out[k++] = t;
-        }
-        return k;
+    // Tiles holding any cell of the nine of a stencil's axis (cells wrap modulo P),
+    // by the cell of the origin: those from its first cell's to its last one's.
+    // There are three where the last tile is narrower than eight cells and the
+    // stencil reaches from the tile before it to the one behind the wrap.
+    struct AxisTiles {
+        int origin, count, tile[3];
     };
+    std::vector<AxisTiles> axis(P);
+    for (int K = 0; K < P; ++K) {
+        const int lo = wrapi(K - kR, P), hi = wrapi(K + kR, P), last = hi / T;
+        AxisTiles &a = axis[K];
+        a.origin = K / T;
+        a.tile[0] = lo / T;
+        a.count = 1;
+        // (on a grid below 2T cells a wrapped stencil may end in the tile it starts in)
+        for (int t = a.tile[0]; t != last || (a.count == 1 && lo > hi && NT > 1);) {
+            t = t + 1 < NT ? t + 1 : 0;
+            if (t != a.tile[0]) a.tile[a.count++] = t;
+        }
+    }
     // Angles are split into contiguous ranges, one per host thread; each
     // thread counts its samples per tile and later places them at its own
     // offsets, so every tile keeps the theta-major sample order.
@@ -111,11 +116,10 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
                 const int fy = (int)std::floor(tn * y0);
                 const int KX = n + fx, KY = n + fy;  // in [0, P)
                 cell[ip] = make_int2(KX, KY);
-                fcnt[(KY / T) * NT + KX / T]++;
-                int xs[3], ys[3];
-                const int nx = axis_tiles(KX, xs), ny = axis_tiles(KY, ys);
-                for (int a = 0; a < ny; ++a)
-                    for (int b = 0; b < nx; ++b) acnt[ys[a] * NT + xs[b]]++;
+                const AxisTiles &ax = axis[KX], &ay = axis[KY];
+                fcnt[ay.origin * NT + ax.origin]++;
+                for (int a = 0; a < ay.count; ++a)
+                    for (int b = 0; b < ax.count; ++b) acnt[ay.tile[a] * NT + ax.tile[b]]++;
             }
         }
     };
@@ -153,12 +157,10 @@ HostPlan build_plan(const float *theta, int n, int ntheta, int T, int fwd_cap, f
             for (int th = rg.first; th < rg.second; ++th)
                 for (int k = 1; k < n; ++k, ++ip) {
                     const uint32_t id = (uint32_t)th * (uint32_t)n + (uint32_t)k;
-                    const int2 c = cell[ip];
-                    p.fwd_pts[fp[(c.y / T) * NT + c.x / T]++] = id;
-                    int xs[3], ys[3];
-                    const int nx = axis_tiles(c.x, xs), ny = axis_tiles(c.y, ys);
-                    for (int a = 0; a < ny; ++a)
-                        for (int b = 0; b < nx; ++b) p.adj_pts[ap[ys[a] * NT + xs[b]]++] = id;
+                    const AxisTiles &ax = axis[cell[ip].x], &ay = axis[cell[ip].y];
+                    p.fwd_pts[fp[ay.origin * NT + ax.origin]++] = id;
+                    for (int a = 0; a < ay.count; ++a)
+                        for (int b = 0; b < ax.count; ++b) p.adj_pts[ap[ay.tile[a] * NT + ax.tile[b]]++] = id;
                 }
         };
         parallel_for(nthr, place);

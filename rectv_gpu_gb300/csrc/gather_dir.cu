@@ -417,6 +417,7 @@ __global__ void __launch_bounds__(256)
     __syncthreads();
     const int cell = threadIdx.x >> 3, ci = threadIdx.x & 7;
     float4 *dst = spec + pl * (g.vplane / 2) + ((long long)(y + kVH) * g.vp + kVH + x0 + cell) * 8 + ci;
+    if (!vec_live(g, z0 + nz, pl, 2 * ci & ~3)) return;  // 32 bytes without data
 #pragma unroll
     for (int i = 0; i < kLayoutCells / 32; ++i) {
         const float2 a = sh[cell + 32 * i][2 * ci], b = sh[cell + 32 * i][2 * ci + 1];

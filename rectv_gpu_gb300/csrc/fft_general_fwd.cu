@@ -181,13 +181,7 @@ size_t gen_cols_smem(int P, int C) { return (size_t)2 * P * C * sizeof(float2); 
 // Eight values per tile (64-byte runs) while three blocks fit an SM, else four.
 int gen_width(int P) { return gen_cols_smem(P, 8) <= 74 * 1024 ? 8 : 4; }
 int gen_resident(size_t smem, int threads) {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
-    return nsm * std::max(1, std::min((int)((size_t)227 * 1024 / (smem + 1024)), 1024 / threads));
+    return sm_count() * std::max(1, std::min((int)((size_t)227 * 1024 / (smem + 1024)), 1024 / threads));
 }
 
 void launch_gen_fft_fwd(const float *u, float2 *spec, int zb, const float *deapod, const float2 *tw, const GenPlan &p,

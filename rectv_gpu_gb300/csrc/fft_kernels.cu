@@ -688,16 +688,6 @@ void set_attrs_n() {
     CUDA_CHECK(cudaFuncSetAttribute(k_fft_cols<N, C, 1>, attr, (int)ColPass<N, C, 1>::SMEM));
 }
 
-int sm_count() {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
-    return nsm;
-}
-
 template <int N, int DIR>
 void launch_cols(const CUtensorMap &map, const float2 *tw, int zb, int *err, const UsGeo &g, cudaStream_t s) {
     constexpr int C = vec_col_c(N), thr = C * (N / 16);
@@ -737,17 +727,27 @@ void inv_n(float2 *spec, float *u, int zb, float cscale, const float *deapod, co
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
-    if (!encode) {
+    static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+        PFN_cuTensorMapEncodeTiled_v12000 e = nullptr;
         cudaDriverEntryPointQueryResult q;
-        CUDA_CHECK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&encode, 12000,
-                                                    cudaEnableDefault, &q));
-        if (q != cudaDriverEntryPointSuccess || !encode) throw Error(1, "cuTensorMapEncodeTiled unavailable");
-    }
+        CUDA_CHECK(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", (void **)&e, 12000, cudaEnableDefault, &q));
+        if (q != cudaDriverEntryPointSuccess || !e) throw Error(1, "cuTensorMapEncodeTiled unavailable");
+        return e;
+    }();
     return encode;
 }
 
 }  // namespace
+
+int sm_count() {
+    static const int nsm = [] {
+        int dev = 0, v = 0;
+        CUDA_CHECK(cudaGetDevice(&dev));
+        CUDA_CHECK(cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev));
+        return v;
+    }();
+    return nsm;
+}
 
 // P <= 2048: the column passes' two landing tiles and exchange buffer fit in
 // shared memory up to that size

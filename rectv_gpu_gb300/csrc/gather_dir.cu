@@ -435,16 +435,10 @@ void launch_planar_to_vec(const float2 *planar, float2 *spec, int z0, int nz, co
 template <int TG>
 static void gather_dir_t(float2 *hrows, int zb, const GeoDev &gd, const UsGeo &g, const CUtensorMap &vmap,
                          cudaStream_t s) {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
     const int npz = vec_planes(g, zb) / g.jg;
     // planes per block: all of them (the weights are built once) while there
     // are blocks for eight waves of two per SM, fewer for small problems
-    const long long want = 16LL * nsm;
+    const long long want = 16LL * sm_count();
     int per = (int)std::max<long long>(1, std::min<long long>(npz, (long long)gd.n_dfwd_items * npz / want));
     per = std::min(per, std::max(1, g.zper));
     const dim3 gs(gd.n_dfwd_items, (npz + per - 1) / per);

@@ -325,7 +325,6 @@ struct Handle {
         ug.ntheta = ntheta;
         ug.m = m;
         ug.P = P;
-        ug.hp = P / 2 + 1;
         ug.tn = (float)(2 * n);
         ug.inv2n = (float)(1.0 / (2.0 * n));
         ug.wexp = (float)(kPiUsfft * kPiUsfft / (double)mu_us);

@@ -43,7 +43,6 @@ void cufft_check(cufftResult e, const char *what, const char *file, int line);
 struct UsGeo {
     int n, ntheta, m;   // detector width, projections, time samples
     int P;              // oversampled grid side 2n
-    int hp;             // half-plane row length P/2+1 (complex)
     float tn;           // (float)(2n)
     float inv2n;        // 1/(2n)
     float wexp;         // pi^2/mu
@@ -207,6 +206,8 @@ bool group_directions(const float *theta, int n, int ntheta, double tol_cells, d
 // 2w+1 of the tile (lo | hi << 16), then the first row of every ray and the
 // table size as 16-bit values; padded to 16 bytes.
 __host__ __device__ constexpr int adj_info_words(int nseg) { return (4 + 8 * nseg + (nseg + 2) / 2 + 3) & ~3; }
+
+int sm_count();  // of the current device (fft_kernels.cu)
 
 // ---- USFFT kernel launchers (usfft_kernels.cu) ----
 // deapodised, padded and modulated images for cuFFT's R2C (planar_pitch)

@@ -590,13 +590,7 @@ void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &
     const long long nunits = (long long)npairs * gd.n_adj_busy;
     if (nunits == 0) return;
     if (nunits > 2147483647LL - 262144) throw Error(1, "adjoint grid too large");
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        CUDA_CHECK(cudaGetDevice(&dev));
-        CUDA_CHECK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    }
-    const int grid = (int)std::min<long long>(nunits, g.sc_grid > 0 ? g.sc_grid : nsm);
+    const int grid = (int)std::min<long long>(nunits, g.sc_grid > 0 ? g.sc_grid : sm_count());
     if (!gd.adj_tabs || !gd.adj_info) throw Error(1, "adjoint table segmentation missing");
     CUDA_CHECK(cudaMemsetAsync(gd.sc_next, 0, sizeof(int), s));
     k_scatter_tc<<<grid, kThr, kScSmemBytes, s>>>(rowsc, spec, gd.adj_recs, gd.adj_items, gd.adj_tabs,

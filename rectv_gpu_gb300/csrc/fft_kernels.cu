@@ -291,9 +291,9 @@ __global__ void __launch_bounds__(kRowThreads, 2)
             v[r] = make_float2(0.f, 0.f);
             if (r >= 4 && r < 12) {  // X = t + N1 r in [n/2, 3n/2)
                 const int x = t + N1 * (r - 4), X = x + n / 2;
-                const float d = (X & 1) ? -__ldg(dp + x) : __ldg(dp + x);
-                if (oka) v[r].x = __ldg(ua + x) * (d * sy);
-                if (okb) v[r].y = __ldg(ub + x) * (d * sy1);
+                const float d = (X & 1) ? -__ldg(dp + x) : __ldg(dp + x), w = d * sy;
+                if (oka) v[r].x = __ldg(ua + x) * w;
+                if (okb) v[r].y = __ldg(ub + x) * (YP ? d * sy1 : w);
             }
         }
     }
@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kRowThreads, 2)
             row[(long long)k * 16] = make_float2(o.x, o.y);
             row[((long long)g.vp + k) * 16] = make_float2(o.z, o.w);
         } else {
-            *reinterpret_cast<float4 *>(row + (long long)k * 16) = o;
+            reinterpret_cast<float4 *>(row)[(long long)k * 8] = o;
         }
     }
 }

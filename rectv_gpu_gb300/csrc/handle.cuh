@@ -143,9 +143,13 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
     L.spec_elems = std::max<size_t>((size_t)(L.planes() * vec_plane), (size_t)2 * (n + 1) * (n + 1) * (m + 1) * (nzp + 1));
     if (!L.pad_fft && !L.gen_fft) {
         // 2D cuFFT calls over as many slices as keep the planar images near the L2 (whole planes
-        // of the vector layout, but never more slices than there are), of equal size
+        // of the vector layout, but never more slices than there are), of equal size.  A slice
+        // that takes most of the L2 gains nothing from it: there as many as 1 GB takes (5 slices
+        // of width 736, 16 samples: 21.6 ms an iteration, 22.2 one at a time; 8 slices of width
+        // 230: 3.6 ms in 64 MB, 3.7 in one call)
         const double img = (double)m * P * planar_pitch(n) * 8.0;
-        const int most = (int)std::max(1.0, std::min((double)L.zb, 64e6 / img));
+        const double group = img > 32e6 ? std::min(1e9, std::max(64e6, budget / 4)) : 64e6;
+        const int most = (int)std::max(1.0, std::min((double)L.zb, group / img));
         const int calls = (L.zb + most - 1) / most, even = (L.zb + calls - 1) / calls;
         L.vec_slices = std::min(L.zb, (even + L.zs - 1) / L.zs * L.zs);
         L.planar_elems = (size_t)L.vec_slices * m * P * planar_pitch(n);

@@ -153,6 +153,8 @@ inline Layout make_layout(int n, int ntheta, int m, int nz, int nzp, double batc
         const int calls = (L.zb + most - 1) / most, even = (L.zb + calls - 1) / calls;
         L.vec_slices = std::min(L.zb, (even + L.zs - 1) / L.zs * L.zs);
         L.planar_elems = (size_t)L.vec_slices * m * P * planar_pitch(n);
+        // the per-ray adjoint's planar images of all slices lie in the spectra, whole calls of them
+        L.spec_elems = std::max(L.spec_elems, (size_t)((L.zb + L.vec_slices - 1) / L.vec_slices) * L.planar_elems);
     }
     const double nt = (double)ntheta * n;
     double b = 3.0 * L.nzc * L.slab * 4 + (double)nz * nt * 4 + 3.0 * 4 * L.nchunks * L.gp * 4;
@@ -273,6 +275,8 @@ struct Handle {
     float2 *rows_adj = nullptr;  // the adjoint's row spectra [zb][ntheta][n/2+1]
     bool own_rows() const { return fused_rows || gen_rows; }
     bool own_fft() const { return pad_fft || gen_fft; }
+    // the per-ray scatters add straight into planar images (in spec) where cuFFT inverts them
+    bool planar_adj() const { return !own_fft() && !gd.dirs; }
 
     // session
     bool session = false;
@@ -796,7 +800,7 @@ struct Handle {
     // u += tau R_apr^T of the row spectra rowsc [zb][ntheta][n/2+1]
     void adjoint_rows(const float2 *rowsc, float *u, float tau) {
         // Re IFFT2 of the scattered grids as a C2R of their Hermitian part
-        launch_scatter_adj(rowsc, spec, zb, gd, ug, stream);
+        launch_scatter_adj(rowsc, spec, zb, gd, ug, planar_adj(), stream);
         if (pad_fft) {
             launch_pad_fft_inv_accum(spec, u, zb, tau, gd.deapod, fft_tw, fft_map, gd.err, ug, stream);
         } else if (gen_fft) {
@@ -804,11 +808,12 @@ struct Handle {
         } else {
             for (int z = 0; z < zb; z += vec_slices) {
                 const int nzg = std::min(vec_slices, zb - z);
-                launch_vec_to_planar(spec, planar, z, nzg, ug, stream);
-                CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], reinterpret_cast<cufftComplex *>(planar),
-                                         reinterpret_cast<cufftReal *>(planar)));
-                launch_crop_accum_real(reinterpret_cast<const float *>(planar), u + (long long)z * slab, nzg, tau,
-                                       gd.deapod, ug, stream);
+                float2 *img = planar_adj() ? spec + (long long)z * m * ug.P * planar_pitch(n) : planar;
+                if (!planar_adj()) launch_vec_to_planar(spec, planar, z, nzg, ug, stream);
+                CUFFT_CHECK(cufftExecC2R(plan[kC2R2D], reinterpret_cast<cufftComplex *>(img),
+                                         reinterpret_cast<cufftReal *>(img)));
+                launch_crop_accum_real(reinterpret_cast<const float *>(img), u + (long long)z * slab, nzg, tau, gd.deapod,
+                                       ug, stream);
             }
         }
     }
@@ -1143,10 +1148,13 @@ struct Handle {
                     : 1 + ng * (((m >= 8 && gd.n_fwd_tc_items > 0) ? 1 : 0) + (gd.n_fwd_items > 0 ? 1 : 0));
         const int fwd_k = (own_fft() ? 2 : 2 * calls) + 1 + gather_k + 1;
         const int fwd_f = (own_fft() ? 0 : calls) + (own_rows() ? 0 : 1);
-        // adjoint: [row preparation], one scatter per group (direction path: the
-        // mixing and the scatter, and the fold of the border), then columns and
-        // rows (the layout change and the crop per cuFFT call)
-        const int adj_k = (own_rows() ? 0 : 1) + (gd.dirs ? 2 * ng + 1 : ng) + (own_fft() ? 2 : 2 * calls);
+        // adjoint: [row preparation], [zeros where planes are partly filled], one scatter
+        // per group (direction path: the mixing and the scatter, and the fold of the
+        // border), then columns and rows (per cuFFT call the layout change, on the
+        // direction path, and the crop)
+        const int zero_k = !gd.dirs && !planar_adj() && vec_groups(ug, zb, 4) < 4 ? 1 : 0;
+        const int adj_k = (own_rows() ? 0 : 1) + zero_k + (gd.dirs ? 2 * ng + 1 : ng) +
+                          (own_fft() ? 2 : (gd.dirs ? 2 : 1) * calls);
         const int adj_f = (own_rows() ? 0 : 1) + (own_fft() ? 0 : calls);
         // per outer iteration: titer inner steps per batch (forward, graddiv,
         // adjoint), one shrink per batch, the two-stage rho reduction
@@ -1204,7 +1212,7 @@ struct Handle {
         for (int r = 0; r < reps; ++r) {
             switch (which) {
                 case 0: launch_gather_fwd(spec, rows, zb, gd, ug, gd.dirs ? &dir_tmap : &tc_tmap, stream); break;
-                case 1: launch_scatter_adj(own_rows() ? rows_adj : rows, spec, zb, gd, ug, stream); break;
+                case 1: launch_scatter_adj(own_rows() ? rows_adj : rows, spec, zb, gd, ug, planar_adj(), stream); break;
                 case 2:  // the inner steps after the first (w = mu - rho psi as stored by the last iteration)
                     launch_graddiv(U[cur], U[cur], U[(cur + 1) % 3], psi, mu, wdual, titer > 1 ? 2 : 0, rho_d, 0,
                                    nchunks, tv, stream);

@@ -221,8 +221,10 @@ void launch_finish_fwd(const float2 *rows, const float *gdata, float *out, int z
 void launch_finish_fwd_real(const float *rows, const float *gdata, float *out, int zb, float tau, int residual,
                             const UsGeo &g, cudaStream_t s);
 void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaStream_t s);
+// the adjoint's Hermitian half planes from the row spectra; planar (per-ray kernels
+// only): as planar images [zb m][P][planar_pitch] for cuFFT
 void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
-                        const UsGeo &g, cudaStream_t s);
+                        const UsGeo &g, bool planar, cudaStream_t s);
 // cropped, deapodised and added into u, from cuFFT's C2R output (rows of 2 planar_pitch floats)
 void launch_crop_accum_real(const float *out, float *u, int zb, float tau, const float *deapod, const UsGeo &g,
                             cudaStream_t s);
@@ -234,7 +236,7 @@ void gather_tc_prepare();
 // tensor-core scatter (scatter_tc.cu): all adjoint items, time samples [16 jgrp, 16 jgrp + 16),
 // added into the zeroed Hermitian half planes of the C2R inverse
 void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jgrp,
-                       cudaStream_t s);
+                       bool planar, cudaStream_t s);
 void scatter_tc_prepare();
 void launch_adj_records(AdjRec *recs, const GeoDev &gd, const UsGeo &g, cudaStream_t s);
 // entries per scatter table, and the 32-bit words of a table's segmentation

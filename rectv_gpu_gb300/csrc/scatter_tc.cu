@@ -260,6 +260,7 @@ void launch_adj_tabinfo(const GeoDev &gd, cudaStream_t s) {
     LAUNCH_CHECK("k_adj_tabinfo");
 }
 
+template <bool PLANAR>
 __global__ void __launch_bounds__(kThr, 1)
     k_scatter_tc(const float2 *__restrict__ rowsc, float2 *__restrict__ spec, const AdjRec *__restrict__ recs,
                  const int4 *__restrict__ items, const int4 *__restrict__ tabs, const int *__restrict__ tab_base,
@@ -556,14 +557,15 @@ __global__ void __launch_bounds__(kThr, 1)
         // (8 slices, 1440 angles, width 480, 16 samples: 1.99 and 1.72 ms, this form
         // 1.55, all with units in fixed order) ----
         if (zok) {
-            float2 *base = spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
+            float2 *base = adj_base<PLANAR>(spec, g, z, jgrp);
             const float sg = ((cx + cy) & 1) ? -0.5f : 0.5f;
 #pragma unroll
             for (int j = 0; j < 16; j += 2) {  // (the sample after an odd last one adds zeros)
                 if (j >= g.tg || jbase + j >= g.m) break;
-                add_hermitian<false>(base, g, txi * kT + cx, tyi * kT + cy, j,
-                                     make_float4(sg * acc[2 * j], sg * acc[2 * j + 1], sg * acc[2 * j + 2],
-                                                 sg * acc[2 * j + 3]));
+                add_hermitian<false, PLANAR>(base, g, txi * kT + cx, tyi * kT + cy, j,
+                                             make_float4(sg * acc[2 * j], sg * acc[2 * j + 1], sg * acc[2 * j + 2],
+                                                         sg * acc[2 * j + 3]),
+                                             jbase + j + 1 < g.m);
             }
         }
     }  // units
@@ -577,11 +579,12 @@ __global__ void __launch_bounds__(kThr, 1)
 constexpr size_t kScSmemBytes = sizeof(ScTcSmem);
 
 void scatter_tc_prepare() {
-    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScSmemBytes));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScSmemBytes));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScSmemBytes));
 }
 
 void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd, const UsGeo &g, int jgrp,
-                       cudaStream_t s) {
+                       bool planar, cudaStream_t s) {
     if (g.T != kT) throw Error(1, "tile size must be 16");
     if (!gd.adj_recs) throw Error(1, "adjoint geometry records missing");
     // items with samples (sorted by count, so the empty tiles, whose half
@@ -593,9 +596,9 @@ void launch_scatter_tc(const float2 *rowsc, float2 *spec, int zb, const GeoDev &
     const int grid = (int)std::min<long long>(nunits, g.sc_grid > 0 ? g.sc_grid : sm_count());
     if (!gd.adj_tabs || !gd.adj_info) throw Error(1, "adjoint table segmentation missing");
     CUDA_CHECK(cudaMemsetAsync(gd.sc_next, 0, sizeof(int), s));
-    k_scatter_tc<<<grid, kThr, kScSmemBytes, s>>>(rowsc, spec, gd.adj_recs, gd.adj_items, gd.adj_tabs,
-                                                  gd.adj_tab_base, gd.adj_info, gd.kmat, gd.shiftadj, g, zb, npairs,
-                                                  (int)nunits, jgrp, gd.sc_next, gd.err);
+    (planar ? k_scatter_tc<true> : k_scatter_tc<false>)<<<grid, kThr, kScSmemBytes, s>>>(
+        rowsc, spec, gd.adj_recs, gd.adj_items, gd.adj_tabs, gd.adj_tab_base, gd.adj_info, gd.kmat, gd.shiftadj, g, zb,
+        npairs, (int)nunits, jgrp, gd.sc_next, gd.err);
     LAUNCH_CHECK("k_scatter_tc");
 }
 

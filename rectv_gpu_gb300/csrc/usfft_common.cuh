@@ -53,18 +53,35 @@ __device__ __forceinline__ void tap_weights(int f, float p0, const UsGeo &g, flo
 // so X(k)/2 goes to H(k) and conj(X(k))/2 to H(-k) where they lie in the half
 // plane (at most two adds per value, onto zeros: the sum does not depend on
 // their order).  v is X / 2 with the pre-IFFT fftshift sign.  ONE: sample j alone.
-template <bool ONE>
+// PLANAR: the half planes are the planar images cuFFT transforms (base: the
+// first of the group's time samples; sample j + 1 is added where there is one).
+template <bool ONE, bool PLANAR>
 __device__ __forceinline__ void add_hermitian(float2 *__restrict__ base, const UsGeo &g, int KX, int KY, int j,
-                                              const float4 &v) {
+                                              const float4 &v, bool two) {
     const int P = g.P, half = P / 2;
     if (KY >= P || KX >= P) return;
     auto add = [&](int X, int Y, const float4 &a) {
+        if constexpr (PLANAR) {
+            const int pitch = planar_pitch(g.n);
+            float2 *d = base + (long long)j * P * pitch + (long long)Y * pitch + X;
+            atomicAdd(d, make_float2(a.x, a.y));
+            if (!ONE && two) atomicAdd(d + (long long)P * pitch, make_float2(a.z, a.w));
+            return;
+        }
         float2 *d = base + ((long long)(Y + kVH) * g.vp + X + kVH) * 16 + j;
         if constexpr (ONE) atomicAdd(d, make_float2(a.x, a.y));
         else atomicAdd(reinterpret_cast<float4 *>(d), a);
     };
     if (KX <= half) add(KX, KY, v);
     if (KX >= half || KX == 0) add(KX ? P - KX : 0, KY ? P - KY : 0, make_float4(v.x, -v.y, v.z, -v.w));
+}
+
+// where the samples of slice z, group jgrp are added: its entries of its plane, or
+// its first planar image
+template <bool PLANAR>
+__device__ __forceinline__ float2 *adj_base(float2 *spec, const UsGeo &g, int z, int jgrp) {
+    if constexpr (PLANAR) return spec + ((long long)z * g.m + 16 * jgrp) * g.P * planar_pitch(g.n);
+    else return spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
 }
 
 }  // namespace rectv

@@ -420,7 +420,7 @@ void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaS
 //     complex time-sample accumulators, held in registers.
 // The tile is added once at the end into the zeroed Hermitian half planes.
 // ---------------------------------------------------------------------------
-template <int MP, int T>
+template <int MP, int T, bool PLANAR>
 __global__ void __launch_bounds__(T * T, 3)
     k_scatter_adj(const float2 *__restrict__ rowsc, float2 *__restrict__ spec,
                   const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
@@ -564,23 +564,24 @@ __global__ void __launch_bounds__(T * T, 3)
     }
     // ---- the cell's sums into the half planes ----
     const int ly = tid / T, lx = tid - (tid / T) * T;
-    float2 *base = spec + vec_plane_of(g, z, jgrp) * g.vplane + vec_entry(g, z);
+    float2 *base = adj_base<PLANAR>(spec, g, z, jgrp);
     const float sg = ((lx + ly) & 1) ? -0.5f : 0.5f;
 #pragma unroll
     for (int j = 0; j < MP; j += 2) {  // (the sample after an odd last one adds zeros)
         if (jbase + j >= g.m) break;
         const int i = MP > 1 ? j + 1 : 0;
-        add_hermitian<MP == 1>(base, g, txi * T + lx, tyi * T + ly, j, make_float4(sg * ar[j], sg * ai[j], sg * ar[i], sg * ai[i]));
+        add_hermitian<MP == 1, PLANAR>(base, g, txi * T + lx, tyi * T + ly, j,
+                                       make_float4(sg * ar[j], sg * ai[j], sg * ar[i], sg * ai[i]), jbase + j + 1 < g.m);
     }
 }
 
 template <int MP, int T>
 static void scatter_adj_t(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
-                          const UsGeo &g, int jgrp, cudaStream_t s) {
+                          const UsGeo &g, int jgrp, bool planar, cudaStream_t s) {
     const size_t smem = sizeof(ScatterSmem<T>);
     dim3 gs(gd.n_adj_items, zb);
-    k_scatter_adj<MP, T><<<gs, T * T, smem, s>>>(rowsc, spec, gd.adj_pts, gd.adj_items, gd.sincos, gd.kmat,
-                                               gd.shiftadj, g, jgrp);
+    (planar ? k_scatter_adj<MP, T, true> : k_scatter_adj<MP, T, false>)<<<gs, T * T, smem, s>>>(
+        rowsc, spec, gd.adj_pts, gd.adj_items, gd.sincos, gd.kmat, gd.shiftadj, g, jgrp);
     LAUNCH_CHECK("k_scatter_adj");
 }
 
@@ -594,7 +595,11 @@ __global__ void __launch_bounds__(256) k_vec_zero(float4 *__restrict__ spec, UsG
 }
 
 // the half planes of zb slices to zero
-static void zero_planes(float2 *spec, int zb, const UsGeo &g, cudaStream_t s) {
+static void zero_planes(float2 *spec, int zb, bool planar, const UsGeo &g, cudaStream_t s) {
+    if (planar) {
+        CUDA_CHECK(cudaMemsetAsync(spec, 0, sizeof(float2) * (size_t)zb * g.m * g.P * planar_pitch(g.n), s));
+        return;
+    }
     const int npl = vec_planes(g, zb), q = 2 * vec_groups(g, zb, 4);  // whole 32-byte sectors
     const dim3 gr(g.P, npl);
     float4 *p = reinterpret_cast<float4 *>(spec);
@@ -609,26 +614,26 @@ static void zero_planes(float2 *spec, int zb, const UsGeo &g, cudaStream_t s) {
 }
 
 void launch_scatter_adj(const float2 *rowsc, float2 *spec, int zb, const GeoDev &gd,
-                        const UsGeo &g, cudaStream_t s) {
+                        const UsGeo &g, bool planar, cudaStream_t s) {
     if (g.T != 16) throw Error(1, "tile size must be 16");
     if (gd.dirs) {  // rays grouped by direction, into the vector layout's half planes (scatter_dir.cu)
         launch_scatter_dir(rowsc, spec, zb, gd, g, s);
         return;
     }
     // the per-ray kernels add into zeroed half planes
-    zero_planes(spec, zb, g, s);
+    zero_planes(spec, zb, planar, g, s);
     const int mp = mp_for(g.m);
     for (int jg = 0; jg < g.jg; ++jg) {
         if (gd.tc_scatter) {  // from 8 time samples up
-            launch_scatter_tc(rowsc, spec, zb, gd, g, jg, s);
+            launch_scatter_tc(rowsc, spec, zb, gd, g, jg, planar, s);
             continue;
         }
         switch (mp) {
-            case 1: scatter_adj_t<1, 16>(rowsc, spec, zb, gd, g, jg, s); break;
-            case 2: scatter_adj_t<2, 16>(rowsc, spec, zb, gd, g, jg, s); break;
-            case 4: scatter_adj_t<4, 16>(rowsc, spec, zb, gd, g, jg, s); break;
-            case 8: scatter_adj_t<8, 16>(rowsc, spec, zb, gd, g, jg, s); break;
-            default: scatter_adj_t<16, 16>(rowsc, spec, zb, gd, g, jg, s); break;
+            case 1: scatter_adj_t<1, 16>(rowsc, spec, zb, gd, g, jg, planar, s); break;
+            case 2: scatter_adj_t<2, 16>(rowsc, spec, zb, gd, g, jg, planar, s); break;
+            case 4: scatter_adj_t<4, 16>(rowsc, spec, zb, gd, g, jg, planar, s); break;
+            case 8: scatter_adj_t<8, 16>(rowsc, spec, zb, gd, g, jg, planar, s); break;
+            default: scatter_adj_t<16, 16>(rowsc, spec, zb, gd, g, jg, planar, s); break;
         }
     }
 }
@@ -665,7 +670,8 @@ static void set_attrs() {
     const int fs = (int)((T + 2 * kR) * (T + 2 * kR) * MP * sizeof(float2) + sizeof(EntryTab));
     const int as = (int)sizeof(ScatterSmem<T>);
     CUDA_CHECK(cudaFuncSetAttribute(k_gather_fwd<MP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, fs));
-    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
 }
 
 void usfft_prepare() {

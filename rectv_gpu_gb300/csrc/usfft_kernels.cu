@@ -169,6 +169,8 @@ __global__ void __launch_bounds__(kThreads)
             int KX = txi * T - kR + col;
             KX += (KX < 0) ? P : 0;
             KX -= (KX >= P) ? P : 0;
+            KY = min(KY, P - 1);  // (a grid smaller than the footprint: cells past its second copy, never used)
+            KX = min(KX, P - 1);
             const int sy = KX <= half ? KY : (KY ? P - KY : 0), sx = KX <= half ? KX : P - KX;
             const float2 *src = img0 + ((long long)(sy + kVH) * g.vp + sx + kVH) * 16 + j;
             float2 *dst = tile + cell * MP + j;

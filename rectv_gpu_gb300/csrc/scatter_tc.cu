@@ -124,7 +124,8 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d, uint32_t a, uint64_t b, 
 // ---------------------------------------------------------------------------
 // Geometry records of the adjoint plan: one block per work item, one thread
 // per entry.  The stencil origin is taken modulo the periodic grid nearest to
-// the tile (wrap TOMO_ADJ, kernels_radonusfft.cuh:40-64).
+// the tile (wrap TOMO_ADJ, kernels_radonusfft.cuh:40-64); on a grid below two
+// tiles a cell takes every tap that wraps onto it.
 // ---------------------------------------------------------------------------
 __global__ void k_adj_records(AdjRec *__restrict__ recs, const uint32_t *__restrict__ pts,
                               const int4 *__restrict__ items, const float2 *__restrict__ sincos,
@@ -149,11 +150,17 @@ __global__ void k_adj_records(AdjRec *__restrict__ recs, const uint32_t *__restr
         int mask = 0;
 #pragma unroll
         for (int c = 0; c < kT; ++c) {
-            const int bx = c - dx, by = c - dy;
+            int bx = c - dx, by = c - dy;
+            if (P < 2 * kT) {
+                bx = (bx + P) % P;
+                by = (by + P) % P;
+            }
             r.wx[c] = ((unsigned)bx < (unsigned)kTaps) ? tap_weight(fx, bx, x0, g) : 0.f;
             const bool iny = (unsigned)by < (unsigned)kTaps;
             r.wy[c] = iny ? tap_weight(fy, by, y0, g) : 0.f;
             mask |= iny ? (1 << c) : 0;
+            for (int b = bx + P; P < kTaps && b < kTaps; b += P) r.wx[c] += tap_weight(fx, b, x0, g);
+            for (int b = by + P; P < kTaps && b < kTaps; b += P) r.wy[c] += tap_weight(fy, b, y0, g);
         }
         r.thm = (th << 16) | mask;
         r.k = k;

@@ -420,9 +420,11 @@ void launch_adj_prep(const float *h, float *rowsr, int zb, const UsGeo &g, cudaS
 //     ray's single-complex grid V_ray (shared memory);
 //  2. thread = cell adds conj(K'(theta, j)) V_ray(cell) to the cell's MP
 //     complex time-sample accumulators, held in registers.
-// The tile is added once at the end into the zeroed Hermitian half planes.
+// The tile is added once at the end into the zeroed Hermitian half planes
+// (add_hermitian).  WRAP: the grid is below two tiles (always one of cuFFT's), a
+// stencil may wrap into the tile it starts in (tested per tap: 4 % of the time).
 // ---------------------------------------------------------------------------
-template <int MP, int T, bool PLANAR>
+template <int MP, int T, bool PLANAR, bool WRAP>
 __global__ void __launch_bounds__(T * T, 3)
     k_scatter_adj(const float2 *__restrict__ rowsc, float2 *__restrict__ spec,
                   const uint32_t *__restrict__ pts, const int4 *__restrict__ items,
@@ -536,7 +538,11 @@ __global__ void __launch_bounds__(T * T, 3)
                 float *vs = sm.v[s][0];
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
-                    const int cy = dy + ta[i], cx = dx + tb[i];
+                    int cy = dy + ta[i], cx = dx + tb[i];
+                    if constexpr (WRAP) {
+                        cy = ta[i] < kTaps ? (cy + 2 * P) % P : T;
+                        cx = (cx + 2 * P) % P;
+                    }
                     if ((unsigned)cy < (unsigned)T && (unsigned)cx < (unsigned)T) {
                         const float w = tab.w[e][tb[i]] * tab.w[e][kTaps + ta[i]];
                         const unsigned sa = (unsigned)__cvta_generic_to_shared(vs + cy * T + cx);
@@ -582,7 +588,10 @@ static void scatter_adj_t(const float2 *rowsc, float2 *spec, int zb, const GeoDe
                           const UsGeo &g, int jgrp, bool planar, cudaStream_t s) {
     const size_t smem = sizeof(ScatterSmem<T>);
     dim3 gs(gd.n_adj_items, zb);
-    (planar ? k_scatter_adj<MP, T, true> : k_scatter_adj<MP, T, false>)<<<gs, T * T, smem, s>>>(
+    if (!planar && g.P < 2 * T) throw Error(1, "grid below two tiles: planar images only");
+    (!planar         ? k_scatter_adj<MP, T, false, false>
+     : g.P >= 2 * T ? k_scatter_adj<MP, T, true, false>
+                    : k_scatter_adj<MP, T, true, true>)<<<gs, T * T, smem, s>>>(
         rowsc, spec, gd.adj_pts, gd.adj_items, gd.sincos, gd.kmat, gd.shiftadj, g, jgrp);
     LAUNCH_CHECK("k_scatter_adj");
 }
@@ -672,8 +681,9 @@ static void set_attrs() {
     const int fs = (int)((T + 2 * kR) * (T + 2 * kR) * MP * sizeof(float2) + sizeof(EntryTab));
     const int as = (int)sizeof(ScatterSmem<T>);
     CUDA_CHECK(cudaFuncSetAttribute(k_gather_fwd<MP, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, fs));
-    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
-    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
+    CUDA_CHECK(cudaFuncSetAttribute(k_scatter_adj<MP, T, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, as));
 }
 
 void usfft_prepare() {

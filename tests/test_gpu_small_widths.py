@@ -43,3 +43,10 @@ def _case(torch, n, m):
 def test_forward(lib_built, torch_cuda, n, m):
     e = _case(torch_cuda, n, m)
     assert e[0] < OP_TOL, e
+
+
+@pytest.mark.parametrize("m", [1, 3, 8, 16])
+@pytest.mark.parametrize("n", list(range(2, 17)) + [24])
+def test_adjoint(lib_built, torch_cuda, n, m):
+    e = _case(torch_cuda, n, m)
+    assert e[1] < OP_TOL, e

@@ -17,8 +17,10 @@
 // the spectrum is read, and each ray stores n/2 + 1 values instead of n:
 //     H(k) = f(k)/2 sum_j [ 2 Re K' (S1_j + delta S1perp_j) + conj K' C_j ]
 // (an opposite ray takes the conjugate sum).  The offset correction of C is
-// left out: its weights are below 1.1e-5 of the stencil's peak and delta is
-// below 2e-3 cells, so the term is below 1e-8 of S1 (FP32 rounding: 6e-8).
+// left out: its weights are 1.1e-5 of the stencil's peak, they change by 5.7 of
+// themselves per cell, and delta is below 2e-3 cells, so the term is below 1.2e-7 of
+// the peak, at the outermost samples (carried along, it left the operator's
+// error at width 1024 at 2.73e-7, where the other roundings stood then).
 //
 // The spectra come in the vector layout (UsGeo): 16 (slice, time sample)
 // values of a cell are 128 contiguous bytes, so the 25x25-cell footprint of a

@@ -50,7 +50,8 @@
 //     H(c) += wx1 (wy1 M0 + (wy2 - wy1) M2) + (wx2 - wx1) wy2 M2
 // with the axis weights w1 on the stencil of p and w2 on the mirrored one, and
 // to first order in the rays' offsets wx1 wy1' + wx1' wy1 times M0perp =
-// sum_theta delta Re K' v (left out on the edges' M2 terms: below 1e-8 of M0).
+// sum_theta delta Re K' v (left out on the edges' M2 terms: below 1.2e-7 of the
+// stencil's peak at the outermost samples, as in gather_dir.cu).
 // Against a scatter of every position this halves the entries, and every cell
 // of the half plane belongs to one block, which stores it once: no atomics
 // and no clearing.
